@@ -6,9 +6,8 @@ all-to-all), the experts' SwiGLU FFN as two grouped tcgen05 GEMMs over all local
 Without gradients nothing of a layer's forward returns to the host: dispatch -> grouped GEMM with
 the SwiGLU epilogue -> grouped GEMM straight into the combine buffer -> combine.  With gradients
 the two communication steps run as autograd functions whose backward passes reuse the same kernels
-(parallel/ep.py) and the expert GEMMs are :class:`GroupedLinear` (forward and input gradient on the
-grouped kernel; the weight gradient, a GEMM with a ragged inner dimension, is a per-expert matmul
-and reads the group boundaries on the host).
+(parallel/ep.py) and the expert GEMMs are :class:`GroupedLinear` (output, input gradient and weight
+gradient each one grouped launch that reads the group boundaries on the device).
 
 Reference parity: none -- the reference keeps NCCL's all-to-all buffers alive across
 ncclPause / ncclResume (README.md:132) and leaves the layer to the framework above it."""
@@ -18,7 +17,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..ops.gemm import grouped_gemm_bf16, interleave_gate_up
+from ..ops.gemm import grouped_gemm_bf16, grouped_gemm_input_grad, grouped_gemm_weight_grad, interleave_gate_up
 from ..ops.moe import MoeDispatcher
 from ..parallel.ep import ep_combine, ep_dispatch
 
@@ -37,16 +36,10 @@ class GroupedLinear(torch.autograd.Function):
         g_out = g_out.contiguous()
         g_rows = g_w = None
         if ctx.needs_input_grad[0]:
-            # d rows = g_out @ w: the same grouped kernel on the transposed matrices
             g_rows = torch.zeros_like(rows)
-            grouped_gemm_bf16(g_out, w.transpose(1, 2).contiguous(), offsets, out=g_rows, rows_hint=rows.shape[0])
+            grouped_gemm_input_grad(g_out, w.contiguous(), offsets, out=g_rows, rows_hint=rows.shape[0])
         if ctx.needs_input_grad[1]:
-            offs = offsets.tolist()
-            g_w = torch.zeros_like(w)
-            for e in range(w.shape[0]):
-                lo, hi = offs[e], offs[e + 1]
-                if hi > lo:
-                    g_w[e] = g_out[lo:hi].t() @ rows[lo:hi]
+            g_w = grouped_gemm_weight_grad(g_out, rows.contiguous(), offsets)
         return g_rows, g_w, None
 
 

@@ -1,7 +1,8 @@
 """Tensor-core GEMMs of the library (hand-written tcgen05 / TMEM / TMA kernels).
 
-All take bf16 CUDA tensors with K contiguous: ``a`` is [M, K] (activations), ``b`` is [N, K]
-(a ``torch.nn.Linear`` weight), the result is [M, N] = a @ b.T in bf16 with fp32 accumulation.
+All take bf16 CUDA tensors, accumulate in fp32 and give bf16.  The forward products take ``a`` as
+[M, K] (activations) and ``b`` as [N, K] (a ``torch.nn.Linear`` weight): a @ b.T.  The gradients'
+products read the same tensors as they lie, with no transposed copies.
 
 Reference parity: none -- the reference contains no GEMM and no fused operator (its plugin is
 host code only, amem_nccl_plugin/Makefile:36).
@@ -52,6 +53,31 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
     return out
 
 
+def _by_k(a: torch.Tensor, b: torch.Tensor, m: int, n: int, k: int, a_by_k: bool, stream) -> torch.Tensor:
+    if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
+        raise TypeError("bf16 tensors expected")
+    if not (a.is_cuda and b.is_cuda and a.is_contiguous() and b.is_contiguous()):
+        raise ValueError("contiguous CUDA tensors expected")
+    out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
+    lib = B.load_library()
+    B.check(lib.amemGemmBf16Strided(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, int(a_by_k), 1, _stream(stream)), "amemGemmBf16Strided")
+    return out
+
+
+def gemm_input_grad(gy: torch.Tensor, w: torch.Tensor, stream=None) -> torch.Tensor:
+    """gy[M, N] @ w[N, K] on one GPU: the input gradient of :func:`gemm_bf16`, from the weight as it lies."""
+    if _on_host(gy, w):
+        return (gy.float() @ w.float()).to(gy.dtype)
+    return _by_k(gy, w, gy.shape[0], w.shape[1], w.shape[0], False, stream)
+
+
+def gemm_weight_grad(gy: torch.Tensor, x: torch.Tensor, stream=None) -> torch.Tensor:
+    """gy[T, N].T @ x[T, K] on one GPU: the weight gradient of :func:`gemm_bf16`, any number of rows T."""
+    if _on_host(gy, x):
+        return gy.t() @ x
+    return _by_k(gy, x, gy.shape[1], x.shape[1], gy.shape[0], True, stream)
+
+
 def interleave_gate_up(w13: torch.Tensor, ffn: int) -> torch.Tensor:
     """[..., 2 * ffn, K] with the gate rows first and the up rows second  ->  the same rows in
     alternating blocks of 32 gate rows and 32 up rows, the layout the SwiGLU epilogue of
@@ -63,6 +89,15 @@ def interleave_gate_up(w13: torch.Tensor, ffn: int) -> torch.Tensor:
     gate = w13[..., :ffn, :].reshape(*lead, ffn // 32, 1, 32, K)
     up = w13[..., ffn:, :].reshape(*lead, ffn // 32, 1, 32, K)
     return torch.cat([gate, up], dim=-3).reshape(*lead, 2 * ffn, K).contiguous()
+
+
+def _check_grouped(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, groups: int) -> None:
+    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or offsets.dtype != torch.int32:
+        raise TypeError("bf16 operands and int32 offsets expected")
+    if not (w.is_cuda and offsets.is_cuda and a.is_contiguous() and w.is_contiguous() and offsets.is_contiguous()):
+        raise ValueError("contiguous CUDA tensors expected")
+    if offsets.numel() != groups + 1:
+        raise ValueError(f"{groups} groups need {groups + 1} offsets, got {offsets.numel()}")
 
 
 def grouped_gemm_bf16(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor | None = None,
@@ -85,18 +120,51 @@ def grouped_gemm_bf16(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, o
                 h = (torch.nn.functional.silu(h[:, :, 0]) * h[:, :, 1]).reshape(h.shape[0], N // 2)
             res[offs[e]:offs[e + 1]] = h.to(a.dtype)
         return res
-    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or offsets.dtype != torch.int32:
-        raise TypeError("bf16 operands and int32 offsets expected")
-    if not (w.is_cuda and offsets.is_cuda and a.is_contiguous() and w.is_contiguous() and offsets.is_contiguous()):
-        raise ValueError("contiguous CUDA tensors expected")
     groups, N, K = w.shape
-    if a.shape[1] != K or offsets.numel() != groups + 1:
-        raise ValueError(f"shapes do not fit: a {tuple(a.shape)}, w {tuple(w.shape)}, {offsets.numel()} offsets")
+    _check_grouped(a, w, offsets, groups)
+    if a.shape[1] != K:
+        raise ValueError(f"shapes do not fit: a {tuple(a.shape)}, w {tuple(w.shape)}")
     rows_cap = a.shape[0]
     out = torch.empty(rows_cap, N // 2 if swiglu else N, dtype=torch.bfloat16, device=a.device) if out is None else out
     lib = B.load_library()
     B.check(lib.amemGroupedGemmBf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, rows_cap,
                                     int(rows_hint or 0), N, K, 1 if swiglu else 0, _stream(stream)), "amemGroupedGemmBf16")
+    return out
+
+
+def grouped_gemm_input_grad(g: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor | None = None,
+                            rows_hint: int | None = None, stream=None) -> torch.Tensor:
+    """For every group e: out[rows of e] = g[rows of e] @ w[e] with ``w`` bf16 [groups, N, K] as it is
+    stored for :func:`grouped_gemm_bf16`.  Rows outside every group are left untouched."""
+    groups, N, K = w.shape
+    if not g.is_cuda:
+        offs = offsets.tolist()
+        res = torch.zeros(g.shape[0], K, dtype=g.dtype) if out is None else out
+        for e in range(groups):
+            res[offs[e]:offs[e + 1]] = (g[offs[e]:offs[e + 1]].float() @ w[e].float()).to(g.dtype)
+        return res
+    out = torch.empty(g.shape[0], K, dtype=torch.bfloat16, device=g.device) if out is None else out
+    _check_grouped(g, w, offsets, groups)
+    if g.shape[1] != N:
+        raise ValueError(f"shapes do not fit: g {tuple(g.shape)}, w {tuple(w.shape)}")
+    B.check(B.load_library().amemGroupedGemmBf16Input(g.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
+                                                      int(rows_hint or 0), N, K, _stream(stream)), "amemGroupedGemmBf16Input")
+    return out
+
+
+def grouped_gemm_weight_grad(g: torch.Tensor, a: torch.Tensor, offsets: torch.Tensor, stream=None) -> torch.Tensor:
+    """bf16 [groups, N, K]: for every group e, g[rows of e].T @ a[rows of e] (zeros without rows).  The
+    group boundaries are read on the device."""
+    groups, N, K = offsets.numel() - 1, g.shape[1], a.shape[1]
+    if not g.is_cuda:
+        offs = offsets.tolist()
+        return torch.stack([g[offs[e]:offs[e + 1]].t() @ a[offs[e]:offs[e + 1]] for e in range(groups)])
+    _check_grouped(g, a, offsets, groups)
+    if g.shape[0] != a.shape[0]:
+        raise ValueError(f"shapes do not fit: g {tuple(g.shape)}, a {tuple(a.shape)}")
+    out = torch.empty(groups, N, K, dtype=torch.bfloat16, device=g.device)
+    B.check(B.load_library().amemGroupedGemmBf16Weight(g.data_ptr(), a.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
+                                                       N, K, _stream(stream)), "amemGroupedGemmBf16Weight")
     return out
 
 

@@ -14,17 +14,24 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from ..ops.gemm import all_gather_gemm, gemm_bf16, gemm_reduce_scatter
+from ..ops.gemm import all_gather_gemm, gemm_input_grad, gemm_reduce_scatter, gemm_weight_grad
 
 
 def _wgrad(gy: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
-    """gw[N, K] = gy[M, N].T @ x[M, K] on the library's tcgen05 GEMM, whose operands are both
-    K-major: A = gy.T [N, M], B = x.T [K, M] (two transposing copies, then one tensor-core pass
-    with fp32 accumulation over the M tokens).  Token counts that are not a multiple of 8 (the
-    16-byte row rule of the TMA loads) fall back to a PyTorch matmul."""
-    if gy.is_cuda and gy.shape[0] % 8 == 0 and gy.dtype == torch.bfloat16 and x.dtype == torch.bfloat16:
-        return gemm_bf16(gy.t().contiguous(), x.t().contiguous())
+    """gw[N, K] = gy[M, N].T @ x[M, K] on the library's tcgen05 GEMM, which reads both operands as they lie."""
+    if gy.is_cuda and gy.dtype == torch.bfloat16 and x.dtype == torch.bfloat16:
+        return gemm_weight_grad(gy.contiguous(), x.contiguous())
     return gy.t() @ x
+
+
+def _gathered(comm, shard: torch.Tensor) -> torch.Tensor:
+    """The rows of every rank (the shard itself on one rank)."""
+    shard = shard.contiguous()
+    if comm.nranks == 1:
+        return shard
+    full = torch.empty(shard.shape[0] * comm.nranks, shard.shape[1], dtype=shard.dtype, device=shard.device)
+    comm.all_gather(shard, full)
+    return full
 
 
 class _ColumnFn(torch.autograd.Function):
@@ -41,11 +48,10 @@ class _ColumnFn(torch.autograd.Function):
         comm = ctx.comm
         x_shard, w = ctx.saved_tensors
         gy = gy.contiguous()
-        # dx_shard = reduce_scatter_rows(gy @ w): the mirrored fused kernel, B = w.T [K, N_local]
-        gx = gemm_reduce_scatter(comm, gy, w.t().contiguous())
-        x_full = torch.empty(x_shard.shape[0] * comm.nranks, x_shard.shape[1], dtype=x_shard.dtype, device=x_shard.device)
-        comm.all_gather(x_shard.contiguous(), x_full)
-        gw = _wgrad(gy, x_full)
+        # dx_shard = reduce_scatter_rows(gy @ w): the mirrored fused kernel, B = w.T [K, N_local]; one
+        # rank has nothing to scatter and its GEMM reads w as it lies
+        gx = gemm_input_grad(gy, w.contiguous()) if comm.nranks == 1 else gemm_reduce_scatter(comm, gy, w.t().contiguous())
+        gw = _wgrad(gy, _gathered(comm, x_shard))
         return gx, gw, None
 
 
@@ -64,10 +70,8 @@ class _RowFn(torch.autograd.Function):
         x, w = ctx.saved_tensors
         gy_shard = gy_shard.contiguous()
         # dx = all_gather_rows(gy_shard) @ w  -> fused all-gather GEMM with B = w.T [K_local, N]
-        gx = all_gather_gemm(comm, gy_shard, w.t().contiguous())
-        gy_full = torch.empty(gy_shard.shape[0] * comm.nranks, gy_shard.shape[1], dtype=gy_shard.dtype, device=gy_shard.device)
-        comm.all_gather(gy_shard, gy_full)
-        gw = _wgrad(gy_full, x)
+        gx = gemm_input_grad(gy_shard, w.contiguous()) if comm.nranks == 1 else all_gather_gemm(comm, gy_shard, w.t().contiguous())
+        gw = _wgrad(_gathered(comm, gy_shard), x)
         return gx, gw, None
 
 

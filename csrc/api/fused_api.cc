@@ -13,6 +13,7 @@
 #include "../core/log.h"
 #include "../include/nccl.h"
 #include "../kernels/gemm_ag_cta_movers.h"
+#include "../kernels/gemm_pair.h"
 #include "../kernels/gemm_sm100.h"
 #include "../kernels/moe.h"
 #include "../vmm/tracked.h"
@@ -147,9 +148,87 @@ Status gemm_process_words(int dev, CtrlBlock** ctrl_out, uint32_t** status_out) 
 }
 }  // namespace
 
+namespace {
+const unsigned long long kGemmTimeoutNs = 5ull * 1000000000ull;
+
+// One launch of the SM-pair kernel, with the process's status words.
+Status run_pair(PairProblem& p, cudaStream_t stream) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  CtrlBlock* ctrl = nullptr;
+  uint32_t* status = nullptr;
+  AMEM_TRY(gemm_process_words(dev, &ctrl, &status));
+  p.status = status;
+  p.timeout_ns = kGemmTimeoutNs;
+  const int sms = gemm_default_grid(dev);
+  // the stream's workspace for cut tiles (shared with the one-SM kernel: launches of one stream take turns)
+  SplitKWs* ws = nullptr;
+  if (p.mode == kPairPlain && env_long("AMEM_GEMM_SPLITK", 1) && !Registry::instance().is_paused(0)) ws = splitk_workspace(dev, stream, sms);
+  if (ws && gemm_splitk_ws_bytes(sms) >= pair_gemm_ws_bytes(sms) && gemm_splitk_ctr_words(sms) >= pair_gemm_ctr_words(sms)) {
+    p.sk_ws = ws->partials;
+    p.sk_ctr = ws->counters;
+  }
+  AMEM_TRY(launch_pair_gemm(p, sms, stream));
+  if (status[0] && ws) cudaMemsetAsync(ws->counters, 0, gemm_splitk_ctr_words(sms) * sizeof(uint32_t), stream);   // an earlier launch gave up: perhaps mid-count
+  if (status[0]) return fail(kInternalError, "tcgen05 GEMM reported a device-side wait timeout (code %u)", status[0]);
+  return kSuccess;
+}
+
+PairProblem pair_plain(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn) {
+  PairProblem p;
+  memset(&p, 0, sizeof(p));
+  p.A = A;
+  p.B = B;
+  p.C = C;
+  p.M = M;
+  p.N = N;
+  p.K = K;
+  p.a_mn = a_mn;
+  p.b_mn = b_mn;
+  p.mode = kPairPlain;
+  p.groups = 1;
+  return p;
+}
+
+// A [rows_cap, K] times the matrices of its rows' groups, stored [groups, N, K] or (b_by_k) [groups, K, N].
+PairProblem pair_grouped(const void* A, const void* B, void* C, const int* group_off, int groups, int rows_cap, int rows_hint, int N, int K,
+                         int b_by_k, int epilogue) {
+  PairProblem p = pair_plain(A, B, C, rows_cap, N, K, 0, b_by_k);
+  p.mode = kPairGroupedRows;
+  p.epilogue = epilogue;
+  p.group_off = group_off;
+  p.groups = groups;
+  // every group ends in a partly filled row tile: count about half a tile of waste per group
+  const int hint = rows_hint > 0 ? rows_hint : rows_cap;
+  p.row_tiles_hint = (hint + 255) / 256 + groups / 2;
+  return p;
+}
+
+// Whether the plain product runs on SM pairs.  AMEM_GEMM_PAIR = 0 / 1 forces; a forced tile height
+// of the one-SM kernel (AMEM_GEMM_TALL) means that kernel.
+bool pair_pays(const PairProblem& p) {
+  if (!pair_gemm_takes(p)) return false;
+  const long f = env_long("AMEM_GEMM_PAIR", -1);
+  if (f >= 0) return f != 0;
+  if (env_long("AMEM_GEMM_TALL", -1) >= 0) return false;
+  return p.M > kGemmBM;
+}
+}  // namespace
+
 extern "C" {
 
-// The tiling amemGemmBf16 would use on a GPU with `sms` SMs (no GPU needed: planning is host
+// C[M, N] = A * B with either operand stored by its contraction index: a_by_k = 0: A [M, K], 1: A [K, M];
+// b_by_k = 0: B [N, K], 1: B [K, N].  (0, 0), (0, 1) and (1, 1) are built: a Linear's output, its input
+// gradient and its weight gradient.  K may be any number where both operands are stored by K.
+ncclResult_t amemGemmBf16Strided(const void* A, const void* B, void* C, int M, int N, int K, int a_by_k, int b_by_k, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return R(fail(kInvalidArgument, "empty GEMM %d x %d x %d", M, N, K));
+  if (!A || !B || !C) return R(fail(kInvalidArgument, "GEMM: null buffer"));
+  PairProblem p = pair_plain(A, B, C, M, N, K, a_by_k != 0, b_by_k != 0);
+  if (!pair_gemm_takes(p)) return R(fail(kInvalidArgument, "rows must be 16-byte aligned: M=%d N=%d K=%d", M, N, K));
+  return R(run_pair(p, stream));
+}
+
+// The tiling of the one-SM form on a GPU with `sms` SMs (no GPU needed: planning is host
 // arithmetic).  Outputs may be null.
 ncclResult_t amemGemmPlan(int M, int N, int K, int sms, int* tile_rows, int* tile_cols, int* tail_slices) {
   Status s = check_shape(M, N, K);
@@ -183,6 +262,8 @@ ncclResult_t amemAllGatherGemmPlan(int nranks, int rows_per_rank, int K, int* mo
 ncclResult_t amemGemmBf16(const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream) {
   Status s = check_shape(M, N, K);
   if (s != kSuccess) return R(s);
+  PairProblem pair = pair_plain(A, B, C, M, N, K, 0, 0);
+  if (pair_pays(pair)) return R(run_pair(pair, stream));
   int dev = 0;
   cudaGetDevice(&dev);
   CtrlBlock* ctrl_dev = nullptr;
@@ -239,7 +320,7 @@ ncclResult_t amemGemmBf16(const void* A, const void* B, void* C, int M, int N, i
 // Grouped GEMM: C[rows of group e, :] = A[rows of group e, :] * B[e]^T for every group, one launch.
 // A: bf16 [rows_cap, K]; group_off: DEVICE int32 [groups + 1] (row offsets, e.g. expert_offsets of
 // amemMoeDispatch — the host never reads them); B: bf16 [groups, N, K]; C: bf16 [rows_cap, N], or
-// [rows_cap, N / 2] with epilogue = 1 (SwiGLU of 32-column gate / up blocks, see GemmEpilogue).
+// [rows_cap, N / 2] with epilogue = 1 (SwiGLU of 32-column gate / up blocks, see kPairSwiGLU32).
 // rows_hint: the number of rows the caller expects (sizes the tile width; any value is correct).
 ncclResult_t amemGroupedGemmBf16(const void* A, const void* B, void* C, const int* group_off, int groups, int rows_cap, int rows_hint,
                                  int N, int K, int epilogue, cudaStream_t stream) {
@@ -247,9 +328,16 @@ ncclResult_t amemGroupedGemmBf16(const void* A, const void* B, void* C, const in
   if (s != kSuccess) return R(s);
   if (!A || !B || !C || !group_off) return R(fail(kInvalidArgument, "grouped GEMM: null buffer"));
   if (groups <= 0 || groups > 256) return R(fail(kInvalidArgument, "grouped GEMM: %d groups (1..256)", groups));
-  if (epilogue != kEpiStore && epilogue != kEpiSwiGLU) return R(fail(kInvalidArgument, "grouped GEMM: unknown epilogue %d", epilogue));
-  if (epilogue == kEpiSwiGLU && N % 64) return R(fail(kInvalidArgument, "grouped GEMM: the SwiGLU epilogue needs N to be a multiple of 64, got %d", N));
+  if (epilogue != kPairStore && epilogue != kPairSwiGLU32) return R(fail(kInvalidArgument, "grouped GEMM: unknown epilogue %d", epilogue));
+  if (epilogue == kPairSwiGLU32 && N % 64) return R(fail(kInvalidArgument, "grouped GEMM: the SwiGLU epilogue needs N to be a multiple of 64, got %d", N));
   if ((long long)groups * N > 0x7fffffffLL) return R(fail(kInvalidArgument, "grouped GEMM: groups * N does not fit 31 bits"));
+  PairProblem p = pair_grouped(A, B, C, group_off, groups, rows_cap, rows_hint, N, K, 0, epilogue);
+  // 256-row tiles pay from about 64 rows a group up (8 groups of 4096 x 1536: 8 rows each 0.9x the 128-row
+  // tiles' time, 2048 rows each 1.2x)
+  if ((long)(rows_hint > 0 ? rows_hint : rows_cap) >= 64L * groups) {
+    if (!pair_gemm_takes(p)) return R(fail(kInvalidArgument, "grouped GEMM: buffers must be 16-byte aligned"));
+    return R(run_pair(p, stream));
+  }
   int dev = 0;
   cudaGetDevice(&dev);
   CtrlBlock* ctrl = nullptr;
@@ -287,6 +375,35 @@ ncclResult_t amemGroupedGemmBf16(const void* A, const void* B, void* C, const in
   s = launch_gemm(g, stream);
   if (s == kSuccess && status[0]) s = fail(kInternalError, "tcgen05 GEMM reported a device-side wait timeout (code %u)", status[0]);
   return R(s);
+}
+
+// The input gradient of the above: C[rows of group e, K] = A[rows of group e, N] * B[e] with the weights
+// as they are stored for the forward product, bf16 [groups, N, K].
+ncclResult_t amemGroupedGemmBf16Input(const void* A, const void* B, void* C, const int* group_off, int groups, int rows_cap, int rows_hint,
+                                      int N, int K, cudaStream_t stream) {
+  Status s = check_shape(rows_cap, N, K);
+  if (s != kSuccess) return R(s);
+  if (!A || !B || !C || !group_off) return R(fail(kInvalidArgument, "grouped GEMM: null buffer"));
+  if (groups <= 0 || groups > 256) return R(fail(kInvalidArgument, "grouped GEMM: %d groups (1..256)", groups));
+  PairProblem p = pair_grouped(A, B, C, group_off, groups, rows_cap, rows_hint, K, N, 1, kPairStore);
+  if (!pair_gemm_takes(p)) return R(fail(kInvalidArgument, "grouped GEMM: buffers must be 16-byte aligned"));
+  return R(run_pair(p, stream));
+}
+
+// The weight gradient: C[e] = A[rows of group e]^T * B[rows of group e], bf16 [groups, N, K], from
+// A: bf16 [rows_cap, N] (output gradients) and B: bf16 [rows_cap, K] (inputs).  A group without rows gets zeros.
+ncclResult_t amemGroupedGemmBf16Weight(const void* A, const void* B, void* C, const int* group_off, int groups, int rows_cap, int N, int K,
+                                       cudaStream_t stream) {
+  Status s = check_shape(rows_cap, N, K);
+  if (s != kSuccess) return R(s);
+  if (!A || !B || !C || !group_off) return R(fail(kInvalidArgument, "grouped GEMM: null buffer"));
+  if (groups <= 0 || groups > 256) return R(fail(kInvalidArgument, "grouped GEMM: %d groups (1..256)", groups));
+  PairProblem p = pair_plain(A, B, C, N, K, rows_cap, 1, 1);
+  p.mode = kPairGroupedK;
+  p.group_off = group_off;
+  p.groups = groups;
+  if (!pair_gemm_takes(p)) return R(fail(kInvalidArgument, "grouped GEMM: buffers must be 16-byte aligned"));
+  return R(run_pair(p, stream));
 }
 
 }  // extern "C"
@@ -348,6 +465,10 @@ ncclResult_t amemAllGatherGemm(const void* a_shard, const void* B, void* C, int 
   if (M % n) return R(fail(kInvalidArgument, "M=%d is not divisible by %d ranks", M, n));
   int rpr = M / n;
   if ((s = c->prepare_stream(stream)) != kSuccess) return R(s);
+  if (n == 1) {   // nothing to gather
+    PairProblem pair = pair_plain(a_shard, B, C, M, N, K, 0, 0);
+    if (pair_pays(pair)) return R(run_pair(pair, stream));
+  }
   if (n > 1 && !gemm_ag_uses_mover_warps(n)) return R(ag_gemm_cta_movers(c, a_shard, B, C, M, N, K, stream));
   GemmLaunch g;
   memset(&g, 0, sizeof(g));
@@ -416,6 +537,10 @@ ncclResult_t amemGemmReduceScatter(const void* A, const void* B, void* out, int 
   int rpr = M / n;
   if ((rpr + kGemmBM - 1) / kGemmBM > kMaxUnits) return R(fail(kInvalidArgument, "more than %d rows per rank", kGemmBM * kMaxUnits));
   if ((s = c->prepare_stream(stream)) != kSuccess) return R(s);
+  if (n == 1) {   // nothing to scatter
+    PairProblem pair = pair_plain(A, B, out, M, N, K, 0, 0);
+    if (pair_pays(pair)) return R(run_pair(pair, stream));
+  }
   GemmLaunch g;
   memset(&g, 0, sizeof(g));
   fill_fused(c, &g.p);

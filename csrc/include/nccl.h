@@ -205,8 +205,13 @@ ncclResult_t amemAllReduceAlgo(const void* sendbuff, void* recvbuff, size_t coun
  * row-major with K contiguous, the layout of activations and of Linear weights).  N and K must
  * be multiples of 8. */
 ncclResult_t amemGemmBf16(const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream);
-/* The tiling amemGemmBf16 picks for a problem on a GPU with `sms` SMs: tile rows (128 or 256), tile
- * columns, K-slices of the last wave (1 = not split).  Host arithmetic only; outputs may be NULL. */
+/* The same product with either operand stored by its contraction index: a_by_k: A is [K, M], b_by_k: B is
+ * [K, N].  Built: (0, 0), (0, 1) -- a Linear's input gradient from its weight as it lies -- and (1, 1), its
+ * weight gradient (K is then any number).  The contiguous extents must be multiples of 8. */
+ncclResult_t amemGemmBf16Strided(const void* A, const void* B, void* C, int M, int N, int K, int a_by_k, int b_by_k, cudaStream_t stream);
+/* The tiling of the one-SM form of the GEMM (the fused all-gather GEMM's) for a GPU with `sms` SMs: tile
+ * rows (128 or 256), tile columns, K-slices of the last wave (1 = not split).  Host arithmetic only;
+ * outputs may be NULL. */
 /* Variant (1 one-shot, 2 two-shot, 3 NVLS, 0 n/a), grid and chunk the library picks for a collective
  * (kind: 0 all-reduce, 1 all-gather, 2 reduce-scatter, 3 broadcast, 4 reduce, 5 all-to-all) on `nranks`
  * GPUs; stage_bytes 0 = default staging.  Host arithmetic only. */
@@ -225,6 +230,13 @@ ncclResult_t amemDebugDirtyCanary(ncclComm_t comm); /* test hook: dirties the gu
  * gate rows and 32 up rows and C is bf16 [rows_cap, N / 2] = silu(gate) * up. */
 ncclResult_t amemGroupedGemmBf16(const void* A, const void* B, void* C, const int* group_off, int groups, int rows_cap, int rows_hint,
                                  int N, int K, int epilogue, cudaStream_t stream);
+/* The gradients of the grouped product, from the operands as they lie: amemGroupedGemmBf16Input gives
+ * C[rows of e, K] = A[rows of e, N] * B[e] (B bf16 [groups, N, K]); amemGroupedGemmBf16Weight gives
+ * C[e] = A[rows of e]^T * B[rows of e], bf16 [groups, N, K], zeros for a group without rows. */
+ncclResult_t amemGroupedGemmBf16Input(const void* A, const void* B, void* C, const int* group_off, int groups, int rows_cap, int rows_hint,
+                                      int N, int K, cudaStream_t stream);
+ncclResult_t amemGroupedGemmBf16Weight(const void* A, const void* B, void* C, const int* group_off, int groups, int rows_cap, int N, int K,
+                                       cudaStream_t stream);
 ncclResult_t amemGemmPlan(int M, int N, int K, int sms, int* tile_rows, int* tile_cols, int* tail_slices);
 /* Schedule of amemAllGatherGemm for nranks ranks (1 = mover warps in every CTA, 0 = dedicated mover CTAs), rows of a
    shard per ready flag and ready flags per source rank.  Host arithmetic, no GPU needed. */
