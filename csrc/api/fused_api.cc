@@ -3,6 +3,7 @@
 // back; here the collective rides inside the GEMM kernel (kernels/gemm_sm100.cu).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -14,6 +15,7 @@
 #include "../include/nccl.h"
 #include "../kernels/gemm_ag_cta_movers.h"
 #include "../kernels/gemm_pair.h"
+#include "../kernels/gemm_skinny.h"
 #include "../kernels/gemm_sm100.h"
 #include "../kernels/moe.h"
 #include "../vmm/tracked.h"
@@ -151,6 +153,22 @@ Status gemm_process_words(int dev, CtrlBlock** ctrl_out, uint32_t** status_out) 
 namespace {
 const unsigned long long kGemmTimeoutNs = 5ull * 1000000000ull;
 
+// The stream's workspace for tiles that are cut along K (all GEMM kernels share it: launches of one stream
+// take turns and leave its counters at zero); null while the process is paused, or where none can be made.
+SplitKWs* stream_workspace(int dev, cudaStream_t stream, int sms) {
+  if (!env_long("AMEM_GEMM_SPLITK", 1) || Registry::instance().is_paused(0)) return nullptr;
+  if (gemm_splitk_ws_bytes(sms) < std::max(pair_gemm_ws_bytes(sms), skinny_gemm_ws_bytes(sms))) return nullptr;
+  if (gemm_splitk_ctr_words(sms) < std::max(pair_gemm_ctr_words(sms), skinny_gemm_ctr_words(sms))) return nullptr;
+  return splitk_workspace(dev, stream, sms);
+}
+
+// An earlier launch may have given up on a wait, perhaps in mid-count.
+Status check_waits(uint32_t* status, SplitKWs* ws, int sms, cudaStream_t stream) {
+  if (!status[0]) return kSuccess;
+  if (ws) cudaMemsetAsync(ws->counters, 0, gemm_splitk_ctr_words(sms) * sizeof(uint32_t), stream);
+  return fail(kInternalError, "tcgen05 GEMM reported a device-side wait timeout (code %u)", status[0]);
+}
+
 // One launch of the SM-pair kernel, with the process's status words.
 Status run_pair(PairProblem& p, cudaStream_t stream) {
   int dev = 0;
@@ -161,17 +179,13 @@ Status run_pair(PairProblem& p, cudaStream_t stream) {
   p.status = status;
   p.timeout_ns = kGemmTimeoutNs;
   const int sms = gemm_default_grid(dev);
-  // the stream's workspace for cut tiles (shared with the one-SM kernel: launches of one stream take turns)
-  SplitKWs* ws = nullptr;
-  if (p.mode == kPairPlain && env_long("AMEM_GEMM_SPLITK", 1) && !Registry::instance().is_paused(0)) ws = splitk_workspace(dev, stream, sms);
-  if (ws && gemm_splitk_ws_bytes(sms) >= pair_gemm_ws_bytes(sms) && gemm_splitk_ctr_words(sms) >= pair_gemm_ctr_words(sms)) {
+  SplitKWs* ws = p.mode == kPairPlain ? stream_workspace(dev, stream, sms) : nullptr;
+  if (ws) {
     p.sk_ws = ws->partials;
     p.sk_ctr = ws->counters;
   }
   AMEM_TRY(launch_pair_gemm(p, sms, stream));
-  if (status[0] && ws) cudaMemsetAsync(ws->counters, 0, gemm_splitk_ctr_words(sms) * sizeof(uint32_t), stream);   // an earlier launch gave up: perhaps mid-count
-  if (status[0]) return fail(kInternalError, "tcgen05 GEMM reported a device-side wait timeout (code %u)", status[0]);
-  return kSuccess;
+  return check_waits(status, ws, sms, stream);
 }
 
 PairProblem pair_plain(const void* A, const void* B, void* C, int M, int N, int K, int a_mn, int b_mn) {
@@ -204,6 +218,50 @@ PairProblem pair_grouped(const void* A, const void* B, void* C, const int* group
   return p;
 }
 
+SkinnyProblem skinny(const void* A, const void* W, void* C, int rows, int N, int K, const int* group_off, int groups, int rows_per_group, int epilogue) {
+  SkinnyProblem p;
+  memset(&p, 0, sizeof(p));
+  p.A = A;
+  p.W = W;
+  p.C = C;
+  p.rows = rows;
+  p.N = N;
+  p.K = K;
+  p.group_off = group_off;
+  p.groups = groups;
+  p.rows_per_group = rows_per_group;
+  p.epilogue = epilogue;
+  return p;
+}
+
+// Whether a product's time is that of reading its weights: few rows (per group, as expected).
+// AMEM_GEMM_SKINNY = 0 / 1 forces.
+bool skinny_pays(const SkinnyProblem& p) {
+  if (!skinny_gemm_takes(p)) return false;
+  const long f = env_long("AMEM_GEMM_SKINNY", -1);
+  if (f >= 0) return f != 0;
+  if (!p.group_off && (env_long("AMEM_GEMM_TALL", -1) >= 0 || env_long("AMEM_GEMM_PAIR", -1) >= 0)) return false;
+  return p.group_off ? p.rows_per_group < 96 : p.rows <= 64;
+}
+
+Status run_skinny(SkinnyProblem& p, cudaStream_t stream) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  CtrlBlock* ctrl = nullptr;
+  uint32_t* status = nullptr;
+  AMEM_TRY(gemm_process_words(dev, &ctrl, &status));
+  p.status = status;
+  p.timeout_ns = kGemmTimeoutNs;
+  const int sms = gemm_default_grid(dev);
+  SplitKWs* ws = stream_workspace(dev, stream, sms);
+  if (ws) {
+    p.ws = ws->partials;
+    p.ctr = ws->counters;
+  }
+  AMEM_TRY(launch_skinny_gemm(p, sms, stream));
+  return check_waits(status, ws, sms, stream);
+}
+
 // Whether the plain product runs on SM pairs.  AMEM_GEMM_PAIR = 0 / 1 forces; a forced tile height
 // of the one-SM kernel (AMEM_GEMM_TALL) means that kernel.
 bool pair_pays(const PairProblem& p) {
@@ -211,7 +269,19 @@ bool pair_pays(const PairProblem& p) {
   const long f = env_long("AMEM_GEMM_PAIR", -1);
   if (f >= 0) return f != 0;
   if (env_long("AMEM_GEMM_TALL", -1) >= 0) return false;
-  return p.M > kGemmBM;
+  return true;
+}
+
+// A * B^T on the kernel for few rows or on SM pairs; *done is false where the one-SM kernel is to run
+// (forced by the environment, or C is not 16-byte aligned).
+Status run_plain(const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream, bool* done) {
+  *done = true;
+  SkinnyProblem few = skinny(A, B, C, M, N, K, nullptr, 1, M, kPairStore);
+  if (skinny_pays(few)) return run_skinny(few, stream);
+  PairProblem pair = pair_plain(A, B, C, M, N, K, 0, 0);
+  if (pair_pays(pair)) return run_pair(pair, stream);
+  *done = false;
+  return kSuccess;
 }
 }  // namespace
 
@@ -262,8 +332,8 @@ ncclResult_t amemAllGatherGemmPlan(int nranks, int rows_per_rank, int K, int* mo
 ncclResult_t amemGemmBf16(const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream) {
   Status s = check_shape(M, N, K);
   if (s != kSuccess) return R(s);
-  PairProblem pair = pair_plain(A, B, C, M, N, K, 0, 0);
-  if (pair_pays(pair)) return R(run_pair(pair, stream));
+  bool done = false;
+  if ((s = run_plain(A, B, C, M, N, K, stream, &done)) != kSuccess || done) return R(s);
   int dev = 0;
   cudaGetDevice(&dev);
   CtrlBlock* ctrl_dev = nullptr;
@@ -332,49 +402,10 @@ ncclResult_t amemGroupedGemmBf16(const void* A, const void* B, void* C, const in
   if (epilogue == kPairSwiGLU32 && N % 64) return R(fail(kInvalidArgument, "grouped GEMM: the SwiGLU epilogue needs N to be a multiple of 64, got %d", N));
   if ((long long)groups * N > 0x7fffffffLL) return R(fail(kInvalidArgument, "grouped GEMM: groups * N does not fit 31 bits"));
   PairProblem p = pair_grouped(A, B, C, group_off, groups, rows_cap, rows_hint, N, K, 0, epilogue);
-  // 256-row tiles pay from about 64 rows a group up (8 groups of 4096 x 1536: 8 rows each 0.9x the 128-row
-  // tiles' time, 2048 rows each 1.2x)
-  if ((long)(rows_hint > 0 ? rows_hint : rows_cap) >= 64L * groups) {
-    if (!pair_gemm_takes(p)) return R(fail(kInvalidArgument, "grouped GEMM: buffers must be 16-byte aligned"));
-    return R(run_pair(p, stream));
-  }
-  int dev = 0;
-  cudaGetDevice(&dev);
-  CtrlBlock* ctrl = nullptr;
-  uint32_t* status = nullptr;
-  if ((s = gemm_process_words(dev, &ctrl, &status)) != kSuccess) return R(s);
-  GemmLaunch g;
-  memset(&g, 0, sizeof(g));
-  g.p.M = rows_cap;
-  g.p.N = N;
-  g.p.K = K;
-  g.p.mode = kGemmGrouped;
-  g.p.C = C;
-  g.p.ldc = epilogue == kEpiSwiGLU ? N / 2 : N;
-  g.p.rows_per_rank = rows_cap;
-  g.p.group_off = group_off;
-  g.p.groups = groups;
-  g.p.epilogue = epilogue;
-  g.p.coll.rank = 0;
-  g.p.coll.nranks = 1;
-  g.p.coll.ctrl[0] = ctrl;
-  g.p.coll.status = status;
-  g.p.coll.timeout_ns = 5ull * 1000000000ull;
-  g.p.fflags[0] = (FusedFlags*)(ctrl + 1);
-  const int sms = gemm_default_grid(dev);
-  // every group ends in a partly filled row tile: count about half a tile of waste per group
-  const int hint = rows_hint > 0 ? rows_hint : rows_cap;
-  const int row_tiles = (hint + kGemmBM - 1) / kGemmBM + groups / 2;
-  int bn = gemm_pick_bn(row_tiles, N, sms);
-  if (epilogue == kEpiSwiGLU) bn = bn >= 224 ? 256 : (bn >= 160 ? 192 : 128);
-  g.p.bn = bn;
-  if ((s = make_tensor_map_bf16(&g.map_a, A, rows_cap, K, K, kGemmBM)) != kSuccess) return R(s);
-  g.map_a_local = g.map_a;
-  if ((s = make_tensor_map_bf16(&g.map_b, B, (uint64_t)groups * N, K, K, g.p.bn)) != kSuccess) return R(s);
-  g.grid = sms;
-  s = launch_gemm(g, stream);
-  if (s == kSuccess && status[0]) s = fail(kInternalError, "tcgen05 GEMM reported a device-side wait timeout (code %u)", status[0]);
-  return R(s);
+  SkinnyProblem few = skinny(A, B, C, rows_cap, N, K, group_off, groups, (rows_hint > 0 ? rows_hint : rows_cap) / groups, epilogue);
+  if (skinny_pays(few)) return R(run_skinny(few, stream));
+  if (!pair_gemm_takes(p)) return R(fail(kInvalidArgument, "grouped GEMM: buffers must be 16-byte aligned"));
+  return R(run_pair(p, stream));
 }
 
 // The input gradient of the above: C[rows of group e, K] = A[rows of group e, N] * B[e] with the weights
@@ -466,8 +497,8 @@ ncclResult_t amemAllGatherGemm(const void* a_shard, const void* B, void* C, int 
   int rpr = M / n;
   if ((s = c->prepare_stream(stream)) != kSuccess) return R(s);
   if (n == 1) {   // nothing to gather
-    PairProblem pair = pair_plain(a_shard, B, C, M, N, K, 0, 0);
-    if (pair_pays(pair)) return R(run_pair(pair, stream));
+    bool done = false;
+    if ((s = run_plain(a_shard, B, C, M, N, K, stream, &done)) != kSuccess || done) return R(s);
   }
   if (n > 1 && !gemm_ag_uses_mover_warps(n)) return R(ag_gemm_cta_movers(c, a_shard, B, C, M, N, K, stream));
   GemmLaunch g;
@@ -538,8 +569,8 @@ ncclResult_t amemGemmReduceScatter(const void* A, const void* B, void* out, int 
   if ((rpr + kGemmBM - 1) / kGemmBM > kMaxUnits) return R(fail(kInvalidArgument, "more than %d rows per rank", kGemmBM * kMaxUnits));
   if ((s = c->prepare_stream(stream)) != kSuccess) return R(s);
   if (n == 1) {   // nothing to scatter
-    PairProblem pair = pair_plain(A, B, out, M, N, K, 0, 0);
-    if (pair_pays(pair)) return R(run_pair(pair, stream));
+    bool done = false;
+    if ((s = run_plain(A, B, out, M, N, K, stream, &done)) != kSuccess || done) return R(s);
   }
   GemmLaunch g;
   memset(&g, 0, sizeof(g));

@@ -30,6 +30,7 @@
 #include "../core/log.h"
 #include "coll_device.cuh"
 #include "gemm_pair.h"
+#include "pdl.cuh"
 #include "sm100_prims.cuh"
 
 namespace amem {
@@ -196,6 +197,7 @@ pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMa
   const int cluster = blockIdx.x / 2, clusters = gridDim.x / 2;
   volatile int* abort = &ctl->abort;
   const int bn = p.bn, half = bn / 2;
+  pdl_launch_dependents();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -216,6 +218,7 @@ pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMa
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
+  pdl_wait();   // from here on: what earlier kernels wrote is read, what they read may be overwritten
   const int out_cols = p.epilogue == kPairStore ? p.N : p.N / 2;
   const int tiles_n = (p.N + bn - 1) / bn;
   if (warp == 2) {
@@ -569,8 +572,24 @@ static_assert(A_BYTES == (HM / 64) * CHUNK_BYTES, "B's chunks follow A's without
 static_assert((MAX_SLICES - 1) * SLOT_FLOATS * 4 / MAX_SLICES <= STAGES * STAGE_BYTES, "the exchanged chunks must fit the operand ring");
 static_assert(kSmemBytes <= 227 * 1024, "operand ring, staging and control words must fit one SM's shared memory");
 
+template <int A_MN, int B_MN, int CUT>
+Status launch_one(const Params& p, const CUtensorMap& ma, const CUtensorMap& mb, int grid, cudaStream_t stream) {
+  static cudaError_t ready = cudaFuncSetAttribute((const void*)pair_kernel<A_MN, B_MN, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+  if (ready != cudaSuccess) return fail(kCudaError, "cudaFuncSetAttribute(%zu bytes of shared memory): %s", kSmemBytes, cudaGetErrorString(ready));
+  cudaError_t e = launch_overlapped(pair_kernel<A_MN, B_MN, CUT>, dim3(grid), dim3(THREADS), kSmemBytes, stream, p, ma, mb);
+  if (e != cudaSuccess) return fail(kCudaError, "pair gemm launch failed: %s", cudaGetErrorString(e));
+  return kSuccess;
+}
+
+template <int A_MN, int B_MN>
+Status launch(const Params& p, const CUtensorMap& ma, const CUtensorMap& mb, int grid, cudaStream_t stream) {
+  return p.slices > 1 ? launch_one<A_MN, B_MN, 1>(p, ma, mb, grid, stream) : launch_one<A_MN, B_MN, 0>(p, ma, mb, grid, stream);
+}
+
+}  // namespace pairk
+
 // [z][outer][inner] bf16 array with a box of box_inner x box_outer
-Status make_map(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t z, uint32_t box_outer) {
+Status make_bf16_map(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t z, uint32_t box_outer) {
   typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
   static EncodeFn fn = [] {
@@ -600,23 +619,6 @@ Status make_map(CUtensorMap* out, const void* base, uint64_t inner, uint64_t out
                                      (unsigned long long)outer, (unsigned long long)z);
   return kSuccess;
 }
-
-template <int A_MN, int B_MN, int CUT>
-Status launch_one(const Params& p, const CUtensorMap& ma, const CUtensorMap& mb, int grid, cudaStream_t stream) {
-  static cudaError_t ready = cudaFuncSetAttribute((const void*)pair_kernel<A_MN, B_MN, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-  if (ready != cudaSuccess) return fail(kCudaError, "cudaFuncSetAttribute(%zu bytes of shared memory): %s", kSmemBytes, cudaGetErrorString(ready));
-  pair_kernel<A_MN, B_MN, CUT><<<grid, THREADS, kSmemBytes, stream>>>(p, ma, mb);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return fail(kCudaError, "pair gemm launch failed: %s", cudaGetErrorString(e));
-  return kSuccess;
-}
-
-template <int A_MN, int B_MN>
-Status launch(const Params& p, const CUtensorMap& ma, const CUtensorMap& mb, int grid, cudaStream_t stream) {
-  return p.slices > 1 ? launch_one<A_MN, B_MN, 1>(p, ma, mb, grid, stream) : launch_one<A_MN, B_MN, 0>(p, ma, mb, grid, stream);
-}
-
-}  // namespace pairk
 
 int pair_gemm_pick_bn(long row_tiles, int N, int clusters, int k_blocks, int* slices) {
   int best = pairk::BN_MAX, best_s = 1;
@@ -677,11 +679,11 @@ Status launch_pair_gemm(const PairProblem& d, int sms, cudaStream_t stream) {
   p.bn = pair_gemm_pick_bn(row_tiles, d.N, clusters, (d.K + pairk::BK - 1) / pairk::BK, may_cut ? &p.slices : nullptr);
   if (d.epilogue != kPairStore) p.bn = p.bn > 192 ? 256 : (p.bn > 128 ? 192 : 128);   // gate and up columns in blocks of 32, half a tile each
   CUtensorMap ma, mb;
-  if (d.a_mn) AMEM_TRY(pairk::make_map(&ma, d.A, d.M, d.K, 1, 64));
-  else AMEM_TRY(pairk::make_map(&ma, d.A, d.K, d.M, 1, pairk::HM));
+  if (d.a_mn) AMEM_TRY(make_bf16_map(&ma, d.A, d.M, d.K, 1, 64));
+  else AMEM_TRY(make_bf16_map(&ma, d.A, d.K, d.M, 1, pairk::HM));
   const uint64_t z = d.mode == kPairGroupedRows ? d.groups : 1;
-  if (d.b_mn) AMEM_TRY(pairk::make_map(&mb, d.B, d.N, d.K, z, 64));
-  else AMEM_TRY(pairk::make_map(&mb, d.B, d.K, d.N, z, p.bn / 2));
+  if (d.b_mn) AMEM_TRY(make_bf16_map(&mb, d.B, d.N, d.K, z, 64));
+  else AMEM_TRY(make_bf16_map(&mb, d.B, d.K, d.N, z, p.bn / 2));
   if (p.slices > 1) p.slices = std::min(p.slices, (d.epilogue == kPairStore ? p.bn : p.bn / 2) / 32);   // a chunk of the result per slice
   const long tiles = d.mode == kPairGroupedRows ? clusters : row_tiles * ((d.N + p.bn - 1) / p.bn) * p.slices;
   const int grid = 2 * (int)std::min<long>(clusters, std::max<long>(1, tiles));

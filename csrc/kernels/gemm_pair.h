@@ -52,4 +52,7 @@ Status launch_pair_gemm(const PairProblem& p, int sms, cudaStream_t stream);
 // blocks of 64; *slices receives the number of cuts (1: none).
 int pair_gemm_pick_bn(long row_tiles, int N, int clusters, int k_blocks, int* slices);
 
+// Tensor map of a bf16 array [z][outer][inner] with boxes of 64 (inner) x box_outer in the 128-byte swizzle.
+Status make_bf16_map(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t z, uint32_t box_outer);
+
 }  // namespace amem
