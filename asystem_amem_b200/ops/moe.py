@@ -70,7 +70,7 @@ class MoeDispatcher:
         counts = torch.empty(self.experts_per_rank, dtype=torch.int32, device=x.device)
         offsets = torch.empty(self.experts_per_rank + 1, dtype=torch.int32, device=x.device)
         send_pos = torch.empty(T, k, dtype=torch.int32, device=x.device)
-        dropped = torch.zeros(1, dtype=torch.int32, device=x.device)
+        dropped = torch.empty(1, dtype=torch.int32, device=x.device)   # every word of the four is written by the kernels
         st = (stream or torch.cuda.current_stream()).cuda_stream
         B.check(self.comm.lib.amemMoeDispatchCounted(x.data_ptr(), topk_idx.data_ptr(), T, k, self.d, self.E, self.capacity,
                                                      counts.data_ptr(), offsets.data_ptr(), send_pos.data_ptr(), dropped.data_ptr(),

@@ -1,225 +1,433 @@
 // MoE dispatch / combine kernels (sm_100a).  See moe.h for the scheme.  Three launches make a
-// dispatch -- count (per-segment expert histograms), plan (scan + exchange of the histograms
+// dispatch (one, on a single rank with few pairs) -- count (per-segment expert histograms), plan (scan + exchange of the histograms
 // between ranks + row offsets), scatter (rows written into the owners' buffers over NVLink) --
 // and one launch makes a combine.  Peers are reached with plain 16-byte loads and stores; all
 // cross-rank waits go through the bounded block barrier of coll_device.cuh.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "../core/log.h"
 #include "coll_device.cuh"
 #include "moe.h"
+#include "pdl.cuh"
 
 namespace amem {
 namespace moek {
 
-constexpr int kThreads = 256;
 
-struct Launch {
-  int segments;
-  int combine_ctas;
-};
+constexpr int kThreads = 1024;        // count, plan, scatter: one CTA per SM, 32 warps
+constexpr int kCombineThreads = 256;  // up to two CTAs per SM, 128 registers a thread
+constexpr int kWarps = kThreads / 32;
+// One launch does a whole dispatch of one rank up to this many pairs: every CTA then works out the
+// positions of ALL pairs for itself and nothing has to be exchanged.
+constexpr int kOneLaunchPairs = 2 * kThreads;
+
+// Segment `seg` of the pairs: whole tokens, so that one CTA holds all choices of a token.
+__device__ __forceinline__ void segment_of(const MoeArgs& a, int seg, int segments, int& lo, int& hi) {
+  const int per = (a.T + segments - 1) / segments;
+  lo = min(a.T, seg * per) * a.k;
+  hi = min(a.T, (seg + 1) * per) * a.k;
+}
+__device__ __forceinline__ int expert_of(const MoeArgs& a, int pair) {   // -1: no such expert, the pair goes nowhere
+  const int e = a.topk_idx[pair];
+  return e >= 0 && e < a.E ? e : -1;
+}
 
 // ---- K1: histogram of expert ids per contiguous segment of (token, choice) pairs
 __device__ void count_body(const MoeArgs& a, int seg, int segments) {
   __shared__ int hist[kMoeMaxExperts];
   for (int e = threadIdx.x; e < a.E; e += blockDim.x) hist[e] = 0;
   __syncthreads();
-  const int P = a.T * a.k;
-  const int per = (P + segments - 1) / segments;
-  const int lo = min(P, seg * per), hi = min(P, lo + per);
+  int lo, hi;
+  segment_of(a, seg, segments, lo, hi);
   for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    int e = a.topk_idx[i];
-    if (e >= 0 && e < a.E) atomicAdd(&hist[e], 1);
+    const int e = expert_of(a, i);
+    if (e >= 0) atomicAdd(&hist[e], 1);
   }
   __syncthreads();
   for (int e = threadIdx.x; e < a.E; e += blockDim.x) a.seg_hist[seg * a.E + e] = hist[e];
+}
+
+// Where the rows of every expert lie: offsets of my pairs in the owners' buffers, counts and offsets of
+// my own experts.  cnt[s][e] = pairs of rank s for expert e.  Called by a whole CTA.
+__device__ void place_experts(const MoeArgs& a, const int (*cnt)[kMoeMaxExperts], int* send_off, bool write_own) {
+  const int n = a.coll.nranks, r = a.coll.rank, E = a.E, El = E / n;
+  // one warp per owner: a running sum over its experts, 32 at a time
+  for (int owner = threadIdx.x / 32; owner < n; owner += blockDim.x / 32) {
+    const int lane = threadIdx.x % 32;
+    int carry = 0;
+    for (int l0 = 0; l0 < El; l0 += 32) {
+      const int el = l0 + lane, e = owner * El + el;
+      int total = 0, before_me = 0;
+      if (el < El)
+        for (int s = 0; s < n; ++s) {
+          if (s == r) before_me = total;
+          total += cnt[s][e];
+        }
+      int sum = total;
+#pragma unroll
+      for (int d = 1; d < 32; d *= 2) {
+        const int o = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane >= d) sum += o;
+      }
+      const int first = carry + sum - total;
+      if (el < El) {
+        send_off[e] = first + before_me;
+        if (owner == r && write_own) {
+          // rows land expert after expert, so the ones beyond the capacity are exactly the tail of
+          // this sequence: clamping the running total gives the counts of the rows actually stored
+          const int cap = a.capacity_rows, lo = min(first, cap), hi = min(first + total, cap);
+          a.expert_counts[el] = hi - lo;
+          a.expert_offsets[el] = lo;
+          if (el == El - 1) {
+            a.expert_offsets[El] = hi;
+            if (a.dropped_rows) *a.dropped_rows = max(0, first + total - cap);
+          }
+        }
+      }
+      carry += __shfl_sync(0xffffffffu, sum, 31);
+    }
+  }
 }
 
 // ---- K2: one CTA per rank.  Scan the segment histograms, all-gather the per-expert totals
 // through the control blocks, derive where my rows start in every owner's buffer.
 __device__ void plan_body(const MoeArgs& a, int segments, int* s_abort) {
   __shared__ int cnt[kMaxRanks][kMoeMaxExperts];
-  const int n = a.coll.nranks, r = a.coll.rank, E = a.E, El = a.E / n;
+  const int n = a.coll.nranks, r = a.coll.rank, E = a.E;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nwarps = blockDim.x / 32;
   dev::Proto p;
   dev::proto_begin(p, a.coll, 0, 1, s_abort);
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int run = 0;
-    for (int s = 0; s < segments; ++s) {
-      a.seg_base[s * E + e] = run;
-      run += a.seg_hist[s * E + e];
+  // A warp takes an expert, a lane four neighbouring segments: the loads of an expert are in flight
+  // together (one thread per expert walked 128 dependent steps: 41 us for 64 experts, now 8).
+  for (int e = warp; e < E; e += nwarps) {
+    int carry = 0;
+    for (int s0 = 0; s0 < segments; s0 += 128) {
+      int h[4], sum = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int s = s0 + lane * 4 + j;
+        h[j] = s < segments ? a.seg_hist[s * E + e] : 0;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sum += h[j];
+      int scan = sum;
+#pragma unroll
+      for (int d = 1; d < 32; d *= 2) {
+        const int o = __shfl_up_sync(0xffffffffu, scan, d);
+        if (lane >= d) scan += o;
+      }
+      int run = carry + scan - sum;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int s = s0 + lane * 4 + j;
+        if (s < segments) a.seg_base[s * E + e] = run;
+        run += h[j];
+      }
+      carry += __shfl_sync(0xffffffffu, scan, 31);
     }
-    cnt[r][e] = run;
+    if (lane == 0) cnt[r][e] = carry;
   }
-  // peers may still read the totals of the previous dispatch: they signal this barrier only
-  // after they have left it
-  dev::block_barrier(p);
-  for (int e = threadIdx.x; e < E; e += blockDim.x)
-    for (int q = 0; q < n; ++q) a.coll.ctrl[q]->xchg[r][e] = (uint32_t)cnt[r][e];
-  dev::block_barrier(p);
-  for (int i = threadIdx.x; i < n * E; i += blockDim.x) {
-    int s = i / E, e = i % E;
-    cnt[s][e] = (int)dev::ld_volatile(&a.coll.ctrl[r]->xchg[s][e]);
+  if (n > 1) {
+    // peers may still read the totals of the previous dispatch: they signal this barrier only
+    // after they have left it
+    dev::block_barrier(p);
+    for (int e = threadIdx.x; e < E; e += blockDim.x)
+      for (int q = 0; q < n; ++q) a.coll.ctrl[q]->xchg[r][e] = (uint32_t)cnt[r][e];
+    dev::block_barrier(p);
+    for (int i = threadIdx.x; i < n * E; i += blockDim.x) {
+      int s = i / E, e = i % E;
+      cnt[s][e] = (int)dev::ld_volatile(&a.coll.ctrl[r]->xchg[s][e]);
+    }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int owner = e / El, first = owner * El;
-    int off = 0;
-    for (int e2 = first; e2 < e; ++e2)
-      for (int s = 0; s < n; ++s) off += cnt[s][e2];
-    for (int s = 0; s < r; ++s) off += cnt[s][e];
-    a.send_off[e] = off;
-  }
-  if (threadIdx.x == 0) {
-    // rows land expert after expert, so the ones beyond the capacity are exactly the tail of
-    // this sequence: clamping the running total gives the counts of the rows actually stored
-    const int cap = a.capacity_rows;
-    int run = 0;
-    for (int el = 0; el < El; ++el) {
-      int c = 0;
-      for (int s = 0; s < n; ++s) c += cnt[s][r * El + el];
-      const int lo = min(run, cap), hi = min(run + c, cap);
-      a.expert_counts[el] = hi - lo;
-      a.expert_offsets[el] = lo;
-      run += c;
-    }
-    a.expert_offsets[El] = min(run, cap);
-    if (a.dropped_rows) *a.dropped_rows = max(0, run - cap);
-  }
+  place_experts(a, cnt, a.send_off, true);
   dev::proto_end(p);
 }
 
-// ---- K3: every pair's row goes to its final place in the owner's receive buffer
-__device__ void scatter_body(const MoeArgs& a, int seg, int segments, int* s_abort) {
-  __shared__ int run[kMoeMaxExperts];
+// Positions of up to blockDim.x pairs at once: thread i holds expert e (-1: none) of pair i of the chunk;
+// run[e] = rows of expert e placed before the chunk, updated.  Rows keep pair order inside an expert.
+// whist: [warps][E | 1] scratch.  Called by a whole CTA.
+__device__ int chunk_positions(int e, int E, int* run, int* whist) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nwarps = blockDim.x / 32;
+  const int stride = E | 1;   // odd: a column of the table lies in 32 banks
+  for (int i = threadIdx.x; i < nwarps * stride; i += blockDim.x) whist[i] = 0;
+  __syncthreads();
+  const unsigned same = __match_any_sync(0xffffffffu, e);
+  const int before = __popc(same & ((1u << lane) - 1u));
+  if (e >= 0 && before == 0) whist[warp * stride + e] = __popc(same);
+  __syncthreads();
+  for (int x = warp; x < E; x += nwarps) {   // exclusive sums over the warps: a warp per expert (at most 32 warps)
+    const int c = lane < nwarps ? whist[lane * stride + x] : 0, start = run[x];
+    int sum = c;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+      const int o = __shfl_up_sync(0xffffffffu, sum, d);
+      if (lane >= d) sum += o;
+    }
+    if (lane < nwarps) whist[lane * stride + x] = start + sum - c;
+    if (lane == 31) run[x] = start + sum;
+  }
+  __syncthreads();
+  return e >= 0 ? whist[warp * stride + e] + before : -1;
+}
+
+// Copies the rows of the chunk's tokens to the positions of their pairs: a warp takes 4 KB of a token's
+// row at a time, reads it once and stores it to every choice.  c_pos / c_exp: the chunk's pairs.
+__device__ void copy_rows(const MoeArgs& a, int base, int count, const int* c_pos, const int* c_exp, int first_warp, int all_warps) {
+  const int lane = threadIdx.x % 32, El = a.E / a.coll.nranks;
+  const size_t row_bytes = (size_t)a.d * 2;
+  const int nvec = (int)(row_bytes / 16), parts = (nvec + 255) / 256;
+  const int t0 = base / a.k, t1 = (base + count - 1) / a.k;
+  for (int item = first_warp; item < (t1 - t0 + 1) * parts; item += all_warps) {
+    const int t = t0 + item / parts, v0 = (item % parts) * 256 + lane;
+    const uint4* src = (const uint4*)((const char*)a.x + (size_t)t * row_bytes);
+    uint4 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (v0 + j * 32 < nvec) v[j] = __ldg(src + v0 + j * 32);
+    const int j0 = max(t * a.k, base) - base, j1 = min((t + 1) * a.k, base + count) - base;
+    for (int c = j0; c < j1; ++c) {
+      const int pos = c_pos[c];
+      if (pos < 0) continue;
+      uint4* dst = (uint4*)(a.recv[c_exp[c] / El] + (size_t)pos * row_bytes);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (v0 + j * 32 < nvec) dst[v0 + j * 32] = v[j];
+    }
+  }
+}
+
+// The pairs of a segment to their places; run[e]: where this segment's rows of expert e begin.  Bound by
+// the rows' stores (16384 tokens x 8 choices x 8 KB: a row read per pair and 8 warps an SM 467 us; each
+// token read once by 32 warps an SM, with the counting 238; 185 are the rows' bytes).
+__device__ void scatter_segment(const MoeArgs& a, int seg, int segments, int* run, int* whist) {
   __shared__ int c_pos[kThreads];
   __shared__ int c_exp[kThreads];
-  const int n = a.coll.nranks, E = a.E, El = a.E / n;
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nwarps = blockDim.x / 32;
-  dev::Proto p;
-  dev::proto_begin(p, a.coll, seg, segments, s_abort);
-  for (int e = threadIdx.x; e < E; e += blockDim.x) run[e] = a.send_off[e] + a.seg_base[seg * E + e];
-  __syncthreads();
-  const int P = a.T * a.k;
-  const int per = (P + segments - 1) / segments;
-  const int lo = min(P, seg * per), hi = min(P, lo + per);
-  const size_t row_bytes = (size_t)a.d * 2;
+  int lo, hi;
+  segment_of(a, seg, segments, lo, hi);
   for (int base = lo; base < hi; base += blockDim.x) {
     const int i = base + threadIdx.x;
-    int e = -1;
-    if (i < hi) {
-      e = a.topk_idx[i];
-      if (e < 0 || e >= E) e = -1;
-    }
-    int pos = -1;
-    // warps take turns so that rows keep token order inside (source, expert)
-    for (int w = 0; w < nwarps; ++w) {
-      if (warp == w) {
-        unsigned valid = __ballot_sync(0xffffffffu, e >= 0);
-        if (e >= 0) {
-          unsigned same = __match_any_sync(valid, e);
-          int before = __popc(same & ((1u << lane) - 1u));
-          int start = run[e];
-          __syncwarp(valid);
-          if (before == 0) run[e] = start + __popc(same);
-          pos = start + before;
-        }
-      }
-      __syncthreads();
-    }
-    if (pos >= a.capacity_rows) pos = -1;  // no room at the owner: not sent (the plan kernel counted it)
+    const int e = i < hi ? expert_of(a, i) : -1;
+    int pos = chunk_positions(e, a.E, run, whist);
+    if (pos >= a.capacity_rows) pos = -1;  // no room at the owner: not sent (place_experts counted it)
     if (i < hi) a.send_pos[i] = pos;
     c_pos[threadIdx.x] = pos;
     c_exp[threadIdx.x] = e;
     __syncthreads();
-    const int in_chunk = min((int)blockDim.x, hi - base);
-    for (int j = warp; j < in_chunk; j += nwarps) {
-      int pj = c_pos[j];
-      if (pj < 0) continue;
-      int owner = c_exp[j] / El;
-      const uint4* src = (const uint4*)((const char*)a.x + (size_t)((base + j) / a.k) * row_bytes);
-      uint4* dst = (uint4*)(a.recv[owner] + (size_t)pj * row_bytes);
-      const int nvec = (int)(row_bytes / 16);
-      int v = lane;
-      for (; v + 96 < nvec; v += 128) {
-        uint4 t0 = src[v], t1 = src[v + 32], t2 = src[v + 64], t3 = src[v + 96];
-        dst[v] = t0;
-        dst[v + 32] = t1;
-        dst[v + 64] = t2;
-        dst[v + 96] = t3;
-      }
-      for (; v < nvec; v += 32) dst[v] = src[v];
-    }
+    copy_rows(a, base, min((int)blockDim.x, hi - base), c_pos, c_exp, threadIdx.x / 32, blockDim.x / 32);
     __syncthreads();
   }
+}
+
+// ---- K3: every pair's row goes to its final place in the owner's receive buffer.
+__device__ void scatter_body(const MoeArgs& a, int seg, int segments, int* s_abort) {
+  extern __shared__ int whist[];
+  __shared__ int run[kMoeMaxExperts];
+  dev::Proto p;
+  dev::proto_begin(p, a.coll, seg, segments, s_abort);
+  for (int e = threadIdx.x; e < a.E; e += blockDim.x) run[e] = a.send_off[e] + a.seg_base[seg * a.E + e];
+  scatter_segment(a, seg, segments, run, whist);
   // my rows are out; when this barrier passes on every block of a rank, every rank's rows for
   // it have landed (all ranks run the same number of blocks)
   dev::block_barrier(p);
   dev::proto_end(p);
 }
 
-// ---- combine: out[t] = sum_j w[t,j] * y_owner(t,j)[row(t,j)]
-__device__ void combine_body(const MoeArgs& a, int cta, int nctas, int* s_abort) {
-  const int n = a.coll.nranks, El = a.E / n;
+// ---- K2 and K3 of a communicator of one rank: every CTA sums the histograms itself (a few hundred
+// bytes per expert, out of L2), so no single CTA's scan stands between counting and copying (41 us of
+// the 512 for 64 experts).  CTA 0 writes the tables.
+__device__ void place_and_scatter_body(const MoeArgs& a, int seg, int segments) {
+  extern __shared__ int whist[];
+  __shared__ int run[kMoeMaxExperts];
+  __shared__ int before[kMoeMaxExperts];
+  __shared__ int cnt[1][kMoeMaxExperts];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nwarps = blockDim.x / 32;
-  dev::Proto p;
-  dev::proto_begin(p, a.coll, cta, nctas, s_abort);
-  dev::block_barrier(p);  // the expert outputs of every rank are complete
-  const int nvec = a.d / 8;
-  __nv_bfloat16* out = (__nv_bfloat16*)a.out;
-  for (int t = cta * nwarps + warp; t < a.T; t += nctas * nwarps) {
-    for (int cv = lane; cv < nvec; cv += 32) {
-      float acc[8];
+  for (int e = warp; e < a.E; e += nwarps) {
+    int total = 0, mine = 0;
+    for (int s = lane; s < segments; s += 32) {
+      const int h = a.seg_hist[s * a.E + e];
+      total += h;
+      if (s < seg) mine += h;
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) {
+      cnt[0][e] = total;
+      before[e] = mine;
+    }
+  }
+  __syncthreads();
+  place_experts(a, cnt, run, seg == 0);
+  __syncthreads();
+  for (int e = threadIdx.x; e < a.E; e += blockDim.x) run[e] += before[e];
+  __syncthreads();
+  scatter_segment(a, seg, segments, run, whist);
+}
+
+// ---- the whole dispatch of a communicator of one rank, for few pairs (see kOneLaunchPairs).  CTA 0
+// writes the tables, every CTA copies its share of the rows.
+__device__ void small_dispatch_body(const MoeArgs& a, int cta, int nctas) {
+  extern __shared__ int whist[];
+  __shared__ int run[kMoeMaxExperts];
+  __shared__ int off[kMoeMaxExperts];
+  __shared__ int cnt[1][kMoeMaxExperts];
+  __shared__ int c_pos[kThreads];
+  __shared__ int c_exp[kThreads];
+  const int P = a.T * a.k;
+  for (int e = threadIdx.x; e < a.E; e += blockDim.x) cnt[0][e] = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < P; i += blockDim.x) {
+    const int e = expert_of(a, i);
+    if (e >= 0) atomicAdd(&cnt[0][e], 1);
+  }
+  __syncthreads();
+  place_experts(a, cnt, off, cta == 0);
+  __syncthreads();
+  for (int e = threadIdx.x; e < a.E; e += blockDim.x) run[e] = off[e];
+  __syncthreads();
+  for (int base = 0; base < P; base += blockDim.x) {
+    const int i = base + threadIdx.x;
+    const int e = i < P ? expert_of(a, i) : -1;
+    int pos = chunk_positions(e, a.E, run, whist);
+    if (pos >= a.capacity_rows) pos = -1;
+    if (i < P && cta == 0) a.send_pos[i] = pos;
+    c_pos[threadIdx.x] = pos;
+    c_exp[threadIdx.x] = e;
+    __syncthreads();
+    copy_rows(a, base, min((int)blockDim.x, P - base), c_pos, c_exp, (threadIdx.x / 32) * nctas + cta, nctas * (blockDim.x / 32));
+    __syncthreads();
+  }
+}
+
+// ---- combine: out[t] = sum_j w[t,j] * y_owner(t,j)[row(t,j)].  A warp takes VPL x 512 bytes of a token's
+// result at a time, KC choices at once, so that 8 to 16 loads are in flight per lane whatever their number (16384 x 8 rows of 8 KB: a token per warp and one vector at a time 434 us, so 227, 185 being the
+// rows' bytes; 8192 x 2 rows 96 and 42).
+template <int KC, int VPL>
+__device__ void combine_items(const MoeArgs& a, int cta, int nctas) {
+  const bool one = a.coll.nranks == 1;
+  const int El = a.E / a.coll.nranks;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nwarps = blockDim.x / 32;
+  const int nvec = a.d / 8, parts = (nvec + 32 * VPL - 1) / (32 * VPL);
+  uint4* out = (uint4*)a.out;
+  for (long item = (long)warp * nctas + cta; item < (long)a.T * parts; item += (long)nctas * nwarps) {
+    const int t = (int)(item / parts), v0 = (int)(item - (long)t * parts) * 32 * VPL + lane;
+    float acc[VPL][8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] = 0.f;
-      for (int j0 = 0; j0 < a.k; j0 += 8) {
-        uint4 raw[8];
-        float w[8];
+    for (int u = 0; u < VPL; ++u)
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          int j = j0 + jj;
-          w[jj] = 0.f;
-          raw[jj] = make_uint4(0, 0, 0, 0);
-          if (j < a.k) {
-            int pos = a.send_pos[t * a.k + j];
-            if (pos >= 0) {
-              int owner = a.topk_idx[t * a.k + j] / El;
-              w[jj] = a.topk_w[t * a.k + j];
-              raw[jj] = *(const uint4*)(a.ybuf[owner] + ((size_t)pos * a.d + (size_t)cv * 8) * 2);
-            }
+      for (int q = 0; q < 8; ++q) acc[u][q] = 0.f;
+    for (int j0 = 0; j0 < a.k; j0 += KC) {
+      uint4 raw[KC][VPL];
+      float w[KC];
+      if (KC < 8) {
+        // lane jj looks up choice j0 + jj, the others get it from there
+        float my_w = 0.f;
+        const uint4* my_row = nullptr;
+        if (lane < KC && j0 + lane < a.k) {
+          const size_t at = (size_t)t * a.k + j0 + lane;
+          const int pos = a.send_pos[at];
+          if (pos >= 0) {
+            my_w = a.topk_w[at];
+            my_row = (const uint4*)(a.ybuf[one ? 0 : a.topk_idx[at] / El] + (size_t)pos * a.d * 2);
           }
         }
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          const __nv_bfloat16* h = (const __nv_bfloat16*)&raw[jj];
+        for (int jj = 0; jj < KC; ++jj) {
+          const uint4* row = (const uint4*)__shfl_sync(0xffffffffu, (unsigned long long)my_row, jj);
+          w[jj] = __shfl_sync(0xffffffffu, my_w, jj);
 #pragma unroll
-          for (int q = 0; q < 8; ++q) acc[q] = fmaf(w[jj], __bfloat162float(h[q]), acc[q]);
+          for (int u = 0; u < VPL; ++u) raw[jj][u] = row && v0 + u * 32 < nvec ? row[v0 + u * 32] : make_uint4(0, 0, 0, 0);
+        }
+      } else {
+        // (with eight choices every lane looks all of them up: shared row pointers need more registers
+        // than two CTAs an SM leave, 309 us instead of 227 for 16384 x 8 rows)
+#pragma unroll
+        for (int jj = 0; jj < KC; ++jj) {
+          const int j = j0 + jj;
+          w[jj] = 0.f;
+#pragma unroll
+          for (int u = 0; u < VPL; ++u) raw[jj][u] = make_uint4(0, 0, 0, 0);
+          if (j < a.k) {
+            const int pos = a.send_pos[(size_t)t * a.k + j];
+            if (pos >= 0) {
+              const int owner = a.topk_idx[(size_t)t * a.k + j] / El;
+              w[jj] = a.topk_w[(size_t)t * a.k + j];
+              const uint4* row = (const uint4*)(a.ybuf[owner] + (size_t)pos * a.d * 2);
+#pragma unroll
+              for (int u = 0; u < VPL; ++u)
+                if (v0 + u * 32 < nvec) raw[jj][u] = row[v0 + u * 32];
+            }
+          }
         }
       }
-      alignas(16) __nv_bfloat16 res[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) res[q] = __float2bfloat16_rn(acc[q]);
-      *(uint4*)(out + (size_t)t * a.d + (size_t)cv * 8) = *(const uint4*)res;
+      for (int jj = 0; jj < KC; ++jj)
+#pragma unroll
+        for (int u = 0; u < VPL; ++u) {
+          const __nv_bfloat16* h = (const __nv_bfloat16*)&raw[jj][u];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) acc[u][q] = fmaf(w[jj], __bfloat162float(h[q]), acc[u][q]);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < VPL; ++u) {
+      if (v0 + u * 32 < nvec) {
+        alignas(16) __nv_bfloat16 res[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) res[q] = __float2bfloat16_rn(acc[u][q]);
+        out[(size_t)t * nvec + v0 + u * 32] = *(const uint4*)res;
+      }
     }
   }
+}
+template <int KC, int VPL>
+__device__ void combine_body(const MoeArgs& a, int cta, int nctas, int* s_abort) {
+  dev::Proto p;
+  dev::proto_begin(p, a.coll, cta, nctas, s_abort);
+  if (a.coll.nranks > 1) dev::block_barrier(p);  // the expert outputs of every rank are complete
+  combine_items<KC, VPL>(a, cta, nctas);
   // nobody may overwrite its expert outputs while a peer still reads them
-  dev::block_barrier(p);
+  if (a.coll.nranks > 1) dev::block_barrier(p);
   dev::proto_end(p);
 }
 
 // ---- kernels: one rank per launch, and all ranks of an emulated communicator per launch
-__global__ void __launch_bounds__(kThreads) count_kernel(const __grid_constant__ MoeArgs a) { count_body(a, blockIdx.x, gridDim.x); }
+__global__ void __launch_bounds__(kThreads) count_kernel(const __grid_constant__ MoeArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  count_body(a, blockIdx.x, gridDim.x);
+}
 __global__ void __launch_bounds__(kThreads) plan_kernel(const __grid_constant__ MoeArgs a, int segments) {
   __shared__ int s_abort;
+  pdl_launch_dependents();
+  pdl_wait();
   plan_body(a, segments, &s_abort);
 }
 __global__ void __launch_bounds__(kThreads) scatter_kernel(const __grid_constant__ MoeArgs a) {
   __shared__ int s_abort;
+  pdl_launch_dependents();
+  pdl_wait();
   scatter_body(a, blockIdx.x, gridDim.x, &s_abort);
 }
-__global__ void __launch_bounds__(kThreads) combine_kernel(const __grid_constant__ MoeArgs a) {
+__global__ void __launch_bounds__(kThreads) place_and_scatter_kernel(const __grid_constant__ MoeArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  place_and_scatter_body(a, blockIdx.x, gridDim.x);
+}
+__global__ void __launch_bounds__(kThreads) small_dispatch_kernel(const __grid_constant__ MoeArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  small_dispatch_body(a, blockIdx.x, gridDim.x);
+}
+template <int KC, int VPL>
+__global__ void __launch_bounds__(kCombineThreads, 2) combine_kernel(const __grid_constant__ MoeArgs a) {
   __shared__ int s_abort;
-  combine_body(a, blockIdx.x, gridDim.x, &s_abort);
+  pdl_launch_dependents();
+  pdl_wait();
+  combine_body<KC, VPL>(a, blockIdx.x, gridDim.x, &s_abort);
 }
 __global__ void __launch_bounds__(kThreads) count_kernel_emu(const MoeArgs* __restrict__ all) { count_body(all[blockIdx.y], blockIdx.x, gridDim.x); }
 __global__ void __launch_bounds__(kThreads) plan_kernel_emu(const MoeArgs* __restrict__ all, int segments) {
@@ -230,57 +438,72 @@ __global__ void __launch_bounds__(kThreads) scatter_kernel_emu(const MoeArgs* __
   __shared__ int s_abort;
   scatter_body(all[blockIdx.y], blockIdx.x, gridDim.x, &s_abort);
 }
-__global__ void __launch_bounds__(kThreads) combine_kernel_emu(const MoeArgs* __restrict__ all) {
+__global__ void __launch_bounds__(kCombineThreads, 2) combine_kernel_emu(const MoeArgs* __restrict__ all) {
   __shared__ int s_abort;
-  combine_body(all[blockIdx.y], blockIdx.x, gridDim.x, &s_abort);
+  combine_body<8, 2>(all[blockIdx.y], blockIdx.x, gridDim.x, &s_abort);
 }
+
+// Per-warp histograms of chunk_positions: at most 33 KB.
+size_t whist_bytes(int E) { return (size_t)kWarps * (E | 1) * sizeof(int); }
 
 }  // namespace moek
 
-static Status launched(const char* what) {
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return fail(kCudaError, "%s launch failed: %s", what, cudaGetErrorString(e));
-  return kSuccess;
-}
-
-Status launch_moe_dispatch(const MoeArgs& a, cudaStream_t stream) {
-  moek::count_kernel<<<kMoeSegments, moek::kThreads, 0, stream>>>(a);
-  AMEM_TRY(launched("moe count"));
-  moek::plan_kernel<<<1, moek::kThreads, 0, stream>>>(a, kMoeSegments);
-  AMEM_TRY(launched("moe plan"));
-  moek::scatter_kernel<<<kMoeSegments, moek::kThreads, 0, stream>>>(a);
-  return launched("moe scatter");
-}
-
-Status launch_moe_combine(const MoeArgs& a, cudaStream_t stream) {
-  moek::combine_kernel<<<2 * kMoeSegments, moek::kThreads, 0, stream>>>(a);
-  return launched("moe combine");
-}
-
-template <typename K>
-static Status coop(K kernel, dim3 grid, void** params, cudaStream_t stream, const char* what) {
-  cudaError_t e = cudaLaunchCooperativeKernel((const void*)kernel, grid, dim3(moek::kThreads), params, 0, stream);
+static Status launched(cudaError_t e, const char* what) {
   if (e != cudaSuccess) {
     cudaGetLastError();
-    return fail(kCudaError, "%s cooperative launch failed: %s", what, cudaGetErrorString(e));
+    return fail(kCudaError, "%s launch failed: %s", what, cudaGetErrorString(e));
   }
   return kSuccess;
 }
 
-Status launch_moe_dispatch_emu(const MoeArgs*, const MoeArgs* dev_all, int nranks, cudaStream_t stream) {
+// One rank: launches overlap their predecessor's end.  With peers they are ordinary launches: those
+// kernels wait for the other GPUs' and are not to be scheduled before their turn.
+template <typename... P, typename... A>
+static cudaError_t launch(void (*kernel)(P...), const MoeArgs& a, int grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
+  if (a.coll.nranks == 1) return launch_overlapped(kernel, dim3(grid), dim3(threads), smem, stream, args...);
+  kernel<<<grid, threads, smem, stream>>>(args...);
+  return cudaGetLastError();
+}
+
+Status launch_moe_dispatch(const MoeArgs& a, cudaStream_t stream) {
+  const size_t smem = moek::whist_bytes(a.E);
+  const long pairs = (long)a.T * a.k;
+  if (a.coll.nranks == 1 && pairs <= moek::kOneLaunchPairs) {
+    // as many CTAs as there are 4 KB pieces for their warps (the positions of all pairs are worked out in each)
+    const long pieces = (long)a.T * ((a.d / 8 + 255) / 256);
+    const int grid = (int)std::max<long>(1, std::min<long>(kMoeSegments, (pieces + 7) / 8));
+    return launched(launch(moek::small_dispatch_kernel, a, grid, moek::kThreads, smem, stream, a), "moe dispatch");
+  }
+  AMEM_TRY(launched(launch(moek::count_kernel, a, kMoeSegments, moek::kThreads, 0, stream, a), "moe count"));
+  if (a.coll.nranks == 1) return launched(launch(moek::place_and_scatter_kernel, a, kMoeSegments, moek::kThreads, smem, stream, a), "moe scatter");
+  AMEM_TRY(launched(launch(moek::plan_kernel, a, 1, moek::kThreads, 0, stream, a, kMoeSegments), "moe plan"));
+  return launched(launch(moek::scatter_kernel, a, kMoeSegments, moek::kThreads, smem, stream, a), "moe scatter");
+}
+
+Status launch_moe_combine(const MoeArgs& a, cudaStream_t stream) {
+  auto kernel = a.k <= 2 ? moek::combine_kernel<2, 4> : a.k <= 4 ? moek::combine_kernel<4, 2> : moek::combine_kernel<8, 2>;
+  return launched(launch(kernel, a, 2 * kMoeSegments, moek::kCombineThreads, 0, stream, a), "moe combine");
+}
+
+template <typename K>
+static Status coop(K kernel, dim3 grid, int threads, size_t smem, void** params, cudaStream_t stream, const char* what) {
+  return launched(cudaLaunchCooperativeKernel((const void*)kernel, grid, dim3(threads), params, smem, stream), what);
+}
+
+Status launch_moe_dispatch_emu(const MoeArgs* host_all, const MoeArgs* dev_all, int nranks, cudaStream_t stream) {
   const int segs = 8;
   moek::count_kernel_emu<<<dim3(segs, nranks), moek::kThreads, 0, stream>>>(dev_all);
-  AMEM_TRY(launched("moe count(emu)"));
+  AMEM_TRY(launched(cudaGetLastError(), "moe count(emu)"));
   int segments = segs;
   void* p2[] = {(void*)&dev_all, (void*)&segments};
-  AMEM_TRY(coop(moek::plan_kernel_emu, dim3(1, nranks), p2, stream, "moe plan(emu)"));
+  AMEM_TRY(coop(moek::plan_kernel_emu, dim3(1, nranks), moek::kThreads, 0, p2, stream, "moe plan(emu)"));
   void* p3[] = {(void*)&dev_all};
-  return coop(moek::scatter_kernel_emu, dim3(segs, nranks), p3, stream, "moe scatter(emu)");
+  return coop(moek::scatter_kernel_emu, dim3(segs, nranks), moek::kThreads, moek::whist_bytes(host_all[0].E), p3, stream, "moe scatter(emu)");
 }
 
 Status launch_moe_combine_emu(const MoeArgs*, const MoeArgs* dev_all, int nranks, cudaStream_t stream) {
   void* p[] = {(void*)&dev_all};
-  return coop(moek::combine_kernel_emu, dim3(8, nranks), p, stream, "moe combine(emu)");
+  return coop(moek::combine_kernel_emu, dim3(8, nranks), moek::kCombineThreads, 0, p, stream, "moe combine(emu)");
 }
 
 }  // namespace amem

@@ -18,7 +18,7 @@
 namespace amem {
 
 static const int kMoeMaxExperts = 256;   // CtrlBlock::xchg row length
-static const int kMoeSegments = 128;     // CTAs of the count / scatter kernels
+static const int kMoeSegments = 148;     // CTAs of the count / scatter kernels: one per SM
 
 struct MoeArgs {
   CollArgs coll;

@@ -25,7 +25,7 @@ struct NoAllocScratch {
   int send_off[kNoAllocMaxExperts];                     // first row of every expert
 };
 
-// ~330 KB per GPU, held from the moment the CUDA module of this library is loaded on that GPU (its
+// ~370 KB per GPU, held from the moment the CUDA module of this library is loaded on that GPU (its
 // first use there) to process exit.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoAllocScratch)];
 
