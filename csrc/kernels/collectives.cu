@@ -461,7 +461,9 @@ Status launch_collective(const CollArgs& a, const LaunchPlan& plan, cudaStream_t
     dev::sendrecv_kernel<<<nb, plan.threads, 0, stream>>>(a);
     return check_launch("sendrecv");
   }
-  bool ok = true;
+  bool ok = true, local = false;
+  const Status st_local = launch_local(a, stream, &local);
+  if (local) return st_local;
   if (a.kind == kCollAllReduce && a.algo == kAlgoNvls && a.nranks > 1) {
     if (a.dtype == kF32) dev::nvls_allreduce_kernel<float><<<grid, block, 0, stream>>>(a, plan.chunk_elems);
     else if (a.dtype == kBF16) dev::nvls_allreduce_kernel<__nv_bfloat16><<<grid, block, 0, stream>>>(a, plan.chunk_elems);

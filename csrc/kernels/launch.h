@@ -9,6 +9,9 @@ namespace amem {
 
 // Launches one rank's kernel on `stream`.
 Status launch_collective(const CollArgs& a, const LaunchPlan& plan, cudaStream_t stream);
+// The same for a communicator of one rank, where that is a copy or a scale and cast of aligned buffers;
+// *handled is false where launch_collective has to do it.
+Status launch_local(const CollArgs& a, cudaStream_t stream, bool* handled);
 // Launches every rank of an emulated (single-GPU) communicator as one cooperative grid.
 // `dev_all` points to `nranks` CollArgs in device-readable memory; `a` is any rank's copy
 // (used for type dispatch only).

@@ -1,0 +1,101 @@
+// Collectives of a communicator of one rank: a copy, or a scale and cast, of the operand.  The general
+// kernel runs 128 blocks with two loads in flight per thread and keeps protocol state; here every block
+// moves one piece of 16 KB (copy) or 8192 elements (cast), all its loads ahead of its stores, and nothing
+// else.  100 MB copied: 53 us (3.8 TB/s) before, 31.7 (6.3 TB/s) so, 35.2 with eight blocks an SM that
+// stride over the buffer; bf16 to fp32, the same 50 M elements: 69 us before, 47.0 (6.4 TB/s) so.
+#include <algorithm>
+
+#include "coll_device.cuh"
+#include "launch.h"
+#include "pdl.cuh"
+
+namespace amem {
+namespace localk {
+
+constexpr int THREADS = 256, AHEAD = 4, CAST_AHEAD = 8;
+
+__global__ void __launch_bounds__(THREADS) copy_kernel(const char* __restrict__ src, char* __restrict__ dst, size_t bytes) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const size_t n = bytes / 16, i0 = (size_t)blockIdx.x * THREADS * AHEAD + threadIdx.x;
+  uint4 v[AHEAD];
+#pragma unroll
+  for (int j = 0; j < AHEAD; ++j)
+    if (i0 + j * THREADS < n) v[j] = ((const uint4*)src)[i0 + j * THREADS];
+#pragma unroll
+  for (int j = 0; j < AHEAD; ++j)
+    if (i0 + j * THREADS < n) ((uint4*)dst)[i0 + j * THREADS] = v[j];
+  if (blockIdx.x == 0 && threadIdx.x < bytes % 16) dst[n * 16 + threadIdx.x] = src[n * 16 + threadIdx.x];
+}
+
+template <typename T>
+struct alignas(4 * sizeof(T)) Four {
+  T e[4];
+};
+
+// out = (TO)(scale * in), in fp32; four elements per access, so that a warp covers whole lines on both sides
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(THREADS) scale_kernel(const TI* __restrict__ src, TO* __restrict__ dst, size_t count, float scale) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const size_t n = count / 4, i0 = (size_t)blockIdx.x * THREADS * CAST_AHEAD + threadIdx.x;
+  Four<TI> v[CAST_AHEAD];
+#pragma unroll
+  for (int j = 0; j < CAST_AHEAD; ++j)
+    if (i0 + j * THREADS < n) v[j] = ((const Four<TI>*)src)[i0 + j * THREADS];
+#pragma unroll
+  for (int j = 0; j < CAST_AHEAD; ++j)
+    if (i0 + j * THREADS < n) {
+      Four<TO> o;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) o.e[q] = dev::from_acc<TO, float>(dev::to_acc<TI>(v[j].e[q]) * scale);
+      ((Four<TO>*)dst)[i0 + j * THREADS] = o;
+    }
+  if (blockIdx.x == 0 && threadIdx.x < count % 4) dst[n * 4 + threadIdx.x] = dev::from_acc<TO, float>(dev::to_acc<TI>(src[n * 4 + threadIdx.x]) * scale);
+}
+
+template <typename TI, typename TO>
+cudaError_t scaled(const CollArgs& a, int grid, cudaStream_t stream) {
+  return launch_overlapped(scale_kernel<TI, TO>, dim3(grid), dim3(THREADS), 0, stream, (const TI*)a.send, (TO*)a.recv, (size_t)a.count, a.scale);
+}
+template <typename TI>
+cudaError_t scaled_from(const CollArgs& a, int grid, cudaStream_t stream) {
+  return a.out_dtype == kF32 ? scaled<TI, float>(a, grid, stream) : a.out_dtype == kBF16 ? scaled<TI, __nv_bfloat16>(a, grid, stream)
+                                                                                           : scaled<TI, __half>(a, grid, stream);
+}
+
+bool narrow_float(int t) { return t == kF32 || t == kBF16 || t == kF16; }
+
+}  // namespace localk
+
+// Takes a one-rank collective where it is a plain copy, or a scale and cast among fp32 / bf16 / fp16, of
+// 16-byte aligned buffers; everything else (other types with a scale, odd addresses) is left to the
+// general kernel.  *handled tells.
+Status launch_local(const CollArgs& a, cudaStream_t stream, bool* handled) {
+  using namespace localk;
+  *handled = false;
+  if (a.nranks != 1 || (((uintptr_t)a.send | (uintptr_t)a.recv) & 15)) return kSuccess;
+  if (a.dtype > kBF16 || a.out_dtype > kBF16) return kSuccess;   // 8-bit floats as such: reductions of them are refused there
+  const bool copy = a.dtype == a.out_dtype && (!a.has_scale || (a.scale == 1.0f && narrow_float(a.dtype)));
+  const bool pair = a.dtype == a.out_dtype || a.dtype == kF32 || a.out_dtype == kF32;   // bf16 <-> fp16 is refused
+  const bool scale = narrow_float(a.dtype) && narrow_float(a.out_dtype) && pair;
+  if (!copy && !scale) return kSuccess;
+  if (a.send == a.recv && !copy) return kSuccess;
+  *handled = true;
+  if (a.send == a.recv) return kSuccess;   // in place: nothing to move
+  const size_t items = copy ? a.count * dtype_size(a.dtype) / 16 : a.count / 4, per_block = (size_t)THREADS * (copy ? AHEAD : CAST_AHEAD);
+  const size_t blocks = std::max<size_t>(1, (items + per_block - 1) / per_block);
+  if (blocks > 0x7fffffffu) return fail(kInvalidArgument, "one-rank collective of %zu elements", (size_t)a.count);
+  const int grid = (int)blocks;
+  cudaError_t e;
+  CollArgs s = a;
+  if (!s.has_scale) s.scale = 1.0f;
+  if (copy) e = launch_overlapped(copy_kernel, dim3(grid), dim3(THREADS), 0, stream, (const char*)a.send, (char*)a.recv, a.count * dtype_size(a.dtype));
+  else if (a.dtype == kF32) e = scaled_from<float>(s, grid, stream);
+  else if (a.dtype == kBF16) e = scaled_from<__nv_bfloat16>(s, grid, stream);
+  else e = scaled_from<__half>(s, grid, stream);
+  if (e != cudaSuccess) return fail(kCudaError, "one-rank collective launch failed: %s", cudaGetErrorString(e));
+  return kSuccess;
+}
+
+}  // namespace amem
