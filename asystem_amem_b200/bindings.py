@@ -136,6 +136,10 @@ def load_library(build_if_missing: bool = True) -> ctypes.CDLL:
         "amemMoeCombine": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
         "amemGemmBf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
         "amemGemmBf16Strided": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+        "amemGemmSwiGLU": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+        "amemSwiGLU": [c_void_p, c_void_p, ctypes.c_longlong, c_void_p, ctypes.c_longlong, c_int, c_void_p],
+        "amemSwiGLUGrad": [c_void_p, c_void_p, ctypes.c_longlong, c_void_p, c_void_p, c_void_p, ctypes.c_longlong, c_int, c_void_p],
+        "amemAdamW": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, ctypes.c_longlong] + [ctypes.c_double] * 5 + [ctypes.c_longlong, c_void_p],
         "amemGemmPlan": [c_int, c_int, c_int, c_int, ctypes.POINTER(c_int), ctypes.POINTER(c_int), ctypes.POINTER(c_int)],
         "amemAllGatherGemmPlan": [c_int, c_int, c_int, ctypes.POINTER(c_int), ctypes.POINTER(c_int), ctypes.POINTER(c_int)],
         "amemDeviceWaitProbe": [c_int, c_int, ctypes.POINTER(c_int), ctypes.POINTER(ctypes.c_float)],

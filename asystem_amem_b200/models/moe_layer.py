@@ -15,9 +15,9 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
-import torch.nn.functional as F
 
 from ..ops.gemm import grouped_gemm_bf16, grouped_gemm_input_grad, grouped_gemm_weight_grad, interleave_gate_up
+from ..ops.elementwise import swiglu
 from ..ops.moe import MoeDispatcher
 from ..parallel.ep import ep_combine, ep_dispatch
 
@@ -76,8 +76,7 @@ class MoELayer(nn.Module):
         if torch.is_grad_enabled() and (x.requires_grad or self.w2.requires_grad):
             rows, offsets, send_pos = ep_dispatch(self.dispatcher, x, idx)
             h = GroupedLinear.apply(rows, self.w13, offsets)
-            a = (F.silu(h[:, : self.ffn_dim].float()) * h[:, self.ffn_dim:].float()).to(torch.bfloat16)
-            y = GroupedLinear.apply(a, self.w2, offsets)
+            y = GroupedLinear.apply(swiglu(h).to(torch.bfloat16), self.w2, offsets)
             return ep_combine(self.dispatcher, y, w, idx, send_pos)
         res = self.dispatcher.dispatch(x.contiguous(), idx)
         self.last_dropped = res.dropped
@@ -85,7 +84,7 @@ class MoELayer(nn.Module):
             a = grouped_gemm_bf16(res.recv_x, self._fused_w13(), res.expert_offsets, rows_hint=self.tokens_hint, swiglu=True)
         else:
             h = grouped_gemm_bf16(res.recv_x, self.w13.detach(), res.expert_offsets, rows_hint=self.tokens_hint)
-            a = (F.silu(h[:, : self.ffn_dim].float()) * h[:, self.ffn_dim:].float()).to(torch.bfloat16)
+            a = swiglu(h).to(torch.bfloat16)
         # the second GEMM writes the experts' outputs where the combine reads them
         grouped_gemm_bf16(a, self.w2.detach(), res.expert_offsets, out=self.dispatcher.y, rows_hint=self.tokens_hint)
         return self.dispatcher.combine(idx, w, res.send_pos)

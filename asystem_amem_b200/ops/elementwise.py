@@ -1,0 +1,69 @@
+"""Element-wise passes as single kernels: SwiGLU with its gradient, the AdamW update of a shard.
+
+Reference parity: none -- the reference contains no arithmetic on user data.
+"""
+from __future__ import annotations
+
+import torch
+import torch.nn.functional as F
+
+from .. import bindings as B
+
+
+def _st() -> int:
+    return torch.cuda.current_stream().cuda_stream
+
+
+def _fused(h: torch.Tensor) -> bool:
+    return h.is_cuda and h.dtype == torch.bfloat16 and h.dim() == 2 and h.shape[1] % 16 == 0 and h.data_ptr() % 16 == 0
+
+
+class _SwiGLU(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, h):
+        ctx.save_for_backward(h)
+        return _forward(h)
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, g):
+        (h,) = ctx.saved_tensors
+        g, out = g.contiguous(), torch.empty_like(h)
+        f, p, o = h.shape[1] // 2, h.data_ptr(), out.data_ptr()
+        B.check(B.load_library().amemSwiGLUGrad(p, p + 2 * f, 2 * f, g.data_ptr(), o, o + 2 * f, h.shape[0], f, _st()), "amemSwiGLUGrad")
+        return out
+
+
+def _forward(h: torch.Tensor) -> torch.Tensor:
+    f, p = h.shape[1] // 2, h.data_ptr()
+    out = torch.empty(h.shape[0], f, dtype=h.dtype, device=h.device)
+    B.check(B.load_library().amemSwiGLU(p, p + 2 * f, 2 * f, out.data_ptr(), h.shape[0], f, _st()), "amemSwiGLU")
+    return out
+
+
+def swiglu(h: torch.Tensor) -> torch.Tensor:
+    """silu(h[:, :f]) * h[:, f:] of a [rows, 2 f] tensor in fp32, rounded once to h's type."""
+    if _fused(h):
+        h = h.contiguous()
+        return _SwiGLU.apply(h) if torch.is_grad_enabled() and h.requires_grad else _forward(h)
+    f = h.shape[1] // 2
+    return (F.silu(h[:, :f].float()) * h[:, f:].float()).to(h.dtype)
+
+
+def adamw_step(grad, m, v, master, shard, lr: float, betas, eps: float, weight_decay: float, step: int) -> None:
+    """One AdamW update in place: fp32 ``m``, ``v`` and ``master`` from the fp32 ``grad``; ``shard``
+    receives the new weights in bf16.  ``step`` counts from 1."""
+    flat = (grad, m, v, master, shard)
+    if all(t.is_cuda and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in flat) and shard.dtype == torch.bfloat16 \
+            and all(t.dtype == torch.float32 for t in flat[:4]):
+        B.check(B.load_library().amemAdamW(grad.data_ptr(), m.data_ptr(), v.data_ptr(), master.data_ptr(), shard.data_ptr(), grad.numel(),
+                                           lr, betas[0], betas[1], eps, weight_decay, step, _st()), "amemAdamW")
+        return
+    b1, b2 = betas
+    c1, c2 = 1 - b1 ** step, 1 - b2 ** step
+    m.mul_(b1).add_(grad, alpha=1 - b1)
+    v.mul_(b2).addcmul_(grad, grad, value=1 - b2)
+    if weight_decay:
+        master.mul_(1 - lr * weight_decay)
+    master.addcdiv_(m / c1, (v / c2).sqrt_().add_(eps), value=-lr)
+    shard.copy_(master)

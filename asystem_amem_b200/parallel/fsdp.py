@@ -22,6 +22,8 @@ import math
 import torch
 import torch.nn as nn
 
+from ..ops.elementwise import adamw_step
+
 
 class _ShardedUnit:
     def __init__(self, module: nn.Module, comm, name: str):
@@ -190,13 +192,5 @@ class ShardedAdamW:
     @torch.no_grad()
     def step(self) -> None:
         self.t += 1
-        b1, b2 = self.betas
-        c1, c2 = 1 - b1 ** self.t, 1 - b2 ** self.t
         for u, m, v in zip(self.fsdp.units, self.m, self.v):
-            g = u.grad_shard
-            m.mul_(b1).add_(g, alpha=1 - b1)
-            v.mul_(b2).addcmul_(g, g, value=1 - b2)
-            if self.wd:
-                u.master.mul_(1 - self.lr * self.wd)
-            u.master.addcdiv_(m / c1, (v / c2).sqrt_().add_(self.eps), value=-self.lr)
-        self.fsdp.sync_shards_from_master()
+            adamw_step(u.grad_shard, m, v, u.master, u.shard, self.lr, self.betas, self.eps, self.wd, self.t)

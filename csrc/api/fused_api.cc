@@ -298,6 +298,21 @@ ncclResult_t amemGemmBf16Strided(const void* A, const void* B, void* C, int M, i
   return R(run_pair(p, stream));
 }
 
+// C[M, F] = silu(A * W[0:F]^T) * (A * W[F:2F]^T): the gate / up projection of an MLP and its activation in
+// one pass; W is bf16 [2 F, K], the gate's rows first.
+ncclResult_t amemGemmSwiGLU(const void* A, const void* W, void* C, int M, int F, int K, cudaStream_t stream) {
+  if (F <= 0 || F > 0x3fffffff) return R(fail(kInvalidArgument, "amemGemmSwiGLU: F=%d", F));
+  Status s = check_shape(M, F, K);
+  if (s != kSuccess) return R(s);
+  if (!A || !W || !C) return R(fail(kInvalidArgument, "GEMM: null buffer"));
+  SkinnyProblem few = skinny(A, W, C, M, 2 * F, K, nullptr, 1, M, kPairSwiGLUHalves);
+  if (skinny_pays(few)) return R(run_skinny(few, stream));
+  PairProblem p = pair_plain(A, W, C, M, 2 * F, K, 0, 0);
+  p.epilogue = kPairSwiGLUHalves;
+  if (!pair_gemm_takes(p)) return R(fail(kInvalidArgument, "amemGemmSwiGLU: buffers must be 16-byte aligned"));
+  return R(run_pair(p, stream));
+}
+
 // The tiling of the one-SM form on a GPU with `sms` SMs (no GPU needed: planning is host
 // arithmetic).  Outputs may be null.
 ncclResult_t amemGemmPlan(int M, int N, int K, int sms, int* tile_rows, int* tile_cols, int* tail_slices) {

@@ -1,0 +1,56 @@
+// C entry points of the element-wise passes (kernels/fused_math.cu).  The reference has no counterpart.
+#include <cuda_runtime.h>
+
+#include <cmath>
+
+#include "../core/log.h"
+#include "../include/nccl.h"
+#include "../kernels/fused_math.h"
+
+using namespace amem;
+
+namespace {
+
+inline ncclResult_t R(Status s) {
+  if (s != kSuccess) LOGW("%s: %s", status_name(s), last_error_slot().c_str());
+  return (ncclResult_t)s;
+}
+
+bool aligned16(const void* a, const void* b, const void* c) { return !(((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15); }
+
+}  // namespace
+
+extern "C" {
+
+ncclResult_t amemSwiGLU(const void* gate, const void* up, long long ld, void* act, long long rows, int F, cudaStream_t stream) {
+  if (rows < 0 || F <= 0 || F % 8 || ld < F || ld % 8 || !aligned16(gate, up, act))
+    return R(fail(kInvalidArgument, "amemSwiGLU: rows=%lld F=%d ld=%lld (multiples of 8, 16-byte aligned)", rows, F, ld));
+  return rows == 0 ? ncclSuccess : R(launch_swiglu(gate, up, (long)ld, act, (long)rows, F, stream));
+}
+
+ncclResult_t amemSwiGLUGrad(const void* gate, const void* up, long long ld, const void* g_act, void* g_gate, void* g_up, long long rows, int F,
+                            cudaStream_t stream) {
+  if (rows < 0 || F <= 0 || F % 8 || ld < F || ld % 8 || !aligned16(gate, up, g_act) || !aligned16(g_gate, g_up, nullptr))
+    return R(fail(kInvalidArgument, "amemSwiGLUGrad: rows=%lld F=%d ld=%lld (multiples of 8, 16-byte aligned)", rows, F, ld));
+  return rows == 0 ? ncclSuccess : R(launch_swiglu_grad(gate, up, (long)ld, g_act, g_gate, g_up, (long)rows, F, stream));
+}
+
+ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,
+                       double eps, double weight_decay, long long step, cudaStream_t stream) {
+  if (n < 0 || step < 1 || !aligned16(grad, m, v) || !aligned16(master, shard_bf16, nullptr))
+    return R(fail(kInvalidArgument, "amemAdamW: n=%lld step=%lld (buffers 16-byte aligned)", n, step));
+  if (n == 0) return ncclSuccess;
+  AdamW a;
+  a.lr = (float)lr;
+  a.b1 = (float)beta1;
+  a.one_minus_b1 = (float)(1.0 - beta1);
+  a.b2 = (float)beta2;
+  a.one_minus_b2 = (float)(1.0 - beta2);
+  a.c1 = (float)(1.0 - std::pow(beta1, (double)step));
+  a.c2 = (float)(1.0 - std::pow(beta2, (double)step));
+  a.eps = (float)eps;
+  a.decay = (float)(1.0 - lr * weight_decay);
+  return R(launch_adamw(grad, m, v, master, shard_bf16, (long)n, a, stream));
+}
+
+}  // extern "C"

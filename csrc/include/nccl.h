@@ -209,6 +209,18 @@ ncclResult_t amemGemmBf16(const void* A, const void* B, void* C, int M, int N, i
  * [K, N].  Built: (0, 0), (0, 1) -- a Linear's input gradient from its weight as it lies -- and (1, 1), its
  * weight gradient (K is then any number).  The contiguous extents must be multiples of 8. */
 ncclResult_t amemGemmBf16Strided(const void* A, const void* B, void* C, int M, int N, int K, int a_by_k, int b_by_k, cudaStream_t stream);
+/* C[M,F] = silu(A * W[0:F]^T) * (A * W[F:2F]^T), W bf16 [2 F, K]: an MLP's gate / up projection with its
+ * activation in the epilogue (fp32 accumulators, one rounding). */
+ncclResult_t amemGemmSwiGLU(const void* A, const void* W, void* C, int M, int F, int K, cudaStream_t stream);
+/* act[r,c] = silu(gate[r,c]) * up[r,c] in bf16, and its gradients; gate, up and their gradients have rows
+ * ld elements apart, act and g_act are contiguous; F and ld multiples of 8. */
+ncclResult_t amemSwiGLU(const void* gate, const void* up, long long ld, void* act, long long rows, int F, cudaStream_t stream);
+ncclResult_t amemSwiGLUGrad(const void* gate, const void* up, long long ld, const void* g_act, void* g_gate, void* g_up, long long rows, int F,
+                            cudaStream_t stream);
+/* One AdamW update of n parameters in one pass: fp32 gradient, moments and master weights, bf16 copy of the
+ * new weights; step counts from 1. */
+ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,
+                       double eps, double weight_decay, long long step, cudaStream_t stream);
 /* The tiling of the one-SM form of the GEMM (the fused all-gather GEMM's) for a GPU with `sms` SMs: tile
  * rows (128 or 256), tile columns, K-slices of the last wave (1 = not split).  Host arithmetic only;
  * outputs may be NULL. */

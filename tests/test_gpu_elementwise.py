@@ -1,0 +1,74 @@
+"""The element-wise kernels and the fused gate / up projection against plain torch in fp32 / fp64."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(shape, seed, scale=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, device="cuda", generator=g) * scale).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("rows,f", [(1, 8), (3, 24), (257, 1000), (70, 14336), (0, 64)])
+def test_swiglu_and_its_gradient(rows, f):
+    from asystem_amem_b200.ops import swiglu
+    h = _rand((rows, 2 * f), 1, 3.0)
+    if rows > 2:
+        h[1, 0], h[1, f], h[2, 1] = 80.0, -80.0, -80.0
+    g = _rand((rows, f), 2)
+    a = h.clone().requires_grad_(True)
+    out = swiglu(a)
+    out.backward(g)
+    b = h.double().requires_grad_(True)
+    ref = F.silu(b[:, :f]) * b[:, f:]
+    ref.backward(g.double())
+    # one rounding to bf16 (8 significant bits: at most 2^-8 of the value) of a value computed in fp32, where
+    # 1 + gate * (1 - sigmoid) loses at most 9 of 22 bits next to its zero (bf16 gates stay 0.0028 away)
+    for x, y in ((out, ref), (a.grad, b.grad)):
+        assert torch.all((x.double() - y).abs() <= y.abs() * (2.0 ** -8 + 2.0 ** -12) + 1e-30)
+    assert torch.equal(swiglu(h), out)
+
+
+# rows of both kernels' tiles, features that end inside a 32-column chunk, products cut along K
+@pytest.mark.parametrize("M,f,K", [(1, 8, 64), (16, 64, 1000), (64, 1000, 4096), (65, 104, 72), (129, 264, 4096), (257, 1000, 264), (500, 200, 8192)])
+def test_gate_up_projection(M, f, K):
+    from asystem_amem_b200.ops import gemm_swiglu
+    x, w = _rand((M, K), 3), _rand((2 * f, K), 4, K ** -0.5)
+    h = x.float() @ w.float().t()
+    ref = F.silu(h[:, :f]) * h[:, f:]
+    for _ in range(2):
+        out = gemm_swiglu(x, w)
+        assert (out.float() - ref).abs().max().item() <= 2.0 ** -8 * ref.abs().max().item() + 1e-6
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 1000, 1_000_003])
+@pytest.mark.parametrize("wd", [0.0, 0.1])
+def test_adamw(n, wd):
+    from asystem_amem_b200.ops import adamw_step
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    master = torch.randn(n, device="cuda", generator=gen)
+    m, v, shard = torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda"), torch.empty(n, device="cuda", dtype=torch.bfloat16)
+    p = torch.nn.Parameter(master.double())
+    opt = torch.optim.AdamW([p], lr=1e-2, betas=(0.9, 0.95), eps=1e-8, weight_decay=wd)
+    for step in range(1, 4):
+        grad = torch.randn(n, device="cuda", generator=gen) * 0.1
+        adamw_step(grad, m, v, master, shard, 1e-2, (0.9, 0.95), 1e-8, wd, step)
+        p.grad = grad.double()
+        opt.step()
+    # three updates of about lr each, every operation to 2^-23
+    assert (master.double() - p.detach()).abs().max().item() <= 3 * (p.detach().abs().max().item() * 2.0 ** -23 + 1e-2 * 2.0 ** -20)
+    assert torch.equal(shard, master.to(torch.bfloat16))
+
+
+def test_adamw_other_layouts_take_the_plain_form():
+    from asystem_amem_b200.ops import adamw_step
+    base = [torch.rand(17, device="cuda") for _ in range(4)]
+    got = [t.clone()[1:] for t in base]       # not 16-byte aligned
+    want = [t.clone()[1:].clone() for t in base]
+    for ts in (got, want):
+        shard = torch.empty(16, device="cuda", dtype=torch.bfloat16)
+        adamw_step(*ts, shard, 1e-3, (0.9, 0.95), 1e-8, 0.0, 1)
+    for a, b in zip(got, want):
+        assert torch.allclose(a, b, rtol=1e-5, atol=1e-7)

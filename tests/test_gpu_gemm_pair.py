@@ -6,8 +6,9 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-# One rounding of the fp32 sum to bf16 is at most 2^-9 of the value, the sum's own error (K <= 8192
-# terms in fp32, any order) far below that: 2^-8 of the largest result covers both.
+# One rounding of the fp32 sum to bf16 (8 significant bits) is at most 2^-8 of the value, less where the
+# value is not just above a power of two; the sum's own error (K <= 8192 terms in fp32, any order) is far
+# below: 2^-8 of the largest result covers both.
 REL = 2.0 ** -8
 
 

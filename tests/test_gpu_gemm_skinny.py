@@ -6,7 +6,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-# one rounding to bf16 (2^-9 of the value) and fp32 sums: see test_gpu_gemm_pair.py
+# one rounding to bf16 and fp32 sums: see test_gpu_gemm_pair.py
 REL = 2.0 ** -8
 
 
