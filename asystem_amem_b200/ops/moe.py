@@ -93,6 +93,45 @@ class MoeDispatcher:
                                              self.d, self.E, self.capacity, self.comm._h, st), "amemMoeCombine")
         return out
 
+    # ---- one rank: the same steps between tensors, without the communicator's buffers ----------
+    def local(self, *bf16: torch.Tensor) -> bool:
+        """Whether the one-rank forms below take these [rows, hidden] tensors."""
+        return not self.host and self.comm.nranks == 1 and all(
+            t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[0] > 0 and t.shape[1] == self.d for t in bf16)
+
+    def dispatch_local(self, x: torch.Tensor, topk_idx: torch.Tensor) -> DispatchResult:
+        """``dispatch`` whose rows land in a tensor of their own."""
+        topk_idx = topk_idx.to(torch.int32).contiguous()
+        T, k = topk_idx.shape
+        rows = min(self.capacity, T * k)
+        recv = torch.empty(rows, self.d, dtype=torch.bfloat16, device=x.device)
+        counts = torch.empty(self.E, dtype=torch.int32, device=x.device)
+        offsets = torch.empty(self.E + 1, dtype=torch.int32, device=x.device)
+        send_pos = torch.empty(T, k, dtype=torch.int32, device=x.device)
+        dropped = torch.empty(1, dtype=torch.int32, device=x.device)
+        B.check(self.comm.lib.amemMoeDispatchLocal(x.data_ptr(), topk_idx.data_ptr(), T, k, self.d, self.E, recv.data_ptr(), rows, counts.data_ptr(),
+                                                   offsets.data_ptr(), send_pos.data_ptr(), dropped.data_ptr(), self.comm._h,
+                                                   torch.cuda.current_stream().cuda_stream), "amemMoeDispatchLocal")
+        return DispatchResult(recv, counts, offsets, send_pos, dropped)
+
+    def combine_local(self, y: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.Tensor, send_pos: torch.Tensor) -> torch.Tensor:
+        """``combine`` of the expert outputs ``y``."""
+        y, idx, w, pos = y.contiguous(), topk_idx.to(torch.int32).contiguous(), topk_w.to(torch.float32).contiguous(), send_pos.contiguous()
+        T, k = idx.shape
+        out = torch.empty(T, self.d, dtype=torch.bfloat16, device=y.device)
+        B.check(self.comm.lib.amemMoeCombineLocal(idx.data_ptr(), w.data_ptr(), pos.data_ptr(), y.data_ptr(), y.shape[0], out.data_ptr(), T, k, self.d, self.E,
+                                                  self.comm._h, torch.cuda.current_stream().cuda_stream), "amemMoeCombineLocal")
+        return out
+
+    def combine_grad_local(self, g_out: torch.Tensor, y: torch.Tensor, topk_w: torch.Tensor, send_pos: torch.Tensor):
+        """Gradients of ``combine_local``: (of ``y``, bf16; of the weights, fp32)."""
+        g_out, y, w, pos = g_out.contiguous(), y.contiguous(), topk_w.to(torch.float32).contiguous(), send_pos.contiguous()
+        T, k = w.shape
+        g_y, g_w = torch.empty_like(y), torch.empty(T, k, dtype=torch.float32, device=y.device)
+        B.check(self.comm.lib.amemMoeCombineGradLocal(g_out.data_ptr(), y.data_ptr(), w.data_ptr(), pos.data_ptr(), g_y.data_ptr(), g_w.data_ptr(), y.shape[0],
+                                                      T, k, self.d, self.comm._h, torch.cuda.current_stream().cuda_stream), "amemMoeCombineGradLocal")
+        return g_y, g_w
+
     # ---- host form (mock backend): same row layout as the kernels, built from the library's
     # all-gather and variable-size all-to-all, so that the expert-parallel wrappers and their
     # gradients can be tested as real multi-process runs without a GPU ------------------------

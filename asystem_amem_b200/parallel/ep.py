@@ -17,6 +17,9 @@ runs on the same two kernels and needs no new device code:
   tokens: a combine of the ``[T * k, 1]`` problem with unit weights is that gather.
 * d rows / d x : ``g_x[t] = sum_c g_rows[pos(t, c)]`` is a combine with unit weights.
 
+On one rank nothing has to travel: the steps then run between the caller's tensors, and the backward of
+the combine is one kernel (``MoeDispatcher.combine_grad_local``).
+
 The four steps are plain functions (``dispatch_forward`` ... ``combine_backward``) so that a
 caller which schedules its own backward pass -- or a test that runs several ranks as threads of
 one process, where the autograd engine's single per-device thread could not run the ranks'
@@ -37,19 +40,24 @@ from ..ops.moe import DispatchResult, MoeDispatcher  # noqa: F401
 def dispatch_forward(disp: MoeDispatcher, x: torch.Tensor, idx: torch.Tensor):
     """Returns (rows, expert_offsets, send_pos, total): ``rows`` is a private copy of the
     received rows (the receive buffer is reused by the next dispatch)."""
-    res = disp.dispatch(x.contiguous(), idx)
+    res = disp.dispatch_local(x.contiguous(), idx) if disp.local(x) else disp.dispatch(x.contiguous(), idx)
     total = int(res.expert_offsets[-1].item())  # host sync: the group boundaries are needed on the host anyway
-    return res.recv_x[:total].clone(), res.expert_offsets, res.send_pos, total
+    rows = res.recv_x[:total]
+    return rows if disp.local(x) else rows.clone(), res.expert_offsets, res.send_pos, total
 
 
 def dispatch_backward(disp: MoeDispatcher, g_rows: torch.Tensor, idx: torch.Tensor, send_pos: torch.Tensor) -> torch.Tensor:
     T, k = idx.shape
-    disp.y[: g_rows.shape[0]] = g_rows.to(torch.bfloat16)
     ones = torch.ones(T, k, dtype=torch.float32, device=g_rows.device)
+    if disp.local(g_rows):
+        return disp.combine_local(g_rows, idx, ones, send_pos)
+    disp.y[: g_rows.shape[0]] = g_rows.to(torch.bfloat16)
     return disp.combine(idx, ones, send_pos)
 
 
 def combine_forward(disp: MoeDispatcher, y_rows: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, send_pos: torch.Tensor) -> torch.Tensor:
+    if disp.local(y_rows):
+        return disp.combine_local(y_rows, idx, w, send_pos)
     disp.y[: y_rows.shape[0]] = y_rows.to(torch.bfloat16)
     return disp.combine(idx, w, send_pos)
 
@@ -57,6 +65,8 @@ def combine_forward(disp: MoeDispatcher, y_rows: torch.Tensor, idx: torch.Tensor
 def combine_backward(disp: MoeDispatcher, g_out: torch.Tensor, y_rows: torch.Tensor, idx: torch.Tensor, w: torch.Tensor,
                      send_pos: torch.Tensor):
     """Returns (g_y_rows, g_w)."""
+    if disp.local(g_out, y_rows):
+        return disp.combine_grad_local(g_out, y_rows, w, send_pos)
     T, k = idx.shape
     d = g_out.shape[1]
     flat_idx = idx.reshape(T * k, 1)

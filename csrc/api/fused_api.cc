@@ -632,6 +632,20 @@ ncclResult_t amemMoeBuffers(ncclComm_t comm, int capacity_rows, int d, void** re
   return ncclSuccess;
 }
 
+// small per-communicator work area: tracked scratch of the communicator (every word of it is
+// rewritten by each dispatch before it is read, so nothing has to survive a pause)
+static Status moe_work_area(Comm* c, MoeArgs* a) {
+  void* wp = nullptr;
+  size_t ints = (size_t)kMoeSegments * kMoeMaxExperts * 2 + kMoeMaxExperts + 64;
+  AMEM_TRY(c->local_scratch(0, ints * sizeof(int), &wp));
+  int* w = (int*)wp;
+  a->seg_hist = w;
+  a->seg_base = w + (size_t)kMoeSegments * kMoeMaxExperts;
+  a->send_off = w + (size_t)kMoeSegments * kMoeMaxExperts * 2;
+  a->dropped_rows = w + (size_t)kMoeSegments * kMoeMaxExperts * 2 + kMoeMaxExperts;
+  return kSuccess;
+}
+
 static Status moe_args(Comm* c, int T, int k, int d, int E, int capacity_rows, MoeArgs* a) {
   if (T < 0 || k <= 0 || d <= 0 || d % 8 || E <= 0 || E > kMoeMaxExperts || E % c->nranks())
     return fail(kInvalidArgument, "MoE shape: T=%d k=%d d=%d (multiple of 8) E=%d (<= %d, divisible by %d ranks)", T, k, d, E, kMoeMaxExperts, c->nranks());
@@ -651,17 +665,7 @@ static Status moe_args(Comm* c, int T, int k, int d, int E, int capacity_rows, M
     a->recv[r] = (char*)rx->va[r];
     a->ybuf[r] = (char*)yb->va[r];
   }
-  // small per-communicator work area: tracked scratch of the communicator (every word of it is
-  // rewritten by each dispatch before it is read, so nothing has to survive a pause)
-  void* wp = nullptr;
-  size_t ints = (size_t)kMoeSegments * kMoeMaxExperts * 2 + kMoeMaxExperts + 64;
-  AMEM_TRY(c->local_scratch(0, ints * sizeof(int), &wp));
-  int* w = (int*)wp;
-  a->seg_hist = w;
-  a->seg_base = w + (size_t)kMoeSegments * kMoeMaxExperts;
-  a->send_off = w + (size_t)kMoeSegments * kMoeMaxExperts * 2;
-  a->dropped_rows = w + (size_t)kMoeSegments * kMoeMaxExperts * 2 + kMoeMaxExperts;
-  return kSuccess;
+  return moe_work_area(c, a);
 }
 
 // Routes this rank's T tokens to their experts' ranks.  On return (stream order) this rank's
@@ -702,6 +706,64 @@ ncclResult_t amemMoeDispatchCounted(const void* x, const int* topk_idx, int T, i
     }));
   }
   return R(launch_moe_dispatch(a, stream));
+}
+
+// ---- the same steps on a communicator of one rank, between the caller's own buffers ----------------
+static Status moe_local(ncclComm_t comm, const char* what, int T, int k, int d, int E, int rows, cudaStream_t stream, MoeArgs* a) {
+  if (!comm) return fail(kInvalidArgument, "%s: null communicator", what);
+  Comm* c = reinterpret_cast<Comm*>(comm);
+  AMEM_TRY(c->check_usable(what));
+  if (c->nranks() != 1) return fail(kInvalidUsage, "%s needs a communicator of one rank, this one has %d", what, c->nranks());
+  if (T < 0 || k <= 0 || d <= 0 || d % 8 || E <= 0 || E > kMoeMaxExperts || rows <= 0)
+    return fail(kInvalidArgument, "%s: T=%d k=%d d=%d (multiple of 8) E=%d (<= %d) rows=%d", what, T, k, d, E, kMoeMaxExperts, rows);
+  memset(a, 0, sizeof(*a));
+  c->fill_args(&a->coll);
+  a->T = T;
+  a->k = k;
+  a->d = d;
+  a->E = E;
+  a->capacity_rows = rows;
+  AMEM_TRY(moe_work_area(c, a));
+  return c->prepare_stream(stream);
+}
+
+// amemMoeDispatch into recv, bf16 [capacity_rows, d] of the caller's.
+ncclResult_t amemMoeDispatchLocal(const void* x, const int* topk_idx, int T, int k, int d, int E, void* recv, int capacity_rows, int* expert_counts,
+                                  int* expert_offsets, int* send_pos, int* dropped_rows, ncclComm_t comm, cudaStream_t stream) {
+  MoeArgs a;
+  Status s = moe_local(comm, "amemMoeDispatchLocal", T, k, d, E, capacity_rows, stream, &a);
+  if (s != kSuccess) return R(s);
+  a.x = x;
+  a.topk_idx = topk_idx;
+  a.recv[0] = (char*)recv;
+  a.expert_counts = expert_counts;
+  a.expert_offsets = expert_offsets;
+  a.send_pos = send_pos;
+  if (dropped_rows) a.dropped_rows = dropped_rows;
+  return R(launch_moe_dispatch(a, stream));
+}
+
+// amemMoeCombine from y, bf16 [rows, d] of the caller's.
+ncclResult_t amemMoeCombineLocal(const int* topk_idx, const float* topk_w, const int* send_pos, const void* y, int rows, void* out, int T, int k, int d, int E,
+                                 ncclComm_t comm, cudaStream_t stream) {
+  MoeArgs a;
+  Status s = moe_local(comm, "amemMoeCombineLocal", T, k, d, E, rows, stream, &a);
+  if (s != kSuccess) return R(s);
+  a.topk_idx = topk_idx;
+  a.topk_w = topk_w;
+  a.send_pos = const_cast<int*>(send_pos);
+  a.ybuf[0] = (char*)y;
+  a.out = out;
+  return R(launch_moe_combine(a, stream));
+}
+
+// Its backward: g_y[row(t, j)] = topk_w[t, j] * g_out[t] (bf16) and g_w[t, j] = <g_out[t], y[row(t, j)]> (fp32).
+ncclResult_t amemMoeCombineGradLocal(const void* g_out, const void* y, const float* topk_w, const int* send_pos, void* g_y, float* g_w, int rows, int T, int k,
+                                     int d, ncclComm_t comm, cudaStream_t stream) {
+  MoeArgs a;
+  Status s = moe_local(comm, "amemMoeCombineGradLocal", T, k, d, 1, rows, stream, &a);
+  if (s != kSuccess) return R(s);
+  return R(launch_moe_combine_grad(g_out, y, topk_w, send_pos, g_y, g_w, rows, T, k, d, stream));
 }
 
 // out[T, d] = sum_j topk_w[t, j] * (expert output row of (t, j)), read from the expert ranks'

@@ -266,6 +266,14 @@ ncclResult_t amemGemmReduceScatter(const void* A, const void* B, void* out, int 
  * expert-sorted position (the permutation is fused into the all-to-all); amemMoeCombine pulls
  * the expert outputs back and applies the routing weights in one pass. */
 ncclResult_t amemMoeBuffers(ncclComm_t comm, int capacity_rows, int d, void** recv_x, void** y);
+/* The same on a communicator of one rank between the caller's own buffers, and the combine's backward:
+ * g_y[row(t, j)] = topk_w[t, j] * g_out[t] (bf16), g_w[t, j] = <g_out[t], y[row(t, j)]> (fp32). */
+ncclResult_t amemMoeDispatchLocal(const void* x, const int* topk_idx, int T, int k, int d, int E, void* recv, int capacity_rows, int* expert_counts,
+                                  int* expert_offsets, int* send_pos, int* dropped_rows, ncclComm_t comm, cudaStream_t stream);
+ncclResult_t amemMoeCombineLocal(const int* topk_idx, const float* topk_w, const int* send_pos, const void* y, int rows, void* out, int T, int k, int d, int E,
+                                 ncclComm_t comm, cudaStream_t stream);
+ncclResult_t amemMoeCombineGradLocal(const void* g_out, const void* y, const float* topk_w, const int* send_pos, void* g_y, float* g_w, int rows, int T, int k,
+                                     int d, ncclComm_t comm, cudaStream_t stream);
 ncclResult_t amemMoeDispatch(const void* x, const int* topk_idx, int T, int k, int d, int E, int capacity_rows, int* expert_counts,
                              int* expert_offsets, int* send_pos, ncclComm_t comm, cudaStream_t stream);
 /* The same with one more output: *dropped_rows (device int, may be null) = rows routed to this rank

@@ -57,3 +57,24 @@ def test_dispatch_and_combine(comm, T, k, E, d, room):
         size += y.abs()
     # the sum's own rounding (k fp32 additions) and one rounding to bf16
     assert torch.all((out.double() - ref).abs() <= size * (k + 1) * 2.0 ** -24 + ref.abs() * 2.0 ** -8 + 1e-30)
+
+    # the same steps between tensors, and the combine's backward
+    if valid.any():
+        own = disp.dispatch_local(x, idx.cuda())
+        torch.cuda.synchronize()
+        assert torch.equal(own.send_pos, res.send_pos) and torch.equal(own.expert_offsets, res.expert_offsets) and torch.equal(own.dropped, res.dropped)
+        assert torch.equal(own.recv_x[: kept.numel()], res.recv_x[: kept.numel()])
+        y = disp.y[: kept.numel()].clone()
+        assert torch.equal(disp.combine_local(y, idx.cuda(), w, own.send_pos), out)
+        g_out = torch.randn(T, d, generator=g).to(torch.bfloat16).cuda()
+        g_y, g_w = disp.combine_grad_local(g_out, y, w, own.send_pos)
+        p = pos.cuda().clamp(min=0)
+        hit = (pos >= 0).cuda()
+        tok = torch.arange(T * k, device="cuda") // k
+        dots, sizes = torch.zeros(T * k, device="cuda", dtype=torch.float64), torch.zeros(T * k, device="cuda", dtype=torch.float64)
+        for lo in range(0, T * k, 8192):
+            s = slice(lo, lo + 8192)
+            prod = g_out[tok[s]].double() * y[p[s]].double()
+            dots[s], sizes[s] = prod.sum(1) * hit[s], prod.abs().sum(1)
+        assert torch.all((g_w.reshape(-1).double() - dots).abs() <= sizes * (d / 128 + 16) * 2.0 ** -24 + 1e-30)
+        assert torch.equal(g_y[p[hit]], (g_out[tok[hit]].float() * w.reshape(-1)[hit].unsqueeze(1)).to(torch.bfloat16))
