@@ -25,9 +25,11 @@ class TPMLP(nn.Module):
 
     def forward(self, x_shard: torch.Tensor) -> torch.Tensor:
         """x_shard: bf16 [tokens / tp, dim] -> bf16 [tokens / tp, dim]"""
-        w = self.w13.weight
-        if (self.comm.nranks == 1 and x_shard.is_cuda and self.ffn_local % 8 == 0 and not (torch.is_grad_enabled() and (x_shard.requires_grad or w.requires_grad))
-                and not self.w13._forward_hooks and not self.w13._forward_pre_hooks):
-            # one rank, no gradients: the activation rides in the projection's epilogue
+        plain = type(self.w13) is ColumnParallelLinear and "forward" not in self.w13.__dict__ and not self.w13._forward_hooks and not self.w13._forward_pre_hooks
+        w = self.w13.weight if plain else None
+        if (plain and self.comm.nranks == 1 and x_shard.is_cuda and self.ffn_local % 8 == 0
+                and not (torch.is_grad_enabled() and (x_shard.requires_grad or w.requires_grad))):
+            # one rank, no gradients: the activation rides in the projection's epilogue (a projection that a
+            # program wrapped, hooked or replaced is called as the module that it is)
             return self.w2(gemm_swiglu(x_shard.contiguous(), w.contiguous()))
         return self.w2(swiglu(self.w13(x_shard)).to(torch.bfloat16))

@@ -57,7 +57,8 @@ def adamw_step(grad, m, v, master, shard, lr: float, betas, eps: float, weight_d
     if all(t.is_cuda and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in flat) and shard.dtype == torch.bfloat16 \
             and all(t.dtype == torch.float32 for t in flat[:4]):
         B.check(B.load_library().amemAdamW(grad.data_ptr(), m.data_ptr(), v.data_ptr(), master.data_ptr(), shard.data_ptr(), grad.numel(),
-                                           lr, betas[0], betas[1], eps, weight_decay, step, _st()), "amemAdamW")
+                                           float(lr), float(betas[0]), float(betas[1]), float(eps), float(weight_decay), step, _st()), "amemAdamW")
+        torch.autograd.graph.increment_version([t for t in flat[1:] if not t.is_inference()])   # as an in-place operator does
         return
     b1, b2 = betas
     c1, c2 = 1 - b1 ** step, 1 - b2 ** step

@@ -62,6 +62,41 @@ def test_adamw(n, wd):
     assert torch.equal(shard, master.to(torch.bfloat16))
 
 
+def test_adamw_takes_a_rate_in_a_tensor_and_counts_as_an_in_place_update():
+    from asystem_amem_b200.ops import adamw_step
+    got, want = ([torch.full((8,), 0.5, device="cuda") for _ in range(4)] + [torch.empty(8, device="cuda", dtype=torch.bfloat16)] for _ in range(2))
+    versions = [t._version for t in got]
+    adamw_step(*got, torch.tensor(1e-2), (0.9, 0.95), 1e-8, 0.1, 1)
+    adamw_step(*want, 1e-2, (0.9, 0.95), 1e-8, 0.1, 1)
+    # the rate passed through fp32: 2^-24 of it
+    assert all(torch.allclose(a, b, rtol=2.0 ** -22, atol=0) for a, b in zip(got[:4], want[:4]))
+    assert got[0]._version == versions[0] and all(t._version > n for t, n in zip(got[1:], versions[1:]))
+
+
+def test_a_replaced_projection_is_called():
+    from asystem_amem_b200 import Communicator, get_unique_id
+    from asystem_amem_b200.models import TPMLP
+    from asystem_amem_b200.parallel.tp import ColumnParallelLinear
+
+    class Doubled(ColumnParallelLinear):
+        def forward(self, x):
+            return 2 * super().forward(x)
+
+    comm = Communicator(1, 0, get_unique_id())
+    layer, x = TPMLP(comm, 128, 256), _rand((16, 128), 5)
+    with torch.no_grad():
+        own = Doubled(128, 512, comm)
+        own.weight.copy_(layer.w13.weight)
+        layer.w13 = own
+        out = layer(x)
+        h = 2 * (x.float() @ own.weight.float().t())
+        ref = (F.silu(h[:, :256]) * h[:, 256:]) @ layer.w2.weight.float().t()
+    # bf16 roundings of h, the activation and the result: a few of 2^-9 each, against the largest result
+    assert (out.float() - ref).abs().max().item() <= 2.0 ** -6 * ref.abs().max().item()
+    torch.cuda.synchronize()
+    comm.destroy()
+
+
 def test_adamw_other_layouts_take_the_plain_form():
     from asystem_amem_b200.ops import adamw_step
     base = [torch.rand(17, device="cuda") for _ in range(4)]
