@@ -23,6 +23,14 @@ def _check(a: torch.Tensor, b: torch.Tensor) -> None:
         raise ValueError(f"inner dimensions differ: {tuple(a.shape)} vs {tuple(b.shape)}")
 
 
+def _matrices(a: torch.Tensor, b: torch.Tensor, inner_a: int, inner_b: int) -> None:
+    """Both operands are matrices and agree in the dimension that the product sums over."""
+    if a.dim() != 2 or b.dim() != 2:
+        raise ValueError(f"matrices expected, got {tuple(a.shape)} and {tuple(b.shape)}")
+    if a.shape[inner_a] != b.shape[inner_b]:
+        raise ValueError(f"inner dimensions differ: {tuple(a.shape)} vs {tuple(b.shape)}")
+
+
 def _on_host(a: torch.Tensor, b: torch.Tensor) -> bool:
     """Host tensors (mock backend, no GPU): the operation is composed from the library's
     collective and a PyTorch matmul with fp32 accumulation, so that the parallel wrappers can be
@@ -55,6 +63,9 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
 
 def gemm_swiglu(a: torch.Tensor, w13: torch.Tensor, stream=None) -> torch.Tensor:
     """silu(a @ gate.T) * (a @ up.T) in one pass on one GPU: ``w13`` [2 f, K] holds the gate's rows first."""
+    _matrices(a, w13, 1, 1)
+    if w13.shape[0] % 2:
+        raise ValueError(f"as many gate rows as up rows expected, got {w13.shape[0]} in all")
     f = w13.shape[0] // 2
     if _on_host(a, w13):
         h = _host_matmul(a, w13)
@@ -79,6 +90,7 @@ def _by_k(a: torch.Tensor, b: torch.Tensor, m: int, n: int, k: int, a_by_k: bool
 
 def gemm_input_grad(gy: torch.Tensor, w: torch.Tensor, stream=None) -> torch.Tensor:
     """gy[M, N] @ w[N, K] on one GPU: the input gradient of :func:`gemm_bf16`, from the weight as it lies."""
+    _matrices(gy, w, 1, 0)
     if _on_host(gy, w):
         return (gy.float() @ w.float()).to(gy.dtype)
     return _by_k(gy, w, gy.shape[0], w.shape[1], w.shape[0], False, stream)
@@ -86,6 +98,7 @@ def gemm_input_grad(gy: torch.Tensor, w: torch.Tensor, stream=None) -> torch.Ten
 
 def gemm_weight_grad(gy: torch.Tensor, x: torch.Tensor, stream=None) -> torch.Tensor:
     """gy[T, N].T @ x[T, K] on one GPU: the weight gradient of :func:`gemm_bf16`, any number of rows T."""
+    _matrices(gy, x, 0, 0)
     if _on_host(gy, x):
         return gy.t() @ x
     return _by_k(gy, x, gy.shape[1], x.shape[1], gy.shape[0], True, stream)
@@ -150,6 +163,10 @@ def grouped_gemm_input_grad(g: torch.Tensor, w: torch.Tensor, offsets: torch.Ten
     """For every group e: out[rows of e] = g[rows of e] @ w[e] with ``w`` bf16 [groups, N, K] as it is
     stored for :func:`grouped_gemm_bf16`.  Rows outside every group are left untouched."""
     groups, N, K = w.shape
+    if g.dim() != 2 or g.shape[1] != N:
+        raise ValueError(f"shapes do not fit: g {tuple(g.shape)}, w {tuple(w.shape)}")
+    if out is not None and out.shape != (g.shape[0], K):
+        raise ValueError(f"shapes do not fit: g {tuple(g.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     if not g.is_cuda:
         offs = offsets.tolist()
         res = torch.zeros(g.shape[0], K, dtype=g.dtype) if out is None else out
@@ -158,8 +175,6 @@ def grouped_gemm_input_grad(g: torch.Tensor, w: torch.Tensor, offsets: torch.Ten
         return res
     out = torch.empty(g.shape[0], K, dtype=torch.bfloat16, device=g.device) if out is None else out
     _check_grouped(g, w, offsets, groups)
-    if g.shape[1] != N:
-        raise ValueError(f"shapes do not fit: g {tuple(g.shape)}, w {tuple(w.shape)}")
     B.check(B.load_library().amemGroupedGemmBf16Input(g.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
                                                       int(rows_hint or 0), N, K, _stream(stream)), "amemGroupedGemmBf16Input")
     return out
@@ -168,13 +183,12 @@ def grouped_gemm_input_grad(g: torch.Tensor, w: torch.Tensor, offsets: torch.Ten
 def grouped_gemm_weight_grad(g: torch.Tensor, a: torch.Tensor, offsets: torch.Tensor, stream=None) -> torch.Tensor:
     """bf16 [groups, N, K]: for every group e, g[rows of e].T @ a[rows of e] (zeros without rows).  The
     group boundaries are read on the device."""
+    _matrices(g, a, 0, 0)
     groups, N, K = offsets.numel() - 1, g.shape[1], a.shape[1]
     if not g.is_cuda:
         offs = offsets.tolist()
         return torch.stack([g[offs[e]:offs[e + 1]].t() @ a[offs[e]:offs[e + 1]] for e in range(groups)])
     _check_grouped(g, a, offsets, groups)
-    if g.shape[0] != a.shape[0]:
-        raise ValueError(f"shapes do not fit: g {tuple(g.shape)}, a {tuple(a.shape)}")
     out = torch.empty(groups, N, K, dtype=torch.bfloat16, device=g.device)
     B.check(B.load_library().amemGroupedGemmBf16Weight(g.data_ptr(), a.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
                                                        N, K, _stream(stream)), "amemGroupedGemmBf16Weight")
