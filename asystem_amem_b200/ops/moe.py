@@ -21,6 +21,7 @@ from dataclasses import dataclass
 import torch
 
 from .. import bindings as B
+from .operands import dense
 
 
 def _view(ptr: int, rows: int, d: int, device) -> torch.Tensor:
@@ -66,6 +67,8 @@ class MoeDispatcher:
         topk_idx = topk_idx.to(torch.int32).contiguous()
         if self.host:
             return self._host_dispatch(x, topk_idx)
+        with torch.cuda.stream(stream):     # (None: the current one)
+            x = dense(x)
         T, k = topk_idx.shape
         counts = torch.empty(self.experts_per_rank, dtype=torch.int32, device=x.device)
         offsets = torch.empty(self.experts_per_rank + 1, dtype=torch.int32, device=x.device)
@@ -101,7 +104,7 @@ class MoeDispatcher:
 
     def dispatch_local(self, x: torch.Tensor, topk_idx: torch.Tensor) -> DispatchResult:
         """``dispatch`` whose rows land in a tensor of their own."""
-        topk_idx = topk_idx.to(torch.int32).contiguous()
+        x, topk_idx = dense(x), topk_idx.to(torch.int32).contiguous()
         T, k = topk_idx.shape
         rows = min(self.capacity, T * k)
         recv = torch.empty(rows, self.d, dtype=torch.bfloat16, device=x.device)
@@ -116,7 +119,7 @@ class MoeDispatcher:
 
     def combine_local(self, y: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.Tensor, send_pos: torch.Tensor) -> torch.Tensor:
         """``combine`` of the expert outputs ``y``."""
-        y, idx, w, pos = y.contiguous(), topk_idx.to(torch.int32).contiguous(), topk_w.to(torch.float32).contiguous(), send_pos.contiguous()
+        y, idx, w, pos = dense(y), topk_idx.to(torch.int32).contiguous(), topk_w.to(torch.float32).contiguous(), send_pos.contiguous()
         T, k = idx.shape
         out = torch.empty(T, self.d, dtype=torch.bfloat16, device=y.device)
         B.check(self.comm.lib.amemMoeCombineLocal(idx.data_ptr(), w.data_ptr(), pos.data_ptr(), y.data_ptr(), y.shape[0], out.data_ptr(), T, k, self.d, self.E,
@@ -125,7 +128,7 @@ class MoeDispatcher:
 
     def combine_grad_local(self, g_out: torch.Tensor, y: torch.Tensor, topk_w: torch.Tensor, send_pos: torch.Tensor):
         """Gradients of ``combine_local``: (of ``y``, bf16; of the weights, fp32)."""
-        g_out, y, w, pos = g_out.contiguous(), y.contiguous(), topk_w.to(torch.float32).contiguous(), send_pos.contiguous()
+        g_out, y, w, pos = dense(g_out), dense(y), topk_w.to(torch.float32).contiguous(), send_pos.contiguous()
         T, k = w.shape
         g_y, g_w = torch.empty_like(y), torch.empty(T, k, dtype=torch.float32, device=y.device)
         B.check(self.comm.lib.amemMoeCombineGradLocal(g_out.data_ptr(), y.data_ptr(), w.data_ptr(), pos.data_ptr(), g_y.data_ptr(), g_w.data_ptr(), y.shape[0],

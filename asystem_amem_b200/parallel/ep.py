@@ -37,26 +37,33 @@ import torch
 from ..ops.moe import DispatchResult, MoeDispatcher  # noqa: F401
 
 
+def _between_tensors(disp: MoeDispatcher, rows: torch.Tensor) -> bool:
+    """Whether a one-rank step reads ``rows`` where they are; more of them than the dispatcher's buffers
+    hold are left to the general form, which refuses them."""
+    return disp.local(rows) and rows.shape[0] <= disp.capacity
+
+
 def dispatch_forward(disp: MoeDispatcher, x: torch.Tensor, idx: torch.Tensor):
     """Returns (rows, expert_offsets, send_pos, total): ``rows`` is a private copy of the
     received rows (the receive buffer is reused by the next dispatch)."""
-    res = disp.dispatch_local(x.contiguous(), idx) if disp.local(x) else disp.dispatch(x.contiguous(), idx)
+    local = disp.local(x) and x.shape[0] == idx.shape[0]
+    res = disp.dispatch_local(x.contiguous(), idx) if local else disp.dispatch(x.contiguous(), idx)
     total = int(res.expert_offsets[-1].item())  # host sync: the group boundaries are needed on the host anyway
     rows = res.recv_x[:total]
-    return rows if disp.local(x) else rows.clone(), res.expert_offsets, res.send_pos, total
+    return rows if local else rows.clone(), res.expert_offsets, res.send_pos, total
 
 
 def dispatch_backward(disp: MoeDispatcher, g_rows: torch.Tensor, idx: torch.Tensor, send_pos: torch.Tensor) -> torch.Tensor:
     T, k = idx.shape
     ones = torch.ones(T, k, dtype=torch.float32, device=g_rows.device)
-    if disp.local(g_rows):
+    if _between_tensors(disp, g_rows):
         return disp.combine_local(g_rows, idx, ones, send_pos)
     disp.y[: g_rows.shape[0]] = g_rows.to(torch.bfloat16)
     return disp.combine(idx, ones, send_pos)
 
 
 def combine_forward(disp: MoeDispatcher, y_rows: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, send_pos: torch.Tensor) -> torch.Tensor:
-    if disp.local(y_rows):
+    if _between_tensors(disp, y_rows):
         return disp.combine_local(y_rows, idx, w, send_pos)
     disp.y[: y_rows.shape[0]] = y_rows.to(torch.bfloat16)
     return disp.combine(idx, w, send_pos)
@@ -65,7 +72,7 @@ def combine_forward(disp: MoeDispatcher, y_rows: torch.Tensor, idx: torch.Tensor
 def combine_backward(disp: MoeDispatcher, g_out: torch.Tensor, y_rows: torch.Tensor, idx: torch.Tensor, w: torch.Tensor,
                      send_pos: torch.Tensor):
     """Returns (g_y_rows, g_w)."""
-    if disp.local(g_out, y_rows):
+    if disp.local(g_out) and _between_tensors(disp, y_rows) and w.shape == idx.shape and g_out.shape[0] == idx.shape[0]:
         return disp.combine_grad_local(g_out, y_rows, w, send_pos)
     T, k = idx.shape
     d = g_out.shape[1]

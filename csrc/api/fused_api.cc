@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -632,6 +633,12 @@ ncclResult_t amemMoeBuffers(ncclComm_t comm, int capacity_rows, int d, void** re
   return ncclSuccess;
 }
 
+// The MoE kernels move rows as 16-byte vectors: every row buffer starts on 16 bytes (d is a multiple of 8).
+static Status moe_aligned(const char* what, const void* a, const void* b = nullptr, const void* c = nullptr) {
+  if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) return fail(kInvalidArgument, "%s: row buffers must be 16-byte aligned", what);
+  return kSuccess;
+}
+
 // small per-communicator work area: tracked scratch of the communicator (every word of it is
 // rewritten by each dispatch before it is read, so nothing has to survive a pause)
 static Status moe_work_area(Comm* c, MoeArgs* a) {
@@ -691,6 +698,7 @@ ncclResult_t amemMoeDispatchCounted(const void* x, const int* topk_idx, int T, i
   Status s = c->check_usable("amemMoeDispatch");
   if (s != kSuccess) return R(s);
   MoeArgs a;
+  if ((s = moe_aligned("amemMoeDispatch", x)) != kSuccess) return R(s);
   if ((s = moe_args(c, T, k, d, E, capacity_rows, &a)) != kSuccess) return R(s);
   if ((s = c->prepare_stream(stream)) != kSuccess) return R(s);
   a.x = x;
@@ -709,8 +717,16 @@ ncclResult_t amemMoeDispatchCounted(const void* x, const int* topk_idx, int T, i
 }
 
 // ---- the same steps on a communicator of one rank, between the caller's own buffers ----------------
-static Status moe_local(ncclComm_t comm, const char* what, int T, int k, int d, int E, int rows, cudaStream_t stream, MoeArgs* a) {
+static Status moe_local(ncclComm_t comm, const char* what, int T, int k, int d, int E, int rows, std::initializer_list<const void*> row_bufs,
+                        std::initializer_list<const void*> tables, cudaStream_t stream, MoeArgs* a) {
   if (!comm) return fail(kInvalidArgument, "%s: null communicator", what);
+  for (const void* p : row_bufs) AMEM_TRY(moe_aligned(what, p));
+  if (T > 0) {   // (an empty tensor has no address)
+    for (const void* p : row_bufs)
+      if (!p) return fail(kInvalidArgument, "%s: null buffer", what);
+    for (const void* p : tables)
+      if (!p) return fail(kInvalidArgument, "%s: null buffer", what);
+  }
   Comm* c = reinterpret_cast<Comm*>(comm);
   AMEM_TRY(c->check_usable(what));
   if (c->nranks() != 1) return fail(kInvalidUsage, "%s needs a communicator of one rank, this one has %d", what, c->nranks());
@@ -731,7 +747,7 @@ static Status moe_local(ncclComm_t comm, const char* what, int T, int k, int d, 
 ncclResult_t amemMoeDispatchLocal(const void* x, const int* topk_idx, int T, int k, int d, int E, void* recv, int capacity_rows, int* expert_counts,
                                   int* expert_offsets, int* send_pos, int* dropped_rows, ncclComm_t comm, cudaStream_t stream) {
   MoeArgs a;
-  Status s = moe_local(comm, "amemMoeDispatchLocal", T, k, d, E, capacity_rows, stream, &a);
+  Status s = moe_local(comm, "amemMoeDispatchLocal", T, k, d, E, capacity_rows, {x, recv}, {topk_idx, expert_counts, expert_offsets, send_pos}, stream, &a);
   if (s != kSuccess) return R(s);
   a.x = x;
   a.topk_idx = topk_idx;
@@ -747,7 +763,7 @@ ncclResult_t amemMoeDispatchLocal(const void* x, const int* topk_idx, int T, int
 ncclResult_t amemMoeCombineLocal(const int* topk_idx, const float* topk_w, const int* send_pos, const void* y, int rows, void* out, int T, int k, int d, int E,
                                  ncclComm_t comm, cudaStream_t stream) {
   MoeArgs a;
-  Status s = moe_local(comm, "amemMoeCombineLocal", T, k, d, E, rows, stream, &a);
+  Status s = moe_local(comm, "amemMoeCombineLocal", T, k, d, E, rows, {y, out}, {topk_idx, topk_w, send_pos}, stream, &a);
   if (s != kSuccess) return R(s);
   a.topk_idx = topk_idx;
   a.topk_w = topk_w;
@@ -761,7 +777,7 @@ ncclResult_t amemMoeCombineLocal(const int* topk_idx, const float* topk_w, const
 ncclResult_t amemMoeCombineGradLocal(const void* g_out, const void* y, const float* topk_w, const int* send_pos, void* g_y, float* g_w, int rows, int T, int k,
                                      int d, ncclComm_t comm, cudaStream_t stream) {
   MoeArgs a;
-  Status s = moe_local(comm, "amemMoeCombineGradLocal", T, k, d, 1, rows, stream, &a);
+  Status s = moe_local(comm, "amemMoeCombineGradLocal", T, k, d, 1, rows, {g_out, y, g_y}, {topk_w, send_pos, g_w}, stream, &a);
   if (s != kSuccess) return R(s);
   return R(launch_moe_combine_grad(g_out, y, topk_w, send_pos, g_y, g_w, rows, T, k, d, stream));
 }
@@ -775,6 +791,7 @@ ncclResult_t amemMoeCombine(const int* topk_idx, const float* topk_w, const int*
   Status s = c->check_usable("amemMoeCombine");
   if (s != kSuccess) return R(s);
   MoeArgs a;
+  if ((s = moe_aligned("amemMoeCombine", out)) != kSuccess) return R(s);
   if ((s = moe_args(c, T, k, d, E, capacity_rows, &a)) != kSuccess) return R(s);
   if ((s = c->prepare_stream(stream)) != kSuccess) return R(s);
   a.topk_idx = topk_idx;

@@ -66,6 +66,7 @@ extern "C" int amemMoePermuteNoAlloc(const void* x, const int* topk_idx, int T, 
   if ((long long)T * k > 0x7fffffffLL) return fail(kInvalidArgument, "amemMoePermuteNoAlloc: T*k does not fit 31 bits");
   if (!x || !topk_idx || !recv_x || !expert_counts || !expert_offsets || !send_pos)
     return fail(kInvalidArgument, "amemMoePermuteNoAlloc: null buffer");
+  if (((uintptr_t)x | (uintptr_t)recv_x) & 15) return fail(kInvalidArgument, "amemMoePermuteNoAlloc: x and recv_x must be 16-byte aligned");
   NoAllocScratch* s = nullptr;
   Status st = scratch_for_current_device(&s);
   if (st != kSuccess) return st;

@@ -71,3 +71,69 @@ def test_an_mlp_refuses_a_batch_of_sequences(lib):
     with torch.no_grad(), pytest.raises(ValueError):
         layer(gpu(2, 16, 64))
     assert [name for name, _ in lib.calls if "Gemm" in name] == []
+
+
+# ------------------------------------------------------------------ rows that start at odd addresses
+
+def shifted(*shape):
+    """A contiguous tensor that starts 2 bytes behind a 16-byte boundary."""
+    n = 1
+    for s in shape:
+        n *= s
+    flat = torch.arange(n + 1, dtype=torch.float32).to(BF16)
+    assert flat.data_ptr() % 16 == 0
+    return flat[1:].view(*shape).as_subclass(OnGpu)
+
+
+def _dispatcher(lib, E=4, d=8, capacity=64):
+    from asystem_amem_b200.ops import MoeDispatcher
+    disp = object.__new__(MoeDispatcher)
+    disp.comm, disp.E, disp.d, disp.capacity, disp.experts_per_rank, disp.host = SimpleNamespace(nranks=1, lib=lib, _h=1), E, d, capacity, E, False
+    disp.y, disp.recv_x = gpu(capacity, d), gpu(capacity, d)
+    return disp
+
+
+def test_moe_steps_hand_over_rows_on_16_bytes(lib):
+    from asystem_amem_b200.parallel import ep
+    disp, idx, w, pos = _dispatcher(lib), torch.zeros(6, 2, dtype=torch.int32), torch.ones(6, 2), torch.zeros(6, 2, dtype=torch.int32)
+    disp.dispatch(shifted(6, 8), idx)
+    disp.dispatch_local(shifted(6, 8), idx)
+    ep.combine_forward(disp, shifted(12, 8), idx, w, pos)
+    ep.dispatch_backward(disp, shifted(12, 8), idx, pos)
+    ep.combine_backward(disp, shifted(6, 8), shifted(12, 8), idx, w, pos)
+    rows = {"amemMoeDispatchCounted": [0], "amemMoeDispatchLocal": [0, 6], "amemMoeCombineLocal": [3, 5], "amemMoeCombineGradLocal": [0, 1, 4]}
+    assert {name for name, _ in lib.calls} == set(rows)
+    for name, args in lib.calls:
+        assert all(args[i] % 16 == 0 for i in rows[name]), name
+
+
+def test_moe_steps_between_tensors_take_what_fits_only(lib):
+    """More rows than the dispatcher's buffers hold, or gradients of another number of tokens, take the general form."""
+    from asystem_amem_b200.parallel import ep
+    disp, idx, w, pos = _dispatcher(lib, capacity=8), torch.zeros(6, 2, dtype=torch.int32), torch.ones(6, 2), torch.zeros(6, 2, dtype=torch.int32)
+    for call in (lambda: ep.combine_forward(disp, gpu(12, 8), idx, w, pos), lambda: ep.dispatch_backward(disp, gpu(12, 8), idx, pos),
+                 lambda: ep.combine_backward(disp, gpu(5, 8), gpu(8, 8), idx, w, pos)):
+        with pytest.raises(RuntimeError):
+            call()
+    assert all("Local" not in name for name, _ in lib.calls)
+
+
+def test_moe_entry_points_refuse_unaligned_and_missing_rows(monkeypatch):
+    """The C side says so too (no GPU: the refusal comes before anything else)."""
+    monkeypatch.setenv("AMEM_BACKEND", "mock")
+    from asystem_amem_b200 import Communicator, get_unique_id
+    comm = Communicator(1, 0, get_unique_id())
+    lib = comm.lib
+    ok, odd = 4096, 4098     # never dereferenced
+
+    def status(x, y, table):
+        return {lib.amemMoeDispatchLocal(x, table, 4, 1, 8, 2, y, 4, table, table, table, None, comm._h, None),
+                lib.amemMoeCombineLocal(table, table, table, x, 4, y, 4, 1, 8, 2, comm._h, None),
+                lib.amemMoeCombineGradLocal(x, y, table, table, ok, table, 4, 4, 1, 8, comm._h, None),
+                lib.amemMoeCombineGradLocal(ok, y, table, table, x, table, 4, 4, 1, 8, comm._h, None)}
+
+    for x, y, table in ((odd, ok, ok), (ok, odd, ok), (None, ok, ok), (ok, None, ok), (ok, ok, None)):
+        assert status(x, y, table) == {4}, (x, y, table)      # ncclInvalidArgument
+    assert lib.amemMoeDispatch(odd, ok, 4, 1, 8, 2, 4, ok, ok, ok, comm._h, None) == 4
+    assert lib.amemMoeCombine(ok, ok, ok, odd, 4, 1, 8, 2, 4, comm._h, None) == 4
+    comm.destroy()

@@ -1,0 +1,58 @@
+"""Layers and their gradients on tensors as a program leaves them: gradients that start at any element,
+rows changed in place, results given at any address."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def comm():
+    from asystem_amem_b200 import Communicator, get_unique_id
+    c = Communicator(1, 0, get_unique_id())
+    yield c
+    torch.cuda.synchronize()
+    c.destroy()
+
+
+def _rand(shape, seed, scale=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, device="cuda", generator=g) * scale).to(torch.bfloat16)
+
+
+def _shifted(t):
+    """The same values, contiguous, one element behind a 16-byte boundary."""
+    flat = torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)
+    view = flat[1:].view(t.shape)
+    view.copy_(t)
+    assert view.is_contiguous() and view.data_ptr() % 16
+    return view
+
+
+def test_moe_layer_with_a_gradient_that_starts_at_an_odd_address(comm):
+    from asystem_amem_b200.models import MoELayer
+    layer = MoELayer(comm, 64, 96, 4, 2, tokens_per_rank=33, capacity_factor=1.0)
+    x, g = _rand((33, 64), 1), _rand((33, 64), 2)
+    got = []
+    for grad in (g, _shifted(g)):
+        a = x.clone().requires_grad_(True)
+        layer.zero_grad(set_to_none=True)
+        layer(a).backward(grad)
+        got.append([a.grad] + [p.grad for p in layer.parameters()])
+    assert all(torch.equal(s, t) for s, t in zip(*got))
+
+
+def test_moe_steps_on_rows_at_odd_addresses(comm):
+    from asystem_amem_b200.ops import MoeDispatcher
+    from asystem_amem_b200.parallel import ep
+    T, k, E, d = 21, 3, 5, 72
+    disp = MoeDispatcher(comm, E, d, T * k)
+    idx = torch.randint(0, E, (T, k), generator=torch.Generator().manual_seed(3), dtype=torch.int32).cuda()
+    w, x, y, g = torch.rand(T, k, device="cuda"), _rand((T, d), 4), _rand((T * k, d), 5), _rand((T, d), 6)
+    rows, _, pos, _ = ep.dispatch_forward(disp, x, idx)
+    assert torch.equal(ep.dispatch_forward(disp, _shifted(x), idx)[0], rows)
+    assert torch.equal(disp.dispatch(_shifted(x), idx).recv_x[:T * k], rows)
+    assert torch.equal(ep.combine_forward(disp, _shifted(y), idx, w, pos), ep.combine_forward(disp, y, idx, w, pos))
+    assert torch.equal(ep.dispatch_backward(disp, _shifted(y), idx, pos), ep.dispatch_backward(disp, y, idx, pos))
+    for a, b in zip(ep.combine_backward(disp, _shifted(g), _shifted(y), idx, w, pos), ep.combine_backward(disp, g, y, idx, w, pos)):
+        assert torch.equal(a, b)
