@@ -19,6 +19,7 @@ import torch.nn as nn
 from ..ops.gemm import grouped_gemm_bf16, grouped_gemm_input_grad, grouped_gemm_weight_grad, interleave_gate_up
 from ..ops.elementwise import swiglu
 from ..ops.moe import MoeDispatcher
+from ..ops.operands import dense
 from ..parallel.ep import ep_combine, ep_dispatch
 
 
@@ -33,7 +34,7 @@ class GroupedLinear(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g_out):
         rows, w, offsets = ctx.saved_tensors
-        g_out = g_out.contiguous()
+        g_out = dense(g_out)
         g_rows = g_w = None
         if ctx.needs_input_grad[0]:
             g_rows = torch.zeros_like(rows)

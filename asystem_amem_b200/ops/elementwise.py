@@ -8,6 +8,7 @@ import torch
 import torch.nn.functional as F
 
 from .. import bindings as B
+from .operands import dense
 
 
 def _st() -> int:
@@ -28,7 +29,7 @@ class _SwiGLU(torch.autograd.Function):
     @torch.autograd.function.once_differentiable
     def backward(ctx, g):
         (h,) = ctx.saved_tensors
-        g, out = g.contiguous(), torch.empty_like(h)
+        g, out = dense(g), torch.empty_like(h)
         f, p, o = h.shape[1] // 2, h.data_ptr(), out.data_ptr()
         B.check(B.load_library().amemSwiGLUGrad(p, p + 2 * f, 2 * f, g.data_ptr(), o, o + 2 * f, h.shape[0], f, _st()), "amemSwiGLUGrad")
         return out

@@ -137,3 +137,15 @@ def test_moe_entry_points_refuse_unaligned_and_missing_rows(monkeypatch):
     assert lib.amemMoeDispatch(odd, ok, 4, 1, 8, 2, 4, ok, ok, ok, comm._h, None) == 4
     assert lib.amemMoeCombine(ok, ok, ok, odd, 4, 1, 8, 2, 4, comm._h, None) == 4
     comm.destroy()
+
+
+def test_gradients_at_odd_addresses_reach_the_kernels_on_16_bytes(lib):
+    from asystem_amem_b200.models.moe_layer import GroupedLinear
+    from asystem_amem_b200.ops import swiglu
+    h = gpu(6, 32).requires_grad_(True)
+    swiglu(h).backward(shifted(6, 16))
+    w, offs = gpu(2, 16, 8).requires_grad_(True), torch.tensor([0, 2, 6], dtype=torch.int32).as_subclass(OnGpu)
+    GroupedLinear.apply(gpu(6, 8), w, offs).backward(shifted(6, 16))
+    rows = {"amemSwiGLUGrad": 3, "amemGroupedGemmBf16Weight": 0}
+    seen = {name: args for name, args in lib.calls}
+    assert all(seen[name][i] % 16 == 0 for name, i in rows.items())

@@ -56,3 +56,14 @@ def test_moe_steps_on_rows_at_odd_addresses(comm):
     assert torch.equal(ep.dispatch_backward(disp, _shifted(y), idx, pos), ep.dispatch_backward(disp, y, idx, pos))
     for a, b in zip(ep.combine_backward(disp, _shifted(g), _shifted(y), idx, w, pos), ep.combine_backward(disp, g, y, idx, w, pos)):
         assert torch.equal(a, b)
+
+
+def test_swiglu_with_a_gradient_that_starts_at_an_odd_address():
+    from asystem_amem_b200.ops import swiglu
+    h, g = _rand((33, 48), 7), _rand((33, 24), 8)
+    got = []
+    for grad in (g, _shifted(g)):
+        a = h.clone().requires_grad_(True)
+        swiglu(a).backward(grad)
+        got.append(a.grad)
+    assert torch.equal(*got)
