@@ -8,7 +8,7 @@ import torch
 import torch.nn.functional as F
 
 from .. import bindings as B
-from .operands import dense
+from .operands import dense, on_device_of
 
 
 def _st() -> int:
@@ -31,14 +31,16 @@ class _SwiGLU(torch.autograd.Function):
         (h,) = ctx.saved_tensors
         g, out = dense(g), torch.empty_like(h)
         f, p, o = h.shape[1] // 2, h.data_ptr(), out.data_ptr()
-        B.check(B.load_library().amemSwiGLUGrad(p, p + 2 * f, 2 * f, g.data_ptr(), o, o + 2 * f, h.shape[0], f, _st()), "amemSwiGLUGrad")
+        with on_device_of(h):
+            B.check(B.load_library().amemSwiGLUGrad(p, p + 2 * f, 2 * f, g.data_ptr(), o, o + 2 * f, h.shape[0], f, _st()), "amemSwiGLUGrad")
         return out
 
 
 def _forward(h: torch.Tensor) -> torch.Tensor:
     f, p = h.shape[1] // 2, h.data_ptr()
     out = torch.empty(h.shape[0], f, dtype=h.dtype, device=h.device)
-    B.check(B.load_library().amemSwiGLU(p, p + 2 * f, 2 * f, out.data_ptr(), h.shape[0], f, _st()), "amemSwiGLU")
+    with on_device_of(h):
+        B.check(B.load_library().amemSwiGLU(p, p + 2 * f, 2 * f, out.data_ptr(), h.shape[0], f, _st()), "amemSwiGLU")
     return out
 
 
@@ -55,10 +57,11 @@ def adamw_step(grad, m, v, master, shard, lr: float, betas, eps: float, weight_d
     """One AdamW update in place: fp32 ``m``, ``v`` and ``master`` from the fp32 ``grad``; ``shard``
     receives the new weights in bf16.  ``step`` counts from 1."""
     flat = (grad, m, v, master, shard)
-    if all(t.is_cuda and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in flat) and shard.dtype == torch.bfloat16 \
+    if all(t.is_cuda and t.device == grad.device and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in flat) and shard.dtype == torch.bfloat16 \
             and all(t.dtype == torch.float32 for t in flat[:4]):
-        B.check(B.load_library().amemAdamW(grad.data_ptr(), m.data_ptr(), v.data_ptr(), master.data_ptr(), shard.data_ptr(), grad.numel(),
-                                           float(lr), float(betas[0]), float(betas[1]), float(eps), float(weight_decay), step, _st()), "amemAdamW")
+        with on_device_of(grad):
+            B.check(B.load_library().amemAdamW(grad.data_ptr(), m.data_ptr(), v.data_ptr(), master.data_ptr(), shard.data_ptr(), grad.numel(),
+                                               float(lr), float(betas[0]), float(betas[1]), float(eps), float(weight_decay), step, _st()), "amemAdamW")
         torch.autograd.graph.increment_version([t for t in flat[1:] if not t.is_inference()])   # as an in-place operator does
         return
     b1, b2 = betas

@@ -12,6 +12,7 @@ from __future__ import annotations
 import torch
 
 from .. import bindings as B
+from .operands import on_device_of
 
 
 def _check(a: torch.Tensor, b: torch.Tensor) -> None:
@@ -57,7 +58,8 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
     N = b.shape[0]
     out = torch.empty(M, N, dtype=torch.bfloat16, device=a.device) if out is None else out
     lib = B.load_library()
-    B.check(lib.amemGemmBf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, _stream(stream)), "amemGemmBf16")
+    with on_device_of(a):
+        B.check(lib.amemGemmBf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, _stream(stream)), "amemGemmBf16")
     return out
 
 
@@ -73,7 +75,8 @@ def gemm_swiglu(a: torch.Tensor, w13: torch.Tensor, stream=None) -> torch.Tensor
     _check(a, w13)
     out = torch.empty(a.shape[0], f, dtype=torch.bfloat16, device=a.device)
     lib = B.load_library()
-    B.check(lib.amemGemmSwiGLU(a.data_ptr(), w13.data_ptr(), out.data_ptr(), a.shape[0], f, a.shape[1], _stream(stream)), "amemGemmSwiGLU")
+    with on_device_of(a):
+        B.check(lib.amemGemmSwiGLU(a.data_ptr(), w13.data_ptr(), out.data_ptr(), a.shape[0], f, a.shape[1], _stream(stream)), "amemGemmSwiGLU")
     return out
 
 
@@ -84,7 +87,8 @@ def _by_k(a: torch.Tensor, b: torch.Tensor, m: int, n: int, k: int, a_by_k: bool
         raise ValueError("contiguous CUDA tensors expected")
     out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
     lib = B.load_library()
-    B.check(lib.amemGemmBf16Strided(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, int(a_by_k), 1, _stream(stream)), "amemGemmBf16Strided")
+    with on_device_of(a):
+        B.check(lib.amemGemmBf16Strided(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, int(a_by_k), 1, _stream(stream)), "amemGemmBf16Strided")
     return out
 
 
@@ -153,8 +157,9 @@ def grouped_gemm_bf16(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, o
     rows_cap = a.shape[0]
     out = torch.empty(rows_cap, N // 2 if swiglu else N, dtype=torch.bfloat16, device=a.device) if out is None else out
     lib = B.load_library()
-    B.check(lib.amemGroupedGemmBf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, rows_cap,
-                                    int(rows_hint or 0), N, K, 1 if swiglu else 0, _stream(stream)), "amemGroupedGemmBf16")
+    with on_device_of(a):
+        B.check(lib.amemGroupedGemmBf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, rows_cap,
+                                        int(rows_hint or 0), N, K, 1 if swiglu else 0, _stream(stream)), "amemGroupedGemmBf16")
     return out
 
 
@@ -175,8 +180,9 @@ def grouped_gemm_input_grad(g: torch.Tensor, w: torch.Tensor, offsets: torch.Ten
         return res
     out = torch.empty(g.shape[0], K, dtype=torch.bfloat16, device=g.device) if out is None else out
     _check_grouped(g, w, offsets, groups)
-    B.check(B.load_library().amemGroupedGemmBf16Input(g.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
-                                                      int(rows_hint or 0), N, K, _stream(stream)), "amemGroupedGemmBf16Input")
+    with on_device_of(g):
+        B.check(B.load_library().amemGroupedGemmBf16Input(g.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
+                                                          int(rows_hint or 0), N, K, _stream(stream)), "amemGroupedGemmBf16Input")
     return out
 
 
@@ -190,8 +196,9 @@ def grouped_gemm_weight_grad(g: torch.Tensor, a: torch.Tensor, offsets: torch.Te
         return torch.stack([g[offs[e]:offs[e + 1]].t() @ a[offs[e]:offs[e + 1]] for e in range(groups)])
     _check_grouped(g, a, offsets, groups)
     out = torch.empty(groups, N, K, dtype=torch.bfloat16, device=g.device)
-    B.check(B.load_library().amemGroupedGemmBf16Weight(g.data_ptr(), a.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
-                                                       N, K, _stream(stream)), "amemGroupedGemmBf16Weight")
+    with on_device_of(g):
+        B.check(B.load_library().amemGroupedGemmBf16Weight(g.data_ptr(), a.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
+                                                           N, K, _stream(stream)), "amemGroupedGemmBf16Weight")
     return out
 
 

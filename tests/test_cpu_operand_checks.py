@@ -36,6 +36,7 @@ def lib(monkeypatch):
     rec = Recorder()
     monkeypatch.setattr(B, "load_library", lambda *a, **k: rec)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: SimpleNamespace(cuda_stream=0))
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: -1)
     return rec
 
 
@@ -149,3 +150,38 @@ def test_gradients_at_odd_addresses_reach_the_kernels_on_16_bytes(lib):
     rows = {"amemSwiGLUGrad": 3, "amemGroupedGemmBf16Weight": 0}
     seen = {name: args for name, args in lib.calls}
     assert all(seen[name][i] % 16 == 0 for name, i in rows.items())
+
+
+# ------------------------------------------------------------------ tensors on another device than the current one
+
+def test_launches_make_the_operands_device_current(lib, monkeypatch):
+    from asystem_amem_b200 import ops
+    current = [0]
+
+    class Device:
+        def __init__(self, index):
+            self.index = index
+
+        def __enter__(self):
+            current.append(self.index)
+
+        def __exit__(self, *exc):
+            current.pop()
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[-1])
+    monkeypatch.setattr(torch.cuda, "device", Device)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: SimpleNamespace(cuda_stream=100 + current[-1]))
+    monkeypatch.setattr(OnGpu, "get_device", lambda self: 3, raising=False)
+    offs = torch.tensor([0, 2, 6], dtype=torch.int32).as_subclass(OnGpu)
+    h = gpu(6, 32).requires_grad_(True)
+    ops.swiglu(h).backward(gpu(6, 16))
+    ops.adamw_step(*(gpu(16, dtype=torch.float32) for _ in range(4)), gpu(16), 1e-3, (0.9, 0.95), 1e-8, 0.0, 1)
+    ops.gemm_bf16(gpu(8, 64), gpu(16, 64))
+    ops.gemm_swiglu(gpu(8, 64), gpu(16, 64))
+    ops.gemm_input_grad(gpu(8, 64), gpu(64, 16))
+    ops.gemm_weight_grad(gpu(8, 64), gpu(8, 16))
+    ops.grouped_gemm_bf16(gpu(6, 64), gpu(2, 16, 64), offs)
+    ops.grouped_gemm_input_grad(gpu(6, 16), gpu(2, 16, 64), offs)
+    ops.grouped_gemm_weight_grad(gpu(6, 16), gpu(6, 64), offs)
+    assert len(lib.calls) == 10 and all(args[-1] == 103 for _, args in lib.calls), lib.calls
+    assert current == [0]
