@@ -55,9 +55,10 @@ def swiglu(h: torch.Tensor) -> torch.Tensor:
 
 def adamw_step(grad, m, v, master, shard, lr: float, betas, eps: float, weight_decay: float, step: int) -> None:
     """One AdamW update in place: fp32 ``m``, ``v`` and ``master`` from the fp32 ``grad``; ``shard``
-    receives the new weights in bf16.  ``step`` counts from 1."""
+    receives the new weights in bf16.  ``step`` counts from 1.  One kernel for five tensors of one shape,
+    dense on one GPU; the general form takes, or refuses, what torch does."""
     flat = (grad, m, v, master, shard)
-    if all(t.is_cuda and t.device == grad.device and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in flat) and shard.dtype == torch.bfloat16 \
+    if all(t.is_cuda and t.device == grad.device and t.shape == grad.shape and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in flat) and shard.dtype == torch.bfloat16 \
             and all(t.dtype == torch.float32 for t in flat[:4]):
         with on_device_of(grad):
             B.check(B.load_library().amemAdamW(grad.data_ptr(), m.data_ptr(), v.data_ptr(), master.data_ptr(), shard.data_ptr(), grad.numel(),

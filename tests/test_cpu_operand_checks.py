@@ -185,3 +185,13 @@ def test_launches_make_the_operands_device_current(lib, monkeypatch):
     ops.grouped_gemm_weight_grad(gpu(6, 16), gpu(6, 64), offs)
     assert len(lib.calls) == 10 and all(args[-1] == 103 for _, args in lib.calls), lib.calls
     assert current == [0]
+
+
+@pytest.mark.parametrize("short", range(5))
+def test_adamw_of_different_sizes_is_refused_as_torch_refuses_it(lib, short):
+    from asystem_amem_b200 import ops
+    ts = [gpu(16, dtype=torch.float32) for _ in range(4)] + [gpu(16)]
+    ts[short] = ts[short][:8]
+    with pytest.raises(RuntimeError):
+        ops.adamw_step(*ts, 1e-3, (0.9, 0.95), 1e-8, 0.0, 1)
+    assert lib.calls == []
