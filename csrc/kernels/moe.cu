@@ -454,16 +454,13 @@ __global__ void __launch_bounds__(kThreads) count_kernel(const __grid_constant__
   pdl_wait();
   count_body(a, blockIdx.x, gridDim.x);
 }
+// (plan and scatter run between ranks only and wait for peers: whatever follows them keeps its turn)
 __global__ void __launch_bounds__(kThreads) plan_kernel(const __grid_constant__ MoeArgs a, int segments) {
   __shared__ int s_abort;
-  pdl_launch_dependents();
-  pdl_wait();
   plan_body(a, segments, &s_abort);
 }
 __global__ void __launch_bounds__(kThreads) scatter_kernel(const __grid_constant__ MoeArgs a) {
   __shared__ int s_abort;
-  pdl_launch_dependents();
-  pdl_wait();
   scatter_body(a, blockIdx.x, gridDim.x, &s_abort);
 }
 __global__ void __launch_bounds__(kThreads) place_and_scatter_kernel(const __grid_constant__ MoeArgs a) {
@@ -479,8 +476,10 @@ __global__ void __launch_bounds__(kThreads) small_dispatch_kernel(const __grid_c
 template <int KC, int VPL>
 __global__ void __launch_bounds__(kCombineThreads, 2) combine_kernel(const __grid_constant__ MoeArgs a) {
   __shared__ int s_abort;
-  pdl_launch_dependents();
-  pdl_wait();
+  if (a.coll.nranks == 1) {
+    pdl_launch_dependents();
+    pdl_wait();
+  }
   combine_body<KC, VPL>(a, blockIdx.x, gridDim.x, &s_abort);
 }
 __global__ void __launch_bounds__(kThreads) count_kernel_emu(const MoeArgs* __restrict__ all) { count_body(all[blockIdx.y], blockIdx.x, gridDim.x); }
@@ -510,8 +509,9 @@ static Status launched(cudaError_t e, const char* what) {
   return kSuccess;
 }
 
-// One rank: launches overlap their predecessor's end.  With peers they are ordinary launches: those
-// kernels wait for the other GPUs' and are not to be scheduled before their turn.
+// One rank: launches overlap their predecessor's end, and their successor theirs.  With peers they are
+// ordinary launches and let nobody in early: those kernels wait for the other GPUs', and a successor parked
+// on the SMs meanwhile would keep out the kernel of another stream that a peer's progress may depend on.
 template <typename... P, typename... A>
 static cudaError_t launch(void (*kernel)(P...), const MoeArgs& a, int grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
   if (a.coll.nranks == 1) return launch_overlapped(kernel, dim3(grid), dim3(threads), smem, stream, args...);

@@ -6,7 +6,8 @@
 // access to global memory that another kernel may touch (reads AND writes): the wait returns when the
 // predecessor has completed and its writes are visible.  A kernel that only calls
 // pdl_launch_dependents() lets its successor in earlier; successors that were launched the ordinary way
-// are ordered as ever.
+// are ordered as ever.  A kernel that waits for a peer GPU does not call it: its successor would hold SMs,
+// shared memory and tensor memory for as long as the wait lasts.
 #pragma once
 #include <cuda_runtime.h>
 
