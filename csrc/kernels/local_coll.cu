@@ -14,7 +14,7 @@ namespace localk {
 
 constexpr int THREADS = 256, AHEAD = 4, CAST_AHEAD = 8;
 
-__global__ void __launch_bounds__(THREADS) copy_kernel(const char* __restrict__ src, char* __restrict__ dst, size_t bytes) {
+__global__ void __launch_bounds__(THREADS) copy_kernel(const char* src, char* dst, size_t bytes) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t n = bytes / 16, i0 = (size_t)blockIdx.x * THREADS * AHEAD + threadIdx.x;
@@ -35,7 +35,7 @@ struct alignas(4 * sizeof(T)) Four {
 
 // out = (TO)(scale * in), in fp32; four elements per access, so that a warp covers whole lines on both sides
 template <typename TI, typename TO>
-__global__ void __launch_bounds__(THREADS) scale_kernel(const TI* __restrict__ src, TO* __restrict__ dst, size_t count, float scale) {
+__global__ void __launch_bounds__(THREADS) scale_kernel(const TI* src, TO* dst, size_t count, float scale) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t n = count / 4, i0 = (size_t)blockIdx.x * THREADS * CAST_AHEAD + threadIdx.x;

@@ -187,7 +187,7 @@ __device__ void copy_rows(const MoeArgs& a, int base, int count, const int* c_po
     uint4 v[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      if (v0 + j * 32 < nvec) v[j] = __ldg(src + v0 + j * 32);
+      if (v0 + j * 32 < nvec) v[j] = src[v0 + j * 32];
     const int j0 = max(t * a.k, base) - base, j1 = min((t + 1) * a.k, base + count) - base;
     for (int c = j0; c < j1; ++c) {
       const int pos = c_pos[c];
@@ -400,9 +400,9 @@ __device__ void combine_body(const MoeArgs& a, int cta, int nctas, int* s_abort)
 // product, a sum, a scaled copy and a second dispatch: 0.5 ms for 4096 x 2 rows of 8 KB; 27.5 us so,
 // 25 are the bytes).
 constexpr int kGradThreads = 128;
-__global__ void __launch_bounds__(kGradThreads) combine_grad_kernel(const char* __restrict__ g_out, const char* __restrict__ y, const float* __restrict__ w,
-                                                                    const int* __restrict__ send_pos, char* __restrict__ g_y, float* __restrict__ g_w, int rows, int T, int k,
-                                                                    int d) {
+constexpr int kGradAhead = 4;   // vectors of either row that a thread loads ahead of its stores: all of them up to d = 4096
+__global__ void __launch_bounds__(kGradThreads) combine_grad_kernel(const char* g_out, const char* y, const float* w, const int* send_pos, char* g_y,
+                                                                    float* g_w, int rows, int T, int k, int d) {
   __shared__ float part[kGradThreads / 32];
   pdl_launch_dependents();
   pdl_wait();
@@ -421,18 +421,27 @@ __global__ void __launch_bounds__(kGradThreads) combine_grad_kernel(const char* 
       const uint4* src = (const uint4*)(y + (size_t)pos * row_bytes);
       uint4* dst = (uint4*)(g_y + (size_t)pos * row_bytes);
       float dot = 0.f;
-#pragma unroll 4
-      for (int v = threadIdx.x; v < nvec; v += kGradThreads) {
-        const uint4 gr = __ldg(g + v), yr = __ldg(src + v);
-        const __nv_bfloat16 *gh = (const __nv_bfloat16*)&gr, *yh = (const __nv_bfloat16*)&yr;
-        alignas(16) __nv_bfloat16 res[8];
+      for (int v0 = threadIdx.x; v0 < nvec; v0 += kGradAhead * kGradThreads) {
+        uint4 gr[kGradAhead], yr[kGradAhead];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float gf = __bfloat162float(gh[q]);
-          dot = fmaf(gf, __bfloat162float(yh[q]), dot);
-          res[q] = __float2bfloat16_rn(gf * scale);
-        }
-        dst[v] = *(const uint4*)res;
+        for (int i = 0; i < kGradAhead; ++i)
+          if (v0 + i * kGradThreads < nvec) {
+            gr[i] = g[v0 + i * kGradThreads];
+            yr[i] = src[v0 + i * kGradThreads];
+          }
+#pragma unroll
+        for (int i = 0; i < kGradAhead; ++i)
+          if (v0 + i * kGradThreads < nvec) {
+            const __nv_bfloat16 *gh = (const __nv_bfloat16*)&gr[i], *yh = (const __nv_bfloat16*)&yr[i];
+            alignas(16) __nv_bfloat16 res[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const float gf = __bfloat162float(gh[q]);
+              dot = fmaf(gf, __bfloat162float(yh[q]), dot);
+              res[q] = __float2bfloat16_rn(gf * scale);
+            }
+            dst[v0 + i * kGradThreads] = *(const uint4*)res;
+          }
       }
 #pragma unroll
       for (int o = 16; o > 0; o /= 2) dot += __shfl_xor_sync(0xffffffffu, dot, o);

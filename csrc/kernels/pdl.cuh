@@ -6,7 +6,10 @@
 // access to global memory that another kernel may touch (reads AND writes): the wait returns when the
 // predecessor has completed and its writes are visible.  A kernel that only calls
 // pdl_launch_dependents() lets its successor in earlier; successors that were launched the ordinary way
-// are ordered as ever.  A kernel that waits for a peer GPU does not call it: its successor would hold SMs,
+// are ordered as ever.  Such a kernel takes its buffers as plain pointers: const __restrict__ and __ldg
+// promise data that does not change while the kernel runs, but its predecessor may still be writing when
+// it starts, and only the code's present order would keep such a load behind the wait.  (Loads that are to
+// be in flight together are therefore written ahead of the stores.)  A kernel that waits for a peer GPU does not call it: its successor would hold SMs,
 // shared memory and tensor memory for as long as the wait lasts.
 #pragma once
 #include <cuda_runtime.h>

@@ -39,3 +39,18 @@ def test_kernels_that_wait_for_peers_let_nobody_in_early():
     assert checked >= 6      # plan, scatter, combine, and their emulated forms
     for name in ("collectives.cu", "coll_bodies.inl", "coll_device.cuh", "gemm_sm100.cu", "gemm_ag_cta_movers.cu"):
         assert "pdl_launch_dependents" not in _source(name), name
+
+
+def test_overlapped_kernels_promise_nothing_about_their_inputs():
+    """Neither read-only loads nor restricted pointers in what may start under its predecessor."""
+    overlapped = 0
+    for path in sorted(CSRC.glob("*.cu")):
+        text = _source(path.name)
+        if "pdl.cuh" not in text:
+            continue
+        assert not re.search(r"\b(__ldg|ld\.global\.nc)\b", text), path.name
+        for head, body in _functions(text):
+            if "__global__" in head and "pdl_wait" in body:
+                overlapped += 1
+                assert "__restrict__" not in head, (path.name, head)
+    assert overlapped >= 8
