@@ -451,7 +451,7 @@ pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMa
           __threadfence();
           if (met) {
             // the other slices' parts of this slice's chunks, all in flight at once, into the idle operand
-            // ring (this pair has no other tile): 16 KB a piece, at most 7 / 8 of a 128 KB slot in all
+            // ring (this pair has no other tile): 16 KB a piece, at most most_pieces() of them
             asm volatile("fence.proxy.async;" ::: "memory");
             const int n = ((cols + 31) / 32 - tl.slice + S - 1) / S * (second ? 2 : 1) * (S - 1);
             mbar_expect_tx(&ctl->tail, (uint32_t)n * PIECE_BYTES);
@@ -569,7 +569,19 @@ pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMa
 
 constexpr size_t kSmemBytes = (size_t)STAGES * STAGE_BYTES + EPI_WARPS * EPI_BYTES + sizeof(Ctl) + 1024;
 static_assert(A_BYTES == (HM / 64) * CHUNK_BYTES, "B's chunks follow A's without a gap");
-static_assert((MAX_SLICES - 1) * SLOT_FLOATS * 4 / MAX_SLICES <= STAGES * STAGE_BYTES, "the exchanged chunks must fit the operand ring");
+// Pieces of 32 columns that a slice collects: its share of the chunks, rounded up, from every other slice (12 for
+// 7 slices of a 256-wide tile, of which the first has chunks 0 and 7).  A SwiGLU tile has half the chunks, in two parts,
+// and at most a slice for each of them.
+constexpr int most_pieces() {
+  int most = 0;
+  for (int s = 2; s <= MAX_SLICES; ++s) {
+    const int chunks = BN_MAX / 32, n = (chunks + s - 1) / s * (s - 1), n_swiglu = s <= chunks / 2 ? 2 * ((chunks / 2 + s - 1) / s) * (s - 1) : 0;
+    most = n > most ? n : most;
+    most = n_swiglu > most ? n_swiglu : most;
+  }
+  return most;
+}
+static_assert((size_t)most_pieces() * PIECE_BYTES <= (size_t)STAGES * STAGE_BYTES, "the exchanged chunks must fit the operand ring");
 static_assert(kSmemBytes <= 227 * 1024, "operand ring, staging and control words must fit one SM's shared memory");
 
 template <int A_MN, int B_MN, int CUT>

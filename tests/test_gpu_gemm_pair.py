@@ -97,3 +97,12 @@ def test_swiglu_epilogue(ffn):
         if sl.stop > sl.start:
             h = a[sl].float() @ w[e].float().t()
             _close(out[sl], torch.nn.functional.silu(h[:, :ffn]) * h[:, ffn:])
+
+
+def test_seven_cuts_of_a_wide_tile(on_pairs):
+    """Ten tiles of 256 x 256 on 74 pairs are cut in seven: the first slice collects two chunks from each of
+    the others, the most that the idle operand ring ever holds."""
+    from asystem_amem_b200.ops import gemm_bf16
+    x, w = _rand((2560, 8192), 14), _rand((256, 8192), 15)
+    for _ in range(2):
+        _close(gemm_bf16(x, w), x.float() @ w.float().t())
