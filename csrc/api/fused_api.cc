@@ -156,6 +156,7 @@ const unsigned long long kGemmTimeoutNs = 5ull * 1000000000ull;
 
 // The stream's workspace for tiles that are cut along K (all GEMM kernels share it: launches of one stream
 // take turns and leave its counters at zero); null while the process is paused, or where none can be made.
+// Asked for only by a launch that cuts: it is some 40 MB of mapped memory, which pause and resume then handle too.
 SplitKWs* stream_workspace(int dev, cudaStream_t stream, int sms) {
   if (!env_long("AMEM_GEMM_SPLITK", 1) || Registry::instance().is_paused(0)) return nullptr;
   if (gemm_splitk_ws_bytes(sms) < std::max(pair_gemm_ws_bytes(sms), skinny_gemm_ws_bytes(sms))) return nullptr;
@@ -180,7 +181,7 @@ Status run_pair(PairProblem& p, cudaStream_t stream) {
   p.status = status;
   p.timeout_ns = kGemmTimeoutNs;
   const int sms = gemm_default_grid(dev);
-  SplitKWs* ws = p.mode == kPairPlain ? stream_workspace(dev, stream, sms) : nullptr;
+  SplitKWs* ws = pair_gemm_tiling(p, sms, true).slices > 1 ? stream_workspace(dev, stream, sms) : nullptr;
   if (ws) {
     p.sk_ws = ws->partials;
     p.sk_ctr = ws->counters;
@@ -254,7 +255,7 @@ Status run_skinny(SkinnyProblem& p, cudaStream_t stream) {
   p.status = status;
   p.timeout_ns = kGemmTimeoutNs;
   const int sms = gemm_default_grid(dev);
-  SplitKWs* ws = stream_workspace(dev, stream, sms);
+  SplitKWs* ws = skinny_gemm_cuts(p, sms) ? stream_workspace(dev, stream, sms) : nullptr;
   if (ws) {
     p.ws = ws->partials;
     p.ctr = ws->counters;

@@ -668,6 +668,23 @@ bool pair_gemm_takes(const PairProblem& p) {
   return !(((uintptr_t)p.A | (uintptr_t)p.B | (uintptr_t)p.C) & 15) && a_inner % 8 == 0 && b_inner % 8 == 0 && p.N % 8 == 0 && p.groups <= pairk::MAX_GROUPS;
 }
 
+namespace pairk {
+long row_tiles_of(const PairProblem& d) {   // of 256 rows, over all groups
+  const long one = (d.M + TM - 1) / TM;
+  return d.mode == kPairPlain ? one : d.mode == kPairGroupedK ? one * d.groups : std::max(1, d.row_tiles_hint);
+}
+}  // namespace pairk
+
+PairTiling pair_gemm_tiling(const PairProblem& d, int sms, bool may_cut) {
+  PairTiling t;
+  t.slices = 1;
+  may_cut = may_cut && d.mode == kPairPlain && d.epilogue != kPairSwiGLU32;
+  t.bn = pair_gemm_pick_bn(pairk::row_tiles_of(d), d.N, std::max(1, sms / 2), (d.K + pairk::BK - 1) / pairk::BK, may_cut ? &t.slices : nullptr);
+  if (d.epilogue != kPairStore) t.bn = t.bn > 192 ? 256 : (t.bn > 128 ? 192 : 128);   // gate and up columns in blocks of 32, half a tile each
+  if (t.slices > 1) t.slices = std::min(t.slices, (d.epilogue == kPairStore ? t.bn : t.bn / 2) / 32);   // a chunk of the result per slice
+  return t;
+}
+
 Status launch_pair_gemm(const PairProblem& d, int sms, cudaStream_t stream) {
   pairk::Params p;
   p.C = d.C;
@@ -681,23 +698,19 @@ Status launch_pair_gemm(const PairProblem& d, int sms, cudaStream_t stream) {
   p.status = d.status;
   p.timeout_ns = d.timeout_ns;
   p.ldc = d.epilogue == kPairStore ? d.N : d.N / 2;
-  const int clusters = std::max(1, sms / 2);
-  const long row_tiles_1 = (d.M + pairk::TM - 1) / pairk::TM;
-  const long row_tiles = d.mode == kPairPlain ? row_tiles_1 : d.mode == kPairGroupedK ? row_tiles_1 * d.groups : std::max(1, d.row_tiles_hint);
-  p.slices = 1;
   p.sk_ws = d.sk_ws;
   p.sk_ctr = d.sk_ctr;
-  const bool may_cut = d.mode == kPairPlain && d.epilogue != kPairSwiGLU32 && d.sk_ws && d.sk_ctr;
-  p.bn = pair_gemm_pick_bn(row_tiles, d.N, clusters, (d.K + pairk::BK - 1) / pairk::BK, may_cut ? &p.slices : nullptr);
-  if (d.epilogue != kPairStore) p.bn = p.bn > 192 ? 256 : (p.bn > 128 ? 192 : 128);   // gate and up columns in blocks of 32, half a tile each
+  const PairTiling tiling = pair_gemm_tiling(d, sms, d.sk_ws && d.sk_ctr);
+  p.bn = tiling.bn;
+  p.slices = tiling.slices;
   CUtensorMap ma, mb;
   if (d.a_mn) AMEM_TRY(make_bf16_map(&ma, d.A, d.M, d.K, 1, 64));
   else AMEM_TRY(make_bf16_map(&ma, d.A, d.K, d.M, 1, pairk::HM));
   const uint64_t z = d.mode == kPairGroupedRows ? d.groups : 1;
   if (d.b_mn) AMEM_TRY(make_bf16_map(&mb, d.B, d.N, d.K, z, 64));
   else AMEM_TRY(make_bf16_map(&mb, d.B, d.K, d.N, z, p.bn / 2));
-  if (p.slices > 1) p.slices = std::min(p.slices, (d.epilogue == kPairStore ? p.bn : p.bn / 2) / 32);   // a chunk of the result per slice
-  const long tiles = d.mode == kPairGroupedRows ? clusters : row_tiles * ((d.N + p.bn - 1) / p.bn) * p.slices;
+  const int clusters = std::max(1, sms / 2);
+  const long tiles = d.mode == kPairGroupedRows ? clusters : pairk::row_tiles_of(d) * ((d.N + p.bn - 1) / p.bn) * p.slices;
   const int grid = 2 * (int)std::min<long>(clusters, std::max<long>(1, tiles));
   if (!d.a_mn && !d.b_mn) return pairk::launch<0, 0>(p, ma, mb, grid, stream);
   if (!d.a_mn) return pairk::launch<0, 1>(p, ma, mb, grid, stream);

@@ -47,6 +47,12 @@ size_t pair_gemm_ctr_words(int sms);
 // Whether the operands' addresses and pitches allow TMA (16-byte rule) and the sizes fit.
 bool pair_gemm_takes(const PairProblem& p);
 Status launch_pair_gemm(const PairProblem& p, int sms, cudaStream_t stream);
+// The tiling that launch_pair_gemm takes; slices: cuts of every tile along K (1: none, and the workspace is
+// not touched), more than one only where may_cut says that there is, or would be, a workspace.
+struct PairTiling {
+  int bn, slices;
+};
+PairTiling pair_gemm_tiling(const PairProblem& p, int sms, bool may_cut);
 // Tile width in columns (multiple of 32, 128..256) for `row_tiles` rows of 256-row tiles on `clusters`
 // SM pairs.  With `slices`, a problem that leaves half of the pairs idle may be cut along its k_blocks
 // blocks of 64; *slices receives the number of cuts (1: none).

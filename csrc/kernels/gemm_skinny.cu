@@ -5,7 +5,7 @@
 // so no MMA row and no byte of shared memory goes to padding tokens; and the K blocks of all weight
 // tiles form one sequence that is cut evenly over the SMs, whatever the number of tiles, so every SM
 // keeps its whole ring (up to 11 stages, about 190 KB) of weight loads in flight to the end.
-// (Several groups: whole tiles, see launch_skinny_gemm.)
+// (Several groups: whole tiles, see skinny_gemm_cuts.)
 //
 // A tile cut by such a boundary is finished by whichever of its CTAs comes last: each parks its fp32
 // partial sums (64 KB at most), counts itself in, and the last one adds the parts in order of K -- the
@@ -411,6 +411,19 @@ bool skinny_gemm_takes(const SkinnyProblem& p) {
   return !(((uintptr_t)p.A | (uintptr_t)p.W) & 15) && !((uintptr_t)p.C & 1) && p.K % 8 == 0 && p.groups <= skinnyk::MAX_GROUPS;
 }
 
+bool skinny_gemm_cuts(const SkinnyProblem& d, int sms) {
+  // Several groups: whole tiles, so that every sum runs over K in one go, as on SM pairs (a caller's guess
+  // of the number of rows, which decides between the two kernels, must not show in the result).  One
+  // group: cut where that pays.  A stage takes 0.25 us per SM (16 x 7168 x 8192 uncut: 32.9 us for 128 of
+  // them), the exchange of a cut 3.5 us, and no schedule beats reading the weights (16 x 8192 x 3584, 64
+  // tiles: 17.5 us whole, 18.8 cut; 16 x 7168 x 8192, 56 tiles: 32.9 whole, 27.3 cut).
+  const double w_tiles = (d.N + skinnyk::WM - 1) / skinnyk::WM, nkb = (d.K + skinnyk::BK - 1) / skinnyk::BK;
+  const double read_us = (double)d.N * d.K * 2 / 6.5e6;
+  const double whole_us = std::max(read_us, (double)(((long)w_tiles + sms - 1) / sms) * nkb * 0.25);
+  const double cut_us = std::max(read_us, w_tiles * nkb / sms * 0.25) + 3.5;
+  return !d.group_off && cut_us < whole_us;
+}
+
 Status launch_skinny_gemm(const SkinnyProblem& d, int sms, cudaStream_t stream) {
   namespace k = skinnyk;
   k::Params p;
@@ -423,16 +436,7 @@ Status launch_skinny_gemm(const SkinnyProblem& d, int sms, cudaStream_t stream) 
   p.epilogue = d.epilogue;
   p.groups = d.group_off ? d.groups : 1;
   p.group_off = d.group_off;
-  // Several groups: whole tiles, so that every sum runs over K in one go, as on SM pairs (a caller's guess
-  // of the number of rows, which decides between the two kernels, must not show in the result).  One
-  // group: cut where that pays.  A stage takes 0.25 us per SM (16 x 7168 x 8192 uncut: 32.9 us for 128 of
-  // them), the exchange of a cut 3.5 us, and no schedule beats reading the weights (16 x 8192 x 3584, 64
-  // tiles: 17.5 us whole, 18.8 cut; 16 x 7168 x 8192, 56 tiles: 32.9 whole, 27.3 cut).
-  const double w_tiles = (d.N + k::WM - 1) / k::WM, nkb = (d.K + k::BK - 1) / k::BK;
-  const double read_us = (double)d.N * d.K * 2 / 6.5e6;
-  const double whole_us = std::max(read_us, (double)(((long)w_tiles + sms - 1) / sms) * nkb * 0.25);
-  const double cut_us = std::max(read_us, w_tiles * nkb / sms * 0.25) + 3.5;
-  p.ws = !d.group_off && d.ctr && cut_us < whole_us ? d.ws : nullptr;
+  p.ws = d.ctr && skinny_gemm_cuts(d, sms) ? d.ws : nullptr;
   p.ctr = d.ctr;
   p.status = d.status;
   p.timeout_ns = d.timeout_ns;

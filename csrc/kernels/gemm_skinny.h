@@ -30,6 +30,8 @@ static const int kSkinnyMaxRows = 128;
 
 bool skinny_gemm_takes(const SkinnyProblem& p);
 Status launch_skinny_gemm(const SkinnyProblem& p, int sms, cudaStream_t stream);
+// Whether launch_skinny_gemm would cut tiles along K, given a workspace.
+bool skinny_gemm_cuts(const SkinnyProblem& p, int sms);
 size_t skinny_gemm_ws_bytes(int sms);
 size_t skinny_gemm_ctr_words(int sms);
 

@@ -94,3 +94,25 @@ def test_under_capture_and_back_to_back():
         g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, ref)
+
+
+def test_only_a_product_that_is_cut_makes_a_workspace():
+    """Grouped products and those of whole tiles allocate nothing on a stream that they are the first to use."""
+    from asystem_amem_b200 import mem_stats
+    from asystem_amem_b200.ops import gemm_bf16, gemm_swiglu, grouped_gemm_bf16
+    x, w, offs = _rand((64, 256), 9), _rand((4, 128, 256), 10), torch.tensor([0, 3, 9, 40, 64], dtype=torch.int32, device="cuda")
+    big, wide = _rand((4096, 512), 11), _rand((4096, 512), 12)
+    gemm_bf16(x, w[0])          # the process's own words
+    torch.cuda.synchronize()
+    live = mem_stats()["live_bytes"]
+    side = torch.cuda.Stream(priority=-1)       # of a pool that no other test draws from
+    with torch.cuda.stream(side):
+        grouped_gemm_bf16(x, w, offs, rows_hint=64)
+        gemm_bf16(x, w[0])
+        gemm_swiglu(x, w[0])
+        gemm_bf16(big, wide)
+        side.synchronize()
+        assert mem_stats()["live_bytes"] == live
+        gemm_bf16(_rand((16, 8192), 13), _rand((7168, 8192), 14))      # 56 tiles on 148 SMs: cut
+        side.synchronize()
+        assert mem_stats()["live_bytes"] > live
