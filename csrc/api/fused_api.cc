@@ -274,12 +274,20 @@ bool pair_pays(const PairProblem& p) {
   return true;
 }
 
+// The fused and the one-SM kernels store 16-byte vectors.
+Status check_result(const char* what, const void* C) {
+  if ((uintptr_t)C & 15) return fail(kInvalidArgument, "%s: the result must be 16-byte aligned", what);
+  return kSuccess;
+}
+
 // A * B^T on the kernel for few rows or on SM pairs; *done is false where the one-SM kernel is to run
-// (forced by the environment, or C is not 16-byte aligned).
+// (forced by the environment).  A result that is not 16-byte aligned goes to the kernel for few rows, which
+// stores element by element and takes any number of rows; the others cannot store it.
 Status run_plain(const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream, bool* done) {
   *done = true;
   SkinnyProblem few = skinny(A, B, C, M, N, K, nullptr, 1, M, kPairStore);
-  if (skinny_pays(few)) return run_skinny(few, stream);
+  if (((uintptr_t)C & 15) && !skinny_gemm_takes(few)) return check_result("GEMM", C);
+  if (((uintptr_t)C & 15) || skinny_pays(few)) return run_skinny(few, stream);
   PairProblem pair = pair_plain(A, B, C, M, N, K, 0, 0);
   if (pair_pays(pair)) return run_pair(pair, stream);
   *done = false;
@@ -325,6 +333,36 @@ ncclResult_t amemGemmPlan(int M, int N, int K, int sms, int* tile_rows, int* til
   if (tile_rows) *tile_rows = p.tall ? 2 * kGemmBM : kGemmBM;
   if (tile_cols) *tile_cols = p.bn;
   if (tail_slices) *tail_slices = p.slices;
+  return ncclSuccess;
+}
+
+// What amemGemmBf16 does on a GPU with `sms` SMs (operands and result 16-byte aligned; no GPU needed).
+ncclResult_t amemGemmForm(int M, int N, int K, int sms, int* form, int* tile, int* slices) {
+  Status s = check_shape(M, N, K);
+  if (s != kSuccess) return R(s);
+  if (sms <= 0) return R(fail(kInvalidArgument, "amemGemmForm: sms must be positive"));
+  const bool may_cut = env_long("AMEM_GEMM_SPLITK", 1) != 0;
+  const SkinnyProblem few = skinny(nullptr, nullptr, nullptr, M, N, K, nullptr, 1, M, kPairStore);
+  const PairProblem pair = pair_plain(nullptr, nullptr, nullptr, M, N, K, 0, 0);
+  int f, t, c;
+  if (skinny_pays(few)) {
+    f = 2;
+    t = skinny_gemm_tokens(few);
+    c = may_cut && skinny_gemm_cuts(few, sms) ? 2 : 1;
+  } else if (pair_pays(pair)) {
+    const PairTiling p = pair_gemm_tiling(pair, sms, may_cut);
+    f = 1;
+    t = p.bn;
+    c = p.slices;
+  } else {
+    const GemmPlan p = plan_gemm(M, N, K, sms, may_cut);
+    f = 0;
+    t = p.bn;
+    c = p.slices;
+  }
+  if (form) *form = f;
+  if (tile) *tile = t;
+  if (slices) *slices = c;
   return ncclSuccess;
 }
 
@@ -517,6 +555,7 @@ ncclResult_t amemAllGatherGemm(const void* a_shard, const void* B, void* C, int 
     bool done = false;
     if ((s = run_plain(a_shard, B, C, M, N, K, stream, &done)) != kSuccess || done) return R(s);
   }
+  if ((s = check_result("amemAllGatherGemm", C)) != kSuccess) return R(s);
   if (n > 1 && !gemm_ag_uses_mover_warps(n)) return R(ag_gemm_cta_movers(c, a_shard, B, C, M, N, K, stream));
   GemmLaunch g;
   memset(&g, 0, sizeof(g));
@@ -589,6 +628,7 @@ ncclResult_t amemGemmReduceScatter(const void* A, const void* B, void* out, int 
     bool done = false;
     if ((s = run_plain(A, B, out, M, N, K, stream, &done)) != kSuccess || done) return R(s);
   }
+  if ((s = check_result("amemGemmReduceScatter", out)) != kSuccess) return R(s);
   GemmLaunch g;
   memset(&g, 0, sizeof(g));
   fill_fused(c, &g.p);

@@ -221,6 +221,10 @@ ncclResult_t amemSwiGLUGrad(const void* gate, const void* up, long long ld, cons
  * new weights; step counts from 1. */
 ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,
                        double eps, double weight_decay, long long step, cudaStream_t stream);
+/* What amemGemmBf16 does for a problem on a GPU with `sms` SMs, operands and result 16-byte aligned: *form 2 =
+ * few rows (*tile tokens, *slices 2 where tiles are cut along K), 1 = SM pairs (tiles of 256 x *tile, each cut
+ * in *slices along K), 0 = the one-SM form (see amemGemmPlan).  Host arithmetic only; outputs may be NULL. */
+ncclResult_t amemGemmForm(int M, int N, int K, int sms, int* form, int* tile, int* slices);
 /* The tiling of the one-SM form of the GEMM (the fused all-gather GEMM's) for a GPU with `sms` SMs: tile
  * rows (128 or 256), tile columns, K-slices of the last wave (1 = not split).  Host arithmetic only;
  * outputs may be NULL. */

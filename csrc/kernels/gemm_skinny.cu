@@ -411,6 +411,13 @@ bool skinny_gemm_takes(const SkinnyProblem& p) {
   return !(((uintptr_t)p.A | (uintptr_t)p.W) & 15) && !((uintptr_t)p.C & 1) && p.K % 8 == 0 && p.groups <= skinnyk::MAX_GROUPS;
 }
 
+int skinny_gemm_tokens(const SkinnyProblem& d) {
+  // Tokens per tile: all rows of the one group; with several, twice the expected number, so that most
+  // groups take one tile (a second one re-reads the weight tile, from L2).
+  const int want = d.group_off ? 2 * d.rows_per_group : d.rows;
+  return want <= 16 ? 16 : want <= 32 ? 32 : want <= 64 ? 64 : skinnyk::MAX_NT;
+}
+
 bool skinny_gemm_cuts(const SkinnyProblem& d, int sms) {
   // Several groups: whole tiles, so that every sum runs over K in one go, as on SM pairs (a caller's guess
   // of the number of rows, which decides between the two kernels, must not show in the result).  One
@@ -440,10 +447,7 @@ Status launch_skinny_gemm(const SkinnyProblem& d, int sms, cudaStream_t stream) 
   p.ctr = d.ctr;
   p.status = d.status;
   p.timeout_ns = d.timeout_ns;
-  // Tokens per tile: all rows of the one group; with several, twice the expected number, so that most
-  // groups take one tile (a second one re-reads the weight tile, from L2).
-  const int want = d.group_off ? 2 * d.rows_per_group : d.rows;
-  p.nt = want <= 16 ? 16 : want <= 32 ? 32 : want <= 64 ? 64 : k::MAX_NT;
+  p.nt = skinny_gemm_tokens(d);
   p.stages = std::min(k::MAX_STAGES, k::RING_BYTES / (k::W_BYTES + p.nt * k::BK * 2));
   CUtensorMap mw, ma;
   AMEM_TRY(make_bf16_map(&mw, d.W, d.K, d.N, p.groups, d.epilogue == kPairSwiGLUHalves ? k::WM / 2 : k::WM));

@@ -30,6 +30,7 @@ static const int kSkinnyMaxRows = 128;
 
 bool skinny_gemm_takes(const SkinnyProblem& p);
 Status launch_skinny_gemm(const SkinnyProblem& p, int sms, cudaStream_t stream);
+int skinny_gemm_tokens(const SkinnyProblem& p);   // tokens of a tile: 16, 32, 64 or kSkinnyMaxRows
 // Whether launch_skinny_gemm would cut tiles along K, given a workspace.
 bool skinny_gemm_cuts(const SkinnyProblem& p, int sms);
 size_t skinny_gemm_ws_bytes(int sms);

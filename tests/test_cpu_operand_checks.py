@@ -195,3 +195,38 @@ def test_adamw_of_different_sizes_is_refused_as_torch_refuses_it(lib, short):
     with pytest.raises(RuntimeError):
         ops.adamw_step(*ts, 1e-3, (0.9, 0.95), 1e-8, 0.0, 1)
     assert lib.calls == []
+
+
+# ------------------------------------------------------------------ results, and which kernel writes them
+
+def test_gemm_refuses_a_result_that_no_kernel_can_store(monkeypatch):
+    monkeypatch.setenv("AMEM_BACKEND", "mock")
+    from asystem_amem_b200 import Communicator, get_unique_id
+    comm = Communicator(1, 0, get_unique_id())
+    lib = comm.lib
+    ok, odd = 4096, 4098     # never dereferenced
+    for m in (16, 512):
+        assert lib.amemGemmBf16(odd, ok, odd, m, 64, 64, None) == 4      # ncclInvalidArgument
+        assert lib.amemAllGatherGemm(ok, odd, odd, m, 64, 64, comm._h, None) == 4
+        assert lib.amemGemmReduceScatter(odd, ok, odd, m, 64, 64, comm._h, None) == 4
+        assert lib.amemGemmBf16(ok, ok, ok + 1, m, 64, 64, None) == 4
+    comm.destroy()
+
+
+def test_which_gemm_runs_and_how_it_is_tiled(monkeypatch):
+    """(form, tile, slices) on 148 SMs: 2 = few rows, 1 = SM pairs, 0 = one SM."""
+    import ctypes
+
+    def form(M, N, K):
+        v = [ctypes.c_int() for _ in range(3)]
+        assert B.load_library().amemGemmForm(M, N, K, 148, *map(ctypes.byref, v)) == 0
+        return tuple(x.value for x in v)
+
+    assert form(16, 7168, 8192) == (2, 16, 2)          # 56 weight tiles: cut evenly over the SMs
+    assert form(16, 18944, 3584) == (2, 16, 1)         # a weight tile per SM: whole
+    assert form(64, 512, 4096)[0] == 2 and form(65, 512, 4096)[0] == 1
+    assert form(1000, 3584, 8192) == (1, 224, 1)       # 64 whole tiles for 74 pairs
+    assert form(2560, 256, 8192) == (1, 256, 7)        # the most chunks that a cut tile's ring takes
+    assert form(8192, 7168, 8192) == (1, 256, 1)
+    monkeypatch.setenv("AMEM_GEMM_TALL", "0")
+    assert form(8192, 7168, 8192)[0] == 0

@@ -67,3 +67,18 @@ def test_swiglu_with_a_gradient_that_starts_at_an_odd_address():
         swiglu(a).backward(grad)
         got.append(a.grad)
     assert torch.equal(*got)
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 72, 64), (64, 136, 1000), (65, 72, 64), (300, 264, 520), (1000, 1000, 256)])
+@pytest.mark.parametrize("shift", [1, 4])
+def test_gemm_into_a_result_at_an_odd_address(comm, M, N, K, shift):
+    from asystem_amem_b200.ops import all_gather_gemm, gemm_bf16, gemm_reduce_scatter
+    a, b = _rand((M, K), 9), _rand((N, K), 10)
+    ref = a.float() @ b.float().t()
+    for call in (gemm_bf16, lambda *x, **k: all_gather_gemm(comm, *x, **k), lambda *x, **k: gemm_reduce_scatter(comm, *x, **k)):
+        buf = torch.full((M * N + 16,), 3.0, device="cuda", dtype=torch.bfloat16)
+        out = buf[shift:shift + M * N].view(M, N)
+        call(a, b, out=out)
+        # one rounding to bf16 of fp32 sums: at most 2^-8 of the largest
+        assert (out.float() - ref).abs().max().item() <= 2.0 ** -8 * ref.abs().max().item() + 1e-6
+        assert torch.all(buf[:shift] == 3) and torch.all(buf[shift + M * N:] == 3)
