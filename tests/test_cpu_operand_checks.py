@@ -227,6 +227,6 @@ def test_which_gemm_runs_and_how_it_is_tiled(monkeypatch):
     assert form(64, 512, 4096)[0] == 2 and form(65, 512, 4096)[0] == 1
     assert form(1000, 3584, 8192) == (1, 224, 1)       # 64 whole tiles for 74 pairs
     assert form(2560, 256, 8192) == (1, 256, 7)        # the most chunks that a cut tile's ring takes
-    assert form(8192, 7168, 8192) == (1, 256, 1)
+    assert form(8192, 7168, 8192) == (1, 224, 1)       # 1024 tiles: 14 waves of 74, the last 62 of them
     monkeypatch.setenv("AMEM_GEMM_TALL", "0")
     assert form(8192, 7168, 8192)[0] == 0
