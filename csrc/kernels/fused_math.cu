@@ -1,7 +1,8 @@
 // Element-wise passes of the models and the optimizer, each ONE pass over memory: SwiGLU forward and
-// backward, the AdamW update of a parameter shard.  All are bound by HBM: 16-byte accesses, all loads of a
-// thread ahead of its stores, a block per piece of the data (fewer blocks that stride over it are slower,
-// see local_coll.cu).  Arithmetic is fp32; results are rounded once, where they are stored.
+// backward, the AdamW update of a parameter shard.  AdamW is bound by HBM, SwiGLU by HBM and its arithmetic
+// together: 16-byte accesses, all loads of a thread ahead of its stores, a block per piece of the data (fewer
+// blocks that stride over it are slower, see local_coll.cu).  Arithmetic is fp32; results are rounded once,
+// where they are stored.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -34,15 +35,17 @@ __device__ __forceinline__ Bf8 pack(const float (&f)[8]) {
   for (int q = 0; q < 4; ++q) b.h[q] = __floats2bfloat162_rn(f[2 * q], f[2 * q + 1]);
   return b;
 }
-// Good to a few units of fp32 (the results are rounded to 16 bits); 0 for x below -87, where it is under 2^-126.
-__device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+// 1 + exp(-x): the accurate exponential, and its quotients below rounded to the last bit (the approximate pair lost
+// two to six bits of them and everything below -87.3).
+__device__ __forceinline__ float one_plus_exp(float x) { return 1.f + expf(-x); }
 
 // Threads of a block: x along a row, y over rows, one 16-byte vector each (two or four rows a thread need
 // more registers than the resident warps leave: 99 us instead of 70 for the case below).
 //
 // act[r, c] = silu(gate[r, c]) * up[r, c]; gate and up have rows ld elements apart (the halves of one
-// tensor, or two tensors).  4096 x 2 x 14336: five torch passes 409 us, this one 55.7 (6.3 TB/s; 70 with
-// divisions rounded to the last bit).
+// tensor, or two tensors).  4096 x 2 x 14336: five torch passes 409 us, this one 77.8 (4.5 TB/s; L2 flushed,
+// launch included).  The bytes alone take 54; the rest is the arithmetic (61.4 with the approximate
+// exponential and quotient, which are no substitute for fp32).
 __global__ void __launch_bounds__(THREADS) swiglu_kernel(const char* __restrict__ gate, const char* __restrict__ up, long ld, char* __restrict__ act, long rows,
                                                           int F) {
   const int vecs = F / 8, c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -52,12 +55,13 @@ __global__ void __launch_bounds__(THREADS) swiglu_kernel(const char* __restrict_
     unpack(((const Bf8*)(gate + r * ld * 2))[c], g);
     unpack(((const Bf8*)(up + r * ld * 2))[c], u);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) g[q] = g[q] * sigmoid(g[q]) * u[q];
+    for (int q = 0; q < 8; ++q) g[q] = g[q] / one_plus_exp(g[q]) * u[q];
     ((Bf8*)act)[r * vecs + c] = pack(g);
   }
 }
 
-// d gate = g * up * s * (1 + gate * (1 - s)), d up = g * gate * s, s = sigmoid(gate).  The same size: 90.5 us.
+// d gate = g * up * s * (1 + gate * (1 - s)), d up = g * (gate * s), s = sigmoid(gate).  The same size, measured the
+// same way through autograd: 130 us (110 with the approximate pair).
 __global__ void __launch_bounds__(THREADS) swiglu_grad_kernel(const char* __restrict__ gate, const char* __restrict__ up, long ld, const char* __restrict__ g_act,
                                                                char* __restrict__ g_gate, char* __restrict__ g_up, long rows, int F) {
   const int vecs = F / 8, c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -69,8 +73,8 @@ __global__ void __launch_bounds__(THREADS) swiglu_grad_kernel(const char* __rest
     unpack(((const Bf8*)g_act)[r * vecs + c], g);
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      const float s = sigmoid(a[q]);
-      du[q] = g[q] * (a[q] * s);
+      const float e = one_plus_exp(a[q]), s = 1.f / e;
+      du[q] = g[q] * (a[q] / e);
       da[q] = g[q] * u[q] * s * (1.f + a[q] * (1.f - s));
     }
     ((Bf8*)(g_gate + r * ld * 2))[c] = pack(da);

@@ -107,3 +107,34 @@ def test_adamw_other_layouts_take_the_plain_form():
         adamw_step(*ts, shard, 1e-3, (0.9, 0.95), 1e-8, 0.0, 1)
     for a, b in zip(got, want):
         assert torch.allclose(a, b, rtol=1e-5, atol=1e-7)
+
+
+def test_swiglu_keeps_the_precision_of_fp32():
+    """Every bf16 gate against 64 bits: half a unit of bf16 for the one rounding, and before it expf (1 ulp, as
+    documented), an addition, a quotient and the products at half an ulp each -- for the gradient's 1 + gate *
+    (1 - sigmoid) relative to the size of its terms."""
+    from asystem_amem_b200.ops import swiglu
+    gate = torch.arange(65536, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    gate = gate[torch.isfinite(gate) & (gate.abs() < 1e18)]
+    gate = gate[: gate.numel() // 8 * 8]
+    rows = [1.0, -3.140625, 1.0078125e3, 2.0 ** -20, 3.0e36]
+    up = torch.tensor(rows, device="cuda").to(torch.bfloat16).unsqueeze(1).expand(len(rows), gate.numel())
+    h = torch.cat([gate.expand(len(rows), -1), up], dim=1).contiguous().requires_grad_(True)
+    g = torch.full(up.shape, 1.5078125, device="cuda", dtype=torch.bfloat16)
+    out = swiglu(h)
+    (gh,) = torch.autograd.grad(out, h, g)
+    x, u, f = gate.double().expand_as(up), up.double(), gate.numel()
+    s = torch.sigmoid(x)
+    eps = 2.0 ** -24                # half an ulp
+    # where exp(-x) leaves fp32 (x < -88.7) the plain form in fp32 gives zero as well
+    inside = x > -88.7
+
+    def check(got, want, size, ulps):
+        room = 2.0 ** (torch.floor(torch.log2(want.abs().clamp(min=2.0 ** -126))) - 8) + size * ulps * eps + 2.0 ** -133
+        bad = inside & want.abs().lt(3e38) & ((got.double() - want).abs() > room)
+        assert not bad.any(), (x[bad][:5], got[bad][:5], want[bad][:5])
+
+    check(out.detach(), x * s * u, (x * s * u).abs(), 5)
+    check(gh[:, f:], 1.5078125 * x * s, (1.5078125 * x * s).abs(), 5)
+    scale = 1.5078125 * u.abs() * s
+    check(gh[:, :f], 1.5078125 * u * s * (1 + x * (1 - s)), scale * (1 + (x * (1 - s)).abs()), 10)
