@@ -6,6 +6,7 @@ from __future__ import annotations
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from .. import bindings as B
 from .operands import dense, on_device_of
@@ -16,7 +17,8 @@ def _st() -> int:
 
 
 def _fused(h: torch.Tensor) -> bool:
-    return h.is_cuda and h.dtype == torch.bfloat16 and h.dim() == 2 and h.shape[1] % 16 == 0 and h.data_ptr() % 16 == 0
+    """One dense bf16 tensor without a tangent (the kernel knows nothing of forward-mode gradients)."""
+    return forward_ad.unpack_dual(h).tangent is None and h.is_cuda and h.dtype == torch.bfloat16 and h.dim() == 2 and h.shape[1] % 16 == 0 and h.data_ptr() % 16 == 0
 
 
 class _SwiGLU(torch.autograd.Function):

@@ -37,6 +37,8 @@ def lib(monkeypatch):
     monkeypatch.setattr(B, "load_library", lambda *a, **k: rec)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: SimpleNamespace(cuda_stream=0))
     monkeypatch.setattr(torch.cuda, "current_device", lambda: -1)
+    empty = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *args, **kw: empty(*args, **kw).as_subclass(OnGpu))
     return rec
 
 
@@ -66,9 +68,7 @@ def test_products_refuse_other_ranks_and_inner_dimensions(lib, make):
 
 
 def test_an_mlp_refuses_a_batch_of_sequences(lib):
-    from asystem_amem_b200.models import TPMLP
-    layer = TPMLP(SimpleNamespace(nranks=1, lib=lib, _h=1), 64, 32, device="cpu")
-    layer.w13.weight = torch.nn.Parameter(layer.w13.weight.detach().as_subclass(OnGpu), requires_grad=False)
+    layer = _mlp(lib)
     with torch.no_grad(), pytest.raises(ValueError):
         layer(gpu(2, 16, 64))
     assert [name for name, _ in lib.calls if "Gemm" in name] == []
@@ -84,6 +84,10 @@ def shifted(*shape):
     flat = torch.arange(n + 1, dtype=torch.float32).to(BF16)
     assert flat.data_ptr() % 16 == 0
     return flat[1:].view(*shape).as_subclass(OnGpu)
+
+
+def _backward(out, g):
+    torch.autograd.backward(out.as_subclass(torch.Tensor), g)     # (a subclass's own backward() would shed the subclass inside)
 
 
 def _dispatcher(lib, E=4, d=8, capacity=64):
@@ -144,9 +148,9 @@ def test_gradients_at_odd_addresses_reach_the_kernels_on_16_bytes(lib):
     from asystem_amem_b200.models.moe_layer import GroupedLinear
     from asystem_amem_b200.ops import swiglu
     h = gpu(6, 32).requires_grad_(True)
-    swiglu(h).backward(shifted(6, 16))
+    _backward(swiglu(h), shifted(6, 16))
     w, offs = gpu(2, 16, 8).requires_grad_(True), torch.tensor([0, 2, 6], dtype=torch.int32).as_subclass(OnGpu)
-    GroupedLinear.apply(gpu(6, 8), w, offs).backward(shifted(6, 16))
+    _backward(GroupedLinear.apply(gpu(6, 8), w, offs), shifted(6, 16))
     rows = {"amemSwiGLUGrad": 3, "amemGroupedGemmBf16Weight": 0}
     seen = {name: args for name, args in lib.calls}
     assert all(seen[name][i] % 16 == 0 for name, i in rows.items())
@@ -174,7 +178,7 @@ def test_launches_make_the_operands_device_current(lib, monkeypatch):
     monkeypatch.setattr(OnGpu, "get_device", lambda self: 3, raising=False)
     offs = torch.tensor([0, 2, 6], dtype=torch.int32).as_subclass(OnGpu)
     h = gpu(6, 32).requires_grad_(True)
-    ops.swiglu(h).backward(gpu(6, 16))
+    _backward(ops.swiglu(h), gpu(6, 16))
     ops.adamw_step(*(gpu(16, dtype=torch.float32) for _ in range(4)), gpu(16), 1e-3, (0.9, 0.95), 1e-8, 0.0, 1)
     ops.gemm_bf16(gpu(8, 64), gpu(16, 64))
     ops.gemm_swiglu(gpu(8, 64), gpu(16, 64))
@@ -230,3 +234,45 @@ def test_which_gemm_runs_and_how_it_is_tiled(monkeypatch):
     assert form(8192, 7168, 8192) == (1, 224, 1)       # 1024 tiles: 14 waves of 74, the last 62 of them
     monkeypatch.setenv("AMEM_GEMM_TALL", "0")
     assert form(8192, 7168, 8192)[0] == 0
+
+
+# ------------------------------------------------------------------ what a fused path must not pass by
+
+def _mlp(lib):
+    from asystem_amem_b200.models import TPMLP
+    layer = TPMLP(SimpleNamespace(nranks=1, lib=lib, _h=1), 64, 32, device="cpu")
+    for m in (layer.w13, layer.w2):
+        m.weight = torch.nn.Parameter(m.weight.detach().as_subclass(OnGpu), requires_grad=False)
+    return layer
+
+
+def test_tangents_are_carried_or_refused_not_dropped(lib):
+    import torch.autograd.forward_ad as fwad
+    from asystem_amem_b200 import ops
+    layer = _mlp(lib)
+    with fwad.dual_level(), torch.no_grad():
+        h = fwad.make_dual(gpu(4, 32), gpu(4, 32) + 1)
+        out = ops.swiglu(h)
+        assert fwad.unpack_dual(out).tangent is not None
+        assert lib.calls == []
+        with pytest.raises(NotImplementedError):
+            layer(fwad.make_dual(gpu(16, 64), gpu(16, 64)))
+    with torch.no_grad():
+        layer(gpu(16, 64))
+    assert [name for name, _ in lib.calls][-2:] == ["amemGemmSwiGLU", "amemGemmReduceScatter"]
+
+
+def test_hooks_of_the_projection_run(lib):
+    from torch.nn.modules.module import register_module_forward_hook
+    layer, seen = _mlp(lib), []
+    with torch.no_grad():
+        handle = register_module_forward_hook(lambda m, args, out: seen.append(m))
+        try:
+            layer(gpu(16, 64))
+        finally:
+            handle.remove()
+        assert layer.w13 in seen and layer.w2 in seen
+        handle = layer.w13.register_forward_hook(lambda m, args, out: seen.append("own"))
+        layer(gpu(16, 64))
+        handle.remove()
+    assert seen[-1] == "own" and "amemGemmSwiGLU" not in {name for name, _ in lib.calls}
