@@ -48,9 +48,10 @@ def dispatch_forward(disp: MoeDispatcher, x: torch.Tensor, idx: torch.Tensor):
     received rows (the receive buffer is reused by the next dispatch)."""
     local = disp.local(x) and x.shape[0] == idx.shape[0]
     res = disp.dispatch_local(x.contiguous(), idx) if local else disp.dispatch(x.contiguous(), idx)
-    total = int(res.expert_offsets[-1].item())  # host sync: the group boundaries are needed on the host anyway
-    rows = res.recv_x[:total]
-    return rows if local else rows.clone(), res.expert_offsets, res.send_pos, total
+    total = int(res.expert_offsets[-1].item())  # host sync: `rows` has exactly the rows that arrived
+    # (shrunk, not sliced: a view made inside an autograd function could not be changed in place)
+    rows = res.recv_x.resize_(total, disp.d) if local else res.recv_x[:total].clone()
+    return rows, res.expert_offsets, res.send_pos, total
 
 
 def dispatch_backward(disp: MoeDispatcher, g_rows: torch.Tensor, idx: torch.Tensor, send_pos: torch.Tensor) -> torch.Tensor:

@@ -276,3 +276,19 @@ def test_hooks_of_the_projection_run(lib):
         layer(gpu(16, 64))
         handle.remove()
     assert seen[-1] == "own" and "amemGemmSwiGLU" not in {name for name, _ in lib.calls}
+
+
+def test_dispatched_rows_can_be_changed_in_place(lib):
+    from asystem_amem_b200.ops.moe import DispatchResult
+    from asystem_amem_b200.parallel import ep
+    disp = _dispatcher(lib)
+    disp.local = lambda *rows: True
+    disp.dispatch_local = lambda x, idx: DispatchResult(torch.ones(12, 8, dtype=BF16), None, torch.tensor([0, 4, 7, 9, 10], dtype=torch.int32),
+                                                        torch.zeros(6, 2, dtype=torch.int32))
+    disp.combine_local = lambda g, idx, w, pos: g[:6] * 1.0
+    x = torch.zeros(6, 8, dtype=BF16, requires_grad=True)
+    rows, _, _ = ep.ep_dispatch(disp, x, torch.zeros(6, 2, dtype=torch.int32))
+    rows.mul_(2)
+    assert rows.shape == (10, 8) and torch.all(rows == 2)
+    rows.sum().backward()
+    assert torch.all(x.grad == 2)

@@ -58,6 +58,24 @@ def test_moe_steps_on_rows_at_odd_addresses(comm):
         assert torch.equal(a, b)
 
 
+def test_dispatched_rows_changed_in_place(comm):
+    from asystem_amem_b200.ops import MoeDispatcher
+    from asystem_amem_b200.parallel import ep_combine, ep_dispatch
+    T, k, E, d = 21, 2, 4, 64
+    disp = MoeDispatcher(comm, E, d, T * k - 5)      # a few rows find no room
+    idx = torch.randint(0, E, (T, k), generator=torch.Generator().manual_seed(11), dtype=torch.int32).cuda()
+    got = []
+    for in_place in (False, True):
+        x, w = _rand((T, d), 12).requires_grad_(True), torch.full((T, k), 0.5, device="cuda")
+        rows, _, pos = ep_dispatch(disp, x, idx)
+        assert rows.shape == (T * k - 5, d)
+        rows = rows.mul_(2) if in_place else rows * 2
+        out = ep_combine(disp, rows, w, idx, pos)
+        out.backward(_rand((T, d), 13))
+        got.append((out.detach(), x.grad))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 def test_swiglu_with_a_gradient_that_starts_at_an_odd_address():
     from asystem_amem_b200.ops import swiglu
     h, g = _rand((33, 48), 7), _rand((33, 24), 8)
