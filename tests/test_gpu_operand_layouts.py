@@ -60,7 +60,7 @@ def test_moe_steps_on_rows_at_odd_addresses(comm):
 
 def test_dispatched_rows_changed_in_place(comm):
     from asystem_amem_b200.ops import MoeDispatcher
-    from asystem_amem_b200.parallel import ep_combine, ep_dispatch
+    from asystem_amem_b200.parallel.ep import ep_combine, ep_dispatch
     T, k, E, d = 21, 2, 4, 64
     disp = MoeDispatcher(comm, E, d, T * k - 5)      # a few rows find no room
     idx = torch.randint(0, E, (T, k), generator=torch.Generator().manual_seed(11), dtype=torch.int32).cuda()
