@@ -39,5 +39,6 @@ class TPMLP(nn.Module):
         """x_shard: bf16 [tokens / tp, dim] -> bf16 [tokens / tp, dim]"""
         if self.comm.nranks == 1 and x_shard.is_cuda and self.ffn_local % 8 == 0 and self._calls_nothing_else(x_shard):
             # one rank: the activation rides in the projection's epilogue
+            self.w13.comm.begin(x_shard)
             return self.w2(gemm_swiglu(x_shard.contiguous(), self.w13.weight.contiguous()))
         return self.w2(swiglu(self.w13(x_shard)).to(torch.bfloat16))

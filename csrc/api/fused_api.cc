@@ -297,6 +297,13 @@ Status run_plain(const void* A, const void* B, void* C, int M, int N, int K, cud
 
 extern "C" {
 
+ncclResult_t amemCommBegin(ncclComm_t comm, cudaStream_t stream) {
+  if (!comm) return ncclInvalidArgument;
+  Comm* c = reinterpret_cast<Comm*>(comm);
+  const Status s = c->check_usable("amemCommBegin");
+  return R(s == kSuccess ? c->prepare_stream(stream) : s);
+}
+
 // C[M, N] = A * B with either operand stored by its contraction index: a_by_k = 0: A [M, K], 1: A [K, M];
 // b_by_k = 0: B [N, K], 1: B [K, N].  (0, 0), (0, 1) and (1, 1) are built: a Linear's output, its input
 // gradient and its weight gradient.  K may be any number where both operands are stored by K.

@@ -221,6 +221,10 @@ ncclResult_t amemSwiGLUGrad(const void* gate, const void* up, long long ld, cons
  * new weights; step counts from 1. */
 ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,
                        double eps, double weight_decay, long long step, cudaStream_t stream);
+/* Refuses what an operation of the communicator would be refused for (paused, aborted, in error, another device
+ * current) and orders the stream behind the communicator's previous one: for callers whose operation has
+ * nothing to send, because the communicator has one rank, and who run it without the communicator. */
+ncclResult_t amemCommBegin(ncclComm_t comm, cudaStream_t stream);
 /* What amemGemmBf16 does for a problem on a GPU with `sms` SMs, operands and result 16-byte aligned: *form 2 =
  * few rows (*tile tokens, *slices 2 where tiles are cut along K), 1 = SM pairs (tiles of 256 x *tile, each cut
  * in *slices along K), 0 = the one-SM form (see amemGemmPlan).  Host arithmetic only; outputs may be NULL. */

@@ -240,7 +240,7 @@ def test_which_gemm_runs_and_how_it_is_tiled(monkeypatch):
 
 def _mlp(lib):
     from asystem_amem_b200.models import TPMLP
-    layer = TPMLP(SimpleNamespace(nranks=1, lib=lib, _h=1), 64, 32, device="cpu")
+    layer = TPMLP(SimpleNamespace(nranks=1, lib=lib, _h=1, begin=lambda t: lib.amemCommBegin(1, 0)), 64, 32, device="cpu")
     for m in (layer.w13, layer.w2):
         m.weight = torch.nn.Parameter(m.weight.detach().as_subclass(OnGpu), requires_grad=False)
     return layer
@@ -259,7 +259,7 @@ def test_tangents_are_carried_or_refused_not_dropped(lib):
             layer(fwad.make_dual(gpu(16, 64), gpu(16, 64)))
     with torch.no_grad():
         layer(gpu(16, 64))
-    assert [name for name, _ in lib.calls][-2:] == ["amemGemmSwiGLU", "amemGemmReduceScatter"]
+    assert [name for name, _ in lib.calls][-3:] == ["amemCommBegin", "amemGemmSwiGLU", "amemGemmReduceScatter"]
 
 
 def test_hooks_of_the_projection_run(lib):
@@ -292,3 +292,21 @@ def test_dispatched_rows_can_be_changed_in_place(lib):
     assert rows.shape == (10, 8) and torch.all(rows == 2)
     rows.sum().backward()
     assert torch.all(x.grad == 2)
+
+
+def test_a_paused_communicator_of_one_rank_refuses_the_backward_pass(monkeypatch):
+    monkeypatch.setenv("AMEM_BACKEND", "mock")
+    from asystem_amem_b200 import Communicator, get_unique_id
+    from asystem_amem_b200.bindings import NcclError
+    from asystem_amem_b200.parallel import ColumnParallelLinear, RowParallelLinear
+    comm = Communicator(1, 0, get_unique_id())
+    for kind in (ColumnParallelLinear, RowParallelLinear):
+        layer, x = kind(64, 32, comm, device="cpu"), torch.ones(4, 64, dtype=BF16, requires_grad=True)
+        out = layer(x).sum()
+        comm.pause()
+        with pytest.raises(NcclError):
+            out.backward(retain_graph=True)
+        comm.resume()
+        out.backward()
+        assert torch.isfinite(x.grad).all()
+    comm.destroy()
