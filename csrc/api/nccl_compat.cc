@@ -456,6 +456,22 @@ ncclResult_t amemTunerPlan(int kind, size_t count, ncclDataType_t dtype, int nra
   if (chunk_elems) *chunk_elems = p.chunk_elems;
   return ncclSuccess;
 }
+// Blocks of the single-pass form of a collective on a communicator of one rank (buffers 16-byte aligned), with
+// the communicator's blocks bounded to block_cap (0: not bounded); *blocks 0: the general kernel runs.
+ncclResult_t amemLocalPlan(size_t count, ncclDataType_t dtype, ncclDataType_t out_dtype, float scale, int block_cap, size_t* blocks) {
+  if (!blocks || dtype_size(dtype) == 0 || dtype_size(out_dtype) == 0) return ncclInvalidArgument;
+  CollArgs a;
+  memset(&a, 0, sizeof(a));
+  a.nranks = 1;
+  a.count = count;
+  a.dtype = dtype;
+  a.out_dtype = out_dtype;
+  a.scale = scale;
+  a.has_scale = 1;
+  a.recv = (void*)16;   // (another buffer than send)
+  *blocks = local_blocks(a, block_cap);
+  return ncclSuccess;
+}
 // Checks the staging guard of `comm` now (AMEM_CANARY=1; ncclSuccess when the guard is off).
 ncclResult_t amemCheckCanary(ncclComm_t comm) {
   NEED_COMM(comm);

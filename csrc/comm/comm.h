@@ -167,6 +167,7 @@ class Comm {
   bool status_pinned_ = false;
   unsigned long long timeout_ns_ = 0;
   int max_blocks_ = 64;
+  int block_cap_ = 0;   // max_blocks_ where the user set it, 0 where it is the default
   size_t canary_bytes_ = 0;
   bool paused_ = false, aborted_ = false;
   int async_error_ = 0;

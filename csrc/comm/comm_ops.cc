@@ -156,6 +156,7 @@ Status Comm::collective(int kind, const void* send, void* recv, size_t count, in
   ti.p2p_slot_bytes = p2p_slot_bytes_;
   ti.nvls = nvls();
   ti.max_blocks = max_blocks_;
+  ti.block_cap = block_cap_;
   ti.forced_algo = algo;
   // Both operands inside registered windows, at the same offsets on every rank (the caller's
   // contract, as for NCCL's symmetric windows): the all-reduce can work on them in place.

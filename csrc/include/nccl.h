@@ -237,6 +237,9 @@ ncclResult_t amemGemmForm(int M, int N, int K, int sms, int* form, int* tile, in
  * GPUs; stage_bytes 0 = default staging.  Host arithmetic only. */
 ncclResult_t amemTunerPlan(int kind, size_t count, ncclDataType_t dtype, int nranks, int nvls, size_t stage_bytes, int* algo,
                            int* blocks, size_t* chunk_elems);
+/* Blocks of the single-pass form of a collective on a communicator of one rank (*blocks; 0: the general kernel
+ * runs) whose blocks the user bounds to block_cap (maxCTAs, AMEM_MAX_BLOCKS; 0: no bound).  Host arithmetic only. */
+ncclResult_t amemLocalPlan(size_t count, ncclDataType_t dtype, ncclDataType_t out_dtype, float scale, int block_cap, size_t* blocks);
 /* Debug guard behind the staging layout (AMEM_CANARY=1): ncclInternalError if a kernel wrote past it. */
 /* Variable-size all-to-all; counts and displacements in elements, MPI_Alltoallv convention. */
 ncclResult_t amemAlltoAllv(const void* sendbuff, const size_t* sendcounts, const size_t* sdispls, void* recvbuff,

@@ -131,6 +131,7 @@ struct LaunchPlan {
   int blocks;
   int threads;
   size_t chunk_elems;   // elements of the per-chunk unit (meaning depends on kind)
+  int block_cap = 0;    // most blocks the user allows, 0: no bound beyond the default
 };
 
 // ---- staging layout, computed the same way on host and device --------------------------

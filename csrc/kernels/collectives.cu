@@ -462,7 +462,7 @@ Status launch_collective(const CollArgs& a, const LaunchPlan& plan, cudaStream_t
     return check_launch("sendrecv");
   }
   bool ok = true, local = false;
-  const Status st_local = launch_local(a, stream, &local);
+  const Status st_local = launch_local(a, plan.block_cap, stream, &local);
   if (local) return st_local;
   if (a.kind == kCollAllReduce && a.algo == kAlgoNvls && a.nranks > 1) {
     if (a.dtype == kF32) dev::nvls_allreduce_kernel<float><<<grid, block, 0, stream>>>(a, plan.chunk_elems);

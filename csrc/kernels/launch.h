@@ -9,9 +9,11 @@ namespace amem {
 
 // Launches one rank's kernel on `stream`.
 Status launch_collective(const CollArgs& a, const LaunchPlan& plan, cudaStream_t stream);
-// The same for a communicator of one rank, where that is a copy or a scale and cast of aligned buffers;
-// *handled is false where launch_collective has to do it.
-Status launch_local(const CollArgs& a, cudaStream_t stream, bool* handled);
+// The same for a communicator of one rank, where that is a copy or a scale and cast of aligned buffers and
+// takes no more blocks than block_cap (0: any number); *handled is false where launch_collective has to do it.
+Status launch_local(const CollArgs& a, int block_cap, cudaStream_t stream, bool* handled);
+// The blocks launch_local runs for this operation; 0: it does not take it.
+size_t local_blocks(const CollArgs& a, int block_cap);
 // Launches every rank of an emulated (single-GPU) communicator as one cooperative grid.
 // `dev_all` points to `nranks` CollArgs in device-readable memory; `a` is any rank's copy
 // (used for type dispatch only).
@@ -30,6 +32,7 @@ struct TunerInput {
   size_t stage_bytes, p2p_slot_bytes;
   bool nvls;          // multicast mapping available
   int max_blocks;     // upper bound for this communicator (emulated comms use a small one)
+  int block_cap = 0;  // the same where the user set it (maxCTAs, AMEM_MAX_BLOCKS), 0: nobody did
   int forced_algo;    // kAlgoAuto or a variant forced by AMEM_ALGO / the API
   bool window = false;      // all-reduce: both operands lie in registered windows at vector-aligned offsets
   bool window_mc = false;   // ... and the windows have multicast mappings

@@ -68,23 +68,34 @@ bool narrow_float(int t) { return t == kF32 || t == kBF16 || t == kF16; }
 
 }  // namespace localk
 
-// Takes a one-rank collective where it is a plain copy, or a scale and cast among fp32 / bf16 / fp16, of
-// 16-byte aligned buffers; everything else (other types with a scale, odd addresses) is left to the
-// general kernel.  *handled tells.
-Status launch_local(const CollArgs& a, cudaStream_t stream, bool* handled) {
+// What a one-rank collective is as a single pass over aligned buffers: 1 a plain copy, 2 a scale and cast
+// among fp32 / bf16 / fp16, 0 neither (other types with a scale, odd addresses): the general kernel's.
+static int local_form(const CollArgs& a) {
   using namespace localk;
-  *handled = false;
-  if (a.nranks != 1 || (((uintptr_t)a.send | (uintptr_t)a.recv) & 15)) return kSuccess;
-  if (a.dtype > kBF16 || a.out_dtype > kBF16) return kSuccess;   // 8-bit floats as such: reductions of them are refused there
-  const bool copy = a.dtype == a.out_dtype && (!a.has_scale || (a.scale == 1.0f && narrow_float(a.dtype)));
+  if (a.nranks != 1 || (((uintptr_t)a.send | (uintptr_t)a.recv) & 15)) return 0;
+  if (a.dtype > kBF16 || a.out_dtype > kBF16) return 0;   // 8-bit floats as such: reductions of them are refused there
+  if (a.dtype == a.out_dtype && (!a.has_scale || (a.scale == 1.0f && narrow_float(a.dtype)))) return 1;
   const bool pair = a.dtype == a.out_dtype || a.dtype == kF32 || a.out_dtype == kF32;   // bf16 <-> fp16 is refused
-  const bool scale = narrow_float(a.dtype) && narrow_float(a.out_dtype) && pair;
-  if (!copy && !scale) return kSuccess;
-  if (a.send == a.recv && !copy) return kSuccess;
-  *handled = true;
-  if (a.send == a.recv) return kSuccess;   // in place: nothing to move
-  const size_t items = copy ? a.count * dtype_size(a.dtype) / 16 : a.count / 4, per_block = (size_t)THREADS * (copy ? AHEAD : CAST_AHEAD);
+  return narrow_float(a.dtype) && narrow_float(a.out_dtype) && pair && a.send != a.recv ? 2 : 0;
+}
+
+// A block per piece.  Where the user bounds the blocks of a communicator (maxCTAs, AMEM_MAX_BLOCKS), because
+// the other SMs are for something else, what needs more of them is left to the general kernel, which strides.
+size_t local_blocks(const CollArgs& a, int block_cap) {
+  using namespace localk;
+  const int form = local_form(a);
+  if (!form) return 0;
+  const size_t items = form == 1 ? a.count * dtype_size(a.dtype) / 16 : a.count / 4, per_block = (size_t)THREADS * (form == 1 ? AHEAD : CAST_AHEAD);
   const size_t blocks = std::max<size_t>(1, (items + per_block - 1) / per_block);
+  return block_cap > 0 && blocks > (size_t)block_cap ? 0 : blocks;
+}
+
+Status launch_local(const CollArgs& a, int block_cap, cudaStream_t stream, bool* handled) {
+  using namespace localk;
+  const size_t blocks = local_blocks(a, block_cap);
+  const bool copy = local_form(a) == 1;
+  *handled = blocks > 0;
+  if (blocks == 0 || a.send == a.recv) return kSuccess;   // (in place: nothing to move)
   if (blocks > 0x7fffffffu) return fail(kInvalidArgument, "one-rank collective of %zu elements", (size_t)a.count);
   const int grid = (int)blocks;
   cudaError_t e;

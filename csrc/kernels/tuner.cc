@@ -24,6 +24,7 @@ static int env_algo() {
 LaunchPlan plan_collective(const TunerInput& in) {
   LaunchPlan p;
   p.threads = 512;
+  p.block_cap = in.block_cap;
   p.algo = kAlgoAuto;
   const size_t es = dtype_size(in.dtype);
   const int n = in.nranks;
@@ -95,6 +96,7 @@ LaunchPlan plan_collective(const TunerInput& in) {
   // always the same number of blocks: the blocks' operation counts (the packets' flag) then move in
   // lockstep, so a word's flag depends on the operation only, never on which block wrote it
   if (ll) blocks = std::min<long>(4, in.max_blocks);
+  if (blocks_env > 0) p.block_cap = (int)std::min<long>(blocks_env, in.max_blocks);
   if (blocks_env > 0 && !ll) blocks = std::min<long>(blocks_env, in.max_blocks);
   if (blocks > kMaxBlocks) blocks = kMaxBlocks;
   p.blocks = (int)blocks;

@@ -310,3 +310,18 @@ def test_a_paused_communicator_of_one_rank_refuses_the_backward_pass(monkeypatch
         out.backward()
         assert torch.isfinite(x.grad).all()
     comm.destroy()
+
+
+def test_a_bound_on_a_communicators_blocks_holds_on_one_rank():
+    """maxCTAs / AMEM_MAX_BLOCKS: what the single-pass form would need more blocks for goes to the general kernel."""
+    import ctypes
+
+    def blocks(count, cap, tin="bfloat16", tout="bfloat16", scale=1.0):
+        n = ctypes.c_size_t()
+        assert B.load_library().amemLocalPlan(ctypes.c_size_t(count), B.DTYPES[tin], B.DTYPES[tout], ctypes.c_float(scale), cap, ctypes.byref(n)) == 0
+        return n.value
+
+    assert blocks(8192 * 100, 0) == 100 and blocks(8192 * 100, 100) == 100      # 16 KB a block
+    assert blocks(8192 * 100, 99) == 0 and blocks(1, 1) == 1
+    assert blocks(8192 * 10 + 4, 0, tout="float32", scale=0.5) == 11 and blocks(8192 * 10 + 4, 10, tout="float32", scale=0.5) == 0
+    assert blocks(8192, 0, tout="float16", scale=0.5) == 0

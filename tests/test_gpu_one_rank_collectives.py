@@ -64,3 +64,17 @@ def test_what_is_refused_stays_refused(comm):
     with pytest.raises(NcclError):
         comm.reduce_scatter(x.to(torch.bfloat16), x.to(torch.float16), scale=1.0)
     comm.all_gather(f8, torch.empty_like(f8))
+
+
+def test_bounded_blocks(monkeypatch):
+    from asystem_amem_b200 import Communicator, get_unique_id
+    monkeypatch.setenv("AMEM_MAX_BLOCKS", "3")
+    c = Communicator(1, 0, get_unique_id())
+    for n in (1000, 1_000_003):       # one block, and more than three
+        x, wide = _data(n, torch.bfloat16, n), torch.empty(n, device="cuda")
+        out = torch.empty_like(x)
+        c.all_reduce(x, out)
+        c.reduce_scatter(x, wide, scale=0.25)
+        assert torch.equal(out, x) and torch.equal(wide, x.float() * 0.25)
+    torch.cuda.synchronize()
+    c.destroy()
