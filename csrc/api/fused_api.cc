@@ -394,6 +394,7 @@ ncclResult_t amemAllGatherGemmPlan(int nranks, int rows_per_rank, int K, int* mo
 ncclResult_t amemGemmBf16(const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream) {
   Status s = check_shape(M, N, K);
   if (s != kSuccess) return R(s);
+  if (!A || !B || !C) return R(fail(kInvalidArgument, "GEMM: null buffer"));
   bool done = false;
   if ((s = run_plain(A, B, C, M, N, K, stream, &done)) != kSuccess || done) return R(s);
   int dev = 0;

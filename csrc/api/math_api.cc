@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <initializer_list>
 
 #include "../core/log.h"
 #include "../include/nccl.h"
@@ -18,6 +19,13 @@ inline ncclResult_t R(Status s) {
 
 bool aligned16(const void* a, const void* b, const void* c) { return !(((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15); }
 
+// (an empty tensor has no address: asked only where there is something to read)
+bool missing(std::initializer_list<const void*> buffers) {
+  for (const void* p : buffers)
+    if (!p) return true;
+  return false;
+}
+
 }  // namespace
 
 extern "C" {
@@ -25,6 +33,7 @@ extern "C" {
 ncclResult_t amemSwiGLU(const void* gate, const void* up, long long ld, void* act, long long rows, int F, cudaStream_t stream) {
   if (rows < 0 || F <= 0 || F % 8 || ld < F || ld % 8 || !aligned16(gate, up, act))
     return R(fail(kInvalidArgument, "amemSwiGLU: rows=%lld F=%d ld=%lld (multiples of 8, 16-byte aligned)", rows, F, ld));
+  if (rows > 0 && missing({gate, up, act})) return R(fail(kInvalidArgument, "amemSwiGLU: null buffer"));
   return rows == 0 ? ncclSuccess : R(launch_swiglu(gate, up, (long)ld, act, (long)rows, F, stream));
 }
 
@@ -32,6 +41,7 @@ ncclResult_t amemSwiGLUGrad(const void* gate, const void* up, long long ld, cons
                             cudaStream_t stream) {
   if (rows < 0 || F <= 0 || F % 8 || ld < F || ld % 8 || !aligned16(gate, up, g_act) || !aligned16(g_gate, g_up, nullptr))
     return R(fail(kInvalidArgument, "amemSwiGLUGrad: rows=%lld F=%d ld=%lld (multiples of 8, 16-byte aligned)", rows, F, ld));
+  if (rows > 0 && missing({gate, up, g_act, g_gate, g_up})) return R(fail(kInvalidArgument, "amemSwiGLUGrad: null buffer"));
   return rows == 0 ? ncclSuccess : R(launch_swiglu_grad(gate, up, (long)ld, g_act, g_gate, g_up, (long)rows, F, stream));
 }
 
@@ -40,6 +50,7 @@ ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, voi
   if (n < 0 || step < 1 || !aligned16(grad, m, v) || !aligned16(master, shard_bf16, nullptr))
     return R(fail(kInvalidArgument, "amemAdamW: n=%lld step=%lld (buffers 16-byte aligned)", n, step));
   if (n == 0) return ncclSuccess;
+  if (missing({grad, m, v, master, shard_bf16})) return R(fail(kInvalidArgument, "amemAdamW: null buffer"));
   AdamW a;
   a.lr = (float)lr;
   a.b1 = (float)beta1;

@@ -325,3 +325,18 @@ def test_a_bound_on_a_communicators_blocks_holds_on_one_rank():
     assert blocks(8192 * 100, 99) == 0 and blocks(1, 1) == 1
     assert blocks(8192 * 10 + 4, 0, tout="float32", scale=0.5) == 11 and blocks(8192 * 10 + 4, 10, tout="float32", scale=0.5) == 0
     assert blocks(8192, 0, tout="float16", scale=0.5) == 0
+
+
+def test_entry_points_refuse_missing_buffers():
+    lib, ok = B.load_library(), 4096       # never dereferenced
+    for i in range(3):
+        bufs = [ok, ok, ok]
+        bufs[i] = None
+        assert lib.amemSwiGLU(bufs[0], bufs[1], 16, bufs[2], 2, 8, None) == 4      # ncclInvalidArgument
+        assert lib.amemGemmBf16(*bufs, 16, 64, 64, None) == 4
+    for i in range(5):
+        bufs = [ok] * 5
+        bufs[i] = None
+        assert lib.amemSwiGLUGrad(bufs[0], bufs[1], 16, *bufs[2:], 2, 8, None) == 4
+        assert lib.amemAdamW(*bufs, 8, 1e-3, 0.9, 0.95, 1e-8, 0.0, 1, None) == 4
+    assert lib.amemSwiGLU(None, None, 16, None, 0, 8, None) == 0
