@@ -28,6 +28,14 @@ def on_pairs():
     os.environ.pop("AMEM_GEMM_PAIR", None)
 
 
+@pytest.fixture
+def groups_on_pairs():
+    """(Few rows a group would go to the kernel for few rows otherwise.)"""
+    os.environ["AMEM_GEMM_SKINNY"] = "0"
+    yield
+    os.environ.pop("AMEM_GEMM_SKINNY", None)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 8, 8), (128, 128, 64), (129, 136, 72), (255, 264, 328), (257, 1000, 2056), (520, 776, 4096), (300, 256, 8192),
                                    (2200, 2568, 512)])
 def test_products_of_a_linear_and_its_gradients(on_pairs, M, N, K):
@@ -48,7 +56,7 @@ def test_weight_gradient_of_any_number_of_rows(on_pairs, T):
 
 @pytest.mark.parametrize("counts", [(1, 0, 63, 64, 65, 300), (0, 0, 5), (256, 256), (17,), (0, 1000, 31)])
 @pytest.mark.parametrize("N,K", [(192, 128), (264, 72)])
-def test_groups(counts, N, K):
+def test_groups(groups_on_pairs, counts, N, K):
     from asystem_amem_b200.ops import grouped_gemm_bf16, grouped_gemm_input_grad, grouped_gemm_weight_grad
     E, rows, pad = len(counts), sum(counts), 9
     offs = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device="cuda")
@@ -70,7 +78,7 @@ def test_groups(counts, N, K):
             assert torch.all(gw[e] == 0)
 
 
-def test_a_group_does_not_see_its_neighbours_values():
+def test_a_group_does_not_see_its_neighbours_values(groups_on_pairs):
     """Infinities and NaN in the rows and matrices next to a group's own stay out of its results."""
     from asystem_amem_b200.ops import grouped_gemm_bf16, grouped_gemm_input_grad, grouped_gemm_weight_grad
     counts, N, K = (37, 50, 41), 200, 72
@@ -87,7 +95,7 @@ def test_a_group_does_not_see_its_neighbours_values():
 
 
 @pytest.mark.parametrize("ffn", [32, 96, 160, 1024])
-def test_swiglu_epilogue(ffn):
+def test_swiglu_epilogue(groups_on_pairs, ffn):
     from asystem_amem_b200.ops import grouped_gemm_bf16, interleave_gate_up
     offs = torch.tensor([0, 130, 130, 400], dtype=torch.int32, device="cuda")
     a, w = _rand((400, 256), 12), _rand((3, 2 * ffn, 256), 13, 0.1)
