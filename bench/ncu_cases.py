@@ -68,6 +68,34 @@ def main():
         for _ in range(reps):
             grouped_gemm_bf16(x, w13, offs, out=act, rows_hint=rows, swiglu=True)
         torch.cuda.synchronize()
+    elif args.case == "one_gpu":
+        # the kernels of the single-GPU paths in turn, inputs larger than L2 wherever the kernel is bound by memory
+        from asystem_amem_b200 import Communicator, get_unique_id
+        from asystem_amem_b200.ops import MoeDispatcher, adamw_step, gemm_bf16, gemm_swiglu, swiglu
+        bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)  # noqa: E731
+        comm = Communicator(1, 0, get_unique_id())
+        x, w, w13, few = bf(2048, 8192), bf(4096, 8192), bf(2 * 8192, 8192), bf(16, 8192)
+        src, wide = bf(100_000_000), torch.empty(100_000_000, device="cuda")
+        dst = torch.empty_like(src)
+        h, g = bf(4096, 2 * 14336).requires_grad_(True), bf(4096, 14336)
+        f32 = [torch.rand(50_000_000, device="cuda") for _ in range(4)]
+        T, E, k, d = 8192, 64, 8, 4096
+        disp, tok = MoeDispatcher(comm, E, d, T * k), bf(T, d)
+        top = torch.randn(T, E, device="cuda").topk(k, dim=1)
+        idx, tw = top.indices.to(torch.int32), torch.softmax(top.values, dim=1)
+        for _ in range(reps):
+            gemm_bf16(x, w)
+            gemm_bf16(few, w13)
+            gemm_swiglu(few, w13)
+            comm.all_reduce(src, dst)
+            comm.reduce_scatter(src, wide, scale=0.25)
+            torch.autograd.grad(swiglu(h), h, g)
+            adamw_step(*f32, src[:50_000_000], 1e-3, (0.9, 0.95), 1e-8, 0.0, 1)
+            res = disp.dispatch(tok, idx)
+            disp.combine(idx, tw, res.send_pos)
+            disp.combine_grad_local(tok, disp.y, tw, res.send_pos)
+        torch.cuda.synchronize()
+        comm.destroy()
     elif args.case == "window_allreduce":
         world = 4
         n = 32 << 20  # bf16 elements: 64 MiB per rank

@@ -423,7 +423,8 @@ bool skinny_gemm_cuts(const SkinnyProblem& d, int sms) {
   // of the number of rows, which decides between the two kernels, must not show in the result).  One
   // group: cut where that pays.  A stage takes 0.25 us per SM (16 x 7168 x 8192 uncut: 32.9 us for 128 of
   // them), the exchange of a cut 3.5 us, and no schedule beats reading the weights (16 x 8192 x 3584, 64
-  // tiles: 17.5 us whole, 18.8 cut; 16 x 7168 x 8192, 56 tiles: 32.9 whole, 27.3 cut).
+  // tiles: 17.5 us whole, 18.8 cut, and the model, which takes a whole tile for 14, cuts it all the same; 16 x 7168
+  // x 8192, 56 tiles: 32.9 whole, 27.3 cut).
   const double w_tiles = (d.N + skinnyk::WM - 1) / skinnyk::WM, nkb = (d.K + skinnyk::BK - 1) / skinnyk::BK;
   const double read_us = (double)d.N * d.K * 2 / 6.5e6;
   const double whole_us = std::max(read_us, (double)(((long)w_tiles + sms - 1) / sms) * nkb * 0.25);

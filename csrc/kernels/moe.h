@@ -18,7 +18,7 @@
 namespace amem {
 
 static const int kMoeMaxExperts = 256;   // CtrlBlock::xchg row length
-static const int kMoeSegments = 148;     // CTAs of the count / scatter kernels: one per SM
+static const int kMoeSegments = 148;     // CTAs of the count / scatter kernels: one per SM of a B200; any number is correct on any GPU
 
 struct MoeArgs {
   CollArgs coll;

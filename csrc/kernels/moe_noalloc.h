@@ -7,8 +7,8 @@
 //   * an engine that shares the GPU with another one and has already handed every byte it may
 //     use to its own pool, so a cudaMalloc here could fail or eat the neighbour's budget;
 //   * code that runs where an allocation would stall or break what surrounds it.
-// It runs the same count / plan / scatter kernels as amemMoeDispatch on a one-rank
-// "communicator", but the scratch they need (per-segment expert histograms and their scans,
+// It runs the kernels of amemMoeDispatch on a one-rank "communicator" (one launch for few pairs, count and
+// scatter otherwise), but the scratch they need (per-segment expert histograms and their scans,
 // per-expert row offsets, one protocol control block and status words: about 370 KB) sits in a
 // file-scope device array inside the library instead of in allocated memory.
 //
