@@ -67,8 +67,9 @@ class MoeDispatcher:
         topk_idx = topk_idx.to(torch.int32).contiguous()
         if self.host:
             return self._host_dispatch(x, topk_idx)
-        with torch.cuda.stream(stream):     # (None: the current one)
-            x = dense(x)
+        if x.data_ptr() % 16:
+            with torch.cuda.stream(stream):     # (None: the current one)
+                x = dense(x)
         T, k = topk_idx.shape
         counts = torch.empty(self.experts_per_rank, dtype=torch.int32, device=x.device)
         offsets = torch.empty(self.experts_per_rank + 1, dtype=torch.int32, device=x.device)
