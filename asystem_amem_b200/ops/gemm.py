@@ -58,8 +58,7 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
     N = b.shape[0]
     out = torch.empty(M, N, dtype=torch.bfloat16, device=a.device) if out is None else out
     lib = B.load_library()
-    with on_device_of(a):
-        B.check(lib.amemGemmBf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, _stream(stream)), "amemGemmBf16")
+    B.check(lib.amemGemmBf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, _stream(stream)), "amemGemmBf16")
     return out
 
 
@@ -157,9 +156,8 @@ def grouped_gemm_bf16(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, o
     rows_cap = a.shape[0]
     out = torch.empty(rows_cap, N // 2 if swiglu else N, dtype=torch.bfloat16, device=a.device) if out is None else out
     lib = B.load_library()
-    with on_device_of(a):
-        B.check(lib.amemGroupedGemmBf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, rows_cap,
-                                        int(rows_hint or 0), N, K, 1 if swiglu else 0, _stream(stream)), "amemGroupedGemmBf16")
+    B.check(lib.amemGroupedGemmBf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, rows_cap,
+                                    int(rows_hint or 0), N, K, 1 if swiglu else 0, _stream(stream)), "amemGroupedGemmBf16")
     return out
 
 
