@@ -279,11 +279,6 @@ class Communicator:
         B.check(self.lib.ncclCommGetAsyncError(self._h, ctypes.byref(e)), "ncclCommGetAsyncError")
         return e.value
 
-    def begin(self, tensor, stream=None) -> None:
-        """For an operation that this communicator's single rank runs without it: raises where the operation would
-        have been refused (paused, aborted, another device current) and orders the stream like one."""
-        B.check(self.lib.amemCommBegin(self._h, _stream_handle(stream, tensor)), "amemCommBegin")
-
     # -- collectives --------------------------------------------------------------------
     def all_reduce(self, send, recv=None, op: str = "sum", stream=None, algo: str = "auto"):
         recv = send if recv is None else recv

@@ -9,12 +9,18 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
-from torch.autograd import forward_ad
 from torch.nn.modules.module import _has_any_global_hook
 
 from ..ops.gemm import gemm_swiglu
 from ..ops.elementwise import swiglu
+from ..ops.operands import tangents_about
 from ..parallel.tp import ColumnParallelLinear, RowParallelLinear
+
+
+def _calls_its_product_alone(m: nn.Module) -> bool:
+    """Whether m(x) is a projection's product on one rank and nothing else: neither wrapped, hooked nor replaced."""
+    return (type(m) is ColumnParallelLinear and "forward" not in m.__dict__ and not m._forward_hooks and not m._forward_pre_hooks
+            and m.comm.nranks == 1 and not _has_any_global_hook())
 
 
 class TPMLP(nn.Module):
@@ -25,20 +31,13 @@ class TPMLP(nn.Module):
         self.w13 = ColumnParallelLinear(dim, 2 * ffn_dim, comm, device=device)
         self.w2 = RowParallelLinear(ffn_dim, dim, comm, device=device)
 
-    def _calls_nothing_else(self, x_shard: torch.Tensor) -> bool:
-        """Whether w13(x_shard) is the projection's product alone: no gradient of either mode asks for it, and it is
-        neither wrapped, hooked nor replaced."""
-        m = self.w13
-        if type(m) is not ColumnParallelLinear or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks or _has_any_global_hook():
-            return False
-        if torch.is_grad_enabled() and (x_shard.requires_grad or m.weight.requires_grad):
-            return False
-        return all(forward_ad.unpack_dual(t).tangent is None for t in (x_shard, m.weight))
-
     def forward(self, x_shard: torch.Tensor) -> torch.Tensor:
         """x_shard: bf16 [tokens / tp, dim] -> bf16 [tokens / tp, dim]"""
-        if self.comm.nranks == 1 and x_shard.is_cuda and self.ffn_local % 8 == 0 and self._calls_nothing_else(x_shard):
-            # one rank: the activation rides in the projection's epilogue
-            self.w13.comm.begin(x_shard)
-            return self.w2(gemm_swiglu(x_shard.contiguous(), self.w13.weight.contiguous()))
+        if x_shard.is_cuda and self.ffn_local % 8 == 0:
+            w13 = self.w13
+            if _calls_its_product_alone(w13) and not tangents_about():
+                w = w13.weight
+                if not (torch.is_grad_enabled() and (x_shard.requires_grad or w.requires_grad)):
+                    # one rank, no gradients: the activation rides in the projection's epilogue
+                    return self.w2(gemm_swiglu(x_shard.contiguous(), w.contiguous(), comm=w13.comm))
         return self.w2(swiglu(self.w13(x_shard)).to(torch.bfloat16))

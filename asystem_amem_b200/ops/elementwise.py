@@ -6,10 +6,9 @@ from __future__ import annotations
 
 import torch
 import torch.nn.functional as F
-from torch.autograd import forward_ad
 
 from .. import bindings as B
-from .operands import dense, on_device_of
+from .operands import dense, on_operands_device, tangents_about
 
 
 def _st() -> int:
@@ -17,8 +16,7 @@ def _st() -> int:
 
 
 def _fused(h: torch.Tensor) -> bool:
-    """One dense bf16 tensor without a tangent (the kernel knows nothing of forward-mode gradients)."""
-    return forward_ad.unpack_dual(h).tangent is None and h.is_cuda and h.dtype == torch.bfloat16 and h.dim() == 2 and h.shape[1] % 16 == 0 and h.data_ptr() % 16 == 0
+    return not tangents_about() and h.is_cuda and h.dtype == torch.bfloat16 and h.dim() == 2 and h.shape[1] % 16 == 0 and h.data_ptr() % 16 == 0
 
 
 class _SwiGLU(torch.autograd.Function):
@@ -31,18 +29,22 @@ class _SwiGLU(torch.autograd.Function):
     @torch.autograd.function.once_differentiable
     def backward(ctx, g):
         (h,) = ctx.saved_tensors
-        g, out = dense(g), torch.empty_like(h)
-        f, p, o = h.shape[1] // 2, h.data_ptr(), out.data_ptr()
-        with on_device_of(h):
-            B.check(B.load_library().amemSwiGLUGrad(p, p + 2 * f, 2 * f, g.data_ptr(), o, o + 2 * f, h.shape[0], f, _st()), "amemSwiGLUGrad")
-        return out
+        return _gradient(h, dense(g))
 
 
+@on_operands_device
+def _gradient(h: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
+    out = torch.empty_like(h)
+    f, p, o = h.shape[1] // 2, h.data_ptr(), out.data_ptr()
+    B.check(B.load_library().amemSwiGLUGrad(p, p + 2 * f, 2 * f, g.data_ptr(), o, o + 2 * f, h.shape[0], f, _st()), "amemSwiGLUGrad")
+    return out
+
+
+@on_operands_device
 def _forward(h: torch.Tensor) -> torch.Tensor:
     f, p = h.shape[1] // 2, h.data_ptr()
     out = torch.empty(h.shape[0], f, dtype=h.dtype, device=h.device)
-    with on_device_of(h):
-        B.check(B.load_library().amemSwiGLU(p, p + 2 * f, 2 * f, out.data_ptr(), h.shape[0], f, _st()), "amemSwiGLU")
+    B.check(B.load_library().amemSwiGLU(p, p + 2 * f, 2 * f, out.data_ptr(), h.shape[0], f, _st()), "amemSwiGLU")
     return out
 
 
@@ -55,6 +57,7 @@ def swiglu(h: torch.Tensor) -> torch.Tensor:
     return (F.silu(h[:, :f].float()) * h[:, f:].float()).to(h.dtype)
 
 
+@on_operands_device
 def adamw_step(grad, m, v, master, shard, lr: float, betas, eps: float, weight_decay: float, step: int) -> None:
     """One AdamW update in place: fp32 ``m``, ``v`` and ``master`` from the fp32 ``grad``; ``shard``
     receives the new weights in bf16.  ``step`` counts from 1.  One kernel for five tensors of one shape,
@@ -62,9 +65,8 @@ def adamw_step(grad, m, v, master, shard, lr: float, betas, eps: float, weight_d
     flat = (grad, m, v, master, shard)
     if all(t.is_cuda and t.device == grad.device and t.shape == grad.shape and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in flat) and shard.dtype == torch.bfloat16 \
             and all(t.dtype == torch.float32 for t in flat[:4]):
-        with on_device_of(grad):
-            B.check(B.load_library().amemAdamW(grad.data_ptr(), m.data_ptr(), v.data_ptr(), master.data_ptr(), shard.data_ptr(), grad.numel(),
-                                               float(lr), float(betas[0]), float(betas[1]), float(eps), float(weight_decay), step, _st()), "amemAdamW")
+        B.check(B.load_library().amemAdamW(grad.data_ptr(), m.data_ptr(), v.data_ptr(), master.data_ptr(), shard.data_ptr(), grad.numel(),
+                                           float(lr), float(betas[0]), float(betas[1]), float(eps), float(weight_decay), step, _st()), "amemAdamW")
         torch.autograd.graph.increment_version([t for t in flat[1:] if not t.is_inference()])   # as an in-place operator does
         return
     b1, b2 = betas

@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from .. import bindings as B
-from .operands import on_device_of
+from .operands import on_operands_device
 
 
 def _check(a: torch.Tensor, b: torch.Tensor) -> None:
@@ -24,12 +24,14 @@ def _check(a: torch.Tensor, b: torch.Tensor) -> None:
         raise ValueError(f"inner dimensions differ: {tuple(a.shape)} vs {tuple(b.shape)}")
 
 
-def _matrices(a: torch.Tensor, b: torch.Tensor, inner_a: int, inner_b: int) -> None:
-    """Both operands are matrices and agree in the dimension that the product sums over."""
-    if a.dim() != 2 or b.dim() != 2:
-        raise ValueError(f"matrices expected, got {tuple(a.shape)} and {tuple(b.shape)}")
-    if a.shape[inner_a] != b.shape[inner_b]:
-        raise ValueError(f"inner dimensions differ: {tuple(a.shape)} vs {tuple(b.shape)}")
+def _matrices(a: torch.Tensor, b: torch.Tensor, inner_a: int, inner_b: int) -> tuple[torch.Size, torch.Size]:
+    """The shapes of two matrices that agree in the dimension that the product sums over; others raise."""
+    sa, sb = a.shape, b.shape       # (building a torch.Size takes a third of a microsecond)
+    if len(sa) != 2 or len(sb) != 2:
+        raise ValueError(f"matrices expected, got {tuple(sa)} and {tuple(sb)}")
+    if sa[inner_a] != sb[inner_b]:
+        raise ValueError(f"inner dimensions differ: {tuple(sa)} vs {tuple(sb)}")
+    return sa, sb
 
 
 def _on_host(a: torch.Tensor, b: torch.Tensor) -> bool:
@@ -62,49 +64,65 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
     return out
 
 
-def gemm_swiglu(a: torch.Tensor, w13: torch.Tensor, stream=None) -> torch.Tensor:
-    """silu(a @ gate.T) * (a @ up.T) in one pass on one GPU: ``w13`` [2 f, K] holds the gate's rows first."""
-    _matrices(a, w13, 1, 1)
-    if w13.shape[0] % 2:
-        raise ValueError(f"as many gate rows as up rows expected, got {w13.shape[0]} in all")
-    f = w13.shape[0] // 2
+def _begin(comm, st: int) -> None:
+    """The launch that follows is an operation of ``comm``, a communicator of one rank: raises where ``comm`` would
+    refuse it (paused, aborted, another device current), orders the stream as for one."""
+    if comm is not None:
+        B.check(comm.lib.amemCommBegin(comm._h, st), "amemCommBegin")
+
+
+@on_operands_device
+def gemm_swiglu(a: torch.Tensor, w13: torch.Tensor, stream=None, comm=None) -> torch.Tensor:
+    """silu(a @ gate.T) * (a @ up.T) in one pass on one GPU: ``w13`` [2 f, K] holds the gate's rows first.
+    ``comm``: the one-rank communicator that this is an operation of, if any."""
+    (M, K), (rows, _) = _matrices(a, w13, 1, 1)
+    if rows % 2:
+        raise ValueError(f"as many gate rows as up rows expected, got {rows} in all")
+    f = rows // 2
     if _on_host(a, w13):
+        _begin(comm, 0)
         h = _host_matmul(a, w13)
         return (torch.nn.functional.silu(h[:, :f]) * h[:, f:]).to(a.dtype)
     _check(a, w13)
-    out = torch.empty(a.shape[0], f, dtype=torch.bfloat16, device=a.device)
+    st = _stream(stream)
+    _begin(comm, st)
+    out = torch.empty(M, f, dtype=torch.bfloat16, device=a.device)
     lib = B.load_library()
-    with on_device_of(a):
-        B.check(lib.amemGemmSwiGLU(a.data_ptr(), w13.data_ptr(), out.data_ptr(), a.shape[0], f, a.shape[1], _stream(stream)), "amemGemmSwiGLU")
+    B.check(lib.amemGemmSwiGLU(a.data_ptr(), w13.data_ptr(), out.data_ptr(), M, f, K, st), "amemGemmSwiGLU")
     return out
 
 
-def _by_k(a: torch.Tensor, b: torch.Tensor, m: int, n: int, k: int, a_by_k: bool, stream) -> torch.Tensor:
+def _by_k(a: torch.Tensor, b: torch.Tensor, m: int, n: int, k: int, a_by_k: bool, st: int) -> torch.Tensor:
     if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
         raise TypeError("bf16 tensors expected")
     if not (a.is_cuda and b.is_cuda and a.is_contiguous() and b.is_contiguous()):
         raise ValueError("contiguous CUDA tensors expected")
     out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
     lib = B.load_library()
-    with on_device_of(a):
-        B.check(lib.amemGemmBf16Strided(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, int(a_by_k), 1, _stream(stream)), "amemGemmBf16Strided")
+    B.check(lib.amemGemmBf16Strided(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, int(a_by_k), 1, st), "amemGemmBf16Strided")
     return out
 
 
-def gemm_input_grad(gy: torch.Tensor, w: torch.Tensor, stream=None) -> torch.Tensor:
-    """gy[M, N] @ w[N, K] on one GPU: the input gradient of :func:`gemm_bf16`, from the weight as it lies."""
-    _matrices(gy, w, 1, 0)
+@on_operands_device
+def gemm_input_grad(gy: torch.Tensor, w: torch.Tensor, stream=None, comm=None) -> torch.Tensor:
+    """gy[M, N] @ w[N, K] on one GPU: the input gradient of :func:`gemm_bf16`, from the weight as it lies.
+    ``comm``: the one-rank communicator that this is an operation of, if any."""
+    (M, N), (_, K) = _matrices(gy, w, 1, 0)
     if _on_host(gy, w):
+        _begin(comm, 0)
         return (gy.float() @ w.float()).to(gy.dtype)
-    return _by_k(gy, w, gy.shape[0], w.shape[1], w.shape[0], False, stream)
+    st = _stream(stream)
+    _begin(comm, st)
+    return _by_k(gy, w, M, K, N, False, st)
 
 
+@on_operands_device
 def gemm_weight_grad(gy: torch.Tensor, x: torch.Tensor, stream=None) -> torch.Tensor:
     """gy[T, N].T @ x[T, K] on one GPU: the weight gradient of :func:`gemm_bf16`, any number of rows T."""
-    _matrices(gy, x, 0, 0)
+    (T, N), (_, K) = _matrices(gy, x, 0, 0)
     if _on_host(gy, x):
         return gy.t() @ x
-    return _by_k(gy, x, gy.shape[1], x.shape[1], gy.shape[0], True, stream)
+    return _by_k(gy, x, N, K, T, True, _stream(stream))
 
 
 def interleave_gate_up(w13: torch.Tensor, ffn: int) -> torch.Tensor:
@@ -161,6 +179,7 @@ def grouped_gemm_bf16(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, o
     return out
 
 
+@on_operands_device
 def grouped_gemm_input_grad(g: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor | None = None,
                             rows_hint: int | None = None, stream=None) -> torch.Tensor:
     """For every group e: out[rows of e] = g[rows of e] @ w[e] with ``w`` bf16 [groups, N, K] as it is
@@ -178,25 +197,24 @@ def grouped_gemm_input_grad(g: torch.Tensor, w: torch.Tensor, offsets: torch.Ten
         return res
     out = torch.empty(g.shape[0], K, dtype=torch.bfloat16, device=g.device) if out is None else out
     _check_grouped(g, w, offsets, groups)
-    with on_device_of(g):
-        B.check(B.load_library().amemGroupedGemmBf16Input(g.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
-                                                          int(rows_hint or 0), N, K, _stream(stream)), "amemGroupedGemmBf16Input")
+    B.check(B.load_library().amemGroupedGemmBf16Input(g.data_ptr(), w.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
+                                                      int(rows_hint or 0), N, K, _stream(stream)), "amemGroupedGemmBf16Input")
     return out
 
 
+@on_operands_device
 def grouped_gemm_weight_grad(g: torch.Tensor, a: torch.Tensor, offsets: torch.Tensor, stream=None) -> torch.Tensor:
     """bf16 [groups, N, K]: for every group e, g[rows of e].T @ a[rows of e] (zeros without rows).  The
     group boundaries are read on the device."""
-    _matrices(g, a, 0, 0)
-    groups, N, K = offsets.numel() - 1, g.shape[1], a.shape[1]
+    (_, N), (_, K) = _matrices(g, a, 0, 0)
+    groups = offsets.numel() - 1
     if not g.is_cuda:
         offs = offsets.tolist()
         return torch.stack([g[offs[e]:offs[e + 1]].t() @ a[offs[e]:offs[e + 1]] for e in range(groups)])
     _check_grouped(g, a, offsets, groups)
     out = torch.empty(groups, N, K, dtype=torch.bfloat16, device=g.device)
-    with on_device_of(g):
-        B.check(B.load_library().amemGroupedGemmBf16Weight(g.data_ptr(), a.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
-                                                           N, K, _stream(stream)), "amemGroupedGemmBf16Weight")
+    B.check(B.load_library().amemGroupedGemmBf16Weight(g.data_ptr(), a.data_ptr(), out.data_ptr(), offsets.data_ptr(), groups, g.shape[0],
+                                                       N, K, _stream(stream)), "amemGroupedGemmBf16Weight")
     return out
 
 

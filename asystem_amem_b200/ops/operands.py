@@ -2,15 +2,27 @@
 device that holds them current."""
 from __future__ import annotations
 
-from contextlib import nullcontext
+from functools import wraps
 
 import torch
+from torch.autograd import forward_ad
 
 
-def on_device_of(t: torch.Tensor):
-    """Context in which the device of ``t`` is current: a launch goes to the current device, wherever
-    its operands lie."""
-    return nullcontext() if t.get_device() == torch.cuda.current_device() else torch.cuda.device(t.get_device())
+def on_operands_device(launch):
+    """``launch(t, ...)`` with the device of ``t`` current: a launch goes to the current device, wherever its
+    operands lie."""
+    @wraps(launch)
+    def call(t, *args, **kw):
+        if t.is_cuda and t.get_device() != torch.cuda.current_device():
+            with torch.cuda.device(t.get_device()):
+                return launch(t, *args, **kw)
+        return launch(t, *args, **kw)
+    return call
+
+
+def tangents_about() -> bool:
+    """Whether a tensor may carry a forward-mode tangent, which the kernels know nothing of."""
+    return forward_ad._current_level >= 0
 
 
 def dense(t: torch.Tensor) -> torch.Tensor:

@@ -24,15 +24,6 @@ def _wgrad(gy: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
     return gy.t() @ x
 
 
-def _alone(comm, t: torch.Tensor) -> bool:
-    """Whether the step has nobody to exchange rows with, and runs without the communicator; it stays an
-    operation of the communicator, so what that refuses is refused."""
-    if comm.nranks > 1:
-        return False
-    comm.begin(t)
-    return True
-
-
 def _gathered(comm, shard: torch.Tensor) -> torch.Tensor:
     """The rows of every rank (the shard itself on one rank)."""
     shard = shard.contiguous()
@@ -59,7 +50,7 @@ class _ColumnFn(torch.autograd.Function):
         gy = gy.contiguous()
         # dx_shard = reduce_scatter_rows(gy @ w): the mirrored fused kernel, B = w.T [K, N_local]; one
         # rank has nothing to scatter and its GEMM reads w as it lies
-        gx = gemm_input_grad(gy, w.contiguous()) if _alone(comm, gy) else gemm_reduce_scatter(comm, gy, w.t().contiguous())
+        gx = gemm_input_grad(gy, w.contiguous(), comm=comm) if comm.nranks == 1 else gemm_reduce_scatter(comm, gy, w.t().contiguous())
         gw = _wgrad(gy, _gathered(comm, x_shard))
         return gx, gw, None
 
@@ -79,7 +70,7 @@ class _RowFn(torch.autograd.Function):
         x, w = ctx.saved_tensors
         gy_shard = gy_shard.contiguous()
         # dx = all_gather_rows(gy_shard) @ w  -> fused all-gather GEMM with B = w.T [K_local, N]
-        gx = gemm_input_grad(gy_shard, w.contiguous()) if _alone(comm, gy_shard) else all_gather_gemm(comm, gy_shard, w.t().contiguous())
+        gx = gemm_input_grad(gy_shard, w.contiguous(), comm=comm) if comm.nranks == 1 else all_gather_gemm(comm, gy_shard, w.t().contiguous())
         gw = _wgrad(_gathered(comm, gy_shard), x)
         return gx, gw, None
 

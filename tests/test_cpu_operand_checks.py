@@ -238,7 +238,7 @@ def test_which_gemm_runs_and_how_it_is_tiled(monkeypatch):
 
 def _mlp(lib):
     from asystem_amem_b200.models import TPMLP
-    layer = TPMLP(SimpleNamespace(nranks=1, lib=lib, _h=1, begin=lambda t: lib.amemCommBegin(1, 0)), 64, 32, device="cpu")
+    layer = TPMLP(SimpleNamespace(nranks=1, lib=lib, _h=1), 64, 32, device="cpu")
     for m in (layer.w13, layer.w2):
         m.weight = torch.nn.Parameter(m.weight.detach().as_subclass(OnGpu), requires_grad=False)
     return layer
