@@ -9,14 +9,15 @@ from torch.autograd import forward_ad
 
 
 def on_operands_device(launch):
-    """``launch(t, ...)`` with the device of ``t`` current: a launch goes to the current device, wherever its
-    operands lie."""
+    """``launch`` with the device of its first tensor current: a launch goes to the current device, wherever
+    its operands lie."""
     @wraps(launch)
-    def call(t, *args, **kw):
-        if t.is_cuda and t.get_device() != torch.cuda.current_device():
+    def call(*args, **kw):
+        t = args[0] if args else next((v for v in kw.values() if isinstance(v, torch.Tensor)), None)
+        if t is not None and t.is_cuda and t.get_device() != torch.cuda.current_device():
             with torch.cuda.device(t.get_device()):
-                return launch(t, *args, **kw)
-        return launch(t, *args, **kw)
+                return launch(*args, **kw)
+        return launch(*args, **kw)
     return call
 
 

@@ -185,7 +185,10 @@ def test_launches_make_the_operands_device_current(lib, monkeypatch):
     ops.gemm_weight_grad(gpu(8, 64), gpu(8, 16))
     ops.grouped_gemm_input_grad(gpu(6, 16), gpu(2, 16, 64), offs)
     ops.grouped_gemm_weight_grad(gpu(6, 16), gpu(6, 64), offs)
-    assert len(lib.calls) == 8 and all(args[-1] == 103 for _, args in lib.calls), lib.calls
+    ops.gemm_input_grad(w=gpu(64, 16), gy=gpu(8, 64))
+    ops.adamw_step(lr=1e-3, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.0, step=1, grad=gpu(16, dtype=torch.float32), m=gpu(16, dtype=torch.float32),
+                   v=gpu(16, dtype=torch.float32), master=gpu(16, dtype=torch.float32), shard=gpu(16))
+    assert len(lib.calls) == 10 and all(args[-1] == 103 for _, args in lib.calls), lib.calls
     assert current == [0]
 
 
