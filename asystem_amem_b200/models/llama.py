@@ -13,6 +13,8 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..ops.elementwise import rms_norm
+
 
 @dataclass
 class LlamaConfig:
@@ -41,9 +43,7 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(dim))
 
     def forward(self, x):
-        v = x.float()
-        v = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + self.eps)
-        return (v * self.weight.float()).to(x.dtype)
+        return rms_norm(x, self.weight, self.eps)
 
 
 def rope_tables(seq: int, head_dim: int, theta: float, device) -> tuple[torch.Tensor, torch.Tensor]:

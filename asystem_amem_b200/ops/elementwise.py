@@ -1,4 +1,5 @@
-"""Element-wise passes as single kernels: SwiGLU with its gradient, the AdamW update of a shard.
+"""Passes over rows as single kernels: SwiGLU and the root-mean-square norm with their gradients, the AdamW
+update of a shard.
 
 Reference parity: none -- the reference contains no arithmetic on user data.
 """
@@ -8,7 +9,7 @@ import torch
 import torch.nn.functional as F
 
 from .. import bindings as B
-from .operands import dense, on_operands_device, tangents_about
+from .operands import dense, on_operands_device, plain_cuda, tangents_about
 
 
 def _st() -> int:
@@ -55,6 +56,63 @@ def swiglu(h: torch.Tensor) -> torch.Tensor:
         return _SwiGLU.apply(h) if torch.is_grad_enabled() and h.requires_grad else _forward(h)
     f = h.shape[1] // 2
     return (F.silu(h[:, :f].float()) * h[:, f:].float()).to(h.dtype)
+
+
+def _rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
+    v = x.float()
+    v = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + eps)
+    return (v * weight.float()).to(x.dtype)
+
+
+@on_operands_device
+def _rms_forward(x: torch.Tensor, weight: torch.Tensor, eps: float, keep: bool):
+    rows, dim = x.numel() // x.shape[-1], x.shape[-1]
+    out = torch.empty_like(x)
+    rstd = torch.empty(rows, dtype=torch.float32, device=x.device) if keep else None
+    B.check(B.load_library().amemRmsNorm(x.data_ptr(), weight.data_ptr(), out.data_ptr(), rstd.data_ptr() if keep else None, rows, dim, float(eps), _st()),
+            "amemRmsNorm")
+    return out, rstd
+
+
+@on_operands_device
+def _rms_gradient(g: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, rstd: torch.Tensor, of_x: bool, of_weight: bool):
+    lib, rows, dim = B.load_library(), rstd.numel(), x.shape[-1]
+    g_x, g_w = torch.empty_like(x) if of_x else None, torch.empty_like(weight) if of_weight else None
+    part = torch.empty(lib.amemRmsNormGradBlocks(rows), dim, dtype=torch.float32, device=x.device) if of_weight else None
+    p = [t if t is None else t.data_ptr() for t in (g_x, part, g_w)]
+    B.check(lib.amemRmsNormGrad(g.data_ptr(), x.data_ptr(), weight.data_ptr(), rstd.data_ptr(), *p, rows, dim, _st()), "amemRmsNormGrad")
+    return g_x, g_w
+
+
+class _RMSNorm(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, weight, eps):
+        out, rstd = _rms_forward(x, weight, eps, True)
+        ctx.save_for_backward(x, weight, rstd)
+        ctx.eps = eps
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        x, weight, rstd = ctx.saved_tensors
+        wanted = ctx.needs_input_grad[:2]
+        if torch.is_grad_enabled():     # a graph of the gradient is wanted: torch's operators make one
+            at = [t for t, w in zip((x, weight), wanted) if w]
+            grads = iter(torch.autograd.grad(_rms_norm(x, weight, ctx.eps), at, g, create_graph=True))
+            return *(next(grads) if w else None for w in wanted), None
+        return *_rms_gradient(dense(g), x, weight, rstd, *wanted), None
+
+
+def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
+    """``x / sqrt(mean(x^2) + eps) * weight`` over the last dimension in fp32, rounded once to x's type.  One
+    kernel for bf16 rows that lie densely on one GPU."""
+    if (x.dtype == weight.dtype == torch.bfloat16 and x.dim() > 0 and x.numel() > 0 and weight.shape == x.shape[-1:] and x.shape[-1] % 8 == 0
+            and x.shape[-1] <= 16384 and x.numel() // x.shape[-1] < 2 ** 31 and plain_cuda(x, weight) and x.is_contiguous() and weight.is_contiguous()
+            and (x.data_ptr() | weight.data_ptr()) % 16 == 0):
+        if torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad):
+            return _RMSNorm.apply(x, weight, eps)
+        return _rms_forward(x, weight, eps, False)[0]
+    return _rms_norm(x, weight, eps)
 
 
 @on_operands_device

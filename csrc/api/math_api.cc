@@ -45,6 +45,21 @@ ncclResult_t amemSwiGLUGrad(const void* gate, const void* up, long long ld, cons
   return rows == 0 ? ncclSuccess : R(launch_swiglu_grad(gate, up, (long)ld, g_act, g_gate, g_up, (long)rows, F, stream));
 }
 
+ncclResult_t amemRmsNorm(const void* x, const void* w, void* y, float* rstd, long long rows, int dim, double eps, cudaStream_t stream) {
+  if (!rms_norm_takes((long)rows, dim) || !aligned16(x, w, y) || missing({x, w, y}))
+    return R(fail(kInvalidArgument, "amemRmsNorm: rows=%lld dim=%d (a multiple of 8 up to 16384, 16-byte aligned)", rows, dim));
+  return R(launch_rms_norm(x, w, y, rstd, (long)rows, dim, (float)eps, stream));
+}
+
+int amemRmsNormGradBlocks(long long rows) { return rms_norm_grad_blocks((long)rows); }
+
+ncclResult_t amemRmsNormGrad(const void* g_y, const void* x, const void* w, const float* rstd, void* g_x, float* part_w, void* g_w, long long rows, int dim,
+                             cudaStream_t stream) {
+  if (!rms_norm_takes((long)rows, dim) || !aligned16(g_y, x, w) || !aligned16(g_x, part_w, nullptr) || missing({g_y, x, w, rstd}) || (g_w && !part_w))
+    return R(fail(kInvalidArgument, "amemRmsNormGrad: rows=%lld dim=%d (a multiple of 8 up to 16384, 16-byte aligned)", rows, dim));
+  return R(launch_rms_norm_grad(g_y, x, w, rstd, g_x, part_w, g_w, (long)rows, dim, stream));
+}
+
 ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,
                        double eps, double weight_decay, long long step, cudaStream_t stream) {
   if (n < 0 || step < 1 || !aligned16(grad, m, v) || !aligned16(master, shard_bf16, nullptr))

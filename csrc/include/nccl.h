@@ -217,6 +217,13 @@ ncclResult_t amemGemmSwiGLU(const void* A, const void* W, void* C, int M, int F,
 ncclResult_t amemSwiGLU(const void* gate, const void* up, long long ld, void* act, long long rows, int F, cudaStream_t stream);
 ncclResult_t amemSwiGLUGrad(const void* gate, const void* up, long long ld, const void* g_act, void* g_gate, void* g_up, long long rows, int F,
                             cudaStream_t stream);
+/* y[r] = x[r] * rstd[r] * w, rstd[r] = 1 / sqrt(mean(x[r]^2) + eps): bf16 rows of dim elements (a multiple of 8 up to
+ * 16384), fp32 inside; rstd (may be NULL) is kept for the gradients.  The gradients g_x and g_w may each be NULL; g_w
+ * needs part_w, fp32 [amemRmsNormGradBlocks(rows)][dim] of work memory. */
+ncclResult_t amemRmsNorm(const void* x, const void* w, void* y, float* rstd, long long rows, int dim, double eps, cudaStream_t stream);
+int amemRmsNormGradBlocks(long long rows);
+ncclResult_t amemRmsNormGrad(const void* g_y, const void* x, const void* w, const float* rstd, void* g_x, float* part_w, void* g_w, long long rows,
+                             int dim, cudaStream_t stream);
 /* One AdamW update of n parameters in one pass: fp32 gradient, moments and master weights, bf16 copy of the
  * new weights; step counts from 1. */
 ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,

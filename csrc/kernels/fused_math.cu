@@ -11,12 +11,14 @@
 
 #include "../core/log.h"
 #include "fused_math.h"
+#include "pdl.cuh"
 
 namespace amem {
 namespace mathk {
 
 constexpr int THREADS = 256;
 constexpr int ADAM_AHEAD = 2;   // groups of four parameters per thread: eight loads in flight
+constexpr int NORM_THREADS = 512, NORM_VECS = 4;   // a row of up to 16384 elements in one block's registers
 
 struct alignas(16) Bf8 {
   __nv_bfloat162 h[4];
@@ -126,6 +128,162 @@ __global__ void __launch_bounds__(THREADS) adamw_kernel(const float* __restrict_
   }
 }
 
+// Sum of v over a block of whole warps; `part` holds a value per warp and is not read again before the next
+// barrier but one, so callers alternate between two of them.
+__device__ __forceinline__ float block_sum(float v, float* part) {
+#pragma unroll
+  for (int o = 16; o > 0; o /= 2) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const int warp = threadIdx.x / 32, warps = blockDim.x / 32;
+  if (threadIdx.x % 32 == 0) part[warp] = v;
+  __syncthreads();
+  float sum = 0.f;
+  for (int i = 0; i < warps; ++i) sum += part[i];
+  return sum;
+}
+
+// y[r] = x[r] * rstd[r] * w with rstd = 1 / sqrt(mean(x[r]^2) + eps): a block per row, which it holds in registers
+// (VECS vectors of eight a thread), so x is read once.
+template <int VECS>
+__global__ void __launch_bounds__(NORM_THREADS) rms_norm_kernel(const char* x, const char* w, char* y, float* rstd, int dim, float eps) {
+  __shared__ float part[NORM_THREADS / 32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int vecs = dim / 8;
+  const long row = blockIdx.x;
+  Bf8 v[VECS], wv[VECS];
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < VECS; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    if (c < vecs) {
+      v[i] = ((const Bf8*)x)[row * vecs + c];
+      wv[i] = ((const Bf8*)w)[c];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < VECS; ++i)
+    if (threadIdx.x + i * blockDim.x < vecs) {
+      float f[8];
+      unpack(v[i], f);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) sum = fmaf(f[q], f[q], sum);
+    }
+  const float r = rsqrtf(block_sum(sum, part) / (float)dim + eps);
+  if (rstd && threadIdx.x == 0) rstd[row] = r;
+#pragma unroll
+  for (int i = 0; i < VECS; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    if (c < vecs) {
+      float f[8], g[8];
+      unpack(v[i], f);
+      unpack(wv[i], g);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) f[q] = f[q] * r * g[q];
+      ((Bf8*)y)[row * vecs + c] = pack(f);
+    }
+  }
+}
+
+// Gradients of the above.  With n = x * rstd: g_x = rstd * (g * w - n * mean(g * w * n)), g_w = sum over rows of
+// g * n.  Blocks stride over the rows and keep the columns' sums in registers; each leaves its sums in
+// part_w [gridDim.x][dim] and rms_norm_weight_grad_kernel adds them in the order of the blocks.
+template <int VECS>
+__global__ void __launch_bounds__(NORM_THREADS) rms_norm_grad_kernel(const char* g_y, const char* x, const char* w, const float* rstd, char* g_x, float* part_w,
+                                                                     long rows, int dim) {
+  __shared__ float part[2][NORM_THREADS / 32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int vecs = dim / 8;
+  Bf8 wv[VECS];
+  float acc[VECS][8];
+#pragma unroll
+  for (int i = 0; i < VECS; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    if (c < vecs) wv[i] = ((const Bf8*)w)[c];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc[i][q] = 0.f;
+  }
+  int flip = 0;
+  for (long row = blockIdx.x; row < rows; row += gridDim.x, flip ^= 1) {
+    Bf8 xv[VECS], gv[VECS];
+    const float r = rstd[row];
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+      const int c = threadIdx.x + i * blockDim.x;
+      if (c < vecs) {
+        xv[i] = ((const Bf8*)x)[row * vecs + c];
+        gv[i] = ((const Bf8*)g_y)[row * vecs + c];
+      }
+    }
+    float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < VECS; ++i)
+      if (threadIdx.x + i * blockDim.x < vecs) {
+        float a[8], g[8], b[8];
+        unpack(xv[i], a);
+        unpack(gv[i], g);
+        unpack(wv[i], b);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const float n = a[q] * r;
+          acc[i][q] = fmaf(g[q], n, acc[i][q]);
+          dot = fmaf(g[q] * b[q], n, dot);
+        }
+      }
+    const float mean = block_sum(dot, part[flip]) / (float)dim;
+    if (g_x) {
+#pragma unroll
+      for (int i = 0; i < VECS; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        if (c < vecs) {
+          float a[8], g[8], b[8];
+          unpack(xv[i], a);
+          unpack(gv[i], g);
+          unpack(wv[i], b);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) a[q] = r * (g[q] * b[q] - a[q] * r * mean);
+          ((Bf8*)g_x)[row * vecs + c] = pack(a);
+        }
+      }
+    }
+  }
+  if (part_w) {
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+      const int c = threadIdx.x + i * blockDim.x;
+      if (c < vecs) {
+        float4* dst = (float4*)(part_w + (size_t)blockIdx.x * dim + c * 8);
+        dst[0] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        dst[1] = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+      }
+    }
+  }
+}
+
+// g_w[c] = sum of `blocks` partial sums: 32 columns a block, a warp per piece of the sum
+__global__ void __launch_bounds__(1024) rms_norm_weight_grad_kernel(const float* part_w, __nv_bfloat16* g_w, int blocks, int dim) {
+  __shared__ float sums[32][33];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32, c = blockIdx.x * 32 + lane;
+  float sum = 0.f;
+  if (c < dim)
+    for (int b = warp; b < blocks; b += 32) sum += part_w[(size_t)b * dim + c];
+  sums[warp][lane] = sum;
+  __syncthreads();
+  sum = sums[lane][warp];
+#pragma unroll
+  for (int o = 16; o > 0; o /= 2) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if (lane == 0 && blockIdx.x * 32 + warp < dim) g_w[blockIdx.x * 32 + warp] = __float2bfloat16_rn(sum);
+}
+
+// Threads of a block for a row of `vecs` vectors, and how many of them each thread takes: 1, 2 or 4
+int norm_threads(int vecs) {
+  int x = 32;
+  while (x < NORM_THREADS && x < vecs) x *= 2;
+  return x;
+}
+
 // x: up to a row's vectors, y: rows, for the kernels with a thread per vector
 void shape_for(long rows, int vecs, dim3* grid, dim3* block) {
   int x = 32;
@@ -140,7 +298,36 @@ Status launched(const char* what) {
   return kSuccess;
 }
 
+Status launched(cudaError_t e, const char* what) {
+  if (e != cudaSuccess) return fail(kCudaError, "%s launch failed: %s", what, cudaGetErrorString(e));
+  return kSuccess;
+}
+
 }  // namespace mathk
+
+bool rms_norm_takes(long rows, int dim) { return rows > 0 && rows <= 0x7fffffffL && dim > 0 && dim % 8 == 0 && dim <= mathk::NORM_THREADS * mathk::NORM_VECS * 8; }
+
+Status launch_rms_norm(const void* x, const void* w, void* y, float* rstd, long rows, int dim, float eps, cudaStream_t stream) {
+  namespace k = mathk;
+  const int threads = k::norm_threads(dim / 8), per = (dim / 8 + threads - 1) / threads;
+  auto kernel = per == 1 ? k::rms_norm_kernel<1> : per == 2 ? k::rms_norm_kernel<2> : k::rms_norm_kernel<4>;
+  return k::launched(launch_overlapped(kernel, dim3((unsigned)rows), dim3(threads), 0, stream, (const char*)x, (const char*)w, (char*)y, rstd, dim, eps), "rms norm");
+}
+
+// Four blocks an SM: enough rows in flight, and few enough partial sums of the weight's gradient (4.8 MB at dim 2048).
+int rms_norm_grad_blocks(long rows) { return (int)std::min(rows, 4L * 148); }
+
+Status launch_rms_norm_grad(const void* g_y, const void* x, const void* w, const float* rstd, void* g_x, float* part_w, void* g_w, long rows, int dim,
+                            cudaStream_t stream) {
+  namespace k = mathk;
+  const int threads = k::norm_threads(dim / 8), per = (dim / 8 + threads - 1) / threads, blocks = rms_norm_grad_blocks(rows);
+  auto kernel = per == 1 ? k::rms_norm_grad_kernel<1> : per == 2 ? k::rms_norm_grad_kernel<2> : k::rms_norm_grad_kernel<4>;
+  AMEM_TRY(k::launched(launch_overlapped(kernel, dim3(blocks), dim3(threads), 0, stream, (const char*)g_y, (const char*)x, (const char*)w, rstd, (char*)g_x,
+                                         part_w, rows, dim), "rms norm gradient"));
+  if (!g_w) return kSuccess;
+  return k::launched(launch_overlapped(k::rms_norm_weight_grad_kernel, dim3((dim + 31) / 32), dim3(1024), 0, stream, (const float*)part_w, (__nv_bfloat16*)g_w,
+                                       blocks, dim), "rms norm weight gradient");
+}
 
 Status launch_swiglu(const void* gate, const void* up, long ld, void* act, long rows, int F, cudaStream_t stream) {
   dim3 grid, block;

@@ -11,6 +11,15 @@ Status launch_swiglu(const void* gate, const void* up, long ld, void* act, long 
 Status launch_swiglu_grad(const void* gate, const void* up, long ld, const void* g_act, void* g_gate, void* g_up, long rows, int F,
                           cudaStream_t stream);
 
+// Root-mean-square norm of bf16 rows (contiguous, 16-byte aligned): y = x * rstd * w, rstd = 1 / sqrt(mean(x^2) + eps) in
+// fp32, kept for the gradients where rstd is given.
+bool rms_norm_takes(long rows, int dim);
+Status launch_rms_norm(const void* x, const void* w, void* y, float* rstd, long rows, int dim, float eps, cudaStream_t stream);
+// Its gradients; either may be null.  part_w: fp32 [rms_norm_grad_blocks(rows)][dim] of work memory for g_w.
+int rms_norm_grad_blocks(long rows);
+Status launch_rms_norm_grad(const void* g_y, const void* x, const void* w, const float* rstd, void* g_x, float* part_w, void* g_w, long rows, int dim,
+                            cudaStream_t stream);
+
 struct AdamW {
   float lr, b1, one_minus_b1, b2, one_minus_b2, c1, c2, eps;   // c1, c2: 1 - b^t
   float decay;                                                 // 1 - lr * weight decay

@@ -43,6 +43,60 @@ def test_gate_up_projection(M, f, K):
         assert (out.float() - ref).abs().max().item() <= 2.0 ** -8 * ref.abs().max().item() + 1e-6
 
 
+# one, two and four vectors a thread, rows that end inside one, more rows than blocks; 16392 and 20: torch's operators
+@pytest.mark.parametrize("rows,dim", [(1, 8), (3, 256), (5, 264), (700, 2048), (601, 4104), (9, 8200), (2, 16384), (2, 16392), (7, 20)])
+def test_rms_norm_and_its_gradients(rows, dim):
+    from asystem_amem_b200.ops import rms_norm
+    x, w, g = _rand((rows, dim), 5, 2.0), _rand((dim,), 6), _rand((rows, dim), 7)
+    x[0] = 0
+    a, b = x.clone().requires_grad_(True), w.clone().requires_grad_(True)
+    out = rms_norm(a, b, 1e-5)
+    out.backward(g)
+    c, d = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    ref = c * torch.rsqrt(c.pow(2).mean(-1, keepdim=True) + 1e-5) * d
+    ref.backward(g.double())
+    # one rounding to bf16 of values computed in fp32: those of the result to a few of its roundings and half that of a
+    # sum of dim squares, the gradients' differences to as much of their larger term, the weight's sum to as many
+    # roundings of its terms as it has
+    assert torch.all((out.double() - ref).abs() <= ref.abs() * (2.0 ** -8 + 2.0 ** -14))
+    r = torch.rsqrt(c.detach().pow(2).mean(-1, keepdim=True) + 1e-5)
+    n, gw = c.detach() * r, g.double() * w.double()
+    larger = r * (gw.abs() + n.abs() * (gw * n).abs().mean(-1, keepdim=True))
+    assert torch.all((a.grad.double() - c.grad).abs() <= c.grad.abs() * 2.0 ** -8 + larger * 2.0 ** -14)
+    terms = (g.double() * n).abs().sum(0)
+    assert torch.all((b.grad.double() - d.grad).abs() <= d.grad.abs() * 2.0 ** -8 + terms * (rows + 16) * 2.0 ** -23)
+    assert torch.equal(rms_norm(x, w, 1e-5), out)
+
+
+def test_rms_norm_in_every_form_that_torch_takes():
+    from torch.func import jvp, vmap
+    from asystem_amem_b200.ops import rms_norm
+    x, w = _rand((6, 64), 8), _rand((64,), 9)
+    want = rms_norm(x, w, 1e-5)
+    close = dict(rtol=2.0 ** -7, atol=1e-6)       # two roundings of one value
+    torch.testing.assert_close(rms_norm(x.t().contiguous().t(), w, 1e-5), want, **close)
+    off = torch.empty(6 * 64 + 1, device="cuda", dtype=torch.bfloat16)[1:].view(6, 64).copy_(x)
+    torch.testing.assert_close(rms_norm(off, w, 1e-5), want, **close)
+    torch.testing.assert_close(rms_norm(x.view(2, 3, 64), w, 1e-5).view(6, 64), want, rtol=0, atol=0)
+    torch.testing.assert_close(rms_norm(x.float(), w, 1e-5), want.float(), **close)
+    torch.testing.assert_close(vmap(lambda r: rms_norm(r, w, 1e-5))(x), want, **close)
+    torch.testing.assert_close(jvp(lambda t: rms_norm(t, w, 1e-5), (x,), (x,))[0], want, **close)
+    assert rms_norm(x[:0], w, 1e-5).shape == (0, 64)
+    # only the input, only the weight, and a gradient of the gradient
+    a = x.clone().requires_grad_(True)
+    (gx,) = torch.autograd.grad(rms_norm(a, w, 1e-5).float().pow(2).sum(), a, create_graph=True)
+    (hx,) = torch.autograd.grad(gx.float().sum(), a)
+    b = x.double().requires_grad_(True)
+    r = b * torch.rsqrt(b.pow(2).mean(-1, keepdim=True) + 1e-5) * w.double()
+    (gr,) = torch.autograd.grad(r.pow(2).sum(), b, create_graph=True)
+    (hr,) = torch.autograd.grad(gr.sum(), b)
+    # some ten roundings to bf16 of terms of the size of the largest
+    assert (hx.double() - hr).abs().max().item() <= 10 * 2.0 ** -8 * max(gr.abs().max().item(), hr.abs().max().item())
+    v = w.clone().requires_grad_(True)
+    rms_norm(x, v, 1e-5).backward(x)
+    assert v.grad is not None and v.grad.shape == v.shape
+
+
 @pytest.mark.parametrize("n", [1, 3, 4, 1000, 1_000_003])
 @pytest.mark.parametrize("wd", [0.0, 0.1])
 def test_adamw(n, wd):
