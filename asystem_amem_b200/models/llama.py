@@ -13,7 +13,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..ops.elementwise import rms_norm
+from ..ops.elementwise import gated, rms_norm, rotate
 
 
 @dataclass
@@ -54,10 +54,7 @@ def rope_tables(seq: int, head_dim: int, theta: float, device) -> tuple[torch.Te
 
 def apply_rope(x, cos, sin):
     # x: [B, H, S, D]
-    x1, x2 = x.float()[..., 0::2], x.float()[..., 1::2]
-    o1 = x1 * cos - x2 * sin
-    o2 = x1 * sin + x2 * cos
-    return torch.stack((o1, o2), dim=-1).flatten(-2).to(x.dtype)
+    return rotate(cos, sin, x)[0]
 
 
 class Attention(nn.Module):
@@ -74,7 +71,7 @@ class Attention(nn.Module):
         q = self.wq(x).view(B, S, self.h, self.hd).transpose(1, 2)
         k = self.wk(x).view(B, S, self.kv, self.hd).transpose(1, 2)
         v = self.wv(x).view(B, S, self.kv, self.hd).transpose(1, 2)
-        q, k = apply_rope(q, cos, sin), apply_rope(k, cos, sin)
+        q, k = rotate(cos, sin, q, k, as_they_lie=True)
         o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=self.kv != self.h)
         return self.wo(o.transpose(1, 2).reshape(B, S, -1))
 
@@ -87,7 +84,7 @@ class SwiGLU(nn.Module):
         self.w2 = nn.Linear(cfg.ffn_dim, cfg.dim, bias=False)
 
     def forward(self, x):
-        return self.w2(F.silu(self.w1(x)) * self.w3(x))
+        return self.w2(gated(self.w1(x), self.w3(x)))
 
 
 class Block(nn.Module):

@@ -5,6 +5,8 @@ Reference parity: none -- the reference contains no arithmetic on user data.
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 import torch.nn.functional as F
 
@@ -113,6 +115,114 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
             return _RMSNorm.apply(x, weight, eps)
         return _rms_forward(x, weight, eps, False)[0]
     return _rms_norm(x, weight, eps)
+
+
+@on_operands_device
+def _gated_forward(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
+    out, f = torch.empty_like(gate), gate.shape[-1]
+    B.check(B.load_library().amemSwiGLU(gate.data_ptr(), up.data_ptr(), f, out.data_ptr(), gate.numel() // f, f, _st()), "amemSwiGLU")
+    return out
+
+
+@on_operands_device
+def _gated_gradient(gate: torch.Tensor, up: torch.Tensor, g: torch.Tensor):
+    g_gate, g_up, f = torch.empty_like(gate), torch.empty_like(up), gate.shape[-1]
+    B.check(B.load_library().amemSwiGLUGrad(gate.data_ptr(), up.data_ptr(), f, g.data_ptr(), g_gate.data_ptr(), g_up.data_ptr(), gate.numel() // f, f, _st()),
+            "amemSwiGLUGrad")
+    return g_gate, g_up
+
+
+class _Gated(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, gate, up):
+        ctx.save_for_backward(gate, up)
+        return _gated_forward(gate, up)
+
+    @staticmethod
+    def backward(ctx, g):
+        gate, up = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            at = [t for t, w in zip((gate, up), ctx.needs_input_grad) if w]
+            grads = iter(torch.autograd.grad(F.silu(gate) * up, at, g, create_graph=True))
+            return tuple(next(grads) if w else None for w in ctx.needs_input_grad)
+        return tuple(t if w else None for t, w in zip(_gated_gradient(gate, up, dense(g)), ctx.needs_input_grad))
+
+
+def gated(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
+    """silu(gate) * up of two tensors of one shape.  One kernel, in fp32 and rounded once, for bf16 that lies densely on
+    one GPU."""
+    if (gate.dtype == up.dtype == torch.bfloat16 and gate.shape == up.shape and gate.dim() > 0 and gate.numel() > 0 and gate.shape[-1] % 8 == 0
+            and plain_cuda(gate, up) and gate.is_contiguous() and up.is_contiguous() and (gate.data_ptr() | up.data_ptr()) % 16 == 0):
+        return _Gated.apply(gate, up) if torch.is_grad_enabled() and (gate.requires_grad or up.requires_grad) else _gated_forward(gate, up)
+    return F.silu(gate) * up
+
+
+def _rotate_plain(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
+    x1, x2 = x.float()[..., 0::2], x.float()[..., 1::2]
+    o1 = x1 * cos - x2 * sin
+    o2 = x1 * sin + x2 * cos
+    return torch.stack((o1, o2), dim=-1).flatten(-2).to(x.dtype)
+
+
+def _tokens_first(x: torch.Tensor) -> bool:
+    """Whether [B, H, S, D] lies as [B, S, H, D], as a projection's output does."""
+    return x.stride(1) < x.stride(2)
+
+
+def _in_vectors(x: torch.Tensor) -> bool:
+    b, h, s, one = x.stride()
+    return one == 1 and (b | h | s) % 8 == 0 and x.data_ptr() % 16 == 0
+
+
+@on_operands_device
+def _rotate_launch(cos: torch.Tensor, sin: torch.Tensor, inverse: bool, tokens_first, *xs: torch.Tensor):
+    n, (batch, _, seq, dim) = len(xs), xs[0].shape
+    outs = []
+    for x, first in zip(xs, tokens_first):
+        h = x.shape[1]
+        st = (seq * h * dim, dim, h * dim, 1) if first else (seq * h * dim, seq * dim, dim, 1)
+        outs.append(torch.empty_strided((batch, h, seq, dim), st, dtype=x.dtype, device=x.device))
+    strides = [st for x, o in zip(xs, outs) for st in (*x.stride()[:3], *o.stride()[:3])]
+    B.check(B.load_library().amemRotate((ctypes.c_void_p * n)(*(x.data_ptr() for x in xs)), (ctypes.c_void_p * n)(*(o.data_ptr() for o in outs)),
+                                        (ctypes.c_int * n)(*(x.shape[1] for x in xs)), (ctypes.c_longlong * (6 * n))(*strides), n, cos.data_ptr(),
+                                        sin.data_ptr(), batch, seq, dim, int(inverse), _st()), "amemRotate")
+    return tuple(outs)
+
+
+class _Rotate(torch.autograd.Function):
+    """A turn; its gradient is the turn back, laid out as the input was."""
+
+    @staticmethod
+    def forward(ctx, cos, sin, inverse, tokens_first, *xs):
+        ctx.save_for_backward(cos, sin)
+        ctx.inverse, ctx.back = inverse, [_tokens_first(x) for x in xs]
+        return _rotate_launch(cos, sin, inverse, tokens_first, *xs)
+
+    @staticmethod
+    def backward(ctx, *gs):
+        cos, sin = ctx.saved_tensors
+        gs = [g if _in_vectors(g) else dense(g) for g in gs]
+        return None, None, None, None, *_Rotate.apply(cos, sin, not ctx.inverse, ctx.back, *gs)
+
+
+def _kernel_turns(cos: torch.Tensor, sin: torch.Tensor, *xs: torch.Tensor) -> bool:
+    batch, seq, dim = xs[0].shape[0], xs[0].shape[2] if xs[0].dim() == 4 else 0, xs[0].shape[-1]
+    return (all(x.dim() == 4 and x.dtype == torch.bfloat16 and x.shape[0] == batch and x.shape[2] == seq and x.shape[3] == dim and x.numel() > 0 for x in xs)
+            and dim % 8 == 0 and batch * seq < 2 ** 31
+            and all(t.dtype == torch.float32 and t.shape == (seq, dim // 2) and t.is_contiguous() and not t.requires_grad for t in (cos, sin))
+            and plain_cuda(*xs, cos, sin) and (cos.data_ptr() | sin.data_ptr()) % 16 == 0 and all(_in_vectors(x) for x in xs))
+
+
+def rotate(cos: torch.Tensor, sin: torch.Tensor, *xs: torch.Tensor, as_they_lie: bool = False):
+    """Rotary embedding of one or two [B, H, S, D] tensors: neighbouring elements turned by the angles of ``cos`` and
+    ``sin`` [S, D / 2].  Computed in fp32 and rounded once; bf16 on one GPU in one kernel.  The results are contiguous, or
+    (``as_they_lie``) laid out as the inputs, whose heads may lie inside the positions."""
+    if _kernel_turns(cos, sin, *xs):
+        layout = [as_they_lie and _tokens_first(x) for x in xs]
+        if torch.is_grad_enabled() and any(x.requires_grad for x in xs):
+            return _Rotate.apply(cos, sin, False, layout, *xs)
+        return _rotate_launch(cos, sin, False, layout, *xs)
+    return tuple(_rotate_plain(x, cos, sin) for x in xs)
 
 
 @on_operands_device

@@ -60,6 +60,27 @@ ncclResult_t amemRmsNormGrad(const void* g_y, const void* x, const void* w, cons
   return R(launch_rms_norm_grad(g_y, x, w, rstd, g_x, part_w, g_w, (long)rows, dim, stream));
 }
 
+ncclResult_t amemRotate(const void* const* in, void* const* out, const int* heads, const long long* strides, int tensors, const float* cos, const float* sin,
+                        int batch, int seq, int dim, int inverse, cudaStream_t stream) {
+  if (tensors < 1 || tensors > 2 || batch <= 0 || seq <= 0 || (long long)batch * seq > 0x7fffffffLL || dim <= 0 || dim % 8 || missing({in, out, heads, strides}) ||
+      missing({cos, sin}) || !aligned16(cos, sin, nullptr))
+    return R(fail(kInvalidArgument, "amemRotate: tensors=%d batch=%d seq=%d dim=%d (a multiple of 8)", tensors, batch, seq, dim));
+  Rotation a = {};
+  for (int i = 0; i < tensors; ++i) {
+    const long long* st = strides + 6 * i;
+    bool fits = heads[i] > 0 && (long long)heads[i] * dim <= 0x3fffffffLL && !missing({in[i], out[i]}) && aligned16(in[i], out[i], nullptr);
+    for (int j = 0; j < 6; ++j) fits = fits && st[j] >= 0 && st[j] % 8 == 0;
+    if (!fits) return R(fail(kInvalidArgument, "amemRotate: tensor %d needs heads, 16-byte aligned rows and strides that are multiples of 8", i));
+    a.t[i] = {(const char*)in[i], (char*)out[i], heads[i], (long)st[0], (long)st[1], (long)st[2], (long)st[3], (long)st[4], (long)st[5]};
+  }
+  a.cos = cos;
+  a.sin = sin;
+  a.seq = seq;
+  a.vecs = dim / 8;
+  a.turn = inverse ? -1.f : 1.f;
+  return R(launch_rotate(a, batch, stream));
+}
+
 ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,
                        double eps, double weight_decay, long long step, cudaStream_t stream) {
   if (n < 0 || step < 1 || !aligned16(grad, m, v) || !aligned16(master, shard_bf16, nullptr))

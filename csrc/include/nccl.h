@@ -224,6 +224,12 @@ ncclResult_t amemRmsNorm(const void* x, const void* w, void* y, float* rstd, lon
 int amemRmsNormGradBlocks(long long rows);
 ncclResult_t amemRmsNormGrad(const void* g_y, const void* x, const void* w, const float* rstd, void* g_x, float* part_w, void* g_w, long long rows,
                              int dim, cudaStream_t stream);
+/* Rotary embedding of one or two bf16 tensors [batch, heads[i], seq, dim]: (o[2j], o[2j+1]) is (x[2j], x[2j+1]) turned by
+ * the angle whose fp32 cosine and sine stand at [position][j] (by its negative with inverse != 0, which is the gradient).
+ * strides: six per tensor, of batch, head and position in elements, first of the input, then of the output; multiples of
+ * 8, the last dimension is dense. */
+ncclResult_t amemRotate(const void* const* in, void* const* out, const int* heads, const long long* strides, int tensors, const float* cos,
+                        const float* sin, int batch, int seq, int dim, int inverse, cudaStream_t stream);
 /* One AdamW update of n parameters in one pass: fp32 gradient, moments and master weights, bf16 copy of the
  * new weights; step counts from 1. */
 ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,

@@ -142,7 +142,8 @@ __device__ __forceinline__ float block_sum(float v, float* part) {
 }
 
 // y[r] = x[r] * rstd[r] * w with rstd = 1 / sqrt(mean(x[r]^2) + eps): a block per row, which it holds in registers
-// (VECS vectors of eight a thread), so x is read once.
+// (VECS vectors of eight a thread), so x is read once.  2048 rows of 2048: 7.6 us cold under ncu, launch included, 2.6 are the
+// bytes (seven torch passes: 47); the rest is the latency of one load, one reduction and one store.
 template <int VECS>
 __global__ void __launch_bounds__(NORM_THREADS) rms_norm_kernel(const char* x, const char* w, char* y, float* rstd, int dim, float eps) {
   __shared__ float part[NORM_THREADS / 32];
@@ -186,7 +187,8 @@ __global__ void __launch_bounds__(NORM_THREADS) rms_norm_kernel(const char* x, c
 
 // Gradients of the above.  With n = x * rstd: g_x = rstd * (g * w - n * mean(g * w * n)), g_w = sum over rows of
 // g * n.  Blocks stride over the rows and keep the columns' sums in registers; each leaves its sums in
-// part_w [gridDim.x][dim] and rms_norm_weight_grad_kernel adds them in the order of the blocks.
+// part_w [gridDim.x][dim] and rms_norm_weight_grad_kernel adds them in the order of the blocks.  The same size: 10.4 + 6.6 us
+// (as torch passes about 130).
 template <int VECS>
 __global__ void __launch_bounds__(NORM_THREADS) rms_norm_grad_kernel(const char* g_y, const char* x, const char* w, const float* rstd, char* g_x, float* part_w,
                                                                      long rows, int dim) {
@@ -277,6 +279,30 @@ __global__ void __launch_bounds__(1024) rms_norm_weight_grad_kernel(const float*
   if (lane == 0 && blockIdx.x * 32 + warp < dim) g_w[blockIdx.x * 32 + warp] = __float2bfloat16_rn(sum);
 }
 
+// (o[2i], o[2i+1]) = (x[2i], x[2i+1]) turned by the angle of (position, i), one tensor or two; a block per token, so its
+// heads share the token's row of the tables out of L1.  q [1, 16, 2048, 128] and k with 4 heads: 8.3 us, 3.2 are the bytes
+// (as torch passes over fp32 copies, forward and backward in the mean: 120).
+__global__ void __launch_bounds__(THREADS) rotate_kernel(const __grid_constant__ Rotation a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int b = blockIdx.x / a.seq, s = blockIdx.x - b * a.seq, first = a.t[0].heads * a.vecs, all = first + a.t[1].heads * a.vecs;
+  for (int i = threadIdx.x; i < all; i += blockDim.x) {
+    const Rotated& t = a.t[i >= first];
+    const int j = i >= first ? i - first : i, h = j / a.vecs, v = j - h * a.vecs;
+    const float4 c = ((const float4*)a.cos)[(long)s * a.vecs + v], n = ((const float4*)a.sin)[(long)s * a.vecs + v];
+    float x[8];
+    unpack(*(const Bf8*)(t.in + (b * t.in_b + h * t.in_h + s * t.in_s) * 2 + v * 16), x);
+    const float cs[4] = {c.x, c.y, c.z, c.w}, sn[4] = {n.x * a.turn, n.y * a.turn, n.z * a.turn, n.w * a.turn};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float x1 = x[2 * q], x2 = x[2 * q + 1];
+      x[2 * q] = x1 * cs[q] - x2 * sn[q];
+      x[2 * q + 1] = x1 * sn[q] + x2 * cs[q];
+    }
+    *(Bf8*)(t.out + (b * t.out_b + h * t.out_h + s * t.out_s) * 2 + v * 16) = pack(x);
+  }
+}
+
 // Threads of a block for a row of `vecs` vectors, and how many of them each thread takes: 1, 2 or 4
 int norm_threads(int vecs) {
   int x = 32;
@@ -327,6 +353,11 @@ Status launch_rms_norm_grad(const void* g_y, const void* x, const void* w, const
   if (!g_w) return kSuccess;
   return k::launched(launch_overlapped(k::rms_norm_weight_grad_kernel, dim3((dim + 31) / 32), dim3(1024), 0, stream, (const float*)part_w, (__nv_bfloat16*)g_w,
                                        blocks, dim), "rms norm weight gradient");
+}
+
+Status launch_rotate(const Rotation& a, int batch, cudaStream_t stream) {
+  const int items = (a.t[0].heads + a.t[1].heads) * a.vecs, threads = std::min(mathk::THREADS, (items + 31) / 32 * 32);
+  return mathk::launched(launch_overlapped(mathk::rotate_kernel, dim3((unsigned)batch * (unsigned)a.seq), dim3(threads), 0, stream, a), "rotary embedding");
 }
 
 Status launch_swiglu(const void* gate, const void* up, long ld, void* act, long rows, int F, cudaStream_t stream) {

@@ -20,6 +20,23 @@ int rms_norm_grad_blocks(long rows);
 Status launch_rms_norm_grad(const void* g_y, const void* x, const void* w, const float* rstd, void* g_x, float* part_w, void* g_w, long rows, int dim,
                             cudaStream_t stream);
 
+// Rotary embedding of bf16 [batch, heads, seq, 8 * vecs] tensors with any strides (in elements, multiples of 8) but a
+// dense last dimension; cos and sin are fp32 [seq, 4 * vecs], turn = 1 or, for the gradients, -1.  The second tensor is
+// left out where it has no heads.
+struct Rotated {
+  const char* in;
+  char* out;
+  int heads;
+  long in_b, in_h, in_s, out_b, out_h, out_s;
+};
+struct Rotation {
+  Rotated t[2];
+  const float *cos, *sin;
+  int seq, vecs;
+  float turn;
+};
+Status launch_rotate(const Rotation& a, int batch, cudaStream_t stream);
+
 struct AdamW {
   float lr, b1, one_minus_b1, b2, one_minus_b2, c1, c2, eps;   // c1, c2: 1 - b^t
   float decay;                                                 // 1 - lr * weight decay

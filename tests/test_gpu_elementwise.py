@@ -97,6 +97,68 @@ def test_rms_norm_in_every_form_that_torch_takes():
     assert v.grad is not None and v.grad.shape == v.shape
 
 
+def _turned(x, cos, sin):
+    x1, x2, c, s = x[..., 0::2], x[..., 1::2], cos.double(), sin.double()
+    return torch.stack((x1 * c - x2 * s, x1 * s + x2 * c), dim=-1).flatten(-2)
+
+
+# heads inside positions (a projection's output), contiguous, and a slice of a wider tensor; blocks of one warp, items
+# that do not fill the last one, more items than threads; 12 is no multiple of 8: torch's operators
+@pytest.mark.parametrize("lie", ["tokens", "heads", "slice"])
+@pytest.mark.parametrize("b,h,kv,s,d", [(1, 1, 1, 1, 8), (2, 3, 1, 5, 24), (1, 16, 4, 33, 128), (2, 20, 20, 7, 256), (1, 2, 1, 3, 12)])
+def test_rotary_embedding_and_its_gradient(lie, b, h, kv, s, d):
+    from asystem_amem_b200.models.llama import apply_rope, rope_tables
+    from asystem_amem_b200.ops import rotate
+    cos, sin = rope_tables(s, d, 10000.0, "cuda")
+
+    def lay(heads, seed):
+        if lie == "heads":
+            return _rand((b, heads, s, d), seed)
+        if lie == "tokens":
+            return _rand((b, s, heads, d), seed).transpose(1, 2)
+        return _rand((b, s, heads + 1, d + 16), seed)[:, :, 1:, 8:8 + d].transpose(1, 2)
+
+    q, k, gq, gk = lay(h, 1), lay(kv, 2), lay(h, 3), lay(kv, 4)
+    a, c = q.clone(memory_format=torch.preserve_format).requires_grad_(True), k.clone(memory_format=torch.preserve_format).requires_grad_(True)
+    for x, y, as_they_lie in ((q, k, True), (a, c, False)):
+        outs = rotate(cos, sin, x, y, as_they_lie=as_they_lie)
+        for t, o in zip((x, y), outs):
+            ref = _turned(t.detach().double(), cos, sin)
+            # one rounding to bf16 of a difference of products in fp32
+            assert torch.all((o.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + t.detach().abs().max().item() * 2.0 ** -22)
+            assert as_they_lie or o.is_contiguous()
+    torch.autograd.backward(outs, (gq, gk))
+    for t, g in ((a, gq), (c, gk)):
+        ref = _turned(g.double(), cos, -sin)
+        assert torch.all((t.grad.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + g.abs().max().item() * 2.0 ** -22)
+    assert torch.equal(apply_rope(q, cos, sin), outs[0]) and apply_rope(q, cos, sin).is_contiguous()
+    # the gradient of the gradient: the map is linear, so the turn itself
+    (g1,) = torch.autograd.grad(rotate(cos, sin, a)[0], a, gq.clone().requires_grad_(True), create_graph=True)
+    assert g1.requires_grad and torch.equal(g1, a.grad)
+
+
+@pytest.mark.parametrize("shape", [(1, 8), (3, 5, 24), (2, 100, 1000), (2, 3, 20), (0, 16)])
+def test_gated_and_its_gradients(shape):
+    from torch.func import vmap
+    from asystem_amem_b200.ops import gated
+    x, u, g = _rand(shape, 11, 3.0), _rand(shape, 12), _rand(shape, 13)
+    a, b = x.clone().requires_grad_(True), u.clone().requires_grad_(True)
+    out = gated(a, b)
+    out.backward(g)
+    c, d = x.double().requires_grad_(True), u.double().requires_grad_(True)
+    ref = F.silu(c) * d
+    ref.backward(g.double())
+    # as swiglu's bound above; torch's operators (rows of 20) round silu and the product of a gradient to bf16 on the way
+    roundings = 1 if shape[-1] % 8 == 0 else 4
+    for y, r in ((out, ref), (a.grad, c.grad), (b.grad, d.grad)):
+        assert torch.all((y.double() - r).abs() <= r.abs() * (roundings * 2.0 ** -8 + 2.0 ** -12) + (1e-30 if roundings == 1 else 2.0 ** -6))
+    assert torch.equal(gated(x, u), out)
+    if x.numel() and len(shape) == 3:
+        torch.testing.assert_close(vmap(gated)(x, u), out.detach(), rtol=3 * 2.0 ** -8, atol=1e-6)   # three roundings
+        (ga,) = torch.autograd.grad(gated(a, b), a, g, create_graph=True)
+        assert ga.requires_grad
+
+
 @pytest.mark.parametrize("n", [1, 3, 4, 1000, 1_000_003])
 @pytest.mark.parametrize("wd", [0.0, 0.1])
 def test_adamw(n, wd):
