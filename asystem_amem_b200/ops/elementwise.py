@@ -226,6 +226,17 @@ def rotate(cos: torch.Tensor, sin: torch.Tensor, *xs: torch.Tensor, as_they_lie:
 
 
 @on_operands_device
+def add_pieces(dst: torch.Tensor, pieces, scale: float = 1.0) -> None:
+    """``dst[at:at + t.numel()] += scale * t`` for every (at, t) of ``pieces``, which do not overlap: contiguous bf16
+    tensors on the GPU that holds ``dst``, a dense fp32 tensor.  One kernel."""
+    n = len(pieces)
+    base, st = dst.data_ptr(), _st()
+    B.check(B.load_library().amemSumPieces((ctypes.c_void_p * n)(*(t.data_ptr() for _, t in pieces)), (ctypes.c_void_p * n)(*(base + 4 * at for at, _ in pieces)),
+                                           (ctypes.c_longlong * n)(*(t.numel() for _, t in pieces)), n, scale, st), "amemSumPieces")
+    torch.autograd.graph.increment_version(dst)      # as an in-place operator does
+
+
+@on_operands_device
 def adamw_step(grad, m, v, master, shard, lr: float, betas, eps: float, weight_decay: float, step: int) -> None:
     """One AdamW update in place: fp32 ``m``, ``v`` and ``master`` from the fp32 ``grad``; ``shard``
     receives the new weights in bf16.  ``step`` counts from 1.  One kernel for five tensors of one shape,

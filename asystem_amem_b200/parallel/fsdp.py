@@ -8,7 +8,8 @@ reduce-scatters the flat gradient with the averaging scale and the bf16 -> fp32 
 the reduce-scatter kernel.  The all-gather of the NEXT unit (forward: i + 1, backward: i - 1) is
 issued on a side stream before the current unit computes, so it runs under that compute; and the
 parameters' ``.grad`` are views into one flat buffer, so the reduce-scatter reads what autograd
-wrote, without a packing pass.  All communicator memory is pausable: ``pause_all()`` between steps
+wrote, without a packing pass (on one rank there is no such buffer: one kernel adds the gradients to
+the shard from where autograd left them).  All communicator memory is pausable: ``pause_all()`` between steps
 gives the staging memory back and ``resume_all()`` restores it without re-initialisation.
 
 Reference parity: none to match -- the reference implements no parallelism strategy, it pauses
@@ -22,7 +23,8 @@ import math
 import torch
 import torch.nn as nn
 
-from ..ops.elementwise import adamw_step
+from ..ops.elementwise import adamw_step, add_pieces
+from ..ops.gemm import _begin
 
 
 class _ShardedUnit:
@@ -50,6 +52,7 @@ class _ShardedUnit:
         self.full = None
         self._prefetched = None       # (buffer, event) of an all-gather issued ahead of time
         self._gflat = None
+        self.direct = n == 1 and dev.type == "cuda"     # gradients go to the shard without a flat buffer between
 
     def prefetch(self, side) -> None:
         """Starts this unit's all-gather on ``side`` (CUDA stream); ``gather`` picks it up."""
@@ -91,7 +94,26 @@ class _ShardedUnit:
             p.data = torch.empty(0, dtype=p.dtype, device=dev)
         self.full = None
 
+    def _add_grads(self) -> bool:
+        """One rank: the sum over ranks is its own gradients, added to the shard from where autograd left them.  Gradients
+        of other types or layouts are left to the general form."""
+        pieces, off = [], 0
+        for p, k in zip(self.params, self.numels):
+            g = p.grad
+            if g is not None:
+                if g.dtype != torch.bfloat16 or g.layout != torch.strided or g.device != self.shard.device or not g.is_contiguous():
+                    return False
+                pieces.append((off, g))
+            off += k
+        _begin(self.comm, torch.cuda.current_stream().cuda_stream)
+        add_pieces(self.grad_shard, pieces)
+        for p in self.params:
+            p.grad = None
+        return True
+
     def reduce_grads(self) -> None:
+        if self.direct and self._add_grads():
+            return
         flat = self._gflat
         if flat is None:                      # gradients were not attached: pack them
             flat = torch.zeros(self.padded, dtype=torch.bfloat16, device=self.shard.device)
@@ -130,7 +152,11 @@ class _UnitFn(torch.autograd.Function):
         unit.gather()
         if unit.prev_unit is not None:
             unit.prev_unit.prefetch(unit.side)      # the backward pass visits the units in reverse
-        unit.attach_flat_grads()
+        if unit.direct:
+            for p in unit.params:
+                p.grad = None
+        else:
+            unit.attach_flat_grads()
         with torch.enable_grad():
             xin = x.detach().requires_grad_(x.is_floating_point())
             y = unit.module(xin, *ctx.extras)

@@ -7,6 +7,7 @@
 #include "../core/log.h"
 #include "../include/nccl.h"
 #include "../kernels/fused_math.h"
+#include "../kernels/launch.h"
 
 using namespace amem;
 
@@ -79,6 +80,26 @@ ncclResult_t amemRotate(const void* const* in, void* const* out, const int* head
   a.vecs = dim / 8;
   a.turn = inverse ? -1.f : 1.f;
   return R(launch_rotate(a, batch, stream));
+}
+
+ncclResult_t amemSumPieces(const void* const* src, float* const* dst, const long long* n, int pieces, double scale, cudaStream_t stream) {
+  if (pieces < 0 || (pieces > 0 && missing({src, dst, n}))) return R(fail(kInvalidArgument, "amemSumPieces: %d pieces", pieces));
+  SumPieces a;
+  a.count = 0;
+  a.scale = (float)scale;
+  for (int i = 0; i < pieces; ++i) {
+    if (n[i] < 0 || (n[i] > 0 && missing({src[i], dst[i]})) || ((uintptr_t)src[i] & 1) || ((uintptr_t)dst[i] & 3))
+      return R(fail(kInvalidArgument, "amemSumPieces: piece %d of %lld elements", i, n[i]));
+  }
+  for (int i = 0; i < pieces; ++i) {
+    if (n[i] > 0) a.piece[a.count++] = {(const __nv_bfloat16*)src[i], dst[i], (size_t)n[i], 0};
+    if (a.count == kMaxPieces || (i == pieces - 1 && a.count > 0)) {
+      const Status s = launch_sum_pieces(a, stream);
+      if (s != kSuccess) return R(s);
+      a.count = 0;
+    }
+  }
+  return ncclSuccess;
 }
 
 ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,

@@ -230,6 +230,8 @@ ncclResult_t amemRmsNormGrad(const void* g_y, const void* x, const void* w, cons
  * 8, the last dimension is dense. */
 ncclResult_t amemRotate(const void* const* in, void* const* out, const int* heads, const long long* strides, int tensors, const float* cos,
                         const float* sin, int batch, int seq, int dim, int inverse, cudaStream_t stream);
+/* dst[i][0 .. n[i]) += scale * src[i][0 .. n[i]) (fp32 += bf16) for every piece i; the pieces of dst do not overlap. */
+ncclResult_t amemSumPieces(const void* const* src, float* const* dst, const long long* n, int pieces, double scale, cudaStream_t stream);
 /* One AdamW update of n parameters in one pass: fp32 gradient, moments and master weights, bf16 copy of the
  * new weights; step counts from 1. */
 ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,

@@ -54,6 +54,48 @@ __global__ void __launch_bounds__(THREADS) scale_kernel(const TI* src, TO* dst, 
   if (blockIdx.x == 0 && threadIdx.x < count % 4) dst[n * 4 + threadIdx.x] = dev::from_acc<TO, float>(dev::to_acc<TI>(src[n * 4 + threadIdx.x]) * scale);
 }
 
+// dst += scale * src over several pieces of memory: the sum over one rank's gradients, tensor by tensor, added to its
+// shard where the tensors lie.  A block per 4096 elements, all its loads ahead of its stores.  67 M elements: 107 us, of
+// which 102 are the bytes (ten an element; through a flat buffer, a reduce-scatter and an add it was 26 and five passes).
+constexpr int SUM_AHEAD = 2;      // vectors of eight elements a thread
+__global__ void __launch_bounds__(THREADS) sum_kernel(const __grid_constant__ SumPieces a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  int p = 0;
+  while (p + 1 < a.count && (int)blockIdx.x >= a.piece[p + 1].first_block) ++p;
+  const SumPiece& piece = a.piece[p];
+  const __nv_bfloat16* src = piece.src;
+  float* dst = piece.dst;
+  const size_t base = (size_t)(blockIdx.x - piece.first_block) * (THREADS * SUM_AHEAD * 8), n = piece.n;
+  if ((((uintptr_t)src | (uintptr_t)dst) & 15) || base + THREADS * SUM_AHEAD * 8 > n) {   // the end of a piece, or one at an odd place
+    for (size_t i = base + threadIdx.x; i < min(n, base + THREADS * SUM_AHEAD * 8); i += THREADS) dst[i] += a.scale * __bfloat162float(src[i]);
+    return;
+  }
+  uint4 v[SUM_AHEAD];
+  float4 d[SUM_AHEAD][2];
+#pragma unroll
+  for (int j = 0; j < SUM_AHEAD; ++j) {
+    const size_t i = base + ((size_t)j * THREADS + threadIdx.x) * 8;
+    v[j] = *(const uint4*)(src + i);
+    d[j][0] = *(const float4*)(dst + i);
+    d[j][1] = *(const float4*)(dst + i + 4);
+  }
+#pragma unroll
+  for (int j = 0; j < SUM_AHEAD; ++j) {
+    const size_t i = base + ((size_t)j * THREADS + threadIdx.x) * 8;
+    const __nv_bfloat162* h = (const __nv_bfloat162*)&v[j];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const float2 x = __bfloat1622float2(h[2 * q]), y = __bfloat1622float2(h[2 * q + 1]);
+      d[j][q].x += a.scale * x.x;
+      d[j][q].y += a.scale * x.y;
+      d[j][q].z += a.scale * y.x;
+      d[j][q].w += a.scale * y.y;
+      *(float4*)(dst + i + 4 * q) = d[j][q];
+    }
+  }
+}
+
 template <typename TI, typename TO>
 cudaError_t scaled(const CollArgs& a, int grid, cudaStream_t stream) {
   return launch_overlapped(scale_kernel<TI, TO>, dim3(grid), dim3(THREADS), 0, stream, (const TI*)a.send, (TO*)a.recv, (size_t)a.count, a.scale);
@@ -88,6 +130,19 @@ size_t local_blocks(const CollArgs& a, int block_cap) {
   const size_t items = form == 1 ? a.count * dtype_size(a.dtype) / 16 : a.count / 4, per_block = (size_t)THREADS * (form == 1 ? AHEAD : CAST_AHEAD);
   const size_t blocks = std::max<size_t>(1, (items + per_block - 1) / per_block);
   return block_cap > 0 && blocks > (size_t)block_cap ? 0 : blocks;
+}
+
+Status launch_sum_pieces(SumPieces& a, cudaStream_t stream) {
+  size_t blocks = 0;
+  for (int i = 0; i < a.count; ++i) {
+    a.piece[i].first_block = (int)blocks;
+    blocks += (a.piece[i].n + localk::THREADS * localk::SUM_AHEAD * 8 - 1) / (localk::THREADS * localk::SUM_AHEAD * 8);
+    if (blocks > 0x7fffffffu) return fail(kInvalidArgument, "sum of gradients: too many elements");
+  }
+  if (blocks == 0) return kSuccess;
+  cudaError_t e = launch_overlapped(localk::sum_kernel, dim3((unsigned)blocks), dim3(localk::THREADS), 0, stream, a);
+  if (e != cudaSuccess) return fail(kCudaError, "sum of gradients: launch failed: %s", cudaGetErrorString(e));
+  return kSuccess;
 }
 
 Status launch_local(const CollArgs& a, int block_cap, cudaStream_t stream, bool* handled) {
