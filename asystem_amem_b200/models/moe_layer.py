@@ -18,7 +18,7 @@ import torch.nn as nn
 
 from ..ops.gemm import grouped_gemm_bf16, grouped_gemm_input_grad, grouped_gemm_weight_grad, interleave_gate_up
 from ..ops.elementwise import swiglu
-from ..ops.moe import MoeDispatcher
+from ..ops.moe import MoeDispatcher, route
 from ..ops.operands import dense
 from ..parallel.ep import ep_combine, ep_dispatch
 
@@ -70,9 +70,7 @@ class MoELayer(nn.Module):
         return self._w13_fused[1]
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        logits = (x @ self.router.t()).float()
-        top = logits.topk(self.k, dim=1)
-        idx, w = top.indices.to(torch.int32), torch.softmax(top.values, dim=1)
+        idx, w = route(x, self.router, self.k)
         fusable = self.ffn_dim % 32 == 0 and x.is_cuda
         if torch.is_grad_enabled() and (x.requires_grad or self.w2.requires_grad):
             rows, offsets, send_pos = ep_dispatch(self.dispatcher, x, idx)

@@ -21,7 +21,7 @@ from dataclasses import dataclass
 import torch
 
 from .. import bindings as B
-from .operands import dense
+from .operands import dense, on_operands_device, plain_cuda
 
 
 def _view(ptr: int, rows: int, d: int, device) -> torch.Tensor:
@@ -29,6 +29,61 @@ def _view(ptr: int, rows: int, d: int, device) -> torch.Tensor:
     class _Holder:
         __cuda_array_interface__ = {"shape": (rows * d,), "typestr": "<i2", "data": (ptr, False), "version": 3}
     return torch.as_tensor(_Holder(), device=device).view(torch.bfloat16).view(rows, d)
+
+
+def _route_torch(x: torch.Tensor, router: torch.Tensor, k: int) -> tuple[torch.Tensor, torch.Tensor]:
+    top = (x @ router.t()).float().topk(k, dim=1)
+    return top.indices.to(torch.int32), torch.softmax(top.values, dim=1)
+
+
+@on_operands_device
+def _route_launch(x: torch.Tensor, router: torch.Tensor, k: int) -> tuple[torch.Tensor, torch.Tensor]:
+    T, d = x.shape
+    idx, w = torch.empty(T, k, dtype=torch.int32, device=x.device), torch.empty(T, k, dtype=torch.float32, device=x.device)
+    B.check(B.load_library().amemMoeRoute(x.data_ptr(), router.data_ptr(), idx.data_ptr(), w.data_ptr(), T, d, router.shape[0], k,
+                                          torch.cuda.current_stream().cuda_stream), "amemMoeRoute")
+    return idx, w
+
+
+@on_operands_device
+def _route_logits_grad(g_w: torch.Tensor, w: torch.Tensor, idx: torch.Tensor, experts: int) -> torch.Tensor:
+    T, k = idx.shape
+    out = torch.empty(T, experts, dtype=torch.bfloat16, device=w.device)
+    B.check(B.load_library().amemMoeRouteGrad(g_w.data_ptr(), w.data_ptr(), idx.data_ptr(), out.data_ptr(), T, experts, k,
+                                              torch.cuda.current_stream().cuda_stream), "amemMoeRouteGrad")
+    return out
+
+
+class _Route(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, router, k):
+        idx, w = _route_launch(x, router, k)
+        ctx.save_for_backward(x, router, idx, w)
+        ctx.mark_non_differentiable(idx)
+        return idx, w
+
+    @staticmethod
+    def backward(ctx, _g_idx, g_w):
+        x, router, idx, w = ctx.saved_tensors
+        of_x, of_router = ctx.needs_input_grad[:2]
+        if torch.is_grad_enabled():     # a graph of the gradient is wanted: torch's operators make one
+            again = torch.softmax((x @ router.t()).float().gather(1, idx.long()), dim=1)
+            grads = iter(torch.autograd.grad(again, [t for t, n in ((x, of_x), (router, of_router)) if n], g_w, create_graph=True))
+            return next(grads) if of_x else None, next(grads) if of_router else None, None
+        g_logits = _route_logits_grad(g_w.contiguous(), w, idx, router.shape[0])
+        return g_logits @ router if of_x else None, g_logits.t() @ x if of_router else None, None
+
+
+def route(x: torch.Tensor, router: torch.Tensor, k: int) -> tuple[torch.Tensor, torch.Tensor]:
+    """The ``k`` largest of every token's logits ``x @ router.T`` and their softmax, largest first: int32 and fp32
+    [T, k].  One kernel for bf16 rows that lie densely on one GPU (equal logits by the lower expert)."""
+    if (x.dtype == router.dtype == torch.bfloat16 and x.dim() == router.dim() == 2 and x.shape[0] > 0 and x.shape[1] == router.shape[1]
+            and x.shape[1] > 0 and x.shape[1] % 8 == 0 and 0 < k <= router.shape[0] <= 256 and plain_cuda(x, router) and x.is_contiguous()
+            and router.is_contiguous() and (x.data_ptr() | router.data_ptr()) % 16 == 0):
+        if torch.is_grad_enabled() and (x.requires_grad or router.requires_grad):
+            return _Route.apply(x, router, k)
+        return _route_launch(x, router, k)
+    return _route_torch(x, router, k)
 
 
 @dataclass

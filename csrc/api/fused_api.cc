@@ -765,6 +765,20 @@ ncclResult_t amemMoeDispatchCounted(const void* x, const int* topk_idx, int T, i
   return R(launch_moe_dispatch(a, stream));
 }
 
+// Routing and the gradient of its weights down to the logits (no communicator: a rank routes its own tokens).
+ncclResult_t amemMoeRoute(const void* x, const void* router, int* topk_idx, float* topk_w, int T, int d, int E, int k, cudaStream_t stream) {
+  if (T <= 0 || d <= 0 || d % 8 || E <= 0 || E > kMoeMaxExperts || k <= 0 || k > E)
+    return R(fail(kInvalidArgument, "amemMoeRoute: T=%d d=%d (multiple of 8) E=%d (<= %d) k=%d", T, d, E, kMoeMaxExperts, k));
+  if (!x || !router || !topk_idx || !topk_w) return R(fail(kInvalidArgument, "amemMoeRoute: null buffer"));
+  const Status s = moe_aligned("amemMoeRoute", x, router);
+  return R(s == kSuccess ? launch_moe_route(x, router, topk_idx, topk_w, T, d, E, k, stream) : s);
+}
+ncclResult_t amemMoeRouteGrad(const float* g_w, const float* topk_w, const int* topk_idx, void* g_logits, int T, int E, int k, cudaStream_t stream) {
+  if (T <= 0 || E <= 0 || E > kMoeMaxExperts || k <= 0 || k > E) return R(fail(kInvalidArgument, "amemMoeRouteGrad: T=%d E=%d (<= %d) k=%d", T, E, kMoeMaxExperts, k));
+  if (!g_w || !topk_w || !topk_idx || !g_logits) return R(fail(kInvalidArgument, "amemMoeRouteGrad: null buffer"));
+  return R(launch_moe_route_grad(g_w, topk_w, topk_idx, g_logits, T, E, k, stream));
+}
+
 // ---- the same steps on a communicator of one rank, between the caller's own buffers ----------------
 static Status moe_local(ncclComm_t comm, const char* what, int T, int k, int d, int E, int rows, std::initializer_list<const void*> row_bufs,
                         std::initializer_list<const void*> tables, cudaStream_t stream, MoeArgs* a) {

@@ -232,6 +232,11 @@ ncclResult_t amemRotate(const void* const* in, void* const* out, const int* head
                         const float* sin, int batch, int seq, int dim, int inverse, cudaStream_t stream);
 /* dst[i][0 .. n[i]) += scale * src[i][0 .. n[i]) (fp32 += bf16) for every piece i; the pieces of dst do not overlap. */
 ncclResult_t amemSumPieces(const void* const* src, float* const* dst, const long long* n, int pieces, double scale, cudaStream_t stream);
+/* Routing of T tokens, bf16 [T, d] (d a multiple of 8), over E <= 256 experts: the k largest products with the rows of
+ * router, bf16 [E, d], rounded to bf16, largest first (equal ones by the lower expert), and the softmax over them: int32 and
+ * fp32 [T, k].  The gradient of the weights down to the logits is bf16 [T, E]. */
+ncclResult_t amemMoeRoute(const void* x, const void* router, int* topk_idx, float* topk_w, int T, int d, int E, int k, cudaStream_t stream);
+ncclResult_t amemMoeRouteGrad(const float* g_w, const float* topk_w, const int* topk_idx, void* g_logits, int T, int E, int k, cudaStream_t stream);
 /* One AdamW update of n parameters in one pass: fp32 gradient, moments and master weights, bf16 copy of the
  * new weights; step counts from 1. */
 ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,

@@ -142,7 +142,8 @@ __device__ __forceinline__ float block_sum(float v, float* part) {
 }
 
 // y[r] = x[r] * rstd[r] * w with rstd = 1 / sqrt(mean(x[r]^2) + eps): a block per row, which it holds in registers
-// (VECS vectors of eight a thread), so x is read once.
+// (VECS vectors of eight a thread), so x is read once.  2048 rows of 2048: 7.6 us cold under ncu, launch included, 2.6 are the
+// bytes (seven torch passes: 47); the rest is the latency of one load, one reduction and one store.
 template <int VECS>
 __global__ void __launch_bounds__(NORM_THREADS) rms_norm_kernel(const char* x, const char* w, char* y, float* rstd, int dim, float eps) {
   __shared__ float part[NORM_THREADS / 32];
@@ -186,7 +187,8 @@ __global__ void __launch_bounds__(NORM_THREADS) rms_norm_kernel(const char* x, c
 
 // Gradients of the above.  With n = x * rstd: g_x = rstd * (g * w - n * mean(g * w * n)), g_w = sum over rows of
 // g * n.  Blocks stride over the rows and keep the columns' sums in registers; each leaves its sums in
-// part_w [gridDim.x][dim] and rms_norm_weight_grad_kernel adds them in the order of the blocks.
+// part_w [gridDim.x][dim] and rms_norm_weight_grad_kernel adds them in the order of the blocks.  The same size: 10.4 + 6.6 us
+// (as torch passes about 130).
 template <int VECS>
 __global__ void __launch_bounds__(NORM_THREADS) rms_norm_grad_kernel(const char* g_y, const char* x, const char* w, const float* rstd, char* g_x, float* part_w,
                                                                      long rows, int dim) {
@@ -278,7 +280,8 @@ __global__ void __launch_bounds__(1024) rms_norm_weight_grad_kernel(const float*
 }
 
 // (o[2i], o[2i+1]) = (x[2i], x[2i+1]) turned by the angle of (position, i), one tensor or two; a block per token, so its
-// heads share the token's row of the tables out of L1.
+// heads share the token's row of the tables out of L1.  q [1, 16, 2048, 128] and k with 4 heads: 8.3 us, 3.2 are the bytes
+// (as torch passes over fp32 copies, forward and backward in the mean: 120).
 __global__ void __launch_bounds__(THREADS) rotate_kernel(const __grid_constant__ Rotation a) {
   pdl_launch_dependents();
   pdl_wait();

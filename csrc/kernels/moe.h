@@ -53,6 +53,11 @@ Status launch_moe_combine(const MoeArgs& a, cudaStream_t stream);
 // positions at or beyond rows count as dropped).
 Status launch_moe_combine_grad(const void* g_out, const void* y, const float* w, const int* send_pos, void* g_y, float* g_w, int rows, int T, int k,
                                int d, cudaStream_t stream);
+// Routing of T > 0 tokens, bf16 [T, d] with d a multiple of 8, to the k largest of their E <= kMoeMaxExperts logits (x times
+// the rows of router, bf16 [E, d], rounded to bf16; equal ones by the lower expert, NaN above all), largest first:
+// idx int32 and weight fp32 [T, k], the softmax over the chosen.  Its gradient down to the logits, bf16 [T, E].
+Status launch_moe_route(const void* x, const void* router, int* idx, float* weight, int T, int d, int E, int k, cudaStream_t stream);
+Status launch_moe_route_grad(const float* g_w, const float* weight, const int* idx, void* g_logits, int T, int E, int k, cudaStream_t stream);
 // Emulated communicator: all ranks in one cooperative grid per phase.
 Status launch_moe_dispatch_emu(const MoeArgs* host_all, const MoeArgs* dev_all, int nranks, cudaStream_t stream);
 Status launch_moe_combine_emu(const MoeArgs* host_all, const MoeArgs* dev_all, int nranks, cudaStream_t stream);
