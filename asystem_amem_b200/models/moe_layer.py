@@ -24,11 +24,13 @@ from ..parallel.ep import ep_combine, ep_dispatch
 
 
 class GroupedLinear(torch.autograd.Function):
-    """out[rows of group e] = rows @ w[e].T for every group, differentiable."""
+    """out[rows of group e] = rows @ w[e].T for every group, differentiable.  ``covered``: every row belongs to a group, so
+    that the gradient of the rows needs no zeros underneath."""
 
     @staticmethod
-    def forward(ctx, rows, w, offsets):
+    def forward(ctx, rows, w, offsets, covered=False):
         ctx.save_for_backward(rows, w, offsets)
+        ctx.covered = covered
         return grouped_gemm_bf16(rows.contiguous(), w.contiguous(), offsets, rows_hint=rows.shape[0])
 
     @staticmethod
@@ -37,11 +39,11 @@ class GroupedLinear(torch.autograd.Function):
         g_out = dense(g_out)
         g_rows = g_w = None
         if ctx.needs_input_grad[0]:
-            g_rows = torch.zeros_like(rows)
+            g_rows = torch.empty_like(rows) if ctx.covered else torch.zeros_like(rows)
             grouped_gemm_input_grad(g_out, w.contiguous(), offsets, out=g_rows, rows_hint=rows.shape[0])
         if ctx.needs_input_grad[1]:
             g_w = grouped_gemm_weight_grad(g_out, rows.contiguous(), offsets)
-        return g_rows, g_w, None
+        return g_rows, g_w, None, None
 
 
 class MoELayer(nn.Module):
@@ -73,9 +75,9 @@ class MoELayer(nn.Module):
         idx, w = route(x, self.router, self.k)
         fusable = self.ffn_dim % 32 == 0 and x.is_cuda
         if torch.is_grad_enabled() and (x.requires_grad or self.w2.requires_grad):
-            rows, offsets, send_pos = ep_dispatch(self.dispatcher, x, idx)
-            h = GroupedLinear.apply(rows, self.w13, offsets)
-            y = GroupedLinear.apply(swiglu(h).to(torch.bfloat16), self.w2, offsets)
+            rows, offsets, send_pos = ep_dispatch(self.dispatcher, x, idx, all_routed=self.router.shape[0] == self.E)
+            h = GroupedLinear.apply(rows, self.w13, offsets, True)      # `rows` are the rows of the groups and no more
+            y = GroupedLinear.apply(swiglu(h).to(torch.bfloat16), self.w2, offsets, True)
             return ep_combine(self.dispatcher, y, w, idx, send_pos)
         res = self.dispatcher.dispatch(x.contiguous(), idx)
         self.last_dropped = res.dropped

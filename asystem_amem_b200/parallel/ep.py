@@ -43,11 +43,14 @@ def _between_tensors(disp: MoeDispatcher, rows: torch.Tensor) -> bool:
     return disp.local(rows) and rows.shape[0] <= disp.capacity
 
 
-def dispatch_forward(disp: MoeDispatcher, x: torch.Tensor, idx: torch.Tensor):
+def dispatch_forward(disp: MoeDispatcher, x: torch.Tensor, idx: torch.Tensor, all_routed: bool = False):
     """Returns (rows, expert_offsets, send_pos, total): ``rows`` is a private copy of the
-    received rows (the receive buffer is reused by the next dispatch)."""
+    received rows (the receive buffer is reused by the next dispatch).  ``all_routed``: every entry of ``idx`` names an
+    expert, so that one rank knows the total without reading it back."""
     local = disp.local(x) and x.shape[0] == idx.shape[0]
     res = disp.dispatch_local(x.contiguous(), idx) if local else disp.dispatch(x.contiguous(), idx)
+    if local and all_routed:
+        return res.recv_x, res.expert_offsets, res.send_pos, res.recv_x.shape[0]
     total = int(res.expert_offsets[-1].item())  # host sync: `rows` has exactly the rows that arrived
     # (shrunk, not sliced: a view made inside an autograd function could not be changed in place)
     rows = res.recv_x.resize_(total, disp.d) if local else res.recv_x[:total].clone()
@@ -91,8 +94,8 @@ def combine_backward(disp: MoeDispatcher, g_out: torch.Tensor, y_rows: torch.Ten
 
 class _Dispatch(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, idx, disp):
-        rows, offsets, send_pos, _ = dispatch_forward(disp, x, idx)
+    def forward(ctx, x, idx, disp, all_routed):
+        rows, offsets, send_pos, _ = dispatch_forward(disp, x, idx, all_routed)
         ctx.disp = disp
         ctx.save_for_backward(idx, send_pos)
         ctx.mark_non_differentiable(offsets, send_pos)
@@ -101,7 +104,7 @@ class _Dispatch(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g_rows, _g_off, _g_pos):
         idx, send_pos = ctx.saved_tensors
-        return dispatch_backward(ctx.disp, g_rows.contiguous(), idx, send_pos), None, None
+        return dispatch_backward(ctx.disp, g_rows.contiguous(), idx, send_pos), None, None, None
 
 
 class _Combine(torch.autograd.Function):
@@ -118,9 +121,10 @@ class _Combine(torch.autograd.Function):
         return g_y, g_w.to(w.dtype), None, None, None
 
 
-def ep_dispatch(disp: MoeDispatcher, x: torch.Tensor, idx: torch.Tensor):
-    """Differentiable dispatch: (rows grouped by local expert, expert_offsets, send_pos)."""
-    return _Dispatch.apply(x, idx.to(torch.int32).contiguous(), disp)
+def ep_dispatch(disp: MoeDispatcher, x: torch.Tensor, idx: torch.Tensor, all_routed: bool = False):
+    """Differentiable dispatch: (rows grouped by local expert, expert_offsets, send_pos).  ``all_routed``: the caller knows
+    that every entry of ``idx`` names an expert (see :func:`dispatch_forward`)."""
+    return _Dispatch.apply(x, idx.to(torch.int32).contiguous(), disp, all_routed)
 
 
 def ep_combine(disp: MoeDispatcher, y_rows: torch.Tensor, w: torch.Tensor, idx: torch.Tensor, send_pos: torch.Tensor) -> torch.Tensor:
