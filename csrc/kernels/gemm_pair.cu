@@ -518,6 +518,10 @@ pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMa
               uint32_t g[32], u[32];
               read_chunk(second ? cc : 2 * cc, g);
               read_chunk(second ? cc + second : 2 * cc + 32, u);
+              if (lane >= rows) {   // zeros of rows that are none would send the quotient down its slow path, and the warp with it
+#pragma unroll
+                for (int q = 0; q < 32; ++q) g[q] = __float_as_uint(1.f);
+              }
 #pragma unroll
               for (int q = 0; q < 16; ++q) {
                 const float g0 = __uint_as_float(g[2 * q]), g1 = __uint_as_float(g[2 * q + 1]);

@@ -374,7 +374,8 @@ skinny_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensor
           store = gate;
           if (gate) {
 #pragma unroll
-            for (int q = 0; q < CH; ++q) v[q] = v[q] / (1.f + __expf(-v[q])) * ctl->up[pair][q][lane];
+            for (int q = 0; q < CH; ++q)   // (zeros of rows that are none would take the quotient's slow path)
+              if (c + q < tl.rows) v[q] = v[q] / (1.f + __expf(-v[q])) * ctl->up[pair][q][lane];
           }
           f = tl.w_tile * (WM / 2) + pair * 32 + lane;
         } else {
