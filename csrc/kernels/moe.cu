@@ -12,6 +12,7 @@
 #include "coll_device.cuh"
 #include "moe.h"
 #include "pdl.cuh"
+#include "sm100_prims.cuh"
 
 namespace amem {
 namespace moek {
@@ -394,6 +395,152 @@ __device__ void combine_body(const MoeArgs& a, int cta, int nctas, int* s_abort)
   dev::proto_end(p);
 }
 
+// ---- combine of one rank with many choices and long rows: the bulk-copy engine gathers the rows of one token after the
+// other (eight choices and a piece of the row a stage) into a ring that never runs dry, and eight warps add them up; the
+// sums are those of combine_items, choice after choice.  A warp that loads its own rows has none in flight while it looks
+// up the next ones and stores: 16384 x 8 rows of 8 KB 233 us, so 204 (185 are the bytes).  With two choices a stage is too
+// short to pay for its barriers: 8192 x 2 rows 38 us against 49.
+constexpr int kStreamWarps = 8, kStreamThreads = 32 * (kStreamWarps + 1), kStreamRows = 8, kStreamStages = 16;
+constexpr uint32_t kStreamRing = 192 * 1024, kStreamPiece = 8192;   // bytes of the ring; of a row at a time, at most
+constexpr long kStreamMinRows = 4096;    // fewer rows than keep the rings filling for a while: combine_items
+// Equal pieces of a row, multiples of 16 bytes.
+__host__ __device__ inline uint32_t stream_piece(size_t row_bytes) {
+  const size_t parts = (row_bytes + kStreamPiece - 1) / kStreamPiece;
+  return (uint32_t)((row_bytes / 16 + parts - 1) / parts * 16);
+}
+struct StreamCtl {
+  uint64_t full[kStreamStages], empty[kStreamStages];
+  float w[kStreamStages][kStreamRows];
+  uint32_t kept[kStreamStages];   // bit r: row r of the stage is there
+  int abort;
+};
+__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sm100::smem_u32(dst)), "l"(src), "r"(bytes),
+               "r"(sm100::smem_u32(bar)) : "memory");
+}
+__global__ void __launch_bounds__(kStreamThreads, 1) combine_stream_kernel(const __grid_constant__ MoeArgs a, int stages) {
+  extern __shared__ __align__(128) char ring[];   // [stages][min(k, kStreamRows)][piece]
+  __shared__ StreamCtl ctl;
+  pdl_launch_dependents();
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x / 32, 0), lane = threadIdx.x % 32;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      sm100::mbar_init(&ctl.full[s], 1);
+      sm100::mbar_init(&ctl.empty[s], kStreamWarps);
+    }
+    ctl.abort = 0;
+    sm100::mbar_fence_init();
+  }
+  __syncthreads();
+  pdl_wait();
+  const size_t row_bytes = (size_t)a.d * 2;
+  const uint32_t piece = stream_piece(row_bytes);
+  const int kc = min(a.k, kStreamRows), passes = (a.k + kStreamRows - 1) / kStreamRows, parts = (int)((row_bytes + piece - 1) / piece);
+  const int items = a.T * parts;     // (the launch keeps it below 2^30)
+  auto length = [&](int part) { return (uint32_t)min((size_t)piece, row_bytes - (size_t)part * piece); };
+  int stage = 0;
+  uint32_t phase = 0;
+  auto next = [&] {
+    if (++stage == stages) {
+      stage = 0;
+      phase ^= 1u;
+    }
+  };
+  bool ok = true;
+  if (warp == kStreamWarps) {
+    // lane r looks up and fetches row r of a stage; what it looks up for the next stage is on its way meanwhile
+    int pos_next = -1;
+    float w_next = 0.f;
+    auto look_up = [&](int item, int pass) {
+      const int j = pass * kStreamRows + lane;
+      pos_next = -1;
+      w_next = 0.f;
+      if (lane < kc && item < items && j < a.k) {
+        const size_t at = (size_t)(item / parts) * a.k + j;
+        pos_next = a.send_pos[at];
+        w_next = a.topk_w[at];
+      }
+    };
+    look_up(blockIdx.x, 0);
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+      const int part = item % parts;
+      const uint32_t len = length(part);
+      for (int pass = 0; pass < passes; ++pass) {
+        const int pos = pos_next;
+        const float w = w_next;
+        if (pass + 1 < passes) look_up(item, pass + 1);
+        else look_up(item + gridDim.x, 0);
+        const bool row = pos >= 0 && pos < a.capacity_rows;
+        const uint32_t kept = __ballot_sync(0xffffffffu, row);
+        ok = __all_sync(0xffffffffu, sm100::mbar_wait(&ctl.empty[stage], phase ^ 1u, a.coll.timeout_ns, &ctl.abort));
+        if (!ok) break;
+        if (lane < kc) ctl.w[stage][lane] = w;
+        if (lane == 0) ctl.kept[stage] = kept;
+        __syncwarp();
+        if (lane == 0) sm100::mbar_expect_tx(&ctl.full[stage], (uint32_t)__popc(kept) * len);
+        __syncwarp();
+        if (row) bulk_g2s(ring + ((size_t)stage * kc + lane) * piece, a.ybuf[0] + (size_t)pos * row_bytes + (size_t)part * piece, len, &ctl.full[stage]);
+        next();
+      }
+    }
+    if (!ok) {
+      // gave up: copies that are still in flight land within microseconds; wait for them before leaving
+      const unsigned long long begin = sm100::gtimer_ns();
+      while (sm100::gtimer_ns() - begin < 2000000ull) {
+      }
+    }
+  } else {
+    constexpr int VPL = kStreamPiece / 16 / (32 * kStreamWarps);
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+      const int part = item % parts;
+      const uint32_t len = length(part);
+      float acc[VPL][8];
+#pragma unroll
+      for (int u = 0; u < VPL; ++u)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[u][q] = 0.f;
+      for (int pass = 0; pass < passes; ++pass) {
+        ok = __all_sync(0xffffffffu, sm100::mbar_wait(&ctl.full[stage], phase, a.coll.timeout_ns, &ctl.abort));
+        if (!ok) break;
+        const uint32_t kept = ctl.kept[stage];
+        const char* rows = ring + (size_t)stage * kc * piece;
+#pragma unroll
+        for (int j = 0; j < kStreamRows; ++j)
+          if (kept >> j & 1u) {
+            const float w = ctl.w[stage][j];
+#pragma unroll
+            for (int u = 0; u < VPL; ++u) {
+              const uint32_t v = (threadIdx.x + u * 32 * kStreamWarps) * 16;
+              if (v < len) {
+                const uint4 raw = *(const uint4*)(rows + (size_t)j * piece + v);
+                const __nv_bfloat16* h = (const __nv_bfloat16*)&raw;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) acc[u][q] = fmaf(w, __bfloat162float(h[q]), acc[u][q]);
+              }
+            }
+          }
+        __syncwarp();
+        if (lane == 0) sm100::mbar_arrive(&ctl.empty[stage]);
+        next();
+      }
+      if (!ok) break;
+      char* out = (char*)a.out + (size_t)(item / parts) * row_bytes + (size_t)part * piece;
+#pragma unroll
+      for (int u = 0; u < VPL; ++u) {
+        const uint32_t v = (threadIdx.x + u * 32 * kStreamWarps) * 16;
+        if (v < len) {
+          alignas(16) __nv_bfloat16 res[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) res[q] = __float2bfloat16_rn(acc[u][q]);
+          *(uint4*)(out + v) = *(const uint4*)res;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && *(volatile int*)&ctl.abort) dev::report_error(a.coll.status, kDevBarrierTimeout, a.coll.rank, a.coll.rank, (int)blockIdx.x, 0xdead0021u);
+}
+
 // ---- the combine's backward on one rank: for every kept choice j of token t, with row p = row(t, j),
 // g_w[t, j] = <g_out[t], y[p]> and g_y[p] = w[t, j] * g_out[t].  A CTA per token: the token's gradient comes
 // from HBM once, each expert row is read and each gradient row written once (as a gather of the outputs, a
@@ -544,6 +691,16 @@ Status launch_moe_dispatch(const MoeArgs& a, cudaStream_t stream) {
 }
 
 Status launch_moe_combine(const MoeArgs& a, cudaStream_t stream) {
+  const size_t row = (size_t)a.d * 2;
+  const long items = (long)a.T * (long)((row + moek::kStreamPiece - 1) / moek::kStreamPiece);
+  if (a.coll.nranks == 1 && a.k > 4 && row >= 4096 && (long)a.T * a.k >= moek::kStreamMinRows && items < 0x40000000L) {
+    using namespace moek;
+    const uint32_t stage = (uint32_t)std::min(a.k, kStreamRows) * stream_piece(row);
+    const int stages = (int)std::min<uint32_t>(kStreamStages, kStreamRing / stage);
+    static cudaError_t ready = cudaFuncSetAttribute((const void*)combine_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamRing);
+    if (ready != cudaSuccess) return launched(ready, "moe combine (shared memory)");
+    return launched(launch(combine_stream_kernel, a, (int)std::min<long>(items, kMoeSegments), kStreamThreads, stages * stage, stream, a, stages), "moe combine");
+  }
   auto kernel = a.k <= 2 ? moek::combine_kernel<2, 4> : a.k <= 4 ? moek::combine_kernel<4, 2> : moek::combine_kernel<8, 2>;
   return launched(launch(kernel, a, 2 * kMoeSegments, moek::kCombineThreads, 0, stream, a), "moe combine");
 }

@@ -78,3 +78,11 @@ def test_dispatch_and_combine(comm, T, k, E, d, room):
             dots[s], sizes[s] = prod.sum(1) * hit[s], prod.abs().sum(1)
         assert torch.all((g_w.reshape(-1).double() - dots).abs() <= sizes * (d / 128 + 16) * 2.0 ** -24 + 1e-30)
         assert torch.equal(g_y[p[hit]], (g_out[tok[hit]].float() * w.reshape(-1)[hit].unsqueeze(1)).to(torch.bfloat16))
+
+
+# rows of at least 4 KB, more than four choices, in numbers that the bulk-copy engine gathers: five choices, eight, more
+# than a stage takes (with a last pass of one), rows in uneven pieces and in three
+@pytest.mark.parametrize("T,k,E,d", [(1400, 5, 5, 2056), (1000, 8, 64, 4096), (700, 16, 64, 2048), (530, 9, 256, 4104), (170, 33, 64, 12288)])
+@pytest.mark.parametrize("room", [1.0, 0.6])
+def test_combine_by_bulk_copies(comm, T, k, E, d, room):
+    test_dispatch_and_combine(comm, T, k, E, d, room)
