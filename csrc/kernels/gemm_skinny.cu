@@ -422,14 +422,14 @@ int skinny_gemm_tokens(const SkinnyProblem& d) {
 bool skinny_gemm_cuts(const SkinnyProblem& d, int sms) {
   // Several groups: whole tiles, so that every sum runs over K in one go, as on SM pairs (a caller's guess
   // of the number of rows, which decides between the two kernels, must not show in the result).  One
-  // group: cut where that pays.  A stage takes 0.25 us per SM (16 x 7168 x 8192 uncut: 32.9 us for 128 of
-  // them), the exchange of a cut 3.5 us, and no schedule beats reading the weights (16 x 8192 x 3584, 64
-  // tiles: 17.5 us whole, 18.8 cut, and the model, which takes a whole tile for 14, cuts it all the same; 16 x 7168
-  // x 8192, 56 tiles: 32.9 whole, 27.3 cut).
+  // group: cut where that pays.  A stage takes 0.25 us per SM whatever it holds (128 of them 31.4 us with 28 tiles of 128
+  // rows, with 56 and with 112 of 64), the exchange of a cut 6.5 us more than whole tiles take to end, and no schedule
+  // beats reading the weights (back to back, whole / cut: 16 x 8192 x 3584, 64 tiles, 16.2 / 17.7 - 20; 4096 x 4096, 32
+  // tiles, 17.7 / 13.7; 16 x 3584 x 8192, 28 tiles, 31.4 / 17.1; 16 x 7168 x 8192, 56 tiles, 31.7 / 26.3).
   const double w_tiles = (d.N + skinnyk::WM - 1) / skinnyk::WM, nkb = (d.K + skinnyk::BK - 1) / skinnyk::BK;
   const double read_us = (double)d.N * d.K * 2 / 6.5e6;
   const double whole_us = std::max(read_us, (double)(((long)w_tiles + sms - 1) / sms) * nkb * 0.25);
-  const double cut_us = std::max(read_us, w_tiles * nkb / sms * 0.25) + 3.5;
+  const double cut_us = std::max(read_us, w_tiles * nkb / sms * 0.25) + 6.5;
   return !d.group_off && cut_us < whole_us;
 }
 
