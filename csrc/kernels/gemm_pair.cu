@@ -7,8 +7,8 @@
 // what bounds the one-SM form; six stages fit, and with 256 of 512 TMEM columns per tile the
 // epilogue of one tile runs under the main loop of the next.  TMA loads carry no multicast.
 //
-// Roles per CTA: warp 0 loads (and, for the ragged end of a group along K, clears the rows that
-// belong to the next group), warp 1 of the even CTA issues every MMA, warps 2-5 drain TMEM.  The
+// Roles per CTA: warp 0 loads, warp 1 of the even CTA issues every MMA, warps 2-5 drain TMEM, and for groups
+// along K warp 6 clears the rows of a group's last block that belong to the next group.  The
 // `full` barrier of a stage lives in the even CTA and counts the bytes of both; `empty` and the
 // accumulator's `tfull` are signalled in both CTAs by one commit.
 //
@@ -45,7 +45,7 @@ constexpr int STAGES = 6;
 constexpr int A_BYTES = HM * BK * 2, B_BYTES = (BN_MAX / 2) * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int CHUNK_BYTES = 64 * BK * 2;     // MN-major operands: 64 columns x 64 of K per TMA box
 constexpr int EPI_WARPS = 4, EPI_BYTES = 32 * 128;   // staging of one epilogue warp: 32 rows x 128 bytes
-constexpr int THREADS = 32 * (2 + EPI_WARPS);
+constexpr int THREADS = 32 * (2 + EPI_WARPS), CLEAR_WARP = 2 + EPI_WARPS;
 constexpr int MAX_GROUPS = 256;
 constexpr int MAX_SLICES = 8;                        // 32-column chunks of the widest tile: one per slice at least
 constexpr size_t SLOT_FLOATS = (size_t)HM * BN_MAX;  // partial sums of one CTA
@@ -69,7 +69,8 @@ struct __align__(8) Ctl {
   uint64_t empty[STAGES];
   uint64_t tfull[2];
   uint64_t tempty[2];       // used in the even CTA
-  uint64_t tail;            // the ragged last K block of a group has landed in this CTA
+  uint64_t tail;            // the exchanged partial sums have landed in this CTA
+  uint64_t ragged[STAGES];  // the ragged last K block of a group has landed in this CTA
   uint32_t tmem_base;
   int abort;
   int off[MAX_GROUPS + 1];        // group offsets, made monotonic
@@ -132,6 +133,9 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn_sw128(const void* tile) {
   return addr | ((uint64_t)(CHUNK_BYTES >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 
+// Only operands that both lie by their contraction index can have groups along it, and need the warp that clears.
+constexpr int threads_of(int a_mn, int b_mn) { return THREADS + (a_mn && b_mn ? 32 : 0); }
+
 struct Tile {
   int group, m0, n_blk;   // first row of the tile inside the group (or matrix), column block
   int rows;               // rows left from m0 on (may exceed a tile)
@@ -186,7 +190,7 @@ __device__ __forceinline__ Tile tile_at(const Params& p, const Ctl* c, int item,
 
 // CUT: tiles may be cut along K (kept apart: the sum over slices costs registers)
 template <int A_MN, int B_MN, int CUT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads_of(A_MN, B_MN), 1)
 pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b) {
   extern __shared__ char smem_raw[];
   char* ring = (char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -209,6 +213,7 @@ pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMa
       mbar_init(&ctl->tempty[b], 2 * EPI_WARPS);
     }
     mbar_init(&ctl->tail, 1);
+    for (int s = 0; s < STAGES; ++s) mbar_init(&ctl->ragged[s], 1);
     ctl->abort = 0;
     mbar_fence_init();
     tma_prefetch_desc(&map_a);
@@ -271,7 +276,7 @@ pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMa
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     int stage = 0;
-    uint32_t phase = 0, tail_phase = 0;
+    uint32_t phase = 0;
     bool ok = true;
     const int b_chunks = (half + 63) / 64;
     const uint32_t bytes = (uint32_t)(A_BYTES + (B_MN ? b_chunks * CHUNK_BYTES : half * BK * 2));
@@ -287,7 +292,9 @@ pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMa
         char* sb = sa + A_BYTES;
         const int k = tl.k0 + kb * BK;
         // The last K block of a group may reach into the next group's rows (both operands hold rows
-        // there): it lands on a barrier of this CTA first, those rows are cleared, then it counts.
+        // there): it lands on a barrier of this CTA first, where another warp clears those rows and counts it.
+        // (Done here, the loads behind it waited: 149 us for 8 x 1024 rows of 3072 x 4096, 190 for groups of about
+        // that size, 177 so: their row tiles and K blocks are not whole.)
         const bool clear = A_MN && B_MN && p.mode == kPairGroupedK && tl.nk - kb * BK < BK;
         ok = ok && wait_bar(&ctl->empty[stage], phase ^ 1u, p.timeout_ns, abort);
         if (ok) {
@@ -297,8 +304,8 @@ pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMa
             if (rank == 0) mbar_expect_tx(&ctl->full[stage], 2 * bytes);
             uint32_t bar = in_leader(&ctl->full[stage]);
             if (clear) {
-              bar = smem_u32(&ctl->tail);
-              mbar_expect_tx(&ctl->tail, bytes);
+              bar = smem_u32(&ctl->ragged[stage]);
+              mbar_expect_tx(&ctl->ragged[stage], bytes);
             }
             if (A_MN) {
 #pragma unroll
@@ -313,19 +320,6 @@ pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMa
             }
           }
           __syncwarp();
-          if (clear) {
-            ok = wait_bar(&ctl->tail, tail_phase, p.timeout_ns, abort);
-            tail_phase ^= 1u;
-            const int r0 = tl.nk - kb * BK, r1 = (r0 + 15) & ~15;   // the MMAs of this block read r1 rows
-            const int lines = (r1 - r0) * (HM / 64 + b_chunks);
-            for (int i = lane; i < lines * 8; i += 32) {
-              const int l = i / 8, c = l / (r1 - r0), r = r0 + l % (r1 - r0);
-              *(uint4*)(sa + c * CHUNK_BYTES + r * 128 + (i % 8) * 16) = make_uint4(0, 0, 0, 0);   // B's chunks follow A's
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0 && ok) complete_leader(in_leader(&ctl->full[stage]), bytes);
-          }
         }
         if (++stage == STAGES) {
           stage = 0;
@@ -347,6 +341,37 @@ pair_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMa
       while (gtimer_ns() - t0 < 2000000ull) {
       }
     }
+  } else if (A_MN && B_MN && warp == CLEAR_WARP) {
+    // ------------------------------------------------------------ rows of the next group out of a group's last block
+    if (p.mode == kPairGroupedK) {
+      int stage = 0;
+      uint32_t phases = 0;      // of ragged[], a bit each
+      bool ok = true;
+      const int b_chunks = (half + 63) / 64;
+      const uint32_t bytes = (uint32_t)(A_BYTES + b_chunks * CHUNK_BYTES);
+      for (int t = cluster; t < total && ok; t += clusters) {
+        const Tile tl = tile_at<CUT>(p, ctl, t, tiles_n);
+        const int num_kb = (tl.nk + BK - 1) / BK;
+        if (num_kb == 0) continue;
+        const int at = (stage + num_kb - 1) % STAGES, r0 = tl.nk - (num_kb - 1) * BK;
+        stage = (stage + num_kb) % STAGES;
+        if (r0 == BK) continue;
+        ok = wait_bar(&ctl->ragged[at], phases >> at & 1u, p.timeout_ns, abort);
+        phases ^= 1u << at;
+        if (!ok) break;
+        char* sa = ring + (size_t)at * STAGE_BYTES;
+        const int r1 = (r0 + 15) & ~15;   // the MMAs of this block read r1 rows
+        const int lines = (r1 - r0) * (HM / 64 + b_chunks);
+        for (int i = lane; i < lines * 8; i += 32) {
+          const int l = i / 8, c = l / (r1 - r0), r = r0 + l % (r1 - r0);
+          *(uint4*)(sa + c * CHUNK_BYTES + r * 128 + (i % 8) * 16) = make_uint4(0, 0, 0, 0);   // B's chunks follow A's
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) complete_leader(in_leader(&ctl->full[at]), bytes);
+      }
+    }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (even CTA)
     if (rank == 0) {
@@ -592,7 +617,7 @@ template <int A_MN, int B_MN, int CUT>
 Status launch_one(const Params& p, const CUtensorMap& ma, const CUtensorMap& mb, int grid, cudaStream_t stream) {
   static cudaError_t ready = cudaFuncSetAttribute((const void*)pair_kernel<A_MN, B_MN, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
   if (ready != cudaSuccess) return fail(kCudaError, "cudaFuncSetAttribute(%zu bytes of shared memory): %s", kSmemBytes, cudaGetErrorString(ready));
-  cudaError_t e = launch_overlapped(pair_kernel<A_MN, B_MN, CUT>, dim3(grid), dim3(THREADS), kSmemBytes, stream, p, ma, mb);
+  cudaError_t e = launch_overlapped(pair_kernel<A_MN, B_MN, CUT>, dim3(grid), dim3(threads_of(A_MN, B_MN)), kSmemBytes, stream, p, ma, mb);
   if (e != cudaSuccess) return fail(kCudaError, "pair gemm launch failed: %s", cudaGetErrorString(e));
   return kSuccess;
 }
