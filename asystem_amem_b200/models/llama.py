@@ -12,8 +12,9 @@ from dataclasses import dataclass
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
-from ..ops.elementwise import gated, rms_norm, rotate
+from ..ops.elementwise import embedding, gated, rms_norm, rotate
 
 
 @dataclass
@@ -104,7 +105,12 @@ class Embed(nn.Module):
         self.tok = nn.Embedding(cfg.vocab_size, cfg.dim)
 
     def forward(self, ids, cos=None, sin=None):
-        return self.tok(ids)
+        t = self.tok
+        if (type(t) is nn.Embedding and t.padding_idx is None and t.max_norm is None and not t.scale_grad_by_freq and not t.sparse
+                and "forward" not in t.__dict__ and not t._forward_hooks and not t._forward_pre_hooks and not t._backward_hooks
+                and not t._backward_pre_hooks and not _has_any_global_hook()):
+            return embedding(ids, t.weight)
+        return t(ids)
 
 
 class Head(nn.Module):

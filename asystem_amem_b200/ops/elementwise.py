@@ -157,6 +157,37 @@ def gated(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     return F.silu(gate) * up
 
 
+@on_operands_device
+def _embedding_gradient(g: torch.Tensor, ids: torch.Tensor, rows: int) -> torch.Tensor:
+    out = torch.empty(rows, g.shape[-1], dtype=g.dtype, device=g.device)
+    B.check(B.load_library().amemEmbeddingGrad(g.data_ptr(), ids.data_ptr(), out.data_ptr(), ids.numel(), g.shape[-1], rows, _st()), "amemEmbeddingGrad")
+    return out
+
+
+class _Embedding(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, ids, table):
+        ctx.save_for_backward(ids)
+        ctx.rows = table.shape[0]
+        return F.embedding(ids, table)
+
+    @staticmethod
+    def backward(ctx, g):
+        (ids,) = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            return None, torch.ops.aten.embedding_dense_backward(g, ids, ctx.rows, -1, False)
+        return None, _embedding_gradient(dense(g), ids, ctx.rows)
+
+
+def embedding(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
+    """``table[ids]``.  The gradient of a bf16 table on one GPU sums the rows of equal ids in their order, in fp32, in one
+    kernel (up to 16384 of them: every block looks through all ids)."""
+    if (table.requires_grad and torch.is_grad_enabled() and table.dtype == torch.bfloat16 and table.dim() == 2 and table.shape[1] % 8 == 0 and table.shape[1] > 0
+            and ids.dtype == torch.int64 and 0 < ids.numel() <= 16384 and plain_cuda(ids, table) and ids.is_contiguous()):
+        return _Embedding.apply(ids, table)
+    return F.embedding(ids, table)
+
+
 def _rotate_plain(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
     x1, x2 = x.float()[..., 0::2], x.float()[..., 1::2]
     o1 = x1 * cos - x2 * sin

@@ -61,6 +61,12 @@ ncclResult_t amemRmsNormGrad(const void* g_y, const void* x, const void* w, cons
   return R(launch_rms_norm_grad(g_y, x, w, rstd, g_x, part_w, g_w, (long)rows, dim, stream));
 }
 
+ncclResult_t amemEmbeddingGrad(const void* g, const long long* ids, void* g_table, int tokens, int dim, long long rows, cudaStream_t stream) {
+  if (tokens <= 0 || dim <= 0 || dim % 8 || rows <= 0 || missing({g, ids, g_table}) || !aligned16(g, g_table, nullptr))
+    return R(fail(kInvalidArgument, "amemEmbeddingGrad: tokens=%d dim=%d (a multiple of 8) rows=%lld, 16-byte aligned", tokens, dim, rows));
+  return R(launch_embedding_grad(g, ids, g_table, tokens, dim, rows, stream));
+}
+
 ncclResult_t amemRotate(const void* const* in, void* const* out, const int* heads, const long long* strides, int tensors, const float* cos, const float* sin,
                         int batch, int seq, int dim, int inverse, cudaStream_t stream) {
   if (tensors < 1 || tensors > 2 || batch <= 0 || seq <= 0 || (long long)batch * seq > 0x7fffffffLL || dim <= 0 || dim % 8 || missing({in, out, heads, strides}) ||

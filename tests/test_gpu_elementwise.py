@@ -137,6 +137,24 @@ def test_rotary_embedding_and_its_gradient(lie, b, h, kv, s, d):
     assert g1.requires_grad and torch.equal(g1, a.grad)
 
 
+# ids that repeat within and across the 256 that a block looks at, all the same, few of many; columns in two passes
+@pytest.mark.parametrize("shape,rows,d", [((1,), 3, 8), ((2, 300), 40, 24), ((5, 257), 1, 64), ((1000,), 5000, 2056), ((3, 1000), 700, 128)])
+def test_embedding_gradient(shape, rows, d):
+    from asystem_amem_b200.ops import embedding
+    ids = torch.randint(0, rows, shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(21))
+    table, g = _rand((rows, d), 22).requires_grad_(True), _rand((*shape, d), 23)
+    out = embedding(ids, table)
+    out.backward(g)
+    assert torch.equal(out.detach(), table.detach()[ids])
+    ref, size = (torch.zeros(rows, d, device="cuda", dtype=torch.float64).index_add(0, ids.reshape(-1), t.reshape(-1, d).double()) for t in (g, g.abs()))
+    # fp32 sums of as many terms as an id has, rounded once
+    assert torch.all((table.grad.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + size * ids.numel() * 2.0 ** -24)
+    first = table.grad.clone()
+    table.grad = None
+    embedding(ids, table).backward(g)
+    assert torch.equal(table.grad, first)
+
+
 @pytest.mark.parametrize("shape", [(1, 8), (3, 5, 24), (2, 100, 1000), (2, 3, 20), (0, 16)])
 def test_gated_and_its_gradients(shape):
     from torch.func import vmap
