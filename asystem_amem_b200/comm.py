@@ -47,7 +47,10 @@ def _stream_handle(stream, tensor) -> int:
     if stream is not None:
         return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
     if hasattr(tensor, "is_cuda") and tensor.is_cuda:
-        return _torch().cuda.current_stream(tensor.device).cuda_stream
+        torch = _torch()
+        if torch.cuda.is_initialized():     # (the Stream object of the other form takes 3 us to make)
+            return torch._C._cuda_getCurrentRawStream(tensor.get_device())
+        return torch.cuda.current_stream(tensor.device).cuda_stream
     return 0
 
 

@@ -11,11 +11,7 @@ import torch
 import torch.nn.functional as F
 
 from .. import bindings as B
-from .operands import dense, on_operands_device, plain_cuda, tangents_about
-
-
-def _st() -> int:
-    return torch.cuda.current_stream().cuda_stream
+from .operands import current_stream, dense, on_operands_device, plain_cuda, tangents_about
 
 
 def _fused(h: torch.Tensor) -> bool:
@@ -39,7 +35,7 @@ class _SwiGLU(torch.autograd.Function):
 def _gradient(h: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
     out = torch.empty_like(h)
     f, p, o = h.shape[1] // 2, h.data_ptr(), out.data_ptr()
-    B.check(B.load_library().amemSwiGLUGrad(p, p + 2 * f, 2 * f, g.data_ptr(), o, o + 2 * f, h.shape[0], f, _st()), "amemSwiGLUGrad")
+    B.check(B.load_library().amemSwiGLUGrad(p, p + 2 * f, 2 * f, g.data_ptr(), o, o + 2 * f, h.shape[0], f, current_stream()), "amemSwiGLUGrad")
     return out
 
 
@@ -47,7 +43,7 @@ def _gradient(h: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
 def _forward(h: torch.Tensor) -> torch.Tensor:
     f, p = h.shape[1] // 2, h.data_ptr()
     out = torch.empty(h.shape[0], f, dtype=h.dtype, device=h.device)
-    B.check(B.load_library().amemSwiGLU(p, p + 2 * f, 2 * f, out.data_ptr(), h.shape[0], f, _st()), "amemSwiGLU")
+    B.check(B.load_library().amemSwiGLU(p, p + 2 * f, 2 * f, out.data_ptr(), h.shape[0], f, current_stream()), "amemSwiGLU")
     return out
 
 
@@ -71,7 +67,7 @@ def _rms_forward(x: torch.Tensor, weight: torch.Tensor, eps: float, keep: bool):
     rows, dim = x.numel() // x.shape[-1], x.shape[-1]
     out = torch.empty_like(x)
     rstd = torch.empty(rows, dtype=torch.float32, device=x.device) if keep else None
-    B.check(B.load_library().amemRmsNorm(x.data_ptr(), weight.data_ptr(), out.data_ptr(), rstd.data_ptr() if keep else None, rows, dim, float(eps), _st()),
+    B.check(B.load_library().amemRmsNorm(x.data_ptr(), weight.data_ptr(), out.data_ptr(), rstd.data_ptr() if keep else None, rows, dim, float(eps), current_stream()),
             "amemRmsNorm")
     return out, rstd
 
@@ -82,7 +78,7 @@ def _rms_gradient(g: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, rstd: 
     g_x, g_w = torch.empty_like(x) if of_x else None, torch.empty_like(weight) if of_weight else None
     part = torch.empty(lib.amemRmsNormGradBlocks(rows), dim, dtype=torch.float32, device=x.device) if of_weight else None
     p = [t if t is None else t.data_ptr() for t in (g_x, part, g_w)]
-    B.check(lib.amemRmsNormGrad(g.data_ptr(), x.data_ptr(), weight.data_ptr(), rstd.data_ptr(), *p, rows, dim, _st()), "amemRmsNormGrad")
+    B.check(lib.amemRmsNormGrad(g.data_ptr(), x.data_ptr(), weight.data_ptr(), rstd.data_ptr(), *p, rows, dim, current_stream()), "amemRmsNormGrad")
     return g_x, g_w
 
 
@@ -120,14 +116,14 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
 @on_operands_device
 def _gated_forward(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     out, f = torch.empty_like(gate), gate.shape[-1]
-    B.check(B.load_library().amemSwiGLU(gate.data_ptr(), up.data_ptr(), f, out.data_ptr(), gate.numel() // f, f, _st()), "amemSwiGLU")
+    B.check(B.load_library().amemSwiGLU(gate.data_ptr(), up.data_ptr(), f, out.data_ptr(), gate.numel() // f, f, current_stream()), "amemSwiGLU")
     return out
 
 
 @on_operands_device
 def _gated_gradient(gate: torch.Tensor, up: torch.Tensor, g: torch.Tensor):
     g_gate, g_up, f = torch.empty_like(gate), torch.empty_like(up), gate.shape[-1]
-    B.check(B.load_library().amemSwiGLUGrad(gate.data_ptr(), up.data_ptr(), f, g.data_ptr(), g_gate.data_ptr(), g_up.data_ptr(), gate.numel() // f, f, _st()),
+    B.check(B.load_library().amemSwiGLUGrad(gate.data_ptr(), up.data_ptr(), f, g.data_ptr(), g_gate.data_ptr(), g_up.data_ptr(), gate.numel() // f, f, current_stream()),
             "amemSwiGLUGrad")
     return g_gate, g_up
 
@@ -160,7 +156,7 @@ def gated(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 @on_operands_device
 def _embedding_gradient(g: torch.Tensor, ids: torch.Tensor, rows: int) -> torch.Tensor:
     out = torch.empty(rows, g.shape[-1], dtype=g.dtype, device=g.device)
-    B.check(B.load_library().amemEmbeddingGrad(g.data_ptr(), ids.data_ptr(), out.data_ptr(), ids.numel(), g.shape[-1], rows, _st()), "amemEmbeddingGrad")
+    B.check(B.load_library().amemEmbeddingGrad(g.data_ptr(), ids.data_ptr(), out.data_ptr(), ids.numel(), g.shape[-1], rows, current_stream()), "amemEmbeddingGrad")
     return out
 
 
@@ -216,7 +212,7 @@ def _rotate_launch(cos: torch.Tensor, sin: torch.Tensor, inverse: bool, tokens_f
     strides = [st for x, o in zip(xs, outs) for st in (*x.stride()[:3], *o.stride()[:3])]
     B.check(B.load_library().amemRotate((ctypes.c_void_p * n)(*(x.data_ptr() for x in xs)), (ctypes.c_void_p * n)(*(o.data_ptr() for o in outs)),
                                         (ctypes.c_int * n)(*(x.shape[1] for x in xs)), (ctypes.c_longlong * (6 * n))(*strides), n, cos.data_ptr(),
-                                        sin.data_ptr(), batch, seq, dim, int(inverse), _st()), "amemRotate")
+                                        sin.data_ptr(), batch, seq, dim, int(inverse), current_stream()), "amemRotate")
     return tuple(outs)
 
 
@@ -261,7 +257,7 @@ def add_pieces(dst: torch.Tensor, pieces, scale: float = 1.0) -> None:
     """``dst[at:at + t.numel()] += scale * t`` for every (at, t) of ``pieces``, which do not overlap: contiguous bf16
     tensors on the GPU that holds ``dst``, a dense fp32 tensor.  One kernel."""
     n = len(pieces)
-    base, st = dst.data_ptr(), _st()
+    base, st = dst.data_ptr(), current_stream()
     B.check(B.load_library().amemSumPieces((ctypes.c_void_p * n)(*(t.data_ptr() for _, t in pieces)), (ctypes.c_void_p * n)(*(base + 4 * at for at, _ in pieces)),
                                            (ctypes.c_longlong * n)(*(t.numel() for _, t in pieces)), n, scale, st), "amemSumPieces")
     torch.autograd.graph.increment_version(dst)      # as an in-place operator does
@@ -276,7 +272,7 @@ def adamw_step(grad, m, v, master, shard, lr: float, betas, eps: float, weight_d
     if all(t.is_cuda and t.device == grad.device and t.shape == grad.shape and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in flat) and shard.dtype == torch.bfloat16 \
             and all(t.dtype == torch.float32 for t in flat[:4]):
         B.check(B.load_library().amemAdamW(grad.data_ptr(), m.data_ptr(), v.data_ptr(), master.data_ptr(), shard.data_ptr(), grad.numel(),
-                                           float(lr), float(betas[0]), float(betas[1]), float(eps), float(weight_decay), step, _st()), "amemAdamW")
+                                           float(lr), float(betas[0]), float(betas[1]), float(eps), float(weight_decay), step, current_stream()), "amemAdamW")
         torch.autograd.graph.increment_version([t for t in flat[1:] if not t.is_inference()])   # as an in-place operator does
         return
     b1, b2 = betas

@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from .. import bindings as B
-from .operands import on_operands_device
+from .operands import current_stream, on_operands_device
 
 
 def _check(a: torch.Tensor, b: torch.Tensor) -> None:
@@ -47,7 +47,7 @@ def _host_matmul(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
 
 
 def _stream(stream) -> int:
-    return (stream or torch.cuda.current_stream()).cuda_stream
+    return stream.cuda_stream if stream else current_stream()
 
 
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, stream=None) -> torch.Tensor:

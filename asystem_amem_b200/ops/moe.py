@@ -21,7 +21,7 @@ from dataclasses import dataclass
 import torch
 
 from .. import bindings as B
-from .operands import dense, on_operands_device, plain_cuda
+from .operands import current_stream, dense, on_operands_device, plain_cuda
 
 
 def _view(ptr: int, rows: int, d: int, device) -> torch.Tensor:
@@ -41,7 +41,7 @@ def _route_launch(x: torch.Tensor, router: torch.Tensor, k: int) -> tuple[torch.
     T, d = x.shape
     idx, w = torch.empty(T, k, dtype=torch.int32, device=x.device), torch.empty(T, k, dtype=torch.float32, device=x.device)
     B.check(B.load_library().amemMoeRoute(x.data_ptr(), router.data_ptr(), idx.data_ptr(), w.data_ptr(), T, d, router.shape[0], k,
-                                          torch.cuda.current_stream().cuda_stream), "amemMoeRoute")
+                                          current_stream()), "amemMoeRoute")
     return idx, w
 
 
@@ -50,7 +50,7 @@ def _route_logits_grad(g_w: torch.Tensor, w: torch.Tensor, idx: torch.Tensor, ex
     T, k = idx.shape
     out = torch.empty(T, experts, dtype=torch.bfloat16, device=w.device)
     B.check(B.load_library().amemMoeRouteGrad(g_w.data_ptr(), w.data_ptr(), idx.data_ptr(), out.data_ptr(), T, experts, k,
-                                              torch.cuda.current_stream().cuda_stream), "amemMoeRouteGrad")
+                                              current_stream()), "amemMoeRouteGrad")
     return out
 
 
@@ -130,7 +130,7 @@ class MoeDispatcher:
         offsets = torch.empty(self.experts_per_rank + 1, dtype=torch.int32, device=x.device)
         send_pos = torch.empty(T, k, dtype=torch.int32, device=x.device)
         dropped = torch.empty(1, dtype=torch.int32, device=x.device)   # every word of the four is written by the kernels
-        st = (stream or torch.cuda.current_stream()).cuda_stream
+        st = stream.cuda_stream if stream else current_stream()
         B.check(self.comm.lib.amemMoeDispatchCounted(x.data_ptr(), topk_idx.data_ptr(), T, k, self.d, self.E, self.capacity,
                                                      counts.data_ptr(), offsets.data_ptr(), send_pos.data_ptr(), dropped.data_ptr(),
                                                      self.comm._h, st), "amemMoeDispatch")
@@ -147,7 +147,7 @@ class MoeDispatcher:
             return res if out is None else out.copy_(res)
         T, k = topk_idx.shape
         out = torch.empty(T, self.d, dtype=torch.bfloat16, device=topk_w.device) if out is None else out
-        st = (stream or torch.cuda.current_stream()).cuda_stream
+        st = stream.cuda_stream if stream else current_stream()
         B.check(self.comm.lib.amemMoeCombine(topk_idx.data_ptr(), topk_w.data_ptr(), send_pos.data_ptr(), out.data_ptr(), T, k,
                                              self.d, self.E, self.capacity, self.comm._h, st), "amemMoeCombine")
         return out
@@ -170,7 +170,7 @@ class MoeDispatcher:
         dropped = torch.empty(1, dtype=torch.int32, device=x.device)
         B.check(self.comm.lib.amemMoeDispatchLocal(x.data_ptr(), topk_idx.data_ptr(), T, k, self.d, self.E, recv.data_ptr(), rows, counts.data_ptr(),
                                                    offsets.data_ptr(), send_pos.data_ptr(), dropped.data_ptr(), self.comm._h,
-                                                   torch.cuda.current_stream().cuda_stream), "amemMoeDispatchLocal")
+                                                   current_stream()), "amemMoeDispatchLocal")
         return DispatchResult(recv, counts, offsets, send_pos, dropped)
 
     def combine_local(self, y: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.Tensor, send_pos: torch.Tensor) -> torch.Tensor:
@@ -179,7 +179,7 @@ class MoeDispatcher:
         T, k = idx.shape
         out = torch.empty(T, self.d, dtype=torch.bfloat16, device=y.device)
         B.check(self.comm.lib.amemMoeCombineLocal(idx.data_ptr(), w.data_ptr(), pos.data_ptr(), y.data_ptr(), y.shape[0], out.data_ptr(), T, k, self.d, self.E,
-                                                  self.comm._h, torch.cuda.current_stream().cuda_stream), "amemMoeCombineLocal")
+                                                  self.comm._h, current_stream()), "amemMoeCombineLocal")
         return out
 
     def combine_grad_local(self, g_out: torch.Tensor, y: torch.Tensor, topk_w: torch.Tensor, send_pos: torch.Tensor):
@@ -188,7 +188,7 @@ class MoeDispatcher:
         T, k = w.shape
         g_y, g_w = torch.empty_like(y), torch.empty(T, k, dtype=torch.float32, device=y.device)
         B.check(self.comm.lib.amemMoeCombineGradLocal(g_out.data_ptr(), y.data_ptr(), w.data_ptr(), pos.data_ptr(), g_y.data_ptr(), g_w.data_ptr(), y.shape[0],
-                                                      T, k, self.d, self.comm._h, torch.cuda.current_stream().cuda_stream), "amemMoeCombineGradLocal")
+                                                      T, k, self.d, self.comm._h, current_stream()), "amemMoeCombineGradLocal")
         return g_y, g_w
 
     # ---- host form (mock backend): same row layout as the kernels, built from the library's

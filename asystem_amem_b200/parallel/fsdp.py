@@ -25,6 +25,7 @@ import torch.nn as nn
 
 from ..ops.elementwise import adamw_step, add_pieces
 from ..ops.gemm import _begin
+from ..ops.operands import current_stream
 
 
 class _ShardedUnit:
@@ -105,7 +106,7 @@ class _ShardedUnit:
                     return False
                 pieces.append((off, g))
             off += k
-        _begin(self.comm, torch.cuda.current_stream().cuda_stream)
+        _begin(self.comm, current_stream())
         add_pieces(self.grad_shard, pieces)
         for p in self.params:
             p.grad = None
