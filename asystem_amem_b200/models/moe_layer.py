@@ -20,7 +20,7 @@ from ..ops.gemm import grouped_gemm_bf16, grouped_gemm_input_grad, grouped_gemm_
 from ..ops.elementwise import swiglu
 from ..ops.moe import MoeDispatcher, route
 from ..ops.operands import dense
-from ..parallel.ep import ep_combine, ep_dispatch
+from ..parallel.ep import ep_combine, ep_route_dispatch
 
 
 class GroupedLinear(torch.autograd.Function):
@@ -72,13 +72,13 @@ class MoELayer(nn.Module):
         return self._w13_fused[1]
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        idx, w = route(x, self.router, self.k)
         fusable = self.ffn_dim % 32 == 0 and x.is_cuda
         if torch.is_grad_enabled() and (x.requires_grad or self.w2.requires_grad):
-            rows, offsets, send_pos = ep_dispatch(self.dispatcher, x, idx, all_routed=self.router.shape[0] == self.E)
+            rows, offsets, send_pos, idx, w = ep_route_dispatch(self.dispatcher, x, self.router, self.k)
             h = GroupedLinear.apply(rows, self.w13, offsets, True)      # `rows` are the rows of the groups and no more
             y = GroupedLinear.apply(swiglu(h).to(torch.bfloat16), self.w2, offsets, True)
             return ep_combine(self.dispatcher, y, w, idx, send_pos)
+        idx, w = route(x, self.router, self.k)
         res = self.dispatcher.dispatch(x.contiguous(), idx)
         self.last_dropped = res.dropped
         if fusable:

@@ -54,6 +54,13 @@ def _route_logits_grad(g_w: torch.Tensor, w: torch.Tensor, idx: torch.Tensor, ex
     return out
 
 
+def _route_grads_torch(x: torch.Tensor, router: torch.Tensor, idx: torch.Tensor, g_w: torch.Tensor, of_x: bool, of_router: bool):
+    """The gradients of :func:`route`'s weights with a graph of their own."""
+    again = torch.softmax((x @ router.t()).float().gather(1, idx.long()), dim=1)
+    grads = iter(torch.autograd.grad(again, [t for t, n in ((x, of_x), (router, of_router)) if n], g_w, create_graph=True))
+    return next(grads) if of_x else None, next(grads) if of_router else None
+
+
 class _Route(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, router, k):
@@ -67,19 +74,21 @@ class _Route(torch.autograd.Function):
         x, router, idx, w = ctx.saved_tensors
         of_x, of_router = ctx.needs_input_grad[:2]
         if torch.is_grad_enabled():     # a graph of the gradient is wanted: torch's operators make one
-            again = torch.softmax((x @ router.t()).float().gather(1, idx.long()), dim=1)
-            grads = iter(torch.autograd.grad(again, [t for t, n in ((x, of_x), (router, of_router)) if n], g_w, create_graph=True))
-            return next(grads) if of_x else None, next(grads) if of_router else None, None
+            return *_route_grads_torch(x, router, idx, g_w, of_x, of_router), None
         g_logits = _route_logits_grad(g_w.contiguous(), w, idx, router.shape[0])
         return g_logits @ router if of_x else None, g_logits.t() @ x if of_router else None, None
+
+
+def _kernel_routes(x: torch.Tensor, router: torch.Tensor, k: int) -> bool:
+    return (x.dtype == router.dtype == torch.bfloat16 and x.dim() == router.dim() == 2 and x.shape[0] > 0 and x.shape[1] == router.shape[1]
+            and x.shape[1] > 0 and x.shape[1] % 8 == 0 and 0 < k <= router.shape[0] <= 256 and plain_cuda(x, router) and x.is_contiguous()
+            and router.is_contiguous() and (x.data_ptr() | router.data_ptr()) % 16 == 0)
 
 
 def route(x: torch.Tensor, router: torch.Tensor, k: int) -> tuple[torch.Tensor, torch.Tensor]:
     """The ``k`` largest of every token's logits ``x @ router.T`` and their softmax, largest first: int32 and fp32
     [T, k].  One kernel for bf16 rows that lie densely on one GPU (equal logits by the lower expert)."""
-    if (x.dtype == router.dtype == torch.bfloat16 and x.dim() == router.dim() == 2 and x.shape[0] > 0 and x.shape[1] == router.shape[1]
-            and x.shape[1] > 0 and x.shape[1] % 8 == 0 and 0 < k <= router.shape[0] <= 256 and plain_cuda(x, router) and x.is_contiguous()
-            and router.is_contiguous() and (x.data_ptr() | router.data_ptr()) % 16 == 0):
+    if _kernel_routes(x, router, k):
         if torch.is_grad_enabled() and (x.requires_grad or router.requires_grad):
             return _Route.apply(x, router, k)
         return _route_launch(x, router, k)
@@ -190,6 +199,15 @@ class MoeDispatcher:
         B.check(self.comm.lib.amemMoeCombineGradLocal(g_out.data_ptr(), y.data_ptr(), w.data_ptr(), pos.data_ptr(), g_y.data_ptr(), g_w.data_ptr(), y.shape[0],
                                                       T, k, self.d, self.comm._h, current_stream()), "amemMoeCombineGradLocal")
         return g_y, g_w
+
+    def input_grad_local(self, g_rows: torch.Tensor, send_pos: torch.Tensor, idx: torch.Tensor, g_logits: torch.Tensor, router: torch.Tensor) -> torch.Tensor:
+        """The tokens' gradient, bf16: of the rows that ``dispatch_local`` made of them and, through the logits' gradient
+        [T, E], of their routing."""
+        T, k = idx.shape
+        g_x = torch.empty(T, self.d, dtype=torch.bfloat16, device=g_rows.device)
+        B.check(self.comm.lib.amemMoeInputGradLocal(g_rows.data_ptr(), send_pos.data_ptr(), idx.data_ptr(), g_logits.data_ptr(), router.data_ptr(), g_x.data_ptr(),
+                                                    g_rows.shape[0], T, k, self.d, self.E, self.comm._h, current_stream()), "amemMoeInputGradLocal")
+        return g_x
 
     # ---- host form (mock backend): same row layout as the kernels, built from the library's
     # all-gather and variable-size all-to-all, so that the expert-parallel wrappers and their

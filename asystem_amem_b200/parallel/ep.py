@@ -34,7 +34,9 @@ from __future__ import annotations
 
 import torch
 
-from ..ops.moe import DispatchResult, MoeDispatcher  # noqa: F401
+from ..ops.moe import (DispatchResult, MoeDispatcher, _kernel_routes, _route_grads_torch, _route_launch, _route_logits_grad,  # noqa: F401
+                       route)
+from ..ops.operands import dense
 
 
 def _between_tensors(disp: MoeDispatcher, rows: torch.Tensor) -> bool:
@@ -107,6 +109,35 @@ class _Dispatch(torch.autograd.Function):
         return dispatch_backward(ctx.disp, g_rows.contiguous(), idx, send_pos), None, None, None
 
 
+class _RouteDispatch(torch.autograd.Function):
+    """Routing and dispatch of one rank as one step, so that the tokens' gradient, which comes through both, is one sum."""
+
+    @staticmethod
+    def forward(ctx, x, router, disp, k):
+        idx, w = _route_launch(x, router, k)
+        rows, offsets, send_pos, _ = dispatch_forward(disp, x, idx, all_routed=True)
+        ctx.disp = disp
+        ctx.save_for_backward(x, router, idx, w, send_pos)
+        ctx.mark_non_differentiable(offsets, send_pos, idx)
+        return rows, offsets, send_pos, idx, w
+
+    @staticmethod
+    def backward(ctx, g_rows, _g_off, _g_pos, _g_idx, g_w):
+        x, router, idx, w, send_pos = ctx.saved_tensors
+        of_x, of_router = ctx.needs_input_grad[:2]
+        g_x = g_router = None
+        if torch.is_grad_enabled():     # a graph of the routing's gradient is wanted: torch's operators make one
+            if of_x or of_router:
+                g_x, g_router = _route_grads_torch(x, router, idx, g_w, of_x, of_router)
+            return (g_x + dispatch_backward(ctx.disp, g_rows.contiguous(), idx, send_pos) if of_x else None), g_router, None, None
+        g_logits = _route_logits_grad(g_w.contiguous(), w, idx, router.shape[0])
+        if of_x:
+            g_x = ctx.disp.input_grad_local(dense(g_rows), send_pos, idx, g_logits, router)
+        if of_router:
+            g_router = g_logits.t() @ x
+        return g_x, g_router, None, None
+
+
 class _Combine(torch.autograd.Function):
     @staticmethod
     def forward(ctx, y_rows, w, idx, send_pos, disp):
@@ -125,6 +156,15 @@ def ep_dispatch(disp: MoeDispatcher, x: torch.Tensor, idx: torch.Tensor, all_rou
     """Differentiable dispatch: (rows grouped by local expert, expert_offsets, send_pos).  ``all_routed``: the caller knows
     that every entry of ``idx`` names an expert (see :func:`dispatch_forward`)."""
     return _Dispatch.apply(x, idx.to(torch.int32).contiguous(), disp, all_routed)
+
+
+def ep_route_dispatch(disp: MoeDispatcher, x: torch.Tensor, router: torch.Tensor, k: int):
+    """Differentiable routing (:func:`ops.moe.route`) and dispatch: (rows grouped by local expert, expert_offsets, send_pos, idx,
+    w).  One step where one rank's kernels take ``x`` and ``router``, the two otherwise."""
+    if disp.local(x) and router.shape[0] == disp.E and _kernel_routes(x, router, k):
+        return _RouteDispatch.apply(x, router, disp, k)
+    idx, w = route(x, router, k)
+    return *ep_dispatch(disp, x, idx, all_routed=router.shape[0] == disp.E), idx, w
 
 
 def ep_combine(disp: MoeDispatcher, y_rows: torch.Tensor, w: torch.Tensor, idx: torch.Tensor, send_pos: torch.Tensor) -> torch.Tensor:

@@ -845,6 +845,15 @@ ncclResult_t amemMoeCombineGradLocal(const void* g_out, const void* y, const flo
   return R(launch_moe_combine_grad(g_out, y, topk_w, send_pos, g_y, g_w, rows, T, k, d, stream));
 }
 
+// The gradient of the tokens through dispatch and routing: g_x[t] = sum_j g_rows[row(t, j)] + g_logits[t, e_j] * router[e_j].
+ncclResult_t amemMoeInputGradLocal(const void* g_rows, const int* send_pos, const int* topk_idx, const void* g_logits, const void* router, void* g_x, int rows,
+                                   int T, int k, int d, int E, ncclComm_t comm, cudaStream_t stream) {
+  MoeArgs a;
+  Status s = moe_local(comm, "amemMoeInputGradLocal", T, k, d, E, rows, {g_rows, router, g_x}, {send_pos, topk_idx, g_logits}, stream, &a);
+  if (s != kSuccess || T == 0) return R(s);
+  return R(launch_moe_input_grad(g_rows, send_pos, topk_idx, g_logits, router, g_x, rows, T, k, d, E, stream));
+}
+
 // out[T, d] = sum_j topk_w[t, j] * (expert output row of (t, j)), read from the expert ranks'
 // output buffers (the `y` of amemMoeBuffers, rows in the layout the dispatch produced).
 ncclResult_t amemMoeCombine(const int* topk_idx, const float* topk_w, const int* send_pos, void* out, int T, int k, int d, int E,

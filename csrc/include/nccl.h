@@ -240,6 +240,10 @@ ncclResult_t amemSumPieces(const void* const* src, float* const* dst, const long
  * fp32 [T, k].  The gradient of the weights down to the logits is bf16 [T, E]. */
 ncclResult_t amemMoeRoute(const void* x, const void* router, int* topk_idx, float* topk_w, int T, int d, int E, int k, cudaStream_t stream);
 ncclResult_t amemMoeRouteGrad(const float* g_w, const float* topk_w, const int* topk_idx, void* g_logits, int T, int E, int k, cudaStream_t stream);
+/* On a communicator of one rank, the gradient of the tokens through dispatch and routing at once, bf16 [T, d]:
+ * g_x[t] = sum_j g_rows[send_pos[t, j]] + g_logits[t, e_j] * router[e_j], e_j = topk_idx[t, j]. */
+ncclResult_t amemMoeInputGradLocal(const void* g_rows, const int* send_pos, const int* topk_idx, const void* g_logits, const void* router, void* g_x,
+                                   int rows, int T, int k, int d, int E, ncclComm_t comm, cudaStream_t stream);
 /* One AdamW update of n parameters in one pass: fp32 gradient, moments and master weights, bf16 copy of the
  * new weights; step counts from 1. */
 ncclResult_t amemAdamW(const float* grad, float* m, float* v, float* master, void* shard_bf16, long long n, double lr, double beta1, double beta2,

@@ -58,6 +58,11 @@ Status launch_moe_combine_grad(const void* g_out, const void* y, const float* w,
 // idx int32 and weight fp32 [T, k], the softmax over the chosen.  Its gradient down to the logits, bf16 [T, E].
 Status launch_moe_route(const void* x, const void* router, int* idx, float* weight, int T, int d, int E, int k, cudaStream_t stream);
 Status launch_moe_route_grad(const float* g_w, const float* weight, const int* idx, void* g_logits, int T, int E, int k, cudaStream_t stream);
+// Gradient of the tokens on one rank, through the dispatch and the routing at once: g_x[t] = sum over its choices of the row's
+// gradient (g_rows bf16 [rows, d] at send_pos; positions at or beyond rows count as dropped) and of the logit's gradient (g_logits
+// bf16 [T, E]) times the chosen expert's row of router.
+Status launch_moe_input_grad(const void* g_rows, const int* send_pos, const int* idx, const void* g_logits, const void* router, void* g_x, int rows, int T,
+                             int k, int d, int E, cudaStream_t stream);
 // Emulated communicator: all ranks in one cooperative grid per phase.
 Status launch_moe_dispatch_emu(const MoeArgs* host_all, const MoeArgs* dev_all, int nranks, cudaStream_t stream);
 Status launch_moe_combine_emu(const MoeArgs* host_all, const MoeArgs* dev_all, int nranks, cudaStream_t stream);

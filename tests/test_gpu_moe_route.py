@@ -81,3 +81,56 @@ def test_every_form_that_torch_takes():
     a = torch.randn(6, 64, device="cuda", generator=_gen(6)).to(torch.bfloat16).requires_grad_(True)
     (ga,) = torch.autograd.grad(route(a, torch.ones_like(router), 3)[1].sum(), a, create_graph=True)
     assert ga.requires_grad
+
+
+@pytest.fixture(scope="module")
+def comm():
+    from asystem_amem_b200 import Communicator, get_unique_id
+    c = Communicator(1, 0, get_unique_id())
+    yield c
+    torch.cuda.synchronize()
+    c.destroy()
+
+
+# columns that end inside a warp's piece and in a second one, an odd number of choices, more than a warp looks up at once, no room
+# for some rows
+@pytest.mark.parametrize("T,E,k,d,room", [(1, 8, 1, 8, 1.0), (37, 8, 3, 1032, 1.0), (700, 16, 2, 4096, 1.0), (20, 64, 40, 264, 1.0), (300, 8, 2, 72, 0.5)])
+def test_routing_and_dispatch_as_one_step(comm, T, E, k, d, room):
+    from asystem_amem_b200.ops import MoeDispatcher, route
+    from asystem_amem_b200.parallel import ep
+    x0 = torch.randn(T, d, device="cuda", generator=_gen(7)).to(torch.bfloat16)
+    router0 = (torch.randn(E, d, device="cuda", generator=_gen(8)) * d ** -0.5).to(torch.bfloat16)
+    disp = MoeDispatcher(comm, E, d, max(1, int(T * k * room)))
+    got = []
+    for fused in (True, False):
+        x, router = x0.clone().requires_grad_(True), router0.clone().requires_grad_(True)
+        if fused:
+            rows, offsets, pos, idx, w = ep.ep_route_dispatch(disp, x, router, k)
+            assert type(rows.grad_fn).__name__ == "_RouteDispatchBackward"
+        else:
+            idx, w = route(x, router, k)
+            rows, offsets, pos = ep.ep_dispatch(disp, x, idx)
+        g_rows = torch.randn(rows.shape, device="cuda", generator=_gen(9)).to(torch.bfloat16)
+        g_w = torch.randn(w.shape, device="cuda", generator=_gen(10))
+        torch.autograd.backward([rows, w], [g_rows, g_w])
+        got.append([rows.detach(), offsets, pos, idx, w.detach(), router.grad, x.grad])
+    assert all(torch.equal(a, b) for a, b in zip(got[0][:6], got[1][:6]))
+    # in 64 bits from the weights as they came out
+    pos, idx, w, gd = got[0][2].long(), got[0][3].long(), got[0][4].double(), g_w.double()
+    gl = torch.zeros(T, E, device="cuda", dtype=torch.float64).scatter_(1, idx, w * (gd - (w * gd).sum(1, keepdim=True)))
+    spread = torch.zeros_like(gl).scatter_(1, idx, w * (gd.abs() + (w * gd).abs().sum(1, keepdim=True)))
+    picked = torch.where((pos >= 0).unsqueeze(2), g_rows.double()[pos.clamp(min=0)], torch.zeros((), device="cuda", dtype=torch.float64))
+    want, terms = picked.sum(1) + gl @ router0.double(), spread @ router0.double().abs()
+    # one rounding of the sum to bf16, one of each logit's gradient, k + k additions and the softmax's gradient in fp32
+    small = (3 * k + 16) * 2.0 ** -23
+    assert torch.all((got[0][6].double() - want).abs() <= want.abs() * 2.0 ** -8 + terms * (2.0 ** -8 + small) + picked.abs().sum(1) * small + 1e-30)
+
+
+def test_a_graph_through_routing_and_dispatch(comm):
+    from asystem_amem_b200.ops import MoeDispatcher
+    from asystem_amem_b200.parallel import ep
+    x = torch.randn(6, 64, device="cuda", generator=_gen(11)).to(torch.bfloat16).requires_grad_(True)
+    router = torch.randn(8, 64, device="cuda", generator=_gen(12)).to(torch.bfloat16).requires_grad_(True)
+    out = ep.ep_route_dispatch(MoeDispatcher(comm, 8, 64, 12), x, router, 2)
+    (gx,) = torch.autograd.grad(out[4].square().sum() + out[0].float().sum(), x, create_graph=True)
+    assert gx.requires_grad and torch.autograd.grad(gx.float().sum(), router)[0].shape == router.shape
