@@ -9,13 +9,15 @@
 //
 // A tile cut by such a boundary is finished by whichever of its CTAs comes last: each parks its fp32
 // partial sums (64 KB at most), counts itself in, and the last one adds the parts in order of K -- the
-// result does not depend on the order of arrival, and nobody waits for anybody.
+// result does not depend on the order of arrival, and nobody waits for anybody.  With at most half as many tiles
+// as SMs and long shares every tile has an owner, which takes the end of its K blocks and LEAD more of them than its helpers take,
+// so that their parts have long been parked when it is done: it has added them up by then and does not park its own.
 //
 // Accumulator rows are output features, so a warp's store of one token covers 32 consecutive features.
 // SwiGLU pairs a gate warp with the up warp that holds the same features; they meet in shared memory.
 //
-// Measured (B200, weights from HBM, us; one-SM kernel -> this one, floor): 16 x 7168 x 8192 37.5 -> 27.8
-// (18.0: 2.7 until the first stage has landed, 3.5 for the exchange at the end), 8 groups of 3072 x 4096
+// Measured (B200, weights from HBM, us; one-SM kernel -> this one, floor): 16 x 7168 x 8192 37.5 -> 27.8,
+// 25.6 with owners (18.0; 2.7 until the first stage has landed), 8 groups of 3072 x 4096
 // with 8 rows each and SwiGLU 78.7 (SM pairs) -> 46.6 (30.8).  Stays ahead of the SM pairs up to 64 rows,
 // or 96 a group; from there the tokens' share of every stage costs more than the padding it avoids
 // (128 rows: 39.1 against 37.2).
@@ -41,6 +43,10 @@ constexpr int RING_BYTES = 198 * 1024;           // 11 stages of 16 + 2 KB (16 t
 constexpr int EPI_WARPS = 4, THREADS = 32 * (2 + EPI_WARPS);
 constexpr int MAX_GROUPS = 256;
 constexpr int MIN_UNITS = 8;                     // K blocks a CTA takes at least
+// K blocks (0.24 us each) that an owner takes longer than its helpers, and the even share from which owners pay.  Back to back,
+// even shares / leads of 12 / 24 blocks: 16 x 7168 x 8192 (48 blocks a CTA) 26.2 / 25.4 / 25.0 us, 64 x 7168 x 8192 32.5 / 30.5 / 29.7,
+// 16 x 9216 x 8192 31.6 / 30.1 / 29.4; but 16 x 3584 x 8192 (24 blocks) 17.1 / 17.2, 4 x 1024 x 8192 (8) 11.1 / 11.6.
+constexpr int LEAD = 24, MIN_OWNED = 32;
 constexpr int CH = 16;                           // tokens per epilogue chunk
 constexpr size_t SLOT_FLOATS = (size_t)MAX_NT * WM;
 
@@ -66,18 +72,51 @@ struct __align__(8) Ctl {
   float up[2][CH][32];              // SwiGLU: the up projection's values, per gate warp
 };
 
-// The sequence of K blocks and this CTA's share of it.
+// How the K blocks of a product's tiles are shared out: whole tiles; all blocks of all tiles in a row, cut evenly; or the last
+// `own` blocks of tile c for CTA c, its owner, and the others of all tiles in a row, cut evenly over the CTAs behind the owners.
+enum { WHOLE = 0, EVEN = 1, OWNERS = 2 };
+template <int HOW>
 struct Share {
-  int tiles, nkb, ctas;
-  bool cut;
-  __device__ __forceinline__ long lo(int c) const {
-    return cut ? (long)c * ((long)tiles * nkb) / ctas : (long)c * tiles / ctas * nkb;
+  int tiles, nkb, ctas, own;
+  __device__ __forceinline__ Share(const Params& p, int tiles_, int grid) {
+    tiles = tiles_;
+    nkb = (p.K + BK - 1) / BK;
+    const long units = (long)tiles * nkb;
+    ctas = (int)min((long)grid, max(1L, HOW != WHOLE ? units / MIN_UNITS : (long)tiles));
+    own = 0;
+    if (HOW == OWNERS) {
+      const int lead = min(LEAD, (int)(units / ctas) / 2);
+      own = (int)((units - (long)tiles * lead) / ctas) + lead;
+    }
   }
-  __device__ __forceinline__ int owner(long u) const {   // the CTA whose share holds K block u
-    int c = (int)(u * ctas / ((long)tiles * nkb));
+  __device__ __forceinline__ int shared() const { return nkb - own; }   // blocks of a tile that its helpers take
+  __device__ __forceinline__ long lo(int c) const {
+    if (HOW == OWNERS) return (long)(c - tiles) * ((long)tiles * shared()) / (ctas - tiles);
+    return HOW == EVEN ? (long)c * ((long)tiles * nkb) / ctas : (long)c * tiles / ctas * nkb;
+  }
+  __device__ __forceinline__ int holder(long u) const {   // the CTA whose share holds block u of the row
+    int c = HOW == OWNERS ? tiles + (int)(u * (ctas - tiles) / ((long)tiles * shared())) : (int)(u * ctas / ((long)tiles * nkb));
     while (lo(c + 1) <= u) ++c;
     while (lo(c) > u) --c;
     return c;
+  }
+  // This CTA's share, as numbers u0 <= u < u1, and what a run of them from u on is: blocks [kb0, kb1) of tile t.
+  __device__ __forceinline__ void mine(int cta, long& u0, long& u1) const {
+    const bool busy = tiles > 0 && cta < ctas, owner = HOW == OWNERS && cta < tiles;
+    u0 = busy && !owner ? lo(cta) : 0;
+    u1 = !busy ? 0 : owner ? own : lo(cta + 1);
+  }
+  __device__ __forceinline__ void run(int cta, long u, long u1, int& t, int& kb0, int& kb1) const {
+    if (HOW == OWNERS && cta < tiles) {
+      t = cta;
+      kb0 = shared() + (int)u;
+      kb1 = nkb;
+      return;
+    }
+    const int per = HOW == OWNERS ? shared() : nkb;
+    t = (int)(u / per);
+    kb0 = (int)(u - (long)t * per);
+    kb1 = (int)min((long)per, kb0 + (u1 - u));
   }
 };
 
@@ -111,6 +150,20 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const void* map, uint64_t
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ bool test_bar(uint64_t* bar, uint32_t parity) {   // does not block
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}"
+      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ uint32_t count_in(uint32_t* ctr) {
   uint32_t old;
   asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(ctr) : "memory");
@@ -127,6 +180,8 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&v)[16])
       : "memory");
 }
 
+// (Kept apart: in one kernel with the others whole tiles took 0.2 us a launch longer.)
+template <int HOW>
 __global__ void __launch_bounds__(THREADS, 1)
 skinny_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a) {
   extern __shared__ char smem_raw[];
@@ -202,15 +257,10 @@ skinny_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensor
   tc_fence_after_sync();
   const uint32_t tmem_base = ctl->tmem_base;
 
-  Share sh;
-  sh.tiles = ctl->first_tile[p.groups];
-  sh.nkb = (p.K + BK - 1) / BK;
-  sh.cut = p.ws != nullptr;
-  const long units = (long)sh.tiles * sh.nkb;
-  sh.ctas = (int)min((long)gridDim.x, max(1L, sh.cut ? units / MIN_UNITS : (long)sh.tiles));
+  const Share<HOW> sh(p, ctl->first_tile[p.groups], (int)gridDim.x);
   const int cta = blockIdx.x;
-  const bool busy = units > 0 && cta < sh.ctas;
-  const long u0 = busy ? sh.lo(cta) : 0, u1 = busy ? sh.lo(cta + 1) : 0;
+  long u0, u1;
+  sh.mine(cta, u0, u1);
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -219,8 +269,8 @@ skinny_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensor
     bool ok = true;
     const uint32_t bytes = (uint32_t)stage_bytes;
     for (long u = u0; u < u1 && ok;) {
-      const int t = (int)(u / sh.nkb), kb0 = (int)(u - (long)t * sh.nkb);
-      const int kb1 = (int)min((long)sh.nkb, kb0 + (u1 - u));
+      int t, kb0, kb1;
+      sh.run(cta, u, u1, t, kb0, kb1);
       const Tile tl = tile_at(p, ctl, t);
       for (int kb = kb0; kb < kb1 && ok; ++kb) {
         ok = wait_bar(&ctl->empty[stage], phase ^ 1u, p.timeout_ns, abort);
@@ -257,7 +307,8 @@ skinny_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensor
     uint32_t phase = 0;
     bool ok = true;
     for (long u = u0; u < u1 && ok; ++it) {
-      const int kb0 = (int)(u % sh.nkb), kb1 = (int)min((long)sh.nkb, kb0 + (u1 - u));
+      int t, kb0, kb1;
+      sh.run(cta, u, u1, t, kb0, kb1);
       const int buf = it & 1;
       ok = wait_bar(&ctl->tempty[buf], (((uint32_t)it >> 1) & 1u) ^ 1u, p.timeout_ns, abort);
       if (!ok) break;
@@ -294,22 +345,70 @@ skinny_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensor
     int it = 0;
     bool ok = true;
     for (long u = u0; u < u1 && ok; ++it) {
-      const int t = (int)(u / sh.nkb), kb0 = (int)(u - (long)t * sh.nkb);
-      const int kb1 = (int)min((long)sh.nkb, kb0 + (u1 - u));
+      int t, kb0, kb1;
+      sh.run(cta, u, u1, t, kb0, kb1);
       u += kb1 - kb0;
       const Tile tl = tile_at(p, ctl, t);
       const int buf = it & 1;
-      ok = wait_bar(&ctl->tfull[buf], ((uint32_t)it >> 1) & 1u, p.timeout_ns, abort);
-      if (!ok) break;
-      tc_fence_after_sync();
-      const uint32_t acc = tmem_base + (uint32_t)(buf * nt) + ((uint32_t)(lg * 32) << 16);
       const int used = (tl.rows + CH - 1) / CH * CH;   // token columns that matter (rows <= nt, a multiple of CH)
       const int row = lg * 32 + lane;
+      // A cut tile's parts, in order of K: those of CTAs c0, c0 + 1, ... and, with owners, the owner's last.
       int c0 = cta, parts = 1;
-      if (kb0 > 0 || kb1 < sh.nkb) {
-        // cut tile: park this part; whoever comes last adds them all
-        c0 = sh.owner((long)t * sh.nkb);
-        parts = sh.owner((long)t * sh.nkb + sh.nkb - 1) - c0 + 1;
+      const bool is_cut = HOW != WHOLE && (kb0 > 0 || kb1 < sh.nkb);
+      if (is_cut) {
+        const int per = HOW == OWNERS ? sh.shared() : sh.nkb;
+        c0 = sh.holder((long)t * per);
+        parts = sh.holder((long)t * per + per - 1) - c0 + 1 + (HOW == OWNERS ? 1 : 0);
+      }
+      uint32_t* ctr = p.ctr + (HOW == OWNERS ? t : c0);
+      auto part_at = [&](int i) {   // (a part that starts its tile lies in its CTA's second slot)
+        return p.ws + ((size_t)(HOW == OWNERS && i == parts - 1 ? t : c0 + i) * 2 + (i == 0 ? 1 : 0)) * SLOT_FLOATS + row;
+      };
+      // the sum of parts [0, n) of tokens [c, c + CH), in order of K; the loads of four parts are in flight together
+      auto add_parts = [&](int n, int c, float (&v)[CH]) {
+#pragma unroll
+        for (int q = 0; q < CH; ++q) v[q] = 0.f;
+        for (int i0 = 0; i0 < n; i0 += 4) {
+          float x[4][CH];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (i0 + j < n) {
+              const float* src = part_at(i0 + j);
+#pragma unroll
+              for (int q = 0; q < CH; ++q) x[j][q] = __ldcg(src + (size_t)(c + q) * WM);
+            }
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (i0 + j < n) {
+#pragma unroll
+              for (int q = 0; q < CH; ++q) v[q] += x[j][q];
+            }
+        }
+      };
+      const uint32_t full_parity = ((uint32_t)it >> 1) & 1u;
+      bool parked = false;      // the helpers' parts are there before the owner's own
+      if (HOW == OWNERS && cta < sh.tiles) {
+        if (warp == 2) {
+          // until its own is there this warp has nothing else to do than to look for them
+          const unsigned long long begin = gtimer_ns();
+          for (;;) {
+            parked = __shfl_sync(0xffffffffu, lane == 0 ? (int)(ld_acquire(ctr) == (uint32_t)parts - 1u) : 0, 0) != 0;
+            if (parked || __any_sync(0xffffffffu, test_bar(&ctl->tfull[buf], full_parity) || *abort || gtimer_ns() - begin > p.timeout_ns)) break;
+          }
+          if (lane == 0) *(volatile int*)&ctl->last = parked ? 1 : 0;
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI_WARPS) : "memory");
+        parked = *(volatile int*)&ctl->last != 0;
+      }
+      auto accumulated = [&] {
+        ok = wait_bar(&ctl->tfull[buf], full_parity, p.timeout_ns, abort);
+        if (ok) tc_fence_after_sync();
+        return ok;
+      };
+      if (!(HOW == OWNERS && parked) && !accumulated()) break;
+      const uint32_t acc = tmem_base + (uint32_t)(buf * nt) + ((uint32_t)(lg * 32) << 16);
+      if (is_cut && !parked) {
+        // park this part; whoever comes last adds them all
         float* slot = p.ws + ((size_t)cta * 2 + (kb0 == 0 ? 1 : 0)) * SLOT_FLOATS + row;
         for (int c = 0; c < used; c += CH) {
           uint32_t v[CH];
@@ -321,8 +420,8 @@ skinny_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensor
         // (one thread orders the parts of all four warps: barrier, release + acquire at the counter, barrier)
         asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI_WARPS) : "memory");
         if (warp == 2 && lane == 0) {
-          const bool last = count_in(p.ctr + c0) == (uint32_t)parts - 1u;
-          if (last) p.ctr[c0] = 0;
+          const bool last = count_in(ctr) == (uint32_t)parts - 1u;
+          if (last) *ctr = 0;
           *(volatile int*)&ctl->last = last ? 1 : 0;
         }
         asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI_WARPS) : "memory");
@@ -334,33 +433,20 @@ skinny_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensor
           continue;
         }
       }
+      const int there = parked ? parts - 1 : parts;   // parts of a cut tile that lie in memory; an owner's is here
       for (int c = 0; c < used; c += CH) {
         float v[CH];
-        if (parts == 1) {
-          uint32_t raw[CH];
+        uint32_t raw[CH];
+        if (is_cut) add_parts(there, c, v);
+        if (HOW == OWNERS && parked && c == 0) {
+          if (!accumulated()) break;
+          if (warp == 2 && lane == 0) *ctr = 0;    // (all parts but this one have been counted, and this one never is)
+        }
+        if (!is_cut || (HOW == OWNERS && parked)) {
           tmem_ld_32x16(acc + (uint32_t)c, raw);
           tmem_ld_wait();
 #pragma unroll
-          for (int q = 0; q < CH; ++q) v[q] = __uint_as_float(raw[q]);
-        } else {
-#pragma unroll
-          for (int q = 0; q < CH; ++q) v[q] = 0.f;
-          for (int i0 = 0; i0 < parts; i0 += 4) {   // the loads of four parts in flight, added in order of K
-            float x[4][CH];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (i0 + j < parts) {
-                const float* src = p.ws + ((size_t)(c0 + i0 + j) * 2 + (i0 + j == 0 ? 1 : 0)) * SLOT_FLOATS + row;
-#pragma unroll
-                for (int q = 0; q < CH; ++q) x[j][q] = __ldcg(src + (size_t)(c + q) * WM);
-              }
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (i0 + j < parts) {
-#pragma unroll
-                for (int q = 0; q < CH; ++q) v[q] += x[j][q];
-              }
-          }
+          for (int q = 0; q < CH; ++q) v[q] = HOW == OWNERS && is_cut ? v[q] + __uint_as_float(raw[q]) : __uint_as_float(raw[q]);
         }
         int f;
         bool store = true;
@@ -425,7 +511,7 @@ bool skinny_gemm_cuts(const SkinnyProblem& d, int sms) {
   // group: cut where that pays.  A stage takes 0.25 us per SM whatever it holds (128 of them 31.4 us with 28 tiles of 128
   // rows, with 56 and with 112 of 64), the exchange of a cut 6.5 us more than whole tiles take to end, and no schedule
   // beats reading the weights (back to back, whole / cut: 16 x 8192 x 3584, 64 tiles, 16.2 / 17.7 - 20; 4096 x 4096, 32
-  // tiles, 17.7 / 13.7; 16 x 3584 x 8192, 28 tiles, 31.4 / 17.1; 16 x 7168 x 8192, 56 tiles, 31.7 / 26.3).
+  // tiles, 17.7 / 12.7; 16 x 3584 x 8192, 28 tiles, 31.4 / 16.1; 16 x 7168 x 8192, 56 tiles, 31.7 / 25.0).
   const double w_tiles = (d.N + skinnyk::WM - 1) / skinnyk::WM, nkb = (d.K + skinnyk::BK - 1) / skinnyk::BK;
   const double read_us = (double)d.N * d.K * 2 / 6.5e6;
   const double whole_us = std::max(read_us, (double)(((long)w_tiles + sms - 1) / sms) * nkb * 0.25);
@@ -454,9 +540,17 @@ Status launch_skinny_gemm(const SkinnyProblem& d, int sms, cudaStream_t stream) 
   CUtensorMap mw, ma;
   AMEM_TRY(make_bf16_map(&mw, d.W, d.K, d.N, p.groups, d.epilogue == kPairSwiGLUHalves ? k::WM / 2 : k::WM));
   AMEM_TRY(make_bf16_map(&ma, d.A, d.K, d.rows, 1, p.nt));
-  static cudaError_t ready = cudaFuncSetAttribute((const void*)k::skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k::kSmemBytes);
+  static cudaError_t ready = [] {
+    for (const void* f : {(const void*)k::skinny_kernel<k::WHOLE>, (const void*)k::skinny_kernel<k::EVEN>, (const void*)k::skinny_kernel<k::OWNERS>})
+      if (cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k::kSmemBytes); e != cudaSuccess) return e;
+    return cudaSuccess;
+  }();
   if (ready != cudaSuccess) return fail(kCudaError, "cudaFuncSetAttribute(%zu bytes of shared memory): %s", k::kSmemBytes, cudaGetErrorString(ready));
-  cudaError_t e = launch_overlapped(k::skinny_kernel, dim3(sms), dim3(k::THREADS), k::kSmemBytes, stream, p, mw, ma);
+  // Owners need helpers, at least one each (then no helper has parts of more than two tiles), and shares that leave room for a lead.
+  const long tiles = (long)((d.rows + p.nt - 1) / p.nt) * ((d.N + k::WM - 1) / k::WM), units = tiles * ((d.K + k::BK - 1) / k::BK);
+  const bool owners = p.ws && !d.group_off && 2 * tiles <= sms && units / sms >= k::MIN_OWNED;
+  auto kernel = !p.ws ? k::skinny_kernel<k::WHOLE> : owners ? k::skinny_kernel<k::OWNERS> : k::skinny_kernel<k::EVEN>;
+  cudaError_t e = launch_overlapped(kernel, dim3(sms), dim3(k::THREADS), k::kSmemBytes, stream, p, mw, ma);
   if (e != cudaSuccess) return fail(kCudaError, "skinny gemm launch failed: %s", cudaGetErrorString(e));
   return kSuccess;
 }

@@ -47,6 +47,20 @@ def test_plain(forced, M, N, K, cut):
     assert all(torch.equal(o, outs[0]) for o in outs)
 
 
+# long shares of at most half as many tiles as SMs: 56 tiles and their helpers, 37 with a share that just suffices and rows that end
+# inside a chunk, 74 with one helper each, two token blocks a weight tile; gate and up halves
+@pytest.mark.parametrize("M,N,K", [(16, 7168, 8192), (33, 4720, 8192), (64, 9472, 4160), (200, 2304, 8200)])
+def test_tiles_with_owners(forced, M, N, K):
+    from asystem_amem_b200.ops import gemm_bf16, gemm_swiglu
+    a, b = _rand((M, K), 1), _rand((N, K), 2)
+    outs = [gemm_bf16(a, b) for _ in range(6)]
+    h = a.float() @ b.float().t()
+    _close(outs[0], h)
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    h = a.float() @ (b * 0.01).float().t()
+    _close(gemm_swiglu(a, b * 0.01), torch.nn.functional.silu(h[:, :N // 2]) * h[:, N // 2:])
+
+
 @pytest.mark.parametrize("counts", [(3, 0, 17, 40), (0, 0, 5), (9, 7, 8, 8), (200, 1, 0, 130), (0, 0)])
 @pytest.mark.parametrize("ffn,K", [(32, 64), (96, 520), (512, 4096)])
 def test_groups(forced, counts, ffn, K):
