@@ -71,7 +71,10 @@ def main():
     elif args.case == "one_gpu":
         # the kernels of the single-GPU paths in turn, inputs larger than L2 wherever the kernel is bound by memory
         from asystem_amem_b200 import Communicator, get_unique_id
-        from asystem_amem_b200.ops import MoeDispatcher, adamw_step, gemm_bf16, gemm_swiglu, swiglu
+        from asystem_amem_b200.models.llama import rope_tables
+        from asystem_amem_b200.ops import MoeDispatcher, adamw_step, embedding, gemm_bf16, gemm_swiglu, rms_norm, rotate, route, swiglu
+        from asystem_amem_b200.ops.elementwise import add_pieces
+        from asystem_amem_b200.parallel.ep import ep_route_dispatch
         bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)  # noqa: E731
         comm = Communicator(1, 0, get_unique_id())
         x, w, w13, few = bf(2048, 8192), bf(4096, 8192), bf(2 * 8192, 8192), bf(16, 8192)
@@ -83,8 +86,22 @@ def main():
         disp, tok = MoeDispatcher(comm, E, d, T * k), bf(T, d)
         top = torch.randn(T, E, device="cuda").topk(k, dim=1)
         idx, tw = top.indices.to(torch.int32), torch.softmax(top.values, dim=1)
+        norm_x, norm_w = bf(32768, 4096).requires_grad_(True), bf(4096).requires_grad_(True)
+        q, kk = bf(1, 8192, 32, 128).transpose(1, 2), bf(1, 8192, 8, 128).transpose(1, 2)
+        rope = rope_tables(8192, 128, 500000.0, "cuda")
+        table, ids = bf(65536, 4096).requires_grad_(True), torch.randint(0, 65536, (8192,), device="cuda")
+        router, few_disp = bf(8, d).requires_grad_(True), MoeDispatcher(comm, 8, d, T * 2)
+        tok_g = bf(T, d).requires_grad_(True)
         for _ in range(reps):
+            torch.autograd.grad(rms_norm(norm_x, norm_w, 1e-5), (norm_x, norm_w), norm_x.detach())
+            rotate(*rope, q, kk, as_they_lie=True)
+            add_pieces(wide, [(0, src)])
+            torch.autograd.grad(embedding(ids, table), table, tok)
+            route(tok, router.detach(), 2)
+            rows, _, _, _, top_w = ep_route_dispatch(few_disp, tok_g, router, 2)
+            torch.autograd.grad([rows, top_w], (tok_g, router), [rows.detach(), top_w.detach()])
             gemm_bf16(x, w)
+            gemm_bf16(few, w13[:7168])
             gemm_bf16(few, w13)
             gemm_swiglu(few, w13)
             comm.all_reduce(src, dst)
