@@ -37,10 +37,12 @@ def plain_cuda(*tensors: torch.Tensor) -> bool:
     """Whether ``tensors`` are ordinary tensors of one GPU in a program that runs eagerly: what a kernel that
     autograd knows only as a :class:`torch.autograd.Function` can take.  Subclasses, tracing, dispatch modes
     and function transforms (vmap, forward mode) need torch's own operators."""
+    if torch.compiler.is_compiling():       # (first: a compiler follows no further)
+        return False
     device = tensors[0].device
     return (device.type == "cuda" and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.device == device for t in tensors)
             and not tangents_about() and torch._C._functorch.peek_interpreter_stack() is None and torch._C._len_torch_dispatch_stack() == 0
-            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+            and not torch.jit.is_tracing())
 
 
 def dense(t: torch.Tensor) -> torch.Tensor:
