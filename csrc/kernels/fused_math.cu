@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(NORM_THREADS) rms_norm_kernel(const char* x, c
 // Gradients of the above.  With n = x * rstd: g_x = rstd * (g * w - n * mean(g * w * n)), g_w = sum over rows of
 // g * n.  Blocks stride over the rows and keep the columns' sums in registers; each leaves its sums in
 // part_w [gridDim.x][dim] and rms_norm_weight_grad_kernel adds them in the order of the blocks.  The same size: 10.4 + 6.6 us
-// (as torch passes about 130).
+// (as torch passes about 130).  2048 x 8192: 46.1 us, with the next row on its way 39.9, 15 are the bytes.
 template <int VECS>
 __global__ void __launch_bounds__(NORM_THREADS) rms_norm_grad_kernel(const char* g_y, const char* x, const char* w, const float* rstd, char* g_x, float* part_w,
                                                                      long rows, int dim) {
@@ -206,9 +206,12 @@ __global__ void __launch_bounds__(NORM_THREADS) rms_norm_grad_kernel(const char*
     for (int q = 0; q < 8; ++q) acc[i][q] = 0.f;
   }
   int flip = 0;
-  for (long row = blockIdx.x; row < rows; row += gridDim.x, flip ^= 1) {
-    Bf8 xv[VECS], gv[VECS];
-    const float r = rstd[row];
+  // Up to two vectors a thread, the next row is on its way while this one is reduced (four leave no registers for it).
+  constexpr bool AHEAD = VECS <= 2;
+  Bf8 x_next[VECS], g_next[VECS];
+  float r_next = 0.f;
+  auto load = [&](long row, Bf8 (&xv)[VECS], Bf8 (&gv)[VECS], float& r) {
+    r = rstd[row];
 #pragma unroll
     for (int i = 0; i < VECS; ++i) {
       const int c = threadIdx.x + i * blockDim.x;
@@ -216,6 +219,22 @@ __global__ void __launch_bounds__(NORM_THREADS) rms_norm_grad_kernel(const char*
         xv[i] = ((const Bf8*)x)[row * vecs + c];
         gv[i] = ((const Bf8*)g_y)[row * vecs + c];
       }
+    }
+  };
+  if (AHEAD && blockIdx.x < rows) load(blockIdx.x, x_next, g_next, r_next);
+  for (long row = blockIdx.x; row < rows; row += gridDim.x, flip ^= 1) {
+    Bf8 xv[VECS], gv[VECS];
+    float r;
+    if (AHEAD) {
+      r = r_next;
+#pragma unroll
+      for (int i = 0; i < VECS; ++i) {
+        xv[i] = x_next[i];
+        gv[i] = g_next[i];
+      }
+      if (row + gridDim.x < rows) load(row + gridDim.x, x_next, g_next, r_next);
+    } else {
+      load(row, xv, gv, r);
     }
     float dot = 0.f;
 #pragma unroll
@@ -306,7 +325,8 @@ __global__ void __launch_bounds__(THREADS) rotate_kernel(const __grid_constant__
 // Rows of a table's gradient (zeroed before): the first token of an id adds up the rows of all tokens that have it, in
 // their order.  A block per token; it looks through the ids 256 at a time, which is most of its work, so the number of
 // tokens is bounded by the caller.  2048 tokens of a 32768 x 2048 table: 106 us by torch's kernel, 11.8 so (cold, under
-// ncu; the zeros are another 21, as before).
+// ncu; the zeros are another 21, as before).  With the zeros, L2 flushed: 2048 tokens 32 us (torch 146), 8192 of a 65536 x 4096
+// table 122 (861), 16384 206 (1430).
 __global__ void __launch_bounds__(THREADS) embedding_grad_kernel(const char* g, const long long* ids, char* g_table, int tokens, int vecs, long long rows) {
   __shared__ int found[THREADS];
   __shared__ int before[THREADS / 32 + 1];
@@ -315,9 +335,20 @@ __global__ void __launch_bounds__(THREADS) embedding_grad_kernel(const char* g, 
   const int t = blockIdx.x, lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   const long long id = ids[t];
   if (id < 0 || id >= rows) return;
-  int earlier = 0;
+  int earlier = 0, later = 0;
   for (int i = threadIdx.x; i < t; i += THREADS) earlier |= ids[i] == id;
+  for (int i = t + 1 + threadIdx.x; i < tokens; i += THREADS) later |= ids[i] == id;
   if (__syncthreads_or(earlier)) return;
+  if (!__syncthreads_or(later)) {   // the id's only token (its sum is the row)
+    for (int v = threadIdx.x; v < vecs; v += THREADS) {
+      float f[8];
+      unpack(((const Bf8*)g)[(long)t * vecs + v], f);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) f[q] += 0.f;   // (as a sum that starts at zero: no negative zeros)
+      ((Bf8*)g_table)[id * vecs + v] = pack(f);
+    }
+    return;
+  }
   for (int v0 = 0; v0 < vecs; v0 += THREADS) {
     const int v = v0 + threadIdx.x;
     float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -348,10 +379,10 @@ __global__ void __launch_bounds__(THREADS) embedding_grad_kernel(const char* g, 
   }
 }
 
-// Threads of a block for a row of `vecs` vectors, and how many of them each thread takes: 1, 2 or 4
-int norm_threads(int vecs) {
+// Threads of a block for a row of `vecs` vectors, of which each takes up to `most`: 1, 2 or 4
+int norm_threads(int vecs, int most) {
   int x = 32;
-  while (x < NORM_THREADS && x < vecs) x *= 2;
+  while (x < NORM_THREADS && x * most < vecs) x *= 2;
   return x;
 }
 
@@ -380,7 +411,9 @@ bool rms_norm_takes(long rows, int dim) { return rows > 0 && rows <= 0x7fffffffL
 
 Status launch_rms_norm(const void* x, const void* w, void* y, float* rstd, long rows, int dim, float eps, cudaStream_t stream) {
   namespace k = mathk;
-  const int threads = k::norm_threads(dim / 8), per = (dim / 8 + threads - 1) / threads;
+  // With rows for every SM several times over, a row is a matter of bandwidth and a quarter of the threads reduce it for less
+  // (32768 x 4096: 143 us with a vector a thread, 111 so, 82 are the bytes); with few it is one of latency.
+  const int threads = k::norm_threads(dim / 8, rows >= 8 * 148 ? k::NORM_VECS : 1), per = (dim / 8 + threads - 1) / threads;
   auto kernel = per == 1 ? k::rms_norm_kernel<1> : per == 2 ? k::rms_norm_kernel<2> : k::rms_norm_kernel<4>;
   return k::launched(launch_overlapped(kernel, dim3((unsigned)rows), dim3(threads), 0, stream, (const char*)x, (const char*)w, (char*)y, rstd, dim, eps), "rms norm");
 }
@@ -391,7 +424,7 @@ int rms_norm_grad_blocks(long rows) { return (int)std::min(rows, 4L * 148); }
 Status launch_rms_norm_grad(const void* g_y, const void* x, const void* w, const float* rstd, void* g_x, float* part_w, void* g_w, long rows, int dim,
                             cudaStream_t stream) {
   namespace k = mathk;
-  const int threads = k::norm_threads(dim / 8), per = (dim / 8 + threads - 1) / threads, blocks = rms_norm_grad_blocks(rows);
+  const int threads = k::norm_threads(dim / 8, 1), per = (dim / 8 + threads - 1) / threads, blocks = rms_norm_grad_blocks(rows);
   auto kernel = per == 1 ? k::rms_norm_grad_kernel<1> : per == 2 ? k::rms_norm_grad_kernel<2> : k::rms_norm_grad_kernel<4>;
   AMEM_TRY(k::launched(launch_overlapped(kernel, dim3(blocks), dim3(threads), 0, stream, (const char*)g_y, (const char*)x, (const char*)w, rstd, (char*)g_x,
                                          part_w, rows, dim), "rms norm gradient"));
