@@ -337,8 +337,8 @@ __global__ void __launch_bounds__(THREADS) embedding_grad_kernel(const char* g, 
   if (id < 0 || id >= rows) return;
   int earlier = 0, later = 0;
   for (int i = threadIdx.x; i < t; i += THREADS) earlier |= ids[i] == id;
-  for (int i = t + 1 + threadIdx.x; i < tokens; i += THREADS) later |= ids[i] == id;
   if (__syncthreads_or(earlier)) return;
+  for (int i = t + 1 + threadIdx.x; i < tokens; i += THREADS) later |= ids[i] == id;
   if (!__syncthreads_or(later)) {   // the id's only token (its sum is the row)
     for (int v = threadIdx.x; v < vecs; v += THREADS) {
       float f[8];
