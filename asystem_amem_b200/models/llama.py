@@ -1,6 +1,8 @@
 """Llama-3-architecture decoder (RMSNorm, rotary embeddings, grouped-query attention, SwiGLU)
-with random initialisation.  The math is plain PyTorch; the library's part is the
-communication around it (see parallel.fsdp).
+with random initialisation.  The linears and the attention are plain PyTorch; norms, rotary
+embedding, gate and the embedding's gradient run on the library's kernels where their tensors are
+ordinary bf16 of one GPU (ops.elementwise), on PyTorch elsewhere; the communication is around it
+(see parallel.fsdp).
 
 Reference parity: none -- the reference ships no model; this decoder is the workload of the
 train / infer switching benchmark (the RL co-location scenario of README.md:1-60).

@@ -1,5 +1,5 @@
-"""Passes over rows as single kernels: SwiGLU and the root-mean-square norm with their gradients, the AdamW
-update of a shard.
+"""Passes over rows as single kernels: SwiGLU, the root-mean-square norm and the rotary embedding with their
+gradients, an embedding's gradient, the sum of gradients into a shard and its AdamW update.
 
 Reference parity: none -- the reference contains no arithmetic on user data.
 """
