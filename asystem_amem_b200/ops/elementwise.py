@@ -11,7 +11,7 @@ import torch
 import torch.nn.functional as F
 
 from .. import bindings as B
-from .operands import current_stream, dense, on_operands_device, plain_cuda, tangents_about
+from .operands import apart, current_stream, dense, on_operands_device, plain_cuda, tangents_about
 
 
 def _fused(h: torch.Tensor) -> bool:
@@ -95,6 +95,7 @@ class _RMSNorm(torch.autograd.Function):
         x, weight, rstd = ctx.saved_tensors
         wanted = ctx.needs_input_grad[:2]
         if torch.is_grad_enabled():     # a graph of the gradient is wanted: torch's operators make one
+            x, weight = apart(x, weight)
             at = [t for t, w in zip((x, weight), wanted) if w]
             grads = iter(torch.autograd.grad(_rms_norm(x, weight, ctx.eps), at, g, create_graph=True))
             return *(next(grads) if w else None for w in wanted), None
@@ -138,6 +139,7 @@ class _Gated(torch.autograd.Function):
     def backward(ctx, g):
         gate, up = ctx.saved_tensors
         if torch.is_grad_enabled():
+            gate, up = apart(gate, up)
             at = [t for t, w in zip((gate, up), ctx.needs_input_grad) if w]
             grads = iter(torch.autograd.grad(F.silu(gate) * up, at, g, create_graph=True))
             return tuple(next(grads) if w else None for w in ctx.needs_input_grad)

@@ -21,7 +21,7 @@ from dataclasses import dataclass
 import torch
 
 from .. import bindings as B
-from .operands import current_stream, dense, on_operands_device, plain_cuda
+from .operands import apart, current_stream, dense, on_operands_device, plain_cuda
 
 
 def _view(ptr: int, rows: int, d: int, device) -> torch.Tensor:
@@ -56,6 +56,7 @@ def _route_logits_grad(g_w: torch.Tensor, w: torch.Tensor, idx: torch.Tensor, ex
 
 def _route_grads_torch(x: torch.Tensor, router: torch.Tensor, idx: torch.Tensor, g_w: torch.Tensor, of_x: bool, of_router: bool):
     """The gradients of :func:`route`'s weights with a graph of their own."""
+    x, router = apart(x, router)
     again = torch.softmax((x @ router.t()).float().gather(1, idx.long()), dim=1)
     grads = iter(torch.autograd.grad(again, [t for t, n in ((x, of_x), (router, of_router)) if n], g_w, create_graph=True))
     return next(grads) if of_x else None, next(grads) if of_router else None

@@ -45,6 +45,12 @@ def plain_cuda(*tensors: torch.Tensor) -> bool:
             and not torch.jit.is_tracing())
 
 
+def apart(*tensors: torch.Tensor) -> list[torch.Tensor]:
+    """A view of each of ``tensors``, which autograd tells apart even where they are one tensor or one is computed from another:
+    derivatives with respect to the views are the partial ones that a backward function owes."""
+    return [t.view_as(t) for t in tensors]
+
+
 def dense(t: torch.Tensor) -> torch.Tensor:
     """``t`` where it is contiguous and starts on 16 bytes (the kernels move 16-byte vectors), a copy of
     it otherwise: a contiguous view may start at any element."""
