@@ -32,6 +32,7 @@
 #include "gemm_pair.h"
 #include "pdl.cuh"
 #include "sm100_prims.cuh"
+#include "smem_limit.h"
 
 namespace amem {
 namespace pairk {
@@ -615,9 +616,10 @@ static_assert(kSmemBytes <= 227 * 1024, "operand ring, staging and control words
 
 template <int A_MN, int B_MN, int CUT>
 Status launch_one(const Params& p, const CUtensorMap& ma, const CUtensorMap& mb, int grid, cudaStream_t stream) {
-  static cudaError_t ready = cudaFuncSetAttribute((const void*)pair_kernel<A_MN, B_MN, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-  if (ready != cudaSuccess) return fail(kCudaError, "cudaFuncSetAttribute(%zu bytes of shared memory): %s", kSmemBytes, cudaGetErrorString(ready));
-  cudaError_t e = launch_overlapped(pair_kernel<A_MN, B_MN, CUT>, dim3(grid), dim3(threads_of(A_MN, B_MN)), kSmemBytes, stream, p, ma, mb);
+  static OncePerDevice raised;
+  cudaError_t e = allow_smem(raised, pair_kernel<A_MN, B_MN, CUT>, kSmemBytes);
+  if (e != cudaSuccess) return fail(kCudaError, "cudaFuncSetAttribute(%zu bytes of shared memory): %s", kSmemBytes, cudaGetErrorString(e));
+  e = launch_overlapped(pair_kernel<A_MN, B_MN, CUT>, dim3(grid), dim3(threads_of(A_MN, B_MN)), kSmemBytes, stream, p, ma, mb);
   if (e != cudaSuccess) return fail(kCudaError, "pair gemm launch failed: %s", cudaGetErrorString(e));
   return kSuccess;
 }

@@ -30,6 +30,7 @@
 #include "gemm_skinny.h"
 #include "pdl.cuh"
 #include "sm100_prims.cuh"
+#include "smem_limit.h"
 
 namespace amem {
 namespace skinnyk {
@@ -540,17 +541,15 @@ Status launch_skinny_gemm(const SkinnyProblem& d, int sms, cudaStream_t stream) 
   CUtensorMap mw, ma;
   AMEM_TRY(make_bf16_map(&mw, d.W, d.K, d.N, p.groups, d.epilogue == kPairSwiGLUHalves ? k::WM / 2 : k::WM));
   AMEM_TRY(make_bf16_map(&ma, d.A, d.K, d.rows, 1, p.nt));
-  static cudaError_t ready = [] {
-    for (const void* f : {(const void*)k::skinny_kernel<k::WHOLE>, (const void*)k::skinny_kernel<k::EVEN>, (const void*)k::skinny_kernel<k::OWNERS>})
-      if (cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k::kSmemBytes); e != cudaSuccess) return e;
-    return cudaSuccess;
-  }();
-  if (ready != cudaSuccess) return fail(kCudaError, "cudaFuncSetAttribute(%zu bytes of shared memory): %s", k::kSmemBytes, cudaGetErrorString(ready));
   // Owners need helpers, at least one each (then no helper has parts of more than two tiles), and shares that leave room for a lead.
   const long tiles = (long)((d.rows + p.nt - 1) / p.nt) * ((d.N + k::WM - 1) / k::WM), units = tiles * ((d.K + k::BK - 1) / k::BK);
   const bool owners = p.ws && !d.group_off && 2 * tiles <= sms && units / sms >= k::MIN_OWNED;
-  auto kernel = !p.ws ? k::skinny_kernel<k::WHOLE> : owners ? k::skinny_kernel<k::OWNERS> : k::skinny_kernel<k::EVEN>;
-  cudaError_t e = launch_overlapped(kernel, dim3(sms), dim3(k::THREADS), k::kSmemBytes, stream, p, mw, ma);
+  const int how = !p.ws ? k::WHOLE : owners ? k::OWNERS : k::EVEN;
+  auto kernel = how == k::WHOLE ? k::skinny_kernel<k::WHOLE> : how == k::OWNERS ? k::skinny_kernel<k::OWNERS> : k::skinny_kernel<k::EVEN>;
+  static OncePerDevice raised[3];
+  cudaError_t e = allow_smem(raised[how], kernel, k::kSmemBytes);
+  if (e != cudaSuccess) return fail(kCudaError, "cudaFuncSetAttribute(%zu bytes of shared memory): %s", k::kSmemBytes, cudaGetErrorString(e));
+  e = launch_overlapped(kernel, dim3(sms), dim3(k::THREADS), k::kSmemBytes, stream, p, mw, ma);
   if (e != cudaSuccess) return fail(kCudaError, "skinny gemm launch failed: %s", cudaGetErrorString(e));
   return kSuccess;
 }

@@ -13,6 +13,7 @@
 #include "moe.h"
 #include "pdl.cuh"
 #include "sm100_prims.cuh"
+#include "smem_limit.h"
 
 namespace amem {
 namespace moek {
@@ -758,7 +759,8 @@ Status launch_moe_combine(const MoeArgs& a, cudaStream_t stream) {
     using namespace moek;
     const uint32_t stage = (uint32_t)std::min(a.k, kStreamRows) * stream_piece(row);
     const int stages = (int)std::min<uint32_t>(kStreamStages, kStreamRing / stage);
-    static cudaError_t ready = cudaFuncSetAttribute((const void*)combine_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamRing);
+    static OncePerDevice raised;
+    const cudaError_t ready = allow_smem(raised, combine_stream_kernel, kStreamRing);
     if (ready != cudaSuccess) return launched(ready, "moe combine (shared memory)");
     return launched(launch(combine_stream_kernel, a, (int)std::min<long>(items, kMoeSegments), kStreamThreads, stages * stage, stream, a, stages), "moe combine");
   }

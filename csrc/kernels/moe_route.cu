@@ -15,6 +15,7 @@
 #include "../core/log.h"
 #include "moe.h"
 #include "pdl.cuh"
+#include "smem_limit.h"
 
 namespace amem {
 namespace routek {
@@ -162,9 +163,10 @@ template <int MT, int NT, int AHEAD>
 Status launch(const void* x, const void* router, int* idx, float* weight, int T, int d, int E, int k, int threads, cudaStream_t stream) {
   constexpr int tokens = NT * COLS;
   const size_t smem = (size_t)(threads / 32) * MT * ROWS * (tokens + 2) * sizeof(float);
-  static cudaError_t ready = cudaFuncSetAttribute((const void*)route_kernel<MT, NT, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  if (ready != cudaSuccess) return fail(kCudaError, "cudaFuncSetAttribute(routing): %s", cudaGetErrorString(ready));
-  cudaError_t e = launch_overlapped(route_kernel<MT, NT, AHEAD>, dim3((unsigned)(((long)T + tokens - 1) / tokens)), dim3(threads), smem, stream, (const char*)x,
+  static OncePerDevice raised;
+  cudaError_t e = allow_smem(raised, route_kernel<MT, NT, AHEAD>, 96 * 1024);
+  if (e != cudaSuccess) return fail(kCudaError, "cudaFuncSetAttribute(routing): %s", cudaGetErrorString(e));
+  e = launch_overlapped(route_kernel<MT, NT, AHEAD>, dim3((unsigned)(((long)T + tokens - 1) / tokens)), dim3(threads), smem, stream, (const char*)x,
                                     (const char*)router, idx, weight, T, d, E, k);
   if (e != cudaSuccess) return fail(kCudaError, "routing launch failed: %s", cudaGetErrorString(e));
   return kSuccess;
