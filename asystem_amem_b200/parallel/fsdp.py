@@ -120,8 +120,9 @@ class _ShardedUnit:
             flat = torch.zeros(self.padded, dtype=torch.bfloat16, device=self.shard.device)
             off = 0
             for p, k in zip(self.params, self.numels):
-                if p.grad is not None:
-                    flat[off:off + k] = p.grad.reshape(-1)
+                g = p.grad
+                if g is not None:             # (a sparse one where there was no view for autograd to add it to)
+                    flat[off:off + k] = (g if g.layout == torch.strided else g.to_dense()).reshape(-1)
                 off += k
         for p in self.params:
             p.grad = None
