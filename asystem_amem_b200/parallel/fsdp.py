@@ -121,8 +121,8 @@ class _ShardedUnit:
             off = 0
             for p, k in zip(self.params, self.numels):
                 g = p.grad
-                if g is not None:             # (a sparse one where there was no view for autograd to add it to)
-                    flat[off:off + k] = (g if g.layout == torch.strided else g.to_dense()).reshape(-1)
+                if g is not None:             # (a sparse one where there was no view for autograd to add it to: its sums in fp32)
+                    flat[off:off + k] = (g if g.layout == torch.strided else g.float().to_dense()).reshape(-1)
                 off += k
         for p in self.params:
             p.grad = None
