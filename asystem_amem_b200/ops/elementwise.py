@@ -255,13 +255,18 @@ def rotate(cos: torch.Tensor, sin: torch.Tensor, *xs: torch.Tensor, as_they_lie:
 
 
 @on_operands_device
-def add_pieces(dst: torch.Tensor, pieces, scale: float = 1.0) -> None:
+def add_pieces(dst: torch.Tensor, pieces, scale: float = 1.0, comm=None) -> None:
     """``dst[at:at + t.numel()] += scale * t`` for every (at, t) of ``pieces``, which do not overlap: contiguous bf16
-    tensors on the GPU that holds ``dst``, a dense fp32 tensor.  One kernel."""
-    n = len(pieces)
+    tensors on the GPU that holds ``dst``, a dense fp32 tensor.  One kernel.  ``comm``: the one-rank communicator that this is an
+    operation of, if any; its bound on blocks holds."""
+    n, lib = len(pieces), B.load_library()
     base, st = dst.data_ptr(), current_stream()
-    B.check(B.load_library().amemSumPieces((ctypes.c_void_p * n)(*(t.data_ptr() for _, t in pieces)), (ctypes.c_void_p * n)(*(base + 4 * at for at, _ in pieces)),
-                                           (ctypes.c_longlong * n)(*(t.numel() for _, t in pieces)), n, scale, st), "amemSumPieces")
+    args = ((ctypes.c_void_p * n)(*(t.data_ptr() for _, t in pieces)), (ctypes.c_void_p * n)(*(base + 4 * at for at, _ in pieces)),
+            (ctypes.c_longlong * n)(*(t.numel() for _, t in pieces)), n, scale)
+    if comm is None:
+        B.check(lib.amemSumPieces(*args, st), "amemSumPieces")
+    else:
+        B.check(lib.amemSumPiecesLocal(*args, comm._h, st), "amemSumPiecesLocal")
     torch.autograd.graph.increment_version(dst)      # as an in-place operator does
 
 

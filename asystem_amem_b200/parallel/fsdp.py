@@ -24,8 +24,6 @@ import torch
 import torch.nn as nn
 
 from ..ops.elementwise import adamw_step, add_pieces
-from ..ops.gemm import _begin
-from ..ops.operands import current_stream
 
 
 class _ShardedUnit:
@@ -106,8 +104,7 @@ class _ShardedUnit:
                     return False
                 pieces.append((off, g))
             off += k
-        _begin(self.comm, current_stream())
-        add_pieces(self.grad_shard, pieces)
+        add_pieces(self.grad_shard, pieces, comm=self.comm)
         for p in self.params:
             p.grad = None
         return True

@@ -4,6 +4,7 @@
 #include <cmath>
 #include <initializer_list>
 
+#include "../comm/comm.h"
 #include "../core/log.h"
 #include "../include/nccl.h"
 #include "../kernels/fused_math.h"
@@ -88,23 +89,32 @@ ncclResult_t amemRotate(const void* const* in, void* const* out, const int* head
   return R(launch_rotate(a, batch, stream));
 }
 
-ncclResult_t amemSumPieces(const void* const* src, float* const* dst, const long long* n, int pieces, double scale, cudaStream_t stream) {
-  if (pieces < 0 || (pieces > 0 && missing({src, dst, n}))) return R(fail(kInvalidArgument, "amemSumPieces: %d pieces", pieces));
-  SumPieces a;
-  a.count = 0;
-  a.scale = (float)scale;
+static Status sum_pieces(const char* what, const void* const* src, float* const* dst, const long long* n, int pieces, double scale, int block_cap,
+                         cudaStream_t stream) {
+  if (pieces < 0 || (pieces > 0 && missing({src, dst, n}))) return fail(kInvalidArgument, "%s: %d pieces", what, pieces);
   for (int i = 0; i < pieces; ++i) {
     if (n[i] < 0 || (n[i] > 0 && missing({src[i], dst[i]})) || ((uintptr_t)src[i] & 1) || ((uintptr_t)dst[i] & 3))
-      return R(fail(kInvalidArgument, "amemSumPieces: piece %d of %lld elements", i, n[i]));
+      return fail(kInvalidArgument, "%s: piece %d of %lld elements", what, i, n[i]);
   }
-  for (int i = 0; i < pieces; ++i) {
-    if (n[i] > 0) a.piece[a.count++] = {(const __nv_bfloat16*)src[i], dst[i], (size_t)n[i], 0};
-    if (a.count == kMaxPieces || (i == pieces - 1 && a.count > 0)) {
-      const Status s = launch_sum_pieces(a, stream);
-      if (s != kSuccess) return R(s);
-      a.count = 0;
-    }
-  }
+  return launch_sum_pieces(src, dst, n, pieces, (float)scale, block_cap, stream);
+}
+
+ncclResult_t amemSumPieces(const void* const* src, float* const* dst, const long long* n, int pieces, double scale, cudaStream_t stream) {
+  return R(sum_pieces("amemSumPieces", src, dst, n, pieces, scale, 0, stream));
+}
+
+ncclResult_t amemSumPiecesLocal(const void* const* src, float* const* dst, const long long* n, int pieces, double scale, ncclComm_t comm, cudaStream_t stream) {
+  if (!comm) return ncclInvalidArgument;
+  Comm* c = reinterpret_cast<Comm*>(comm);
+  Status s = c->check_usable("amemSumPiecesLocal");
+  if (s == kSuccess && c->nranks() != 1) s = fail(kInvalidArgument, "amemSumPiecesLocal: a communicator of one rank expected");
+  if (s == kSuccess) s = c->prepare_stream(stream);
+  return R(s == kSuccess ? sum_pieces("amemSumPiecesLocal", src, dst, n, pieces, scale, c->block_cap(), stream) : s);
+}
+
+ncclResult_t amemSumPiecesPlan(const long long* n, int pieces, int block_cap, size_t* blocks) {
+  if (!blocks || pieces < 0 || (pieces > 0 && !n)) return ncclInvalidArgument;
+  *blocks = sum_pieces_blocks(n, pieces, block_cap);
   return ncclSuccess;
 }
 

@@ -100,6 +100,7 @@ class Comm {
   uint32_t* status_words() { return status_; }
   unsigned long long timeout_ns() const { return timeout_ns_; }
   int max_blocks() const { return max_blocks_; }
+  int block_cap() const { return block_cap_; }
   EmuGroup* emu() { return emu_.get(); }
 
   Status pause(PauseResumeStats* st);

@@ -235,6 +235,11 @@ ncclResult_t amemRotate(const void* const* in, void* const* out, const int* head
                         const float* sin, int batch, int seq, int dim, int inverse, cudaStream_t stream);
 /* dst[i][0 .. n[i]) += scale * src[i][0 .. n[i]) (fp32 += bf16) for every piece i; the pieces of dst do not overlap. */
 ncclResult_t amemSumPieces(const void* const* src, float* const* dst, const long long* n, int pieces, double scale, cudaStream_t stream);
+/* The same as an operation of a communicator of one rank: refused where that refuses one, and within its bound on blocks.  The plan says
+ * how many blocks the largest of its launches runs where the user bounds them to block_cap (0: no bound); host arithmetic only. */
+ncclResult_t amemSumPiecesLocal(const void* const* src, float* const* dst, const long long* n, int pieces, double scale, ncclComm_t comm,
+                                cudaStream_t stream);
+ncclResult_t amemSumPiecesPlan(const long long* n, int pieces, int block_cap, size_t* blocks);
 /* Routing of T tokens, bf16 [T, d] (d a multiple of 8), over E <= 256 experts: the k largest products with the rows of
  * router, bf16 [E, d], rounded to bf16, largest first (equal ones by the lower expert), and the softmax over them: int32 and
  * fp32 [T, k].  The gradient of the weights down to the logits is bf16 [T, E]. */

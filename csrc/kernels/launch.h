@@ -1,6 +1,5 @@
 // Host-side entry points of the kernel layer: launchers and the variant picker.
 #pragma once
-#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include "../core/status.h"
@@ -15,21 +14,12 @@ Status launch_collective(const CollArgs& a, const LaunchPlan& plan, cudaStream_t
 Status launch_local(const CollArgs& a, int block_cap, cudaStream_t stream, bool* handled);
 // The blocks launch_local runs for this operation; 0: it does not take it.
 size_t local_blocks(const CollArgs& a, int block_cap);
-// dst += scale * src (fp32 += bf16) for up to kMaxPieces pieces of memory, none of them empty, in one launch; fills
-// first_block.
-constexpr int kMaxPieces = 32;
-struct SumPiece {
-  const __nv_bfloat16* src;
-  float* dst;
-  size_t n;
-  int first_block;
-};
-struct SumPieces {
-  SumPiece piece[kMaxPieces];
-  int count;
-  float scale;
-};
-Status launch_sum_pieces(SumPieces& a, cudaStream_t stream);
+// dst[i][0 .. n[i]) += scale * src[i][0 .. n[i]) (fp32 += bf16) for every piece of memory i; a launch per kSumPieces pieces that are
+// not empty, none of more blocks than block_cap (0: any number).
+constexpr int kSumPieces = 32;
+Status launch_sum_pieces(const void* const* src, float* const* dst, const long long* n, int pieces, float scale, int block_cap, cudaStream_t stream);
+// The blocks that each of these launches runs, the largest of them.
+size_t sum_pieces_blocks(const long long* n, int pieces, int block_cap);
 // Launches every rank of an emulated (single-GPU) communicator as one cooperative grid.
 // `dev_all` points to `nranks` CollArgs in device-readable memory; `a` is any rank's copy
 // (used for type dispatch only).

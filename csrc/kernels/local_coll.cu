@@ -55,43 +55,59 @@ __global__ void __launch_bounds__(THREADS) scale_kernel(const TI* src, TO* dst, 
 }
 
 // dst += scale * src over several pieces of memory: the sum over one rank's gradients, tensor by tensor, added to its
-// shard where the tensors lie.  A block per 4096 elements, all its loads ahead of its stores.  67 M elements: 107 us, of
-// which 102 are the bytes (ten an element; through a flat buffer, a reduce-scatter and an add it was 26 and five passes).
+// shard where the tensors lie.  A block per 4096 elements, all its loads ahead of its stores; where the user bounds the blocks, each
+// takes several.  67 M elements: 107 us, of which 102 are the bytes (ten an element; through a flat buffer, a reduce-scatter
+// and an add it was 26 and five passes).
 constexpr int SUM_AHEAD = 2;      // vectors of eight elements a thread
+constexpr size_t SUM_BLOCK = THREADS * SUM_AHEAD * 8;
+struct SumPiece {
+  const __nv_bfloat16* src;
+  float* dst;
+  size_t n;
+  long first_block;
+};
+struct SumPieces {
+  SumPiece piece[kSumPieces];
+  int count;
+  float scale;
+  long blocks;
+};
 __global__ void __launch_bounds__(THREADS) sum_kernel(const __grid_constant__ SumPieces a) {
   pdl_launch_dependents();
   pdl_wait();
   int p = 0;
-  while (p + 1 < a.count && (int)blockIdx.x >= a.piece[p + 1].first_block) ++p;
-  const SumPiece& piece = a.piece[p];
-  const __nv_bfloat16* src = piece.src;
-  float* dst = piece.dst;
-  const size_t base = (size_t)(blockIdx.x - piece.first_block) * (THREADS * SUM_AHEAD * 8), n = piece.n;
-  if ((((uintptr_t)src | (uintptr_t)dst) & 15) || base + THREADS * SUM_AHEAD * 8 > n) {   // the end of a piece, or one at an odd place
-    for (size_t i = base + threadIdx.x; i < min(n, base + THREADS * SUM_AHEAD * 8); i += THREADS) dst[i] += a.scale * __bfloat162float(src[i]);
-    return;
-  }
-  uint4 v[SUM_AHEAD];
-  float4 d[SUM_AHEAD][2];
+  for (long block = blockIdx.x; block < a.blocks; block += gridDim.x) {
+    while (p + 1 < a.count && block >= a.piece[p + 1].first_block) ++p;
+    const SumPiece& piece = a.piece[p];
+    const __nv_bfloat16* src = piece.src;
+    float* dst = piece.dst;
+    const size_t base = (size_t)(block - piece.first_block) * SUM_BLOCK, n = piece.n;
+    if ((((uintptr_t)src | (uintptr_t)dst) & 15) || base + SUM_BLOCK > n) {   // the end of a piece, or one at an odd place
+      for (size_t i = base + threadIdx.x; i < min(n, base + SUM_BLOCK); i += THREADS) dst[i] += a.scale * __bfloat162float(src[i]);
+      continue;
+    }
+    uint4 v[SUM_AHEAD];
+    float4 d[SUM_AHEAD][2];
 #pragma unroll
-  for (int j = 0; j < SUM_AHEAD; ++j) {
-    const size_t i = base + ((size_t)j * THREADS + threadIdx.x) * 8;
-    v[j] = *(const uint4*)(src + i);
-    d[j][0] = *(const float4*)(dst + i);
-    d[j][1] = *(const float4*)(dst + i + 4);
-  }
+    for (int j = 0; j < SUM_AHEAD; ++j) {
+      const size_t i = base + ((size_t)j * THREADS + threadIdx.x) * 8;
+      v[j] = *(const uint4*)(src + i);
+      d[j][0] = *(const float4*)(dst + i);
+      d[j][1] = *(const float4*)(dst + i + 4);
+    }
 #pragma unroll
-  for (int j = 0; j < SUM_AHEAD; ++j) {
-    const size_t i = base + ((size_t)j * THREADS + threadIdx.x) * 8;
-    const __nv_bfloat162* h = (const __nv_bfloat162*)&v[j];
+    for (int j = 0; j < SUM_AHEAD; ++j) {
+      const size_t i = base + ((size_t)j * THREADS + threadIdx.x) * 8;
+      const __nv_bfloat162* h = (const __nv_bfloat162*)&v[j];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const float2 x = __bfloat1622float2(h[2 * q]), y = __bfloat1622float2(h[2 * q + 1]);
-      d[j][q].x += a.scale * x.x;
-      d[j][q].y += a.scale * x.y;
-      d[j][q].z += a.scale * y.x;
-      d[j][q].w += a.scale * y.y;
-      *(float4*)(dst + i + 4 * q) = d[j][q];
+      for (int q = 0; q < 2; ++q) {
+        const float2 x = __bfloat1622float2(h[2 * q]), y = __bfloat1622float2(h[2 * q + 1]);
+        d[j][q].x += a.scale * x.x;
+        d[j][q].y += a.scale * x.y;
+        d[j][q].z += a.scale * y.x;
+        d[j][q].w += a.scale * y.y;
+        *(float4*)(dst + i + 4 * q) = d[j][q];
+      }
     }
   }
 }
@@ -132,17 +148,42 @@ size_t local_blocks(const CollArgs& a, int block_cap) {
   return block_cap > 0 && blocks > (size_t)block_cap ? 0 : blocks;
 }
 
-Status launch_sum_pieces(SumPieces& a, cudaStream_t stream) {
-  size_t blocks = 0;
-  for (int i = 0; i < a.count; ++i) {
-    a.piece[i].first_block = (int)blocks;
-    blocks += (a.piece[i].n + localk::THREADS * localk::SUM_AHEAD * 8 - 1) / (localk::THREADS * localk::SUM_AHEAD * 8);
-    if (blocks > 0x7fffffffu) return fail(kInvalidArgument, "sum of gradients: too many elements");
+// Walks the launches: f(pieces of one of them, its blocks).
+template <typename F>
+static Status sum_launches(const void* const* src, float* const* dst, const long long* n, int pieces, int block_cap, F&& f) {
+  using namespace localk;
+  SumPieces a;
+  a.count = 0;
+  a.blocks = 0;
+  for (int i = 0; i < pieces; ++i) {
+    if (n[i] > 0) {
+      a.piece[a.count++] = {src ? (const __nv_bfloat16*)src[i] : nullptr, dst ? dst[i] : nullptr, (size_t)n[i], a.blocks};
+      a.blocks += (long)(((size_t)n[i] + SUM_BLOCK - 1) / SUM_BLOCK);
+    }
+    if (a.count == kSumPieces || (i == pieces - 1 && a.count > 0)) {
+      AMEM_TRY(f(a, std::min(a.blocks, block_cap > 0 ? (long)block_cap : 0x7fffffffL)));
+      a.count = 0;
+      a.blocks = 0;
+    }
   }
-  if (blocks == 0) return kSuccess;
-  cudaError_t e = launch_overlapped(localk::sum_kernel, dim3((unsigned)blocks), dim3(localk::THREADS), 0, stream, a);
-  if (e != cudaSuccess) return fail(kCudaError, "sum of gradients: launch failed: %s", cudaGetErrorString(e));
   return kSuccess;
+}
+
+Status launch_sum_pieces(const void* const* src, float* const* dst, const long long* n, int pieces, float scale, int block_cap, cudaStream_t stream) {
+  return sum_launches(src, dst, n, pieces, block_cap, [&](localk::SumPieces& a, long blocks) {
+    a.scale = scale;
+    cudaError_t e = launch_overlapped(localk::sum_kernel, dim3((unsigned)blocks), dim3(localk::THREADS), 0, stream, a);
+    return e == cudaSuccess ? kSuccess : fail(kCudaError, "sum of gradients: launch failed: %s", cudaGetErrorString(e));
+  });
+}
+
+size_t sum_pieces_blocks(const long long* n, int pieces, int block_cap) {
+  long most = 0;
+  sum_launches(nullptr, nullptr, n, pieces, block_cap, [&](localk::SumPieces&, long blocks) {
+    most = std::max(most, blocks);
+    return kSuccess;
+  });
+  return (size_t)most;
 }
 
 Status launch_local(const CollArgs& a, int block_cap, cudaStream_t stream, bool* handled) {
