@@ -175,7 +175,10 @@ Status launch(const void* x, const void* router, int* idx, float* weight, int T,
 }  // namespace routek
 
 // Tokens of a block: 8 while that leaves SMs without a block, then 16 and, with few experts, 32, so that the experts' rows
-// are read (out of L2) for more tokens at once.  A block has 16 warps while there is at most one for every SM.
+// are read (out of L2) for more tokens at once.  A block has 16 warps while there is at most one for every SM.  Of 4096 elements, 1 /
+// 1024 / 16384 tokens (us): 8 experts 8.2 / 11.3 / 45, 32 experts 11 / 13 / 57, 64 experts 14 / 16 / 86, 128 experts 27 / 26 / 198,
+// 256 experts 49 / 44 / 344.  From 65 experts on a block has 8 tokens, with one vector in flight: the callers in Python
+// (ops/moe.py, _route_pays) leave to a library product what that makes slower.
 Status launch_moe_route(const void* x, const void* router, int* idx, float* weight, int T, int d, int E, int k, cudaStream_t stream) {
   using namespace routek;
   const int sms = 148, n = T <= COLS * sms ? 1 : T <= 4 * COLS * sms ? 2 : 4;
