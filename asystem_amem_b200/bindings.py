@@ -151,6 +151,7 @@ def load_library(build_if_missing: bool = True) -> ctypes.CDLL:
         "amemSumPieces": [ctypes.POINTER(c_void_p), ctypes.POINTER(c_void_p), ctypes.POINTER(ctypes.c_longlong), c_int, ctypes.c_double, c_void_p],
         "amemSumPiecesLocal": [ctypes.POINTER(c_void_p), ctypes.POINTER(c_void_p), ctypes.POINTER(ctypes.c_longlong), c_int, ctypes.c_double, c_void_p, c_void_p],
         "amemSumPiecesPlan": [ctypes.POINTER(ctypes.c_longlong), c_int, c_int, P(c_size_t)],
+        "amemMoeCombinePlan": [c_int] * 3 + [P(c_int)],
         "amemMoeRoute": [c_void_p] * 4 + [c_int] * 4 + [c_void_p],
         "amemMoeInputGradLocal": [c_void_p] * 6 + [c_int] * 5 + [c_void_p, c_void_p],
         "amemMoeRouteGrad": [c_void_p] * 4 + [c_int] * 3 + [c_void_p],

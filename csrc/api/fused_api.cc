@@ -845,6 +845,12 @@ ncclResult_t amemMoeCombineGradLocal(const void* g_out, const void* y, const flo
   return R(launch_moe_combine_grad(g_out, y, topk_w, send_pos, g_y, g_w, rows, T, k, d, stream));
 }
 
+ncclResult_t amemMoeCombinePlan(int T, int k, int d, int* streams) {
+  if (!streams || T <= 0 || k <= 0 || d <= 0) return ncclInvalidArgument;
+  *streams = moe_combine_streams(T, k, d) ? 1 : 0;
+  return ncclSuccess;
+}
+
 // The gradient of the tokens through dispatch and routing: g_x[t] = sum_j g_rows[row(t, j)] + g_logits[t, e_j] * router[e_j].
 ncclResult_t amemMoeInputGradLocal(const void* g_rows, const int* send_pos, const int* topk_idx, const void* g_logits, const void* router, void* g_x, int rows,
                                    int T, int k, int d, int E, ncclComm_t comm, cudaStream_t stream) {

@@ -309,6 +309,9 @@ ncclResult_t amemGemmReduceScatter(const void* A, const void* B, void* out, int 
  * expert-sorted position (the permutation is fused into the all-to-all); amemMoeCombine pulls
  * the expert outputs back and applies the routing weights in one pass. */
 ncclResult_t amemMoeBuffers(ncclComm_t comm, int capacity_rows, int d, void** recv_x, void** y);
+/* Whether a communicator of one rank gathers the combine's rows by bulk copies (*streams 1) or by the warps' own loads (0).  Host
+ * arithmetic only. */
+ncclResult_t amemMoeCombinePlan(int T, int k, int d, int* streams);
 /* The same on a communicator of one rank between the caller's own buffers, and the combine's backward:
  * g_y[row(t, j)] = topk_w[t, j] * g_out[t] (bf16), g_w[t, j] = <g_out[t], y[row(t, j)]> (fp32). */
 ncclResult_t amemMoeDispatchLocal(const void* x, const int* topk_idx, int T, int k, int d, int E, void* recv, int capacity_rows, int* expert_counts,

@@ -403,7 +403,14 @@ __device__ void combine_body(const MoeArgs& a, int cta, int nctas, int* s_abort)
 // short to pay for its barriers: 8192 x 2 rows 38 us against 49.
 constexpr int kStreamWarps = 8, kStreamThreads = 32 * (kStreamWarps + 1), kStreamRows = 8, kStreamStages = 16;
 constexpr uint32_t kStreamRing = 192 * 1024, kStreamPiece = 8192;   // bytes of the ring; of a row at a time, at most
-constexpr long kStreamMinRows = 4096;    // fewer rows than keep the rings filling for a while: combine_items
+// A stage takes the same time for pieces of 4 KB as for 6 (16384 x 8 rows in 151 - 184 us for 4 to 6 KB, and 195 for 7, 201 for 8), so
+// short pieces are left to combine_items (129 - 182, 209, 240): rows of less than 6 KB but where there are so few of them that
+// looking them up in time is what counts (of 4 KB, stream / items: 4096 x 5 rows 37 / 41, 4096 x 6 41 / 43, 4096 x 8 45 / 45, 8192 x 8
+// 82 / 74), and rows that come to short pieces (of 8208 bytes: 520 x 8 23 / 19, 8192 x 8 191 / 139; of 16400: 8192 x 8 277 / 248).
+// At 6 KB: 16384 x 5 141 / 166, x 6 156 / 172, x 8 184 / 182, 4096 x 12 76 / 88.  Five choices of 8 KB: 150 / 221; four: not
+// taken, a stage of half the rows.  520 x 8 rows of 8 KB: 18.5 either way.
+constexpr long kStreamMinRows = 4096, kStreamFewRows = 24576;
+constexpr uint32_t kStreamShortRow = 4096, kStreamShortPiece = 6144;
 // Equal pieces of a row, multiples of 16 bytes.
 __host__ __device__ inline uint32_t stream_piece(size_t row_bytes) {
   const size_t parts = (row_bytes + kStreamPiece - 1) / kStreamPiece;
@@ -752,11 +759,19 @@ Status launch_moe_dispatch(const MoeArgs& a, cudaStream_t stream) {
   return launched(launch(moek::scatter_kernel, a, kMoeSegments, moek::kThreads, smem, stream, a), "moe scatter");
 }
 
+bool moe_combine_streams(int T, int k, int d) {
+  using namespace moek;
+  const size_t row = (size_t)d * 2, parts = (row + kStreamPiece - 1) / kStreamPiece;
+  const long rows = (long)T * k;
+  if (k <= 4 || row < kStreamShortRow || rows < kStreamMinRows || (long)T * (long)parts >= 0x40000000L) return false;
+  return stream_piece(row) >= kStreamShortPiece || (parts == 1 && rows <= kStreamFewRows);
+}
+
 Status launch_moe_combine(const MoeArgs& a, cudaStream_t stream) {
-  const size_t row = (size_t)a.d * 2;
-  const long items = (long)a.T * (long)((row + moek::kStreamPiece - 1) / moek::kStreamPiece);
-  if (a.coll.nranks == 1 && a.k > 4 && row >= 4096 && (long)a.T * a.k >= moek::kStreamMinRows && items < 0x40000000L) {
+  if (a.coll.nranks == 1 && moe_combine_streams(a.T, a.k, a.d)) {
     using namespace moek;
+    const size_t row = (size_t)a.d * 2;
+    const long items = (long)a.T * (long)((row + kStreamPiece - 1) / kStreamPiece);
     const uint32_t stage = (uint32_t)std::min(a.k, kStreamRows) * stream_piece(row);
     const int stages = (int)std::min<uint32_t>(kStreamStages, kStreamRing / stage);
     static OncePerDevice raised;

@@ -49,6 +49,8 @@ struct MoeArgs {
 
 Status launch_moe_dispatch(const MoeArgs& a, cudaStream_t stream);
 Status launch_moe_combine(const MoeArgs& a, cudaStream_t stream);
+// Whether one rank's combine gathers its rows by bulk copies.
+bool moe_combine_streams(int T, int k, int d);
 // Backward of the combine on one rank: g_w fp32 [T, k] and g_y bf16 [rows, d] (the rows that send_pos names;
 // positions at or beyond rows count as dropped).
 Status launch_moe_combine_grad(const void* g_out, const void* y, const float* w, const int* send_pos, void* g_y, float* g_w, int rows, int T, int k,

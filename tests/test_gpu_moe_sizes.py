@@ -86,3 +86,10 @@ def test_dispatch_and_combine(comm, T, k, E, d, room):
 @pytest.mark.parametrize("room", [1.0, 0.6])
 def test_combine_by_bulk_copies(comm, T, k, E, d, room):
     test_dispatch_and_combine(comm, T, k, E, d, room)
+
+
+# rows in two uneven pieces, long enough to be gathered so
+@pytest.mark.parametrize("T,k,E,d", [(530, 9, 256, 7000)])
+@pytest.mark.parametrize("room", [1.0, 0.6])
+def test_combine_of_rows_in_uneven_pieces(comm, T, k, E, d, room):
+    test_dispatch_and_combine(comm, T, k, E, d, room)
