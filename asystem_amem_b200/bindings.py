@@ -146,6 +146,7 @@ def load_library(build_if_missing: bool = True) -> ctypes.CDLL:
         "amemRmsNormGradBlocks": [ctypes.c_longlong],
         "amemRmsNormGrad": [c_void_p] * 7 + [ctypes.c_longlong, c_int, c_void_p],
         "amemEmbeddingGrad": [c_void_p, c_void_p, c_void_p, c_int, c_int, ctypes.c_longlong, c_void_p],
+        "amemEmbeddingGradShared": [c_void_p] * 4 + [c_int, c_int, ctypes.c_longlong, c_void_p],
         "amemRotate": [ctypes.POINTER(c_void_p), ctypes.POINTER(c_void_p), ctypes.POINTER(c_int), ctypes.POINTER(ctypes.c_longlong), c_int, c_void_p,
                        c_void_p, c_int, c_int, c_int, c_int, c_void_p],
         "amemSumPieces": [ctypes.POINTER(c_void_p), ctypes.POINTER(c_void_p), ctypes.POINTER(ctypes.c_longlong), c_int, ctypes.c_double, c_void_p],

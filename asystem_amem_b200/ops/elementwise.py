@@ -158,7 +158,10 @@ def gated(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 @on_operands_device
 def _embedding_gradient(g: torch.Tensor, ids: torch.Tensor, rows: int) -> torch.Tensor:
     out = torch.empty(rows, g.shape[-1], dtype=g.dtype, device=g.device)
-    B.check(B.load_library().amemEmbeddingGrad(g.data_ptr(), ids.data_ptr(), out.data_ptr(), ids.numel(), g.shape[-1], rows, current_stream()), "amemEmbeddingGrad")
+    n = ids.numel()
+    work = torch.empty((n + 15) // 16 * 16, dtype=torch.uint8, device=g.device)
+    B.check(B.load_library().amemEmbeddingGradShared(g.data_ptr(), ids.data_ptr(), out.data_ptr(), work.data_ptr(), n, g.shape[-1], rows, current_stream()),
+            "amemEmbeddingGrad")
     return out
 
 
@@ -178,8 +181,8 @@ class _Embedding(torch.autograd.Function):
 
 
 def embedding(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
-    """``table[ids]``.  The gradient of a bf16 table on one GPU sums the rows of equal ids in their order, in fp32, in one
-    kernel (up to 16384 of them: every block looks through all ids)."""
+    """``table[ids]``.  The gradient of a bf16 table on one GPU sums the rows of equal ids in fp32, in an order that the ids alone
+    decide, by the library's kernels (up to 16384 ids: every block looks through all of them)."""
     if (table.requires_grad and torch.is_grad_enabled() and table.dtype == torch.bfloat16 and table.dim() == 2 and table.shape[1] % 8 == 0 and table.shape[1] > 0
             and ids.dtype == torch.int64 and 0 < ids.numel() <= 16384 and plain_cuda(ids, table) and ids.is_contiguous()):
         return _Embedding.apply(ids, table)

@@ -62,10 +62,21 @@ ncclResult_t amemRmsNormGrad(const void* g_y, const void* x, const void* w, cons
   return R(launch_rms_norm_grad(g_y, x, w, rstd, g_x, part_w, g_w, (long)rows, dim, stream));
 }
 
-ncclResult_t amemEmbeddingGrad(const void* g, const long long* ids, void* g_table, int tokens, int dim, long long rows, cudaStream_t stream) {
-  if (tokens <= 0 || dim <= 0 || dim % 8 || rows <= 0 || missing({g, ids, g_table}) || !aligned16(g, g_table, nullptr))
+ncclResult_t amemEmbeddingGradShared(const void* g, const long long* ids, void* g_table, void* work, int tokens, int dim, long long rows, cudaStream_t stream) {
+  if (tokens <= 0 || dim <= 0 || dim % 8 || rows <= 0 || missing({g, ids, g_table, work}) || !aligned16(g, g_table, work))
     return R(fail(kInvalidArgument, "amemEmbeddingGrad: tokens=%d dim=%d (a multiple of 8) rows=%lld, 16-byte aligned", tokens, dim, rows));
-  return R(launch_embedding_grad(g, ids, g_table, tokens, dim, rows, stream));
+  return R(launch_embedding_grad(g, ids, g_table, (unsigned char*)work, tokens, dim, rows, stream));
+}
+
+ncclResult_t amemEmbeddingGrad(const void* g, const long long* ids, void* g_table, int tokens, int dim, long long rows, cudaStream_t stream) {
+  void* work = nullptr;
+  if (tokens > 0 && !missing({g, ids, g_table})) {
+    const cudaError_t e = cudaMallocAsync(&work, ((size_t)tokens + 15) / 16 * 16, stream);
+    if (e != cudaSuccess) return R(fail(kCudaError, "amemEmbeddingGrad: %s", cudaGetErrorString(e)));
+  }
+  const ncclResult_t r = amemEmbeddingGradShared(g, ids, g_table, work, tokens, dim, rows, stream);
+  if (work) cudaFreeAsync(work, stream);
+  return r;
 }
 
 ncclResult_t amemRotate(const void* const* in, void* const* out, const int* heads, const long long* strides, int tensors, const float* cos, const float* sin,

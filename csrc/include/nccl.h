@@ -224,9 +224,12 @@ ncclResult_t amemRmsNorm(const void* x, const void* w, void* y, float* rstd, lon
 int amemRmsNormGradBlocks(long long rows);
 ncclResult_t amemRmsNormGrad(const void* g_y, const void* x, const void* w, const float* rstd, void* g_x, float* part_w, void* g_w, long long rows,
                              int dim, cudaStream_t stream);
-/* Gradient of an embedding table, bf16 [rows, dim]: the sums of the rows of g[tokens, dim] that have the same id, in the order
- * of the tokens, fp32 inside; zero where no token points. */
+/* Gradient of an embedding table, bf16 [rows, dim]: the sums of the rows of g[tokens, dim] that have the same id, fp32 inside, in an
+ * order that the ids alone decide; zero where no token points.  The second form takes its work memory, `tokens` bytes rounded
+ * up to 16 at a 16-byte boundary, from the caller; the first allocates it on the stream. */
 ncclResult_t amemEmbeddingGrad(const void* g, const long long* ids, void* g_table, int tokens, int dim, long long rows, cudaStream_t stream);
+ncclResult_t amemEmbeddingGradShared(const void* g, const long long* ids, void* g_table, void* work, int tokens, int dim, long long rows,
+                                     cudaStream_t stream);
 /* Rotary embedding of one or two bf16 tensors [batch, heads[i], seq, dim]: (o[2j], o[2j+1]) is (x[2j], x[2j+1]) turned by
  * the angle whose fp32 cosine and sine stand at [position][j] (by its negative with inverse != 0, which is the gradient).
  * strides: six per tensor, of batch, head and position in elements, first of the input, then of the output; multiples of

@@ -323,22 +323,27 @@ __global__ void __launch_bounds__(THREADS) rotate_kernel(const __grid_constant__
 }
 
 // Rows of a table's gradient (zeroed before): the first token of an id adds up the rows of all tokens that have it, in
-// their order.  A block per token; it looks through the ids 256 at a time, which is most of its work, so the number of
-// tokens is bounded by the caller.  2048 tokens of a 32768 x 2048 table: 106 us by torch's kernel, 11.8 so (cold, under
-// ncu; the zeros are another 21, as before).  With the zeros, L2 flushed: 2048 tokens 32 us (torch 146), 8192 of a 65536 x 4096
-// table 122 (861), 16384 206 (1430).
-__global__ void __launch_bounds__(THREADS) embedding_grad_kernel(const char* g, const long long* ids, char* g_table, int tokens, int vecs, long long rows) {
-  __shared__ int found[THREADS];
-  __shared__ int before[THREADS / 32 + 1];
+// their order, four in flight.  A block per token; it looks through the ids 256 at a time, which is most of its work (they stay in L1: no
+// shared memory to speak of), so the number of tokens is bounded by the caller.  The block of an id of `many` tokens and more would be
+// busy long after the others: it marks the token and leaves the id to embedding_many_kernel.  With the zeros, L2 flushed, us (torch's
+// kernel / every id its block's / so): 2048 tokens of a 32768 x 2048 table drawn evenly 146 / 32 / 34, by Zipf's law 144 / 97 / 48, all of
+// one id 189 / 833 / 46; 16384 of 65536 x 4096 evenly 1397 / 204 / 191, by Zipf's law 1016 / 1285 / 249, half of them one id
+// 1097 / 6458 / 239, all of them 754 / 12983 / 249, each id 70 times 759 / 235 / 155.
+constexpr int MOST = 128, AHEAD = 4;   // of `many`; rows in flight
+__global__ void __launch_bounds__(THREADS, 6) embedding_grad_kernel(const char* g, const long long* ids, char* g_table, unsigned char* marks, int many, int tokens, int vecs,
+                                                                 long long rows) {
+  __shared__ int found[MOST];
+  __shared__ int before[THREADS / 32];
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x, lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   const long long id = ids[t];
+  if (threadIdx.x == 0) marks[t] = 0;
   if (id < 0 || id >= rows) return;
   int earlier = 0, later = 0;
   for (int i = threadIdx.x; i < t; i += THREADS) earlier |= ids[i] == id;
   if (__syncthreads_or(earlier)) return;
-  for (int i = t + 1 + threadIdx.x; i < tokens; i += THREADS) later |= ids[i] == id;
+  for (int i = t + 1 + threadIdx.x; i < tokens; i += THREADS) later += ids[i] == id;
   if (!__syncthreads_or(later)) {   // the id's only token (its sum is the row)
     for (int v = threadIdx.x; v < vecs; v += THREADS) {
       float f[8];
@@ -349,33 +354,206 @@ __global__ void __launch_bounds__(THREADS) embedding_grad_kernel(const char* g, 
     }
     return;
   }
-  for (int v0 = 0; v0 < vecs; v0 += THREADS) {
-    const int v = v0 + threadIdx.x;
+  later = __reduce_add_sync(0xffffffffu, later);
+  if (lane == 0) before[warp] = later;
+  __syncthreads();
+  int all = 1;
+  for (int w = 0; w < THREADS / 32; ++w) all += before[w];
+  if (all >= many) {
+    if (threadIdx.x == 0) marks[t] = 1;
+    return;
+  }
+  for (int base = t, have = 0; have < all && base < tokens; base += THREADS) {
+    const int i = base + threadIdx.x;
+    const bool same = i < tokens && ids[i] == id;
+    if (!__syncthreads_or(same)) continue;
+    const unsigned mask = __ballot_sync(0xffffffffu, same);
+    if (lane == 0) before[warp] = __popc(mask);
+    __syncthreads();
+    int at = have;
+    for (int w = 0; w < THREADS / 32; ++w) {
+      if (w < warp) at += before[w];
+      have += before[w];
+    }
+    if (same) found[at + __popc(mask & ((1u << lane) - 1u))] = i;
+    __syncthreads();
+  }
+  for (int v = threadIdx.x; v < vecs; v += THREADS) {
     float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int base = t; base < tokens; base += THREADS) {
-      const int i = base + threadIdx.x;
-      const bool same = i < tokens && ids[i] == id;
-      if (!__syncthreads_or(same)) continue;
-      const unsigned mask = __ballot_sync(0xffffffffu, same);
-      if (lane == 0) before[warp] = __popc(mask);
-      __syncthreads();
-      int at = 0, all = 0;
-      for (int w = 0; w < THREADS / 32; ++w) {
-        if (w < warp) at += before[w];
-        all += before[w];
-      }
-      if (same) found[at + __popc(mask & ((1u << lane) - 1u))] = i;
-      __syncthreads();
-      if (v < vecs)
-        for (int j = 0; j < all; ++j) {
+    for (int j = 0; j < all; j += AHEAD) {
+      Bf8 x[AHEAD];
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u)
+        if (j + u < all) x[u] = ((const Bf8*)g)[(long)found[j + u] * vecs + v];
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u)
+        if (j + u < all) {
           float f[8];
-          unpack(((const Bf8*)g)[(long)found[j] * vecs + v], f);
+          unpack(x[u], f);
 #pragma unroll
           for (int q = 0; q < 8; ++q) sum[q] += f[q];
         }
+    }
+    ((Bf8*)g_table)[id * vecs + v] = pack(sum);
+  }
+}
+
+// The ids that the kernel above left a mark for.  A block takes consecutive items of (id, slice of its columns): it finds the id's tokens
+// once, and GROUPS groups of threads add a part of the rows each, whose sums are added in the order of the groups.
+constexpr int LOOK = 8;                              // ids a thread looks at in one go
+constexpr int FOUND = 2 * LOOK * THREADS;            // positions that a block keeps
+constexpr int SLICE = 8, GROUPS = THREADS / SLICE;   // vectors of a slice (a line of 128 bytes), groups of threads over its rows
+constexpr int MARKS = 64 * THREADS;                  // marks that a block looks at in one go
+constexpr int MANY_BLOCKS = 2 * 148;
+
+struct Positions {
+  int found[FOUND];
+  int counts[LOOK][THREADS / 32];
+};
+// Appends the tokens i >= at that have `id`, in order, to p->found[0, have) until the ids are through or the next go might not fit; all
+// threads of the block.  Moves `at` on; returns the new number.
+__device__ __forceinline__ int find_tokens(const long long* ids, int tokens, long long id, int& at, int have, Positions* p) {
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  while (at < tokens && have + LOOK * THREADS <= FOUND) {
+    unsigned same[LOOK];
+#pragma unroll
+    for (int j = 0; j < LOOK; ++j) {
+      const int i = at + j * THREADS + threadIdx.x;
+      same[j] = i < tokens && ids[i] == id;
+    }
+#pragma unroll
+    for (int j = 0; j < LOOK; ++j) {
+      same[j] = __ballot_sync(0xffffffffu, same[j]);
+      if (lane == 0) p->counts[j][warp] = __popc(same[j]);
+    }
+    __syncthreads();
+    int before = have;
+#pragma unroll
+    for (int j = 0; j < LOOK; ++j)
+#pragma unroll
+      for (int w = 0; w < THREADS / 32; ++w) {
+        if (w == warp && (same[j] >> lane & 1u)) p->found[before + __popc(same[j] & ((1u << lane) - 1u))] = at + j * THREADS + threadIdx.x;
+        before += p->counts[j][w];
+      }
+    have = before;
+    at += LOOK * THREADS;
+    __syncthreads();
+  }
+  return have;
+}
+
+// sum += the rows rows[from], rows[from + step], ... of g, eight of them in flight, added in this order
+__device__ __forceinline__ void add_rows(const char* g, int vecs, int v, const int* rows, int from, int step, int n, float (&sum)[8]) {
+  for (int j0 = from; j0 < n; j0 += 8 * step) {
+    Bf8 x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (j0 + u * step < n) x[u] = ((const Bf8*)g)[(long)rows[j0 + u * step] * vecs + v];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (j0 + u * step < n) {
+        float f[8];
+        unpack(x[u], f);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) sum[q] += f[q];
+      }
+  }
+}
+
+__global__ void __launch_bounds__(THREADS, 2) embedding_many_kernel(const char* g, const long long* ids, char* g_table, const unsigned char* marks, int tokens,
+                                                                    int vecs) {
+  __shared__ Positions pos;
+  __shared__ int first[LOOK * THREADS], counts[THREADS / 32];
+  __shared__ float sums[THREADS / 32][SLICE][8];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32, group = threadIdx.x / SLICE, sv = threadIdx.x % SLICE, slices = (vecs + SLICE - 1) / SLICE;
+  long turn = blockIdx.x;   // the next items go to the blocks behind those that took the last ones
+  for (long base = 0; base < tokens; base += LOOK * THREADS) {
+    if (base % MARKS == 0) {   // mostly there are none
+      uint4 m[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const long i = base + (j * THREADS + threadIdx.x) * 16;
+        m[j] = i < tokens ? ((const uint4*)marks)[i / 16] : make_uint4(0, 0, 0, 0);   // (their memory is whole vectors)
+      }
+      unsigned any = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) any |= m[j].x | m[j].y | m[j].z | m[j].w;
+      if (!__syncthreads_or((int)any)) {
+        if (tokens - base <= MARKS) return;
+        base += MARKS - LOOK * THREADS;
+        continue;
+      }
+    }
+    // the marked tokens among the next LOOK * THREADS, in order
+    int mine = 0;
+    const long at0 = base + threadIdx.x * LOOK;
+#pragma unroll
+    for (int j = 0; j < LOOK; ++j) mine += at0 + j < tokens && marks[at0 + j] == 1;
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+      const int x = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += x;
+    }
+    if (lane == 31) counts[warp] = upto;
+    __syncthreads();
+    int at = upto - mine, marked = 0;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) {
+      if (w < warp) at += counts[w];
+      marked += counts[w];
+    }
+#pragma unroll
+    for (int j = 0; j < LOOK; ++j)
+      if (at0 + j < tokens && marks[at0 + j] == 1) first[at++] = (int)(at0 + j);
+    __syncthreads();
+    const long items = (long)marked * slices, per = (items + gridDim.x - 1) / gridDim.x;
+    int which = -1, have = 0;
+    bool whole = false;       // found[0, have) are all tokens of the id
+    long long id = 0;
+    for (long item = turn * per; item < min(items, (turn + 1) * per); ++item) {
+      const int w = (int)(item / slices), v = (int)(item - (long)w * slices) * SLICE + sv;
+      if (w != which) {
+        which = w;
+        id = ids[first[w]];
+        whole = false;
+      }
+      float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (whole) {
+        if (v < vecs) add_rows(g, vecs, v, pos.found, group, GROUPS, have, sum);
+      } else {
+        int next = first[w], done = 0;
+        do {
+          have = find_tokens(ids, tokens, id, next, 0, &pos);
+          // token number `done` + j of the id belongs to group (done + j) % GROUPS
+          if (v < vecs) add_rows(g, vecs, v, pos.found, (group - done % GROUPS + GROUPS) % GROUPS, GROUPS, have, sum);
+          whole = done == 0 && next >= tokens;
+          done += have;
+          __syncthreads();
+        } while (next < tokens);
+      }
+      // a warp's groups, then the warps in their order
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], SLICE);
+        sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], 2 * SLICE);
+        if (lane < SLICE) sums[warp][lane][q] = sum[q];
+      }
+      __syncthreads();
+      if (warp == 0 && lane < SLICE && v < vecs) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          sum[q] = 0.f;
+          for (int x = 0; x < THREADS / 32; ++x) sum[q] += sums[x][lane][q];
+        }
+        ((Bf8*)g_table)[id * vecs + v] = pack(sum);
+      }
       __syncthreads();
     }
-    if (v < vecs) ((Bf8*)g_table)[id * vecs + v] = pack(sum);
+    if (items) turn = (turn + gridDim.x - (items + per - 1) / per) % gridDim.x;
+    __syncthreads();
   }
 }
 
@@ -433,11 +611,18 @@ Status launch_rms_norm_grad(const void* g_y, const void* x, const void* w, const
                                        blocks, dim), "rms norm weight gradient");
 }
 
-Status launch_embedding_grad(const void* g, const long long* ids, void* g_table, int tokens, int dim, long long rows, cudaStream_t stream) {
+Status launch_embedding_grad(const void* g, const long long* ids, void* g_table, unsigned char* marks, int tokens, int dim, long long rows, cudaStream_t stream) {
   const cudaError_t e = cudaMemsetAsync(g_table, 0, (size_t)rows * dim * 2, stream);
   if (e != cudaSuccess) return mathk::launched(e, "embedding gradient (zeros)");
-  return mathk::launched(launch_overlapped(mathk::embedding_grad_kernel, dim3(tokens), dim3(mathk::THREADS), 0, stream, (const char*)g, ids, (char*)g_table,
-                                           tokens, dim / 8, rows), "embedding gradient");
+  // The second kernel looks for an id's tokens again, 10 us for 16384 ids: the more there are, the later that is the shorter way.  With 32 /
+  // 64 / 128, us: 128 tokens of an 8192 x 8192 table, 63 of an id, 40 / 83 / 83; 2048 of 32768 x 2048, 4 of an id, 40 / 34 / 34, and by
+  // Zipf's law 52 / 48 / 58; 16384 of 65536 x 4096, 70 of an id, 279 / 267 / 155.
+  const int many = tokens <= 512 ? 32 : tokens <= 4096 ? 64 : mathk::MOST;
+  AMEM_TRY(mathk::launched(launch_overlapped(mathk::embedding_grad_kernel, dim3(tokens), dim3(mathk::THREADS), 0, stream, (const char*)g, ids, (char*)g_table,
+                                             marks, many, tokens, dim / 8, rows), "embedding gradient"));
+  if (tokens < many) return kSuccess;   // no id can have so many
+  return mathk::launched(launch_overlapped(mathk::embedding_many_kernel, dim3(mathk::MANY_BLOCKS), dim3(mathk::THREADS), 0, stream, (const char*)g, ids, (char*)g_table,
+                                           (const unsigned char*)marks, tokens, dim / 8), "embedding gradient (frequent ids)");
 }
 
 Status launch_rotate(const Rotation& a, int batch, cudaStream_t stream) {

@@ -20,9 +20,10 @@ int rms_norm_grad_blocks(long rows);
 Status launch_rms_norm_grad(const void* g_y, const void* x, const void* w, const float* rstd, void* g_x, float* part_w, void* g_w, long rows, int dim,
                             cudaStream_t stream);
 
-// g_table[rows, dim] = the sums of the rows of g[tokens, dim] over equal ids, in the order of the tokens, fp32 inside; zero
-// elsewhere.  Ids outside the table are left out.
-Status launch_embedding_grad(const void* g, const long long* ids, void* g_table, int tokens, int dim, long long rows, cudaStream_t stream);
+// g_table[rows, dim] = the sums of the rows of g[tokens, dim] over equal ids, fp32 inside, in an order that the ids alone decide; zero
+// elsewhere.  Ids outside the table are left out.  marks: `tokens` bytes of work memory in whole 16-byte vectors.
+Status launch_embedding_grad(const void* g, const long long* ids, void* g_table, unsigned char* marks, int tokens, int dim, long long rows,
+                             cudaStream_t stream);
 // Rotary embedding of bf16 [batch, heads, seq, 8 * vecs] tensors with any strides (in elements, multiples of 8) but a
 // dense last dimension; cos and sin are fp32 [seq, 4 * vecs], turn = 1 or, for the gradients, -1.  The second tensor is
 // left out where it has no heads.
