@@ -159,6 +159,7 @@ def load_library(build_if_missing: bool = True) -> ctypes.CDLL:
         "amemAdamW": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, ctypes.c_longlong] + [ctypes.c_double] * 5 + [ctypes.c_longlong, c_void_p],
         "amemGemmPlan": [c_int, c_int, c_int, c_int, ctypes.POINTER(c_int), ctypes.POINTER(c_int), ctypes.POINTER(c_int)],
         "amemCommBegin": [c_void_p, c_void_p],
+        "amemGemmSchedule": [c_int] * 4 + [P(c_int)],
         "amemGemmForm": [c_int, c_int, c_int, c_int, ctypes.POINTER(c_int), ctypes.POINTER(c_int), ctypes.POINTER(c_int)],
         "amemAllGatherGemmPlan": [c_int, c_int, c_int, ctypes.POINTER(c_int), ctypes.POINTER(c_int), ctypes.POINTER(c_int)],
         "amemDeviceWaitProbe": [c_int, c_int, ctypes.POINTER(c_int), ctypes.POINTER(ctypes.c_float)],

@@ -343,6 +343,16 @@ ncclResult_t amemGemmPlan(int M, int N, int K, int sms, int* tile_rows, int* til
   return ncclSuccess;
 }
 
+// How the form for few rows shares out its K blocks; -1 where amemGemmBf16 takes another form.
+ncclResult_t amemGemmSchedule(int M, int N, int K, int sms, int* schedule) {
+  int form;
+  const ncclResult_t r = amemGemmForm(M, N, K, sms, &form, nullptr, nullptr);
+  if (r != ncclSuccess || !schedule) return r;
+  const SkinnyProblem few = skinny(nullptr, nullptr, nullptr, M, N, K, nullptr, 1, M, kPairStore);
+  *schedule = form == 2 ? skinny_gemm_schedule(few, sms, env_long("AMEM_GEMM_SPLITK", 1) != 0 && skinny_gemm_cuts(few, sms)) : -1;
+  return ncclSuccess;
+}
+
 // What amemGemmBf16 does on a GPU with `sms` SMs (operands and result 16-byte aligned; no GPU needed).
 ncclResult_t amemGemmForm(int M, int N, int K, int sms, int* form, int* tile, int* slices) {
   Status s = check_shape(M, N, K);

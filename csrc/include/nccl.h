@@ -264,6 +264,9 @@ ncclResult_t amemCommBegin(ncclComm_t comm, cudaStream_t stream);
  * few rows (*tile tokens, *slices 2 where tiles are cut along K), 1 = SM pairs (tiles of 256 x *tile, each cut
  * in *slices along K), 0 = the one-SM form (see amemGemmPlan).  Host arithmetic only; outputs may be NULL. */
 ncclResult_t amemGemmForm(int M, int N, int K, int sms, int* form, int* tile, int* slices);
+/* How the form for few rows shares out its blocks of K: *schedule 0 = whole tiles, 1 = all of them evenly over the SMs, 2 = a tile's owner
+ * with its helpers; -1: amemGemmBf16 takes another form.  Host arithmetic only. */
+ncclResult_t amemGemmSchedule(int M, int N, int K, int sms, int* schedule);
 /* The tiling of the one-SM form of the GEMM (the fused all-gather GEMM's) for a GPU with `sms` SMs: tile
  * rows (128 or 256), tile columns, K-slices of the last wave (1 = not split).  Host arithmetic only;
  * outputs may be NULL. */

@@ -520,6 +520,15 @@ bool skinny_gemm_cuts(const SkinnyProblem& d, int sms) {
   return !d.group_off && cut_us < whole_us;
 }
 
+int skinny_gemm_schedule(const SkinnyProblem& d, int sms, bool workspace) {
+  namespace k = skinnyk;
+  if (!workspace) return k::WHOLE;
+  // Owners need helpers, at least one each (then no helper has parts of more than two tiles), and shares that leave room for a lead.
+  const int nt = skinny_gemm_tokens(d);
+  const long tiles = (long)((d.rows + nt - 1) / nt) * ((d.N + k::WM - 1) / k::WM), units = tiles * ((d.K + k::BK - 1) / k::BK);
+  return !d.group_off && 2 * tiles <= sms && units / sms >= k::MIN_OWNED ? k::OWNERS : k::EVEN;
+}
+
 Status launch_skinny_gemm(const SkinnyProblem& d, int sms, cudaStream_t stream) {
   namespace k = skinnyk;
   k::Params p;
@@ -541,10 +550,7 @@ Status launch_skinny_gemm(const SkinnyProblem& d, int sms, cudaStream_t stream) 
   CUtensorMap mw, ma;
   AMEM_TRY(make_bf16_map(&mw, d.W, d.K, d.N, p.groups, d.epilogue == kPairSwiGLUHalves ? k::WM / 2 : k::WM));
   AMEM_TRY(make_bf16_map(&ma, d.A, d.K, d.rows, 1, p.nt));
-  // Owners need helpers, at least one each (then no helper has parts of more than two tiles), and shares that leave room for a lead.
-  const long tiles = (long)((d.rows + p.nt - 1) / p.nt) * ((d.N + k::WM - 1) / k::WM), units = tiles * ((d.K + k::BK - 1) / k::BK);
-  const bool owners = p.ws && !d.group_off && 2 * tiles <= sms && units / sms >= k::MIN_OWNED;
-  const int how = !p.ws ? k::WHOLE : owners ? k::OWNERS : k::EVEN;
+  const int how = skinny_gemm_schedule(d, sms, p.ws != nullptr);
   auto kernel = how == k::WHOLE ? k::skinny_kernel<k::WHOLE> : how == k::OWNERS ? k::skinny_kernel<k::OWNERS> : k::skinny_kernel<k::EVEN>;
   static OncePerDevice raised[3];
   cudaError_t e = allow_smem(raised[how], kernel, k::kSmemBytes);

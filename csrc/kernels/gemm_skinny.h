@@ -33,6 +33,9 @@ Status launch_skinny_gemm(const SkinnyProblem& p, int sms, cudaStream_t stream);
 int skinny_gemm_tokens(const SkinnyProblem& p);   // tokens of a tile: 16, 32, 64 or kSkinnyMaxRows
 // Whether launch_skinny_gemm would cut tiles along K, given a workspace.
 bool skinny_gemm_cuts(const SkinnyProblem& p, int sms);
+// How launch_skinny_gemm shares out the K blocks, with a workspace or without: 0 whole tiles, 1 evenly over the SMs, 2 with a tile's owner and
+// its helpers.
+int skinny_gemm_schedule(const SkinnyProblem& p, int sms, bool workspace);
 size_t skinny_gemm_ws_bytes(int sms);
 size_t skinny_gemm_ctr_words(int sms);
 

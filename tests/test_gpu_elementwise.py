@@ -272,3 +272,10 @@ def test_swiglu_keeps_the_precision_of_fp32():
     check(gh[:, f:], 1.5078125 * x * s, (1.5078125 * x * s).abs(), 5)
     scale = 1.5078125 * u.abs() * s
     check(gh[:, :f], 1.5078125 * u * s * (1 + x * (1 - s)), scale * (1 + (x * (1 - s)).abs()), 10)
+
+
+# as many rows as change the forward's threads and more, blocks of the gradient that take three rows and more; one, two and four
+# vectors a thread, the last of them part-filled
+@pytest.mark.parametrize("rows,dim", [(1184, 2048), (2500, 264), (1900, 4104), (1800, 8200)])
+def test_rms_norm_of_many_rows(rows, dim):
+    test_rms_norm_and_its_gradients(rows, dim)

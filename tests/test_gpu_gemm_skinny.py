@@ -130,3 +130,16 @@ def test_only_a_product_that_is_cut_makes_a_workspace():
         gemm_bf16(_rand((16, 8192), 13), _rand((7168, 8192), 14))      # 56 tiles on 148 SMs: cut
         side.synchronize()
         assert mem_stats()["live_bytes"] > live
+
+
+# sizes that run with owners: 74 tiles with one helper each, two token blocks a weight tile and a ragged last block in the owner's share
+# (tests/test_cpu_gemm_schedules.py asks which way they go)
+@pytest.mark.parametrize("M,N,K", [(64, 9472, 7424), (200, 2304, 8456)])
+def test_owners_at_their_limits(forced, M, N, K):
+    test_tiles_with_owners(None, M, N, K)
+
+
+# more rows than one tile takes, cut evenly
+@pytest.mark.parametrize("M,N,K", [(300, 264, 2008)])
+def test_even_cuts_of_several_token_blocks(forced, M, N, K):
+    test_plain(None, M, N, K, True)
