@@ -510,13 +510,19 @@ bool skinny_gemm_cuts(const SkinnyProblem& d, int sms) {
   // Several groups: whole tiles, so that every sum runs over K in one go, as on SM pairs (a caller's guess
   // of the number of rows, which decides between the two kernels, must not show in the result).  One
   // group: cut where that pays.  A stage takes 0.25 us per SM whatever it holds (128 of them 31.4 us with 28 tiles of 128
-  // rows, with 56 and with 112 of 64), the exchange of a cut 6.5 us more than whole tiles take to end, and no schedule
-  // beats reading the weights (back to back, whole / cut: 16 x 8192 x 3584, 64 tiles, 16.2 / 17.7 - 20; 4096 x 4096, 32
-  // tiles, 17.7 / 12.7; 16 x 3584 x 8192, 28 tiles, 31.4 / 16.1; 16 x 7168 x 8192, 56 tiles, 31.7 / 25.0).
-  const double w_tiles = (d.N + skinnyk::WM - 1) / skinnyk::WM, nkb = (d.K + skinnyk::BK - 1) / skinnyk::BK;
+  // rows, with 56 and with 112 of 64), and no schedule beats reading the weights.  The exchange of a cut takes as much longer
+  // than whole tiles take to end as there are tokens' sums to park, and more where shares lie across two tiles than where
+  // MIN_UNITS blocks divide a tile.  Back to back, us, whole / cut: 16 x 3584 x 2048 10.5 / 8.0, 16 x 5120 x 2048 (40 tiles: across)
+  // 10.5 / 10.8, 16 x 8192 x 3584 16.7 / 17.0, 16 x 7168 x 3584 16.3 / 15.5, 4096 x 4096 17.7 / 12.7; 32 x 4096 x 2048 11.0 / 9.8,
+  // 32 x 5120 x 2560 12.9 / 13.8; 64 x 4096 x 2560 13.7 / 17.5, 64 x 7168 x 4096 20.1 / 23.0, 16 x 7168 x 8192 31.7 / 25.0.  Over 864
+  // sizes of 1 to 64 tokens the rule loses 25 us in all on the better way of each (one figure of 6.5 for all: 127).
+  static const double exchange_us[3][2] = {{3.0, 5.0}, {4.2, 6.4}, {6.5, 8.0}};   // 16, 32, 64 tokens; shares in tiles, across them
+  const long w_tiles = (d.N + skinnyk::WM - 1) / skinnyk::WM, nkb = (d.K + skinnyk::BK - 1) / skinnyk::BK;
+  const int nt = skinny_gemm_tokens(d);
+  const bool across = w_tiles * nkb > (long)skinnyk::MIN_UNITS * sms || nkb % skinnyk::MIN_UNITS != 0;
   const double read_us = (double)d.N * d.K * 2 / 6.5e6;
-  const double whole_us = std::max(read_us, (double)(((long)w_tiles + sms - 1) / sms) * nkb * 0.25);
-  const double cut_us = std::max(read_us, w_tiles * nkb / sms * 0.25) + 6.5;
+  const double whole_us = std::max(read_us, (double)((w_tiles + sms - 1) / sms) * nkb * 0.25);
+  const double cut_us = std::max(read_us, (double)(w_tiles * nkb) / sms * 0.25) + exchange_us[nt <= 16 ? 0 : nt <= 32 ? 1 : 2][across];
   return !d.group_off && cut_us < whole_us;
 }
 
