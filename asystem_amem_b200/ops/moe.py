@@ -62,6 +62,18 @@ def _route_grads_torch(x: torch.Tensor, router: torch.Tensor, idx: torch.Tensor,
     return next(grads) if of_x else None, next(grads) if of_router else None
 
 
+def _route_pays(T: int, d: int, E: int) -> bool:
+    """Whether one kernel routes T tokens sooner than a library product, a cast, a top-k and a softmax do.  Every block reads the
+    whole router, so a long one (experts in tiles of 16, 32, 64, 128 or 256, times d) keeps few tokens waiting, and with more than
+    64 experts a block has only 8 tokens to spread that over.  Kernel / torch in us, from cold memory, under a graph:
+    64 x 4096 experts (the layer's default) 14.4 / 26.7 for one token, 86 / 115 for 16384; 64 x 8192 22.6 / 32.8 and 135 / 143;
+    128 x 2048 16.5 / 24.6 and 118 / 145; 256 x 2048 28.7 / 26.8 (28.7 / 30.8 for 32 tokens) and 203 / 240;
+    128 x 4096 26.7 / 28.7 and, for 4096 tokens, 61.4 / 61.5, but 106 / 94 for 8192 and 197 / 160 for 16384; 72 x 4096 24.6 / 28.7,
+    53 / 55, 90 / 82 and 166 / 133; and on the far side 256 x 4096 51.2 / 28.7 and 344 / 275, 64 x 16384 36.9 / 32.8 and 232 / 178."""
+    tiled = max(16, 1 << (E - 1).bit_length())
+    return tiled * d <= 530_000 and (E <= 64 or d <= 2048 or T <= 4096)
+
+
 class _Route(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, router, k):
@@ -80,32 +92,23 @@ class _Route(torch.autograd.Function):
         return g_logits @ router if of_x else None, g_logits.t() @ x if of_router else None, None
 
 
-def _route_pays(T: int, d: int, E: int) -> bool:
-    """Whether one kernel routes T tokens sooner than a library product, a cast, a top-k and a softmax do.  Every block reads the
-    whole router, so a long one (experts in tiles of 16, 32, 64, 128 or 256, times d) keeps few tokens waiting, and with more than
-    64 experts a block has only 8 tokens to spread that over.  Kernel / torch in us, from cold memory, under a graph:
-    64 x 4096 experts (the layer's default) 14.4 / 26.7 for one token, 86 / 115 for 16384; 64 x 8192 22.6 / 32.8 and 135 / 143;
-    128 x 2048 16.5 / 24.6 and 118 / 145; 256 x 2048 28.7 / 26.8 (28.7 / 30.8 for 32 tokens) and 203 / 240;
-    128 x 4096 26.7 / 28.7 and, for 4096 tokens, 61.4 / 61.5, but 106 / 94 for 8192 and 197 / 160 for 16384; 72 x 4096 24.6 / 28.7,
-    53 / 55, 90 / 82 and 166 / 133; and on the far side 256 x 4096 51.2 / 28.7 and 344 / 275, 64 x 16384 36.9 / 32.8 and 232 / 178."""
-    tiled = max(16, 1 << (E - 1).bit_length())
-    return tiled * d <= 530_000 and (E <= 64 or d <= 2048 or T <= 4096)
-
-
 def _kernel_routes(x: torch.Tensor, router: torch.Tensor, k: int) -> bool:
     return (x.dtype == router.dtype == torch.bfloat16 and x.dim() == router.dim() == 2 and x.shape[0] > 0 and x.shape[1] == router.shape[1]
-            and x.shape[1] > 0 and x.shape[1] % 8 == 0 and 0 < k <= router.shape[0] <= 256 and _route_pays(*x.shape, router.shape[0])
-            and plain_cuda(x, router) and x.is_contiguous() and router.is_contiguous() and (x.data_ptr() | router.data_ptr()) % 16 == 0)
+            and x.shape[1] > 0 and x.shape[1] % 8 == 0 and 0 < k <= router.shape[0] <= 256 and plain_cuda(x, router) and x.is_contiguous()
+            and router.is_contiguous() and (x.data_ptr() | router.data_ptr()) % 16 == 0)
 
 
 def route(x: torch.Tensor, router: torch.Tensor, k: int) -> tuple[torch.Tensor, torch.Tensor]:
     """The ``k`` largest of every token's logits ``x @ router.T`` and their softmax, largest first: int32 and fp32
-    [T, k].  One kernel for bf16 rows that lie densely on one GPU (equal logits by the lower expert), where that is the
-    faster way."""
+    [T, k].  One kernel for bf16 rows that lie densely on one GPU (equal logits by the lower expert), without gradients only where
+    that is the faster way.  (With them it always is for one rank's layer: its step takes the routing's gradients in with the
+    dispatch's.  128 x 4096 experts of 512, top-8: 8192 tokens 3.32 ms a training step, 3.38 with torch's routing; 256 experts, 2048
+    tokens 2.95 and 3.02; 8192 4.29 and 4.31.)"""
     if _kernel_routes(x, router, k):
         if torch.is_grad_enabled() and (x.requires_grad or router.requires_grad):
             return _Route.apply(x, router, k)
-        return _route_launch(x, router, k)
+        if _route_pays(*x.shape, router.shape[0]):
+            return _route_launch(x, router, k)
     return _route_torch(x, router, k)
 
 

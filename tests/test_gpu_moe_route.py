@@ -134,3 +134,22 @@ def test_a_graph_through_routing_and_dispatch(comm):
     out = ep.ep_route_dispatch(MoeDispatcher(comm, 8, 64, 12), x, router, 2)
     (gx,) = torch.autograd.grad(out[4].square().sum() + out[0].float().sum(), x, create_graph=True)
     assert gx.requires_grad and torch.autograd.grad(gx.float().sum(), router)[0].shape == router.shape
+
+
+# more experts than one kernel routes in time: torch's operators without gradients, the kernel with them
+@pytest.mark.parametrize("T,E,k,d", [(40, 256, 8, 4096), (4100, 96, 2, 2056)])
+def test_routing_over_many_experts(T, E, k, d):
+    from asystem_amem_b200.ops import route
+    from asystem_amem_b200.ops.moe import _route_pays
+    assert not _route_pays(T, d, E)
+    test_gradients(T, E, k, d)
+    x = torch.randn(T, d, device="cuda", generator=_gen(1)).to(torch.bfloat16)
+    router = (torch.randn(E, d, device="cuda", generator=_gen(2)) * d ** -0.5).to(torch.bfloat16)
+    idx, w = route(x, router, k)
+    logits = x.double() @ router.double().t()
+    chosen = logits.gather(1, idx.long())
+    # as in the test of the gradients: roundings of the logits to bf16
+    kth, off = logits.topk(k, dim=1).values[:, -1:], 2 * 2.0 ** -8 * logits.abs().max(dim=1, keepdim=True).values + 2.0 ** -20
+    assert idx.dtype == torch.int32 and torch.all(chosen >= kth - 2 * 2.0 ** -8 * kth.abs() - 1e-6)
+    ref = torch.softmax(chosen, dim=1)
+    assert torch.all((w.double() - ref).abs() <= ref * (off.exp() - 1) + 1e-37)
