@@ -102,15 +102,22 @@ class _RMSNorm(torch.autograd.Function):
         return *_rms_gradient(dense(g), x, weight, rstd, *wanted), None
 
 
+def _norm_pays(rows: int, dim: int, gradients: bool) -> bool:
+    """Whether one kernel is sooner done than seven passes of torch's: it takes a block per row, so of many short rows it makes
+    the same time as of longer ones.  Forward, kernel / torch, us: 65536 rows of 8 74 / 29, of 72 74 / 72, of 128 74 / 100, 1 M of 72
+    1036 / 946, of 96 1036 / 1190, 8192 of 8 14 / 25; with gradients 65536 of 8 162 / 80, of 64 162 / 199, 1 M of 64 2568 / 2548."""
+    return rows <= 8192 or dim >= (64 if gradients else 80)
+
+
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
     """``x / sqrt(mean(x^2) + eps) * weight`` over the last dimension in fp32, rounded once to x's type.  One
     kernel for bf16 rows that lie densely on one GPU."""
     if (x.dtype == weight.dtype == torch.bfloat16 and x.dim() > 0 and x.numel() > 0 and weight.shape == x.shape[-1:] and x.shape[-1] % 8 == 0
             and x.shape[-1] <= 16384 and x.numel() // x.shape[-1] < 2 ** 31 and plain_cuda(x, weight) and x.is_contiguous() and weight.is_contiguous()
             and (x.data_ptr() | weight.data_ptr()) % 16 == 0):
-        if torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad):
-            return _RMSNorm.apply(x, weight, eps)
-        return _rms_forward(x, weight, eps, False)[0]
+        gradients = torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)
+        if _norm_pays(x.numel() // x.shape[-1], x.shape[-1], gradients):
+            return _RMSNorm.apply(x, weight, eps) if gradients else _rms_forward(x, weight, eps, False)[0]
     return _rms_norm(x, weight, eps)
 
 

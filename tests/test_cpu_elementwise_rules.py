@@ -1,0 +1,11 @@
+"""Which of the decoder's passes go to the kernels: those that they were measured to be the faster way for."""
+import pytest
+
+from asystem_amem_b200.ops import elementwise as EW
+
+
+@pytest.mark.parametrize("rows,dim,gradients,kernel", [(65536, 8, False, False), (65536, 8, True, False), (65536, 64, False, False), (65536, 64, True, True),
+                                                       (1_000_000, 72, False, False), (1_000_000, 96, False, True), (65536, 128, False, True), (4096, 64, False, True), (8192, 8, True, True),
+                                                       (1, 8, False, True), (32768, 4096, True, True)])
+def test_norm(rows, dim, gradients, kernel):
+    assert EW._norm_pays(rows, dim, gradients) == kernel
