@@ -9,3 +9,10 @@ from asystem_amem_b200.ops import elementwise as EW
                                                        (1, 8, False, True), (32768, 4096, True, True)])
 def test_norm(rows, dim, gradients, kernel):
     assert EW._norm_pays(rows, dim, gradients) == kernel
+
+
+def test_gated_rows_are_one():
+    """Many short rows: most of a block's threads would have no vector."""
+    import torch
+    assert EW._as_rows(torch.empty(65536, 64, device="meta")) == (1, 65536 * 64) and EW._as_rows(torch.empty(2, 3, 8, device="meta")) == (1, 48)
+    assert EW._as_rows(torch.empty(2 ** 22, 1024, device="meta")) == (2 ** 22, 1024)
