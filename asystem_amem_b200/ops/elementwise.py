@@ -250,10 +250,16 @@ class _Rotate(torch.autograd.Function):
         return None, None, None, None, *_Rotate.apply(cos, sin, not ctx.inverse, ctx.back, *gs)
 
 
+def _turn_pays(tokens: int, elements: int) -> bool:
+    """Whether one kernel is sooner done than torch's operators with ``elements`` of a token in all tensors: a block per token takes
+    1.1 ns whatever it has to turn (65536 tokens 74 us; torch 60 for 16 elements, 158 for 128)."""
+    return elements >= 24 or tokens <= 16384
+
+
 def _kernel_turns(cos: torch.Tensor, sin: torch.Tensor, *xs: torch.Tensor) -> bool:
     batch, seq, dim = xs[0].shape[0], xs[0].shape[2] if xs[0].dim() == 4 else 0, xs[0].shape[-1]
     return (all(x.dim() == 4 and x.dtype == torch.bfloat16 and x.shape[0] == batch and x.shape[2] == seq and x.shape[3] == dim and x.numel() > 0 for x in xs)
-            and dim % 8 == 0 and batch * seq < 2 ** 31
+            and dim % 8 == 0 and batch * seq < 2 ** 31 and _turn_pays(batch * seq, sum(x.shape[1] for x in xs) * dim)
             and all(t.dtype == torch.float32 and t.shape == (seq, dim // 2) and t.is_contiguous() and not t.requires_grad for t in (cos, sin))
             and plain_cuda(*xs, cos, sin) and (cos.data_ptr() | sin.data_ptr()) % 16 == 0 and all(_in_vectors(x) for x in xs))
 

@@ -16,3 +16,8 @@ def test_gated_rows_are_one():
     import torch
     assert EW._as_rows(torch.empty(65536, 64, device="meta")) == (1, 65536 * 64) and EW._as_rows(torch.empty(2, 3, 8, device="meta")) == (1, 48)
     assert EW._as_rows(torch.empty(2 ** 22, 1024, device="meta")) == (2 ** 22, 1024)
+
+
+@pytest.mark.parametrize("tokens,elements,kernel", [(65536, 16, False), (65536, 8, False), (65536, 128, True), (1, 8, True), (8192, 5120, True)])
+def test_rotary_embedding(tokens, elements, kernel):
+    assert EW._turn_pays(tokens, elements) == kernel
