@@ -136,8 +136,8 @@ def test_a_graph_through_routing_and_dispatch(comm):
     assert gx.requires_grad and torch.autograd.grad(gx.float().sum(), router)[0].shape == router.shape
 
 
-# more experts than one kernel routes in time: torch's operators without gradients, the kernel with them
-@pytest.mark.parametrize("T,E,k,d", [(40, 256, 8, 4096), (4100, 96, 2, 2056)])
+# more experts than one kernel routes in time: torch's operators without gradients and, for many tokens, with them
+@pytest.mark.parametrize("T,E,k,d", [(40, 256, 8, 4096), (8200, 96, 2, 2056)])
 def test_routing_over_many_experts(T, E, k, d):
     from asystem_amem_b200.ops import route
     from asystem_amem_b200.ops.moe import _route_pays
