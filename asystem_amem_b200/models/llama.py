@@ -17,6 +17,7 @@ import torch.nn.functional as F
 from torch.nn.modules.module import _has_any_global_hook
 
 from ..ops.elementwise import embedding, gated, rms_norm, rotate
+from ..ops.operands import concrete
 
 
 @dataclass
@@ -108,7 +109,7 @@ class Embed(nn.Module):
 
     def forward(self, ids, cos=None, sin=None):
         t = self.tok
-        if (not torch.compiler.is_compiling() and type(t) is nn.Embedding and t.padding_idx is None and t.max_norm is None and not t.scale_grad_by_freq and not t.sparse
+        if (concrete(ids) and not torch.compiler.is_compiling() and type(t) is nn.Embedding and t.padding_idx is None and t.max_norm is None and not t.scale_grad_by_freq and not t.sparse
                 and "forward" not in t.__dict__ and not t._forward_hooks and not t._forward_pre_hooks and not t._backward_hooks
                 and not t._backward_pre_hooks and not _has_any_global_hook()):
             return embedding(ids, t.weight)

@@ -11,7 +11,7 @@ import torch
 import torch.nn.functional as F
 
 from .. import bindings as B
-from .operands import apart, current_stream, dense, on_operands_device, plain_cuda, tangents_about
+from .operands import apart, concrete, current_stream, dense, on_operands_device, plain_cuda, tangents_about
 
 
 def _fused(h: torch.Tensor) -> bool:
@@ -112,7 +112,7 @@ def _norm_pays(rows: int, dim: int, gradients: bool) -> bool:
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
     """``x / sqrt(mean(x^2) + eps) * weight`` over the last dimension in fp32, rounded once to x's type.  One
     kernel for bf16 rows that lie densely on one GPU."""
-    if (x.dtype == weight.dtype == torch.bfloat16 and x.dim() > 0 and x.numel() > 0 and weight.shape == x.shape[-1:] and x.shape[-1] % 8 == 0
+    if (concrete(x, weight) and x.dtype == weight.dtype == torch.bfloat16 and x.dim() > 0 and x.numel() > 0 and weight.shape == x.shape[-1:] and x.shape[-1] % 8 == 0
             and x.shape[-1] <= 16384 and x.numel() // x.shape[-1] < 2 ** 31 and plain_cuda(x, weight) and x.is_contiguous() and weight.is_contiguous()
             and (x.data_ptr() | weight.data_ptr()) % 16 == 0):
         gradients = torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)
@@ -162,7 +162,7 @@ class _Gated(torch.autograd.Function):
 def gated(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     """silu(gate) * up of two tensors of one shape.  One kernel, in fp32 and rounded once, for bf16 that lies densely on
     one GPU."""
-    if (gate.dtype == up.dtype == torch.bfloat16 and gate.shape == up.shape and gate.dim() > 0 and gate.numel() > 0 and gate.shape[-1] % 8 == 0
+    if (concrete(gate, up) and gate.dtype == up.dtype == torch.bfloat16 and gate.shape == up.shape and gate.dim() > 0 and gate.numel() > 0 and gate.shape[-1] % 8 == 0
             and plain_cuda(gate, up) and gate.is_contiguous() and up.is_contiguous() and (gate.data_ptr() | up.data_ptr()) % 16 == 0):
         return _Gated.apply(gate, up) if torch.is_grad_enabled() and (gate.requires_grad or up.requires_grad) else _gated_forward(gate, up)
     return F.silu(gate) * up
@@ -196,7 +196,7 @@ class _Embedding(torch.autograd.Function):
 def embedding(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
     """``table[ids]``.  The gradient of a bf16 table on one GPU sums the rows of equal ids in fp32, in an order that the ids alone
     decide, by the library's kernels (up to 16384 ids: every block looks through all of them)."""
-    if (table.requires_grad and torch.is_grad_enabled() and table.dtype == torch.bfloat16 and table.dim() == 2 and table.shape[1] % 8 == 0 and table.shape[1] > 0
+    if (concrete(ids, table) and table.requires_grad and torch.is_grad_enabled() and table.dtype == torch.bfloat16 and table.dim() == 2 and table.shape[1] % 8 == 0 and table.shape[1] > 0
             and ids.dtype == torch.int64 and 0 < ids.numel() <= 16384 and plain_cuda(ids, table) and ids.is_contiguous()):
         return _Embedding.apply(ids, table)
     return F.embedding(ids, table)
@@ -268,7 +268,7 @@ def rotate(cos: torch.Tensor, sin: torch.Tensor, *xs: torch.Tensor, as_they_lie:
     """Rotary embedding of one or two [B, H, S, D] tensors: neighbouring elements turned by the angles of ``cos`` and
     ``sin`` [S, D / 2].  Computed in fp32 and rounded once; bf16 on one GPU in one kernel.  The results are contiguous, or
     (``as_they_lie``) laid out as the inputs, whose heads may lie inside the positions."""
-    if _kernel_turns(cos, sin, *xs):
+    if concrete(cos, sin, *xs) and _kernel_turns(cos, sin, *xs):
         layout = [as_they_lie and _tokens_first(x) for x in xs]
         if torch.is_grad_enabled() and any(x.requires_grad for x in xs):
             return _Rotate.apply(cos, sin, False, layout, *xs)

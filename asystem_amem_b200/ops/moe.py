@@ -21,7 +21,7 @@ from dataclasses import dataclass
 import torch
 
 from .. import bindings as B
-from .operands import apart, current_stream, dense, on_operands_device, plain_cuda
+from .operands import apart, concrete, current_stream, dense, on_operands_device, plain_cuda
 
 
 def _view(ptr: int, rows: int, d: int, device) -> torch.Tensor:
@@ -97,7 +97,7 @@ class _Route(torch.autograd.Function):
 
 
 def _kernel_routes(x: torch.Tensor, router: torch.Tensor, k: int) -> bool:
-    return (x.dtype == router.dtype == torch.bfloat16 and x.dim() == router.dim() == 2 and x.shape[0] > 0 and x.shape[1] == router.shape[1]
+    return (concrete(x, router) and x.dtype == router.dtype == torch.bfloat16 and x.dim() == router.dim() == 2 and x.shape[0] > 0 and x.shape[1] == router.shape[1]
             and x.shape[1] > 0 and x.shape[1] % 8 == 0 and 0 < k <= router.shape[0] <= 256 and plain_cuda(x, router) and x.is_contiguous()
             and router.is_contiguous() and (x.data_ptr() | router.data_ptr()) % 16 == 0)
 

@@ -33,6 +33,11 @@ def tangents_about() -> bool:
     return forward_ad._current_level >= 0
 
 
+def concrete(*values) -> bool:
+    """Whether ``values`` are tensors: a symbolic tracer hands stand-ins through, of which no branch can be asked."""
+    return all(isinstance(v, torch.Tensor) for v in values)
+
+
 def plain_cuda(*tensors: torch.Tensor) -> bool:
     """Whether ``tensors`` are ordinary tensors of one GPU in a program that runs eagerly: what a kernel that
     autograd knows only as a :class:`torch.autograd.Function` can take.  Subclasses, tracing, dispatch modes
