@@ -16,7 +16,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch.nn.modules.module import _has_any_global_hook
 
-from ..ops.elementwise import embedding, gated, rms_norm, rotate
+from ..ops.elementwise import _rms_norm, _rotate_plain, embedding, gated, rms_norm, rotate
 from ..ops.operands import concrete
 
 
@@ -47,7 +47,10 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(dim))
 
     def forward(self, x):
-        return rms_norm(x, self.weight, self.eps)
+        if torch.jit.is_scripting():      # (compiles torch's operators only, and no more of the branches than it takes)
+            return _rms_norm(x, self.weight, self.eps)
+        else:
+            return rms_norm(x, self.weight, self.eps)
 
 
 def rope_tables(seq: int, head_dim: int, theta: float, device) -> tuple[torch.Tensor, torch.Tensor]:
@@ -58,7 +61,10 @@ def rope_tables(seq: int, head_dim: int, theta: float, device) -> tuple[torch.Te
 
 def apply_rope(x, cos, sin):
     # x: [B, H, S, D]
-    return rotate(cos, sin, x)[0]
+    if torch.jit.is_scripting():
+        return _rotate_plain(x, cos, sin)
+    else:
+        return rotate(cos, sin, x)[0]
 
 
 class Attention(nn.Module):
@@ -75,7 +81,10 @@ class Attention(nn.Module):
         q = self.wq(x).view(B, S, self.h, self.hd).transpose(1, 2)
         k = self.wk(x).view(B, S, self.kv, self.hd).transpose(1, 2)
         v = self.wv(x).view(B, S, self.kv, self.hd).transpose(1, 2)
-        q, k = rotate(cos, sin, q, k, as_they_lie=True)
+        if torch.jit.is_scripting():
+            q, k = apply_rope(q, cos, sin), apply_rope(k, cos, sin)
+        else:
+            q, k = rotate(cos, sin, q, k, as_they_lie=True)
         o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=self.kv != self.h)
         return self.wo(o.transpose(1, 2).reshape(B, S, -1))
 
@@ -88,7 +97,10 @@ class SwiGLU(nn.Module):
         self.w2 = nn.Linear(cfg.ffn_dim, cfg.dim, bias=False)
 
     def forward(self, x):
-        return self.w2(gated(self.w1(x), self.w3(x)))
+        if torch.jit.is_scripting():
+            return self.w2(F.silu(self.w1(x)) * self.w3(x))
+        else:
+            return self.w2(gated(self.w1(x), self.w3(x)))
 
 
 class Block(nn.Module):
@@ -108,12 +120,15 @@ class Embed(nn.Module):
         self.tok = nn.Embedding(cfg.vocab_size, cfg.dim)
 
     def forward(self, ids, cos=None, sin=None):
-        t = self.tok
-        if (concrete(ids) and not torch.compiler.is_compiling() and type(t) is nn.Embedding and t.padding_idx is None and t.max_norm is None and not t.scale_grad_by_freq and not t.sparse
-                and "forward" not in t.__dict__ and not t._forward_hooks and not t._forward_pre_hooks and not t._backward_hooks
-                and not t._backward_pre_hooks and not _has_any_global_hook()):
-            return embedding(ids, t.weight)
-        return t(ids)
+        if torch.jit.is_scripting():
+            return self.tok(ids)
+        else:
+            t = self.tok
+            if (concrete(ids) and not torch.compiler.is_compiling() and type(t) is nn.Embedding and t.padding_idx is None and t.max_norm is None
+                    and not t.scale_grad_by_freq and not t.sparse and "forward" not in t.__dict__ and not t._forward_hooks and not t._forward_pre_hooks
+                    and not t._backward_hooks and not t._backward_pre_hooks and not _has_any_global_hook()):
+                return embedding(ids, t.weight)
+            return t(ids)
 
 
 class Head(nn.Module):

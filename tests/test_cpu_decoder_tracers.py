@@ -31,3 +31,11 @@ def test_symbolic_trace(name):
     torch.testing.assert_close(traced(*args), m(*args), rtol=0, atol=0)
     if name == "embed":
         assert any(n.op == "call_module" and n.target == "tok" for n in traced.graph.nodes)
+
+
+@pytest.mark.filterwarnings("ignore::DeprecationWarning")
+@pytest.mark.parametrize("name", ["norm", "swiglu", "embed", "rope", "head", "attention", "block"])
+def test_script(name):
+    m, args = _module(name)
+    with torch.no_grad():
+        torch.testing.assert_close(torch.jit.script(m)(*args), m(*args), rtol=1e-5, atol=1e-5)     # fp32, its passes fused or not
