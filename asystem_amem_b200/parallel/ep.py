@@ -160,8 +160,9 @@ def ep_dispatch(disp: MoeDispatcher, x: torch.Tensor, idx: torch.Tensor, all_rou
 
 def ep_route_dispatch(disp: MoeDispatcher, x: torch.Tensor, router: torch.Tensor, k: int):
     """Differentiable routing (:func:`ops.moe.route`) and dispatch: (rows grouped by local expert, expert_offsets, send_pos, idx,
-    w).  One step where one rank's kernels take ``x`` and ``router``, the two otherwise."""
-    if disp.local(x) and router.shape[0] == disp.E and _kernel_routes(x, router, k):
+    w).  One step where one rank's kernels take ``x`` and ``router`` and ``x`` wants a gradient, the two otherwise (as outputs of one
+    step the rows would want a gradient for the router's sake, and the experts would compute it)."""
+    if x.requires_grad and disp.local(x) and router.shape[0] == disp.E and _kernel_routes(x, router, k):
         return _RouteDispatch.apply(x, router, disp, k)
     idx, w = route(x, router, k)
     return *ep_dispatch(disp, x, idx, all_routed=router.shape[0] == disp.E), idx, w
