@@ -241,13 +241,17 @@ class _Rotate(torch.autograd.Function):
     def forward(ctx, cos, sin, inverse, tokens_first, *xs):
         ctx.save_for_backward(cos, sin)
         ctx.inverse, ctx.back = inverse, [_tokens_first(x) for x in xs]
-        return _rotate_launch(cos, sin, inverse, tokens_first, *xs)
+        outs = _rotate_launch(cos, sin, inverse, tokens_first, *xs)
+        ctx.mark_non_differentiable(*(o for o, wanted in zip(outs, ctx.needs_input_grad[4:]) if not wanted))
+        return outs
 
     @staticmethod
     def backward(ctx, *gs):
         cos, sin = ctx.saved_tensors
-        gs = [g if _in_vectors(g) else dense(g) for g in gs]
-        return None, None, None, None, *_Rotate.apply(cos, sin, not ctx.inverse, ctx.back, *gs)
+        wanted = ctx.needs_input_grad[4:]
+        gs = [g if _in_vectors(g) else dense(g) for g, w in zip(gs, wanted) if w]
+        turned = iter(_Rotate.apply(cos, sin, not ctx.inverse, [b for b, w in zip(ctx.back, wanted) if w], *gs))
+        return None, None, None, None, *(next(turned) if w else None for w in wanted)
 
 
 def _turn_pays(tokens: int, elements: int) -> bool:

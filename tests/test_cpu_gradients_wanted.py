@@ -30,3 +30,27 @@ def test_rows_of_a_routing(monkeypatch, of_x):
     x, router = torch.randn(6, 8, requires_grad=of_x), torch.randn(4, 8, requires_grad=True)
     rows, _, _, _, w = ep.ep_route_dispatch(_Dispatcher(), x, router, 2)
     assert rows.requires_grad == of_x and w.requires_grad
+
+
+@pytest.mark.parametrize("of_q,of_k", [(True, True), (True, False), (False, True)])
+def test_turned_tensors(monkeypatch, of_q, of_k):
+    from asystem_amem_b200.models.llama import rope_tables
+    from asystem_amem_b200.ops import elementwise as EW
+    turned = []
+
+    def launch(cos, sin, inverse, tokens_first, *xs):
+        turned.append(len(xs))
+        return tuple(EW._rotate_plain(x, cos, -sin if inverse else sin) for x in xs)
+    monkeypatch.setattr(EW, "_rotate_launch", launch)
+    cos, sin = rope_tables(3, 8, 10000.0, "cpu")
+    torch.manual_seed(0)
+    q, k = torch.randn(1, 2, 3, 8, requires_grad=of_q), torch.randn(1, 1, 3, 8, requires_grad=of_k)
+    outs = EW._Rotate.apply(cos, sin, False, [False, False], q, k)
+    assert [o.requires_grad for o in outs] == [of_q, of_k]
+    g = [torch.randn_like(o) for o in outs]
+    wanted = [t for t in (q, k) if t.requires_grad]
+    got = torch.autograd.grad([o for o in outs if o.requires_grad], wanted, [a for a, o in zip(g, outs) if o.requires_grad], create_graph=True)
+    want = torch.autograd.grad([EW._rotate_plain(t, cos, sin) for t in wanted], wanted, [a for a, o in zip(g, outs) if o.requires_grad])
+    for a, b in zip(got, want):
+        torch.testing.assert_close(a, b)
+    assert turned == [2, len(wanted)]
