@@ -28,7 +28,7 @@ class _SwiGLU(torch.autograd.Function):
     @torch.autograd.function.once_differentiable
     def backward(ctx, g):
         (h,) = ctx.saved_tensors
-        return _gradient(h, dense(g))
+        return _gradient(dense(h), dense(g))     # (dense: a hook on saved tensors may give them back in any strides)
 
 
 @on_operands_device
@@ -99,7 +99,7 @@ class _RMSNorm(torch.autograd.Function):
             at = [t for t, w in zip((x, weight), wanted) if w]
             grads = iter(torch.autograd.grad(_rms_norm(x, weight, ctx.eps), at, g, create_graph=True))
             return *(next(grads) if w else None for w in wanted), None
-        return *_rms_gradient(dense(g), x, weight, rstd, *wanted), None
+        return *_rms_gradient(dense(g), dense(x), dense(weight), dense(rstd), *wanted), None
 
 
 def _norm_pays(rows: int, dim: int, gradients: bool) -> bool:
@@ -156,7 +156,7 @@ class _Gated(torch.autograd.Function):
             at = [t for t, w in zip((gate, up), ctx.needs_input_grad) if w]
             grads = iter(torch.autograd.grad(F.silu(gate) * up, at, g, create_graph=True))
             return tuple(next(grads) if w else None for w in ctx.needs_input_grad)
-        return tuple(t if w else None for t, w in zip(_gated_gradient(gate, up, dense(g)), ctx.needs_input_grad))
+        return tuple(t if w else None for t, w in zip(_gated_gradient(dense(gate), dense(up), dense(g)), ctx.needs_input_grad))
 
 
 def gated(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
@@ -190,7 +190,7 @@ class _Embedding(torch.autograd.Function):
         (ids,) = ctx.saved_tensors
         if torch.is_grad_enabled():
             return None, torch.ops.aten.embedding_dense_backward(g, ids, ctx.rows, -1, False)
-        return None, _embedding_gradient(dense(g), ids, ctx.rows)
+        return None, _embedding_gradient(dense(g), ids.contiguous(), ctx.rows)
 
 
 def embedding(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
@@ -247,7 +247,7 @@ class _Rotate(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, *gs):
-        cos, sin = ctx.saved_tensors
+        cos, sin = map(dense, ctx.saved_tensors)
         wanted = ctx.needs_input_grad[4:]
         gs = [g if _in_vectors(g) else dense(g) for g, w in zip(gs, wanted) if w]
         turned = iter(_Rotate.apply(cos, sin, not ctx.inverse, [b for b, w in zip(ctx.back, wanted) if w], *gs))

@@ -92,7 +92,7 @@ class _Route(torch.autograd.Function):
         of_x, of_router = ctx.needs_input_grad[:2]
         if torch.is_grad_enabled():     # a graph of the gradient is wanted: torch's operators make one
             return *_route_grads_torch(x, router, idx, g_w, of_x, of_router), None
-        g_logits = _route_logits_grad(g_w.contiguous(), w, idx, router.shape[0])
+        g_logits = _route_logits_grad(g_w.contiguous(), dense(w), dense(idx), router.shape[0])
         return g_logits @ router if of_x else None, g_logits.t() @ x if of_router else None, None
 
 

@@ -130,6 +130,7 @@ class _RouteDispatch(torch.autograd.Function):
             if of_x or of_router:
                 g_x, g_router = _route_grads_torch(x, router, idx, g_w, of_x, of_router)
             return (g_x + dispatch_backward(ctx.disp, g_rows.contiguous(), idx, send_pos) if of_x else None), g_router, None, None
+        w, idx, send_pos, router = map(dense, (w, idx, send_pos, router))
         g_logits = _route_logits_grad(g_w.contiguous(), w, idx, router.shape[0])
         if of_x:
             g_x = ctx.disp.input_grad_local(dense(g_rows), send_pos, idx, g_logits, router)
