@@ -113,6 +113,19 @@ def main():
             disp.combine_grad_local(tok, disp.y, tw, res.send_pos)
         torch.cuda.synchronize()
         comm.destroy()
+    elif args.case == "gradient_sums":
+        # an embedding's gradient, tokens drawn evenly, half of them one id, and 70 an id; gradients into a shard, two sizes
+        from asystem_amem_b200.ops import embedding
+        from asystem_amem_b200.ops.elementwise import add_pieces
+        table = torch.randn(32768, 4096, device="cuda").to(torch.bfloat16).requires_grad_(True)
+        g, evenly = torch.randn(16384, 4096, device="cuda").to(torch.bfloat16), torch.randint(0, 32768, (16384,), device="cuda")
+        half, often = torch.where(torch.rand(16384, device="cuda") < 0.5, 3, evenly), torch.arange(16384, device="cuda") % (16384 // 70)
+        src, wide = torch.randn(100_000_000, device="cuda").to(torch.bfloat16), torch.zeros(100_000_000, device="cuda")
+        for _ in range(reps):
+            for ids in (evenly, half, often):
+                torch.autograd.grad(embedding(ids, table), table, g)
+            add_pieces(wide, [(0, src)])
+        torch.cuda.synchronize()
     elif args.case == "window_allreduce":
         world = 4
         n = 32 << 20  # bf16 elements: 64 MiB per rank
