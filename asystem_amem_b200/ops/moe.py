@@ -21,7 +21,7 @@ from dataclasses import dataclass
 import torch
 
 from .. import bindings as B
-from .operands import apart, concrete, current_stream, dense, on_operands_device, plain_cuda
+from .operands import apart, current_stream, dense, on_operands_device, plain_cuda
 
 
 def _view(ptr: int, rows: int, d: int, device) -> torch.Tensor:
@@ -70,6 +70,8 @@ def _route_pays(T: int, d: int, E: int) -> bool:
     128 x 2048 16.5 / 24.6 and 118 / 145; 256 x 2048 28.7 / 26.8 (28.7 / 30.8 for 32 tokens) and 203 / 240;
     128 x 4096 26.7 / 28.7 and, for 4096 tokens, 61.4 / 61.5, but 106 / 94 for 8192 and 197 / 160 for 16384; 72 x 4096 24.6 / 28.7,
     53 / 55, 90 / 82 and 166 / 133; and on the far side 256 x 4096 51.2 / 28.7 and 344 / 275, 64 x 16384 36.9 / 32.8 and 232 / 178."""
+    if E <= 64 and d <= 8192:
+        return True
     tiled = max(16, 1 << (E - 1).bit_length())
     return tiled * d <= 530_000 and (E <= 64 or d <= 2048 or T <= 4096)
 
@@ -97,7 +99,7 @@ class _Route(torch.autograd.Function):
 
 
 def _kernel_routes(x: torch.Tensor, router: torch.Tensor, k: int) -> bool:
-    return (concrete(x, router) and x.dtype == router.dtype == torch.bfloat16 and x.dim() == router.dim() == 2 and x.shape[0] > 0 and x.shape[1] == router.shape[1]
+    return (x.dtype == router.dtype == torch.bfloat16 and x.dim() == router.dim() == 2 and x.shape[0] > 0 and x.shape[1] == router.shape[1]
             and x.shape[1] > 0 and x.shape[1] % 8 == 0 and 0 < k <= router.shape[0] <= 256 and plain_cuda(x, router) and x.is_contiguous()
             and router.is_contiguous() and (x.data_ptr() | router.data_ptr()) % 16 == 0)
 

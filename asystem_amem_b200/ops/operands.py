@@ -35,7 +35,10 @@ def tangents_about() -> bool:
 
 def concrete(*values) -> bool:
     """Whether ``values`` are tensors: a symbolic tracer hands stand-ins through, of which no branch can be asked."""
-    return all(isinstance(v, torch.Tensor) for v in values)
+    for v in values:
+        if not isinstance(v, torch.Tensor):
+            return False
+    return True
 
 
 def plain_cuda(*tensors: torch.Tensor) -> bool:
